@@ -8,12 +8,17 @@ compiled library is missing the import fails loudly.
 from __future__ import annotations
 
 import ctypes as C
+import importlib.machinery
+import importlib.util
 from pathlib import Path
 
 import os
 
 # SSD_B200_LIB overrides the library location (e.g. to test a differently built copy).
 LIB_PATH = Path(os.environ.get("SSD_B200_LIB") or (Path(__file__).resolve().parent / "lib" / "libssd_b200.so"))
+
+# The native host path of the Python entry points (csrc/ssd_host.cpp).
+HOST_PATH = Path(__file__).resolve().parent / "lib" / "_ssd_host.so"
 
 SSD_F32, SSD_BF16 = 0, 1
 PASS_FWD, PASS_BWD = 0, 1
@@ -177,6 +182,29 @@ def load() -> C.CDLL:
     lib.ssd_compiled_arch.restype = i32
     _lib = lib
     return lib
+
+
+_host = None
+
+
+def host():
+    """The native host module, bound to the C ABI functions of the library that load() opened."""
+    global _host
+    if _host is not None:
+        return _host
+    lib = load()
+    if not HOST_PATH.exists():
+        raise ImportError(f"{HOST_PATH} is missing: run `python -m trading_bot_0_b200.build`. There is no fallback.")
+    import torch  # (its libraries have to be loaded before the module's symbols can be resolved)
+    loader = importlib.machinery.ExtensionFileLoader("_ssd_host", str(HOST_PATH))
+    mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("_ssd_host", loader))
+    loader.exec_module(mod)
+    names = ("ssd_workspace_bytes", "ssd_forward_staged", "ssd_backward_staged", "ssd_state_update", "ssd_last_error",
+             "ssd_conv1d_workspace_bytes", "ssd_conv1d_forward", "ssd_conv1d_backward", "ssd_rmsnorm_workspace_bytes",
+             "ssd_rmsnorm_forward", "ssd_rmsnorm_backward")
+    mod.bind(tuple(C.cast(getattr(lib, n), C.c_void_p).value for n in names), SsdError, torch.OutOfMemoryError)
+    _host = mod
+    return mod
 
 
 def check(rc: int) -> None:

@@ -1,6 +1,6 @@
 """Build the CUDA library in-tree with nvcc for sm_100a (cross-compiles without a GPU).
 
-    python -m trading_bot_0_b200.build            # -> trading_bot_0_b200/lib/libssd_b200.so
+    python -m trading_bot_0_b200.build            # -> trading_bot_0_b200/lib/libssd_b200.so and lib/_ssd_host.so (host path)
     python -m trading_bot_0_b200.build --torch    # also -> lib/libssd_b200_torch.so (libtorch autograd node over the C ABI)
 """
 from __future__ import annotations
@@ -28,7 +28,7 @@ def nvcc_path() -> str:
 
 
 def needs_build() -> bool:
-    if not LIB.exists():
+    if not LIB.exists() or host_needs_build():
         return True
     t = LIB.stat().st_mtime
     deps = list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.h")) + \
@@ -59,8 +59,10 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         cmd = [nvcc_path(), *flags, "-c", str(CSRC / src), "-o", str(obj)]
         return obj, (cmd, subprocess.run(cmd, capture_output=True, text=True))
 
-    with ThreadPoolExecutor(max_workers=len(SOURCES)) as ex:
+    with ThreadPoolExecutor(max_workers=len(SOURCES) + 1) as ex:
+        host = ex.submit(build_host, force)
         results = list(ex.map(compile_one, SOURCES))
+        host.result()
     for obj, run in results:
         if run is None:
             continue
@@ -85,6 +87,37 @@ def host_cxx() -> str:
         if cand and os.path.exists(cand):
             return cand
     raise RuntimeError("no host C++ compiler found")
+
+
+HOST_LIB = PKG / "lib" / "_ssd_host.so"
+HOST_SRC = CSRC / "ssd_host.cpp"
+
+
+def host_needs_build() -> bool:
+    deps = [HOST_SRC, PKG.parent / "include" / "ssd_b200.h", Path(__file__)]
+    return not HOST_LIB.exists() or any(d.stat().st_mtime > HOST_LIB.stat().st_mtime for d in deps)
+
+
+def build_host(force: bool = False) -> Path:
+    """The native host path of the Python entry points: a CPython extension over libtorch (host C++ only).  It gets the
+    library's functions by address when it is loaded, so it is linked to nothing of libssd_b200."""
+    if not force and not host_needs_build():
+        return HOST_LIB
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension as E
+    HOST_LIB.parent.mkdir(parents=True, exist_ok=True)
+    inc = [f"-I{p}" for p in E.include_paths("cuda")] + [f"-I{sysconfig.get_paths()['include']}"]
+    tlib = os.path.join(os.path.dirname(torch.__file__), "lib")
+    cmd = [host_cxx(), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-Wl,--exclude-libs,ALL",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *inc, str(HOST_SRC), "-o", str(HOST_LIB),
+           f"-L{tlib}", "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", f"-Wl,-rpath,{tlib}"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode:
+        sys.stderr.write(r.stdout + r.stderr)
+        raise RuntimeError("g++ failed: " + " ".join(cmd))
+    return HOST_LIB
 
 
 TORCH_LIB = PKG / "lib" / "libssd_b200_torch.so"
