@@ -166,3 +166,22 @@ def test_fused_state_scan_matches_the_staged_two_kernel_path(lib, Bn, L, H, P, G
             assert_close(k + " (staged)", res["staged"][k], ref[k], "bf16")
         tol = 2e-2 if k == "dA" else 2e-3
         assert mean_rel(v, res["staged"][k]) < tol, f"{k}: fused and staged paths differ by {mean_rel(v, res['staged'][k]):.3e}"
+
+
+@pytest.mark.parametrize("L", [1, 100, 129, 255, 383, 641])
+@pytest.mark.parametrize("H,P,N,G,has_z", [(8, 32, 64, 1, False), (4, 64, 64, 2, True), (24, 64, 128, 1, True), (8, 32, 128, 2, False)])
+def test_ragged_forward_runs_on_the_tensor_family(lib, L, H, P, N, G, has_z):
+    """A forward without a backward takes any sequence length: the last chunk's loads zero-fill, its stores drop the rows past
+    the end (the neighbouring batch row and the guard rows stay untouched)."""
+    import trading_bot_0_b200 as T
+    cfg = O.SsdConfig("rag", 2, L, H, P, N, G, 128, "bf16", has_z)
+    inp = O.make_inputs(cfg, with_init_state=True)
+    y_ref, fin_ref = O.ssd_sequential(inp["x"], inp["dt"], inp["A"], inp["B"], inp["C"], inp["D"], inp.get("z"), inp["init_state"])
+    d = to_dev(inp, DEV)
+    buf = torch.full((2, L + 3, H, P), 7.0, dtype=torch.bfloat16, device=DEV)
+    y, fin, ws = T.forward(d["x"], d["dt"], d["A"], d["B"], d["C"], d["D"], d.get("z"), d["init_state"], chunk=128, algo="tensor",
+                           y=buf[:, :L])
+    assert status_word(ws) == 0
+    assert_close("y", y, y_ref, "bf16")
+    assert_close("final_state", fin, fin_ref, "bf16")
+    assert (buf[:, L:] == 7.0).all()

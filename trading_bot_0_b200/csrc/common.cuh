@@ -17,6 +17,7 @@ struct Geo {
   int B, L, H, P, N, G, Q, nc, hpg;  // hpg = heads per group
   long long xsb, xsl, dtsb, dtsl, bsb, bsl, csb, csl, zsb, zsl, ysb, ysl;
   int dt_softplus;                     // step size = softplus(dt + dt_bias) instead of dt + dt_bias
+  int fwd_only;                        // the workspace is too small for a backward: none will follow in it (see forward_geo)
   int onetile;                         // tensor family: the one-tile-per-CTA kernels for every shape (SSD_ALGO_TENSOR_ONETILE)
 };
 

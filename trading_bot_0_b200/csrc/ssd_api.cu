@@ -45,7 +45,7 @@ void after_launch(const char* what, cudaStream_t s) {
 static size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
 
 // Returns 0 or a negative status (error string set).
-static int make_geo(const SsdDims* d, Geo* g) {
+static int make_geo(const SsdDims* d, Geo* g, bool fwd_only = false) {
   if (!d) { set_error("dims is NULL"); return SSD_ERR_NULL_POINTER; }
   if (d->batch <= 0 || d->seqlen <= 0 || d->nheads <= 0 || d->headdim <= 0 || d->dstate <= 0 || d->ngroups <= 0 ||
       d->chunk <= 0) {
@@ -63,6 +63,7 @@ static int make_geo(const SsdDims* d, Geo* g) {
   g->B = d->batch; g->L = d->seqlen; g->H = d->nheads; g->P = d->headdim; g->N = d->dstate; g->G = d->ngroups;
   g->Q = d->chunk; g->nc = (d->seqlen + d->chunk - 1) / d->chunk; g->hpg = d->nheads / d->ngroups;
   g->dt_softplus = d->dt_softplus != 0;
+  g->fwd_only = fwd_only;
   g->onetile = d->algo == SSD_ALGO_TENSOR_ONETILE;
   if (g->B > 65535) { set_error("batch (%d) must be <= 65535 (grid limit)", g->B); return SSD_ERR_UNSUPPORTED; }
   const long long HP = (long long)g->H * g->P, GN = (long long)g->G * g->N;
@@ -91,7 +92,8 @@ static int make_geo(const SsdDims* d, Geo* g) {
     Geo t = *g;
     t.Q = 128;
     t.nc = (t.L + 127) / 128;
-    if (tensor_supported(t, d->dtype, nullptr)) *g = t;
+    t.fwd_only = 1;   // also where only the forward will: both families then cut a sequence into the same chunks
+    if (tensor_supported(t, d->dtype, nullptr)) { t.fwd_only = fwd_only; *g = t; }
   }
   return SSD_OK;
 }
@@ -125,6 +127,33 @@ static void make_layout(const Geo& g, bool has_z, bool tcfam, WsLayout* w) {
 
 static bool family_is_tensor(const Geo& g, const SsdDims* d) {
   return d->algo != SSD_ALGO_FP32_CORES && tensor_supported(g, d->dtype, nullptr);
+}
+
+// Geometry and layout of a forward (or of a call on a forward's workspace).  The tensor family's forward takes any sequence
+// length, its backward multiples of 128 only, and a backward with fwd_saved has to find the workspace as its own family
+// lays it out.  The size of the workspace tells the two apart: one that could not hold a backward's layout belongs to a
+// forward on its own.  `whole` = a full pass on pointers that suit the tensor family; anything else that is ragged stays on
+// the CUDA cores, whose layout fits as well (forward_bytes).
+static int forward_geo(const SsdDims* d, size_t workspace_bytes, bool whole, Geo* g, WsLayout* w) {
+  int rc = make_geo(d, g);
+  if (rc) return rc;
+  const bool has_z = d->has_z != 0;
+  make_layout(*g, has_z, family_is_tensor(*g, d), w);
+  if (g->L % 128 && whole && workspace_bytes < w->total_bwd) {
+    Geo t;
+    make_geo(d, &t, true);
+    if (family_is_tensor(t, d)) {
+      *g = t;
+      make_layout(t, has_z, true, w);
+    }
+  }
+  return SSD_OK;
+}
+static size_t forward_bytes(const SsdDims* d) {
+  Geo g;
+  WsLayout any, fwd;
+  if (forward_geo(d, SIZE_MAX, true, &g, &any) || forward_geo(d, 0, true, &g, &fwd)) return 0;
+  return any.total_fwd > fwd.total_fwd ? any.total_fwd : fwd.total_fwd;
 }
 
 // The CUDA-core kernels put (chunk, head) on one grid axis.
@@ -236,24 +265,25 @@ size_t ssd_workspace_bytes(const SsdDims* dims, int32_t pass) {
   SsdDims d2;
   if (dims) { d2 = *dims; d2.device = -1; }
   if (make_geo(dims ? &d2 : nullptr, &g)) return 0;
+  if (pass != SSD_PASS_BWD) return forward_bytes(&d2);
   WsLayout w;
   make_layout(g, dims->has_z != 0, family_is_tensor(g, dims), &w);
-  return pass == SSD_PASS_BWD ? w.total_bwd : w.total_fwd;
+  return w.total_bwd;
 }
 
 int32_t ssd_forward_staged(const SsdDims* dims, const SsdFwdPtrs* p, void* workspace, size_t workspace_bytes,
                            void* cuda_stream, int32_t stages) {
   clear_error();
   Geo g;
-  int rc = make_geo(dims, &g);
+  WsLayout w;
+  const uintptr_t low = p ? ((uintptr_t)p->x | (uintptr_t)p->Bm | (uintptr_t)p->Cm | (uintptr_t)p->z | (uintptr_t)p->y) & 15 : 0;
+  int rc = forward_geo(dims, workspace_bytes, low == 0 && stages == SSD_STAGE_ALL, &g, &w);
   if (rc) return rc;
   if (!p) { set_error("ptrs is NULL"); return SSD_ERR_NULL_POINTER; }
   if (!p->x || !p->dt || !p->A || !p->Bm || !p->Cm) { set_error("x, dt, A, B, C must be non-NULL"); return SSD_ERR_NULL_POINTER; }
   if ((stages & SSD_STAGE_FINISH) && !p->y) { set_error("y must be non-NULL"); return SSD_ERR_NULL_POINTER; }
   if ((p->z != nullptr) != (dims->has_z != 0)) { set_error("dims.has_z (%d) does not match the z pointer", dims->has_z); return SSD_ERR_BAD_SHAPE; }
   if (stages == 0 || (stages & ~(SSD_STAGE_LOCAL | SSD_STAGE_TOTAL | SSD_STAGE_FINISH | SSD_STAGE_LOCAL_STATES | SSD_STAGE_LOCAL_REST))) { set_error("bad stage mask %d", stages); return SSD_ERR_BAD_SHAPE; }
-  WsLayout w;
-  make_layout(g, dims->has_z != 0, family_is_tensor(g, dims), &w);
   rc = check_ws(workspace, workspace_bytes, w.total_fwd);
   if (rc) return rc;
   cudaStream_t s = (cudaStream_t)cuda_stream;
@@ -398,7 +428,7 @@ int32_t ssd_sp_total_logdecay(const SsdDims* dims, const void* workspace, size_t
   int rc = make_geo(dims, &g);
   if (rc) return rc;
   if (!out) { set_error("out is NULL"); return SSD_ERR_NULL_POINTER; }
-  WsLayout w;
+  WsLayout w;   // the chunk cumsums lie at the same place, in the same chunks, in every family's layout
   make_layout(g, dims->has_z != 0, family_is_tensor(g, dims), &w);
   rc = check_ws(workspace, workspace_bytes, w.total_fwd);
   if (rc) return rc;

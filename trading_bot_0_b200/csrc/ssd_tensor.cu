@@ -3328,7 +3328,9 @@ bool tensor_supported(const Geo& g, int dtype, const char** why) {
   auto no = [&](const char* m) { if (why) *why = m; return false; };
   if (dtype != SSD_BF16) return no("tensor-core kernels need bf16 storage");
   if (g.Q != QT) return no("tensor-core kernels need chunk == 128 (or a multiple of it)");
-  if (g.L % QT) return no("tensor-core kernels need seqlen % 128 == 0");
+  // A ragged tail costs the forward nothing: its loads zero-fill and its stores drop the rows past the end, and the cumsum
+  // kernel gives those positions a step size of zero.  The backward kernels store rows of their own.
+  if (g.L % QT && (!g.fwd_only || g.onetile)) return no("tensor-core kernels need seqlen % 128 == 0, except in a forward without a backward");
   if (!((g.P == 32 || g.P == 64) && (g.N == 64 || g.N == 128))) return no("tensor-core kernels cover headdim in {32,64}, dstate in {64,128}");
   if ((g.hpg * g.P) % 128) return no("heads_per_group * headdim must be a multiple of 128");
   if ((g.xsl % 8) || (g.xsb % 8) || (g.bsl % 8) || (g.bsb % 8) || (g.csl % 8) || (g.csb % 8) || (g.ysl % 8) || (g.ysb % 8) ||
