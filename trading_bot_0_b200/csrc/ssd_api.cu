@@ -42,6 +42,19 @@ void after_launch(const char* what, cudaStream_t s) {
   }
 }
 
+int sm_count() {
+  static std::atomic<int> n[64];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64) return 132;
+  int v = n[dev].load(std::memory_order_relaxed);
+  if (!v) {
+    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+    n[dev].store(v, std::memory_order_relaxed);
+  }
+  return v > 0 ? v : 132;
+}
+
 static size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
 
 // Returns 0 or a negative status (error string set).
@@ -120,7 +133,7 @@ static void make_layout(const Geo& g, bool has_z, bool tcfam, WsLayout* w) {
   w->dyp = take(has_z ? (size_t)g.B * g.L * g.H * g.P * f : 0);
   w->dcsp = take(nq); w->ddtd = take(nq); w->ddot = take(nq);
   w->sdot = take(nbh * (tcfam ? 64 : 1));   // tensor family: up to 64 warp-partial sums per entry
-  w->dapart = take(nbh); w->ddpart = take(nbh);
+  w->dapart = take(nbh); w->ddpart = take(nbh); w->dbpart = take(nbh);
   w->dini = take(nfin);
   w->total_bwd = o;
 }
@@ -287,8 +300,6 @@ int32_t ssd_forward_staged(const SsdDims* dims, const SsdFwdPtrs* p, void* works
   rc = check_ws(workspace, workspace_bytes, w.total_fwd);
   if (rc) return rc;
   cudaStream_t s = (cudaStream_t)cuda_stream;
-  SsdFwdPtrs q = *p;
-  q.final_state = nullptr;  // kernels always leave the final state in the workspace; copied out below
   const int fam = pick_family(g, dims);
   if (fam < 0) return fam;
   if (fam == 1) {
@@ -297,14 +308,7 @@ int32_t ssd_forward_staged(const SsdDims* dims, const SsdFwdPtrs* p, void* works
     for (int i = 0; i < 5; ++i)
       if ((rc = check_align16(names[i], ptrs[i]))) return rc;
   }
-  rc = run_forward(g, dims->dtype, fam == 1, q, (char*)workspace, w, s, stages);
-  if (rc) return rc;
-  if (p->final_state && (stages & (SSD_STAGE_TOTAL | SSD_STAGE_FINISH))) {
-    cudaError_t e = cudaMemcpyAsync(p->final_state, (char*)workspace + w.fin,
-                                    (size_t)g.B * g.H * g.P * g.N * sizeof(float), cudaMemcpyDeviceToDevice, s);
-    if (e != cudaSuccess) { set_error("final_state copy: %s", cudaGetErrorString(e)); return SSD_ERR_CUDA; }
-  }
-  return SSD_OK;
+  return run_forward(g, dims->dtype, fam == 1, *p, (char*)workspace, w, s, stages, workspace_bytes >= w.total_bwd);
 }
 
 int32_t ssd_forward(const SsdDims* dims, const SsdFwdPtrs* p, void* workspace, size_t workspace_bytes,

@@ -34,6 +34,7 @@ __device__ __forceinline__ float ldf_shared(const __nv_bfloat16* p) { return __b
 //   LPR = lanes that share a state row, V = float4 pieces per lane per row, RPW = rows per warp.
 template <typename T, int N>
 __global__ void __launch_bounds__(DEC_THREADS, 8) k_state_update(SsdStepDims d, SsdStepPtrs p) {
+  pdl_wait();
   constexpr int LPR = (N / 4 < 32) ? N / 4 : 32;
   constexpr int V = N / (4 * LPR);
   constexpr int RPW = 32 / LPR;
@@ -132,6 +133,7 @@ constexpr int DEC_STAGES = 3;
 
 template <typename T, int N, int R>
 __global__ void __launch_bounds__(DEC_THREADS) k_state_update_ring(SsdStepDims d, SsdStepPtrs p, long long items) {
+  pdl_wait();
   constexpr int LPR = (N / 4 < 32) ? N / 4 : 32;
   constexpr int V = N / (4 * LPR);
   constexpr int RPW = 32 / LPR;
@@ -245,6 +247,7 @@ __global__ void __launch_bounds__(DEC_THREADS) k_state_update_ring(SsdStepDims d
 // Any other dstate: one warp per state row, lanes stride over n.
 template <typename T>
 __global__ void __launch_bounds__(DEC_THREADS) k_state_update_generic(SsdStepDims d, SsdStepPtrs p) {
+  pdl_wait();
   const int sh = blockIdx.x;
   const int s = sh / d.nheads, h = sh - s * d.nheads;
   const int grp = h / (d.nheads / d.ngroups);
@@ -280,6 +283,7 @@ __global__ void __launch_bounds__(DEC_THREADS) k_state_update_generic(SsdStepDim
 
 __global__ void k_reset_rows(float* state, long long row_elems, const long long* idx, long long count,
                              long long streams) {
+  pdl_wait();
   const long long r = blockIdx.y;
   if (r >= count) return;
   const long long s = idx[r];
@@ -293,6 +297,7 @@ __global__ void k_reset_rows(float* state, long long row_elems, const long long*
 }
 
 __global__ void k_total_logdecay(Geo g, const float* __restrict__ cs, float* __restrict__ out) {
+  pdl_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;  // b*H + h
   if (i >= g.B * g.H) return;
   float v = 0.f;
@@ -306,6 +311,7 @@ __global__ void k_total_logdecay(Geo g, const float* __restrict__ cs, float* __r
 __global__ void k_sp_prefix(const float* __restrict__ gs, const float* __restrict__ gl, int world, int rank,
                             int direction, long long bh, long long elems, const float* __restrict__ init,
                             float* __restrict__ out) {
+  pdl_wait();
   const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   const long long r = blockIdx.y;  // b*H + h
   if (e >= elems) return;
@@ -331,15 +337,10 @@ static bool launch_ring(const SsdStepDims& d, const SsdStepPtrs& p, cudaStream_t
   if (!al(p.x, d.x_stride_s) || !al(p.Bm, d.b_stride_s) || !al(p.Cm, d.c_stride_s) || ((uintptr_t)p.state % 16)) return false;
   const long long items = (long long)d.streams * d.nheads;
   constexpr int smem = DEC_STAGES * STAGE;
-  auto k = k_state_update_ring<T, N, R>;
-  cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);   // per device, so at every launch
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int per_sm = (227 * 1024) / (smem + 1024) < 16 ? (227 * 1024) / (smem + 1024) : 16;
-  long long grid = (long long)sms * (per_sm > 0 ? per_sm : 1);
+  long long grid = (long long)sm_count() * (per_sm > 0 ? per_sm : 1);
   if (grid > items) grid = items;
-  k<<<(unsigned)grid, DEC_THREADS, smem, s>>>(d, p, items);
+  launch<k_state_update_ring<T, N, R>>((unsigned)grid, DEC_THREADS, smem, s, d, p, items);
   return true;
 }
 
@@ -351,12 +352,12 @@ static int decode_t(const SsdStepDims& d, const SsdStepPtrs& p, cudaStream_t s) 
     return SSD_OK;
   }
   switch (d.dstate) {
-    case 16: k_state_update<T, 16><<<blocks, DEC_THREADS, 0, s>>>(d, p); break;
-    case 32: k_state_update<T, 32><<<blocks, DEC_THREADS, 0, s>>>(d, p); break;
-    case 64: k_state_update<T, 64><<<blocks, DEC_THREADS, 0, s>>>(d, p); break;
-    case 128: k_state_update<T, 128><<<blocks, DEC_THREADS, 0, s>>>(d, p); break;
-    case 256: k_state_update<T, 256><<<blocks, DEC_THREADS, 0, s>>>(d, p); break;
-    default: k_state_update_generic<T><<<blocks, DEC_THREADS, 0, s>>>(d, p); break;
+    case 16: launch<k_state_update<T, 16>>(blocks, DEC_THREADS, 0, s, d, p); break;
+    case 32: launch<k_state_update<T, 32>>(blocks, DEC_THREADS, 0, s, d, p); break;
+    case 64: launch<k_state_update<T, 64>>(blocks, DEC_THREADS, 0, s, d, p); break;
+    case 128: launch<k_state_update<T, 128>>(blocks, DEC_THREADS, 0, s, d, p); break;
+    case 256: launch<k_state_update<T, 256>>(blocks, DEC_THREADS, 0, s, d, p); break;
+    default: launch<k_state_update_generic<T>>(blocks, DEC_THREADS, 0, s, d, p); break;
   }
   SSD_CUDA_CHECK_LAUNCH("state_update");
   return SSD_OK;
@@ -373,21 +374,21 @@ int reset_rows(float* state, long long row_elems, const long long* idx, long lon
   const unsigned gx = (unsigned)((n4 + 255) / 256 > 0 ? ((n4 + 255) / 256 < 64 ? (n4 + 255) / 256 : 64) : 1);
   for (long long off = 0; off < count; off += 65535) {
     const long long c = (count - off < 65535) ? count - off : 65535;
-    k_reset_rows<<<dim3(gx, (unsigned)c), 256, 0, s>>>(state, row_elems, idx + off, c, streams);
+    launch<k_reset_rows>(dim3(gx, (unsigned)c), 256, 0, s, state, row_elems, idx + off, c, streams);
   }
   SSD_CUDA_CHECK_LAUNCH("state_reset_rows");
   return SSD_OK;
 }
 
 int sp_total_logdecay(const Geo& g, const float* cs, float* out, cudaStream_t s) {
-  k_total_logdecay<<<cdiv(g.B * g.H, 128), 128, 0, s>>>(g, cs, out);
+  launch<k_total_logdecay>(cdiv(g.B * g.H, 128), 128, 0, s, g, cs, out);
   SSD_CUDA_CHECK_LAUNCH("sp_total_logdecay");
   return SSD_OK;
 }
 
 int sp_prefix_state(const float* gs, const float* gl, int world, int rank, int direction, long long bh,
                     long long elems, const float* init, float* out, cudaStream_t s) {
-  k_sp_prefix<<<dim3((unsigned)((elems + 255) / 256), (unsigned)bh), 256, 0, s>>>(gs, gl, world, rank, direction, bh,
+  launch<k_sp_prefix>(dim3((unsigned)((elems + 255) / 256), (unsigned)bh), 256, 0, s, gs, gl, world, rank, direction, bh,
                                                                                  elems, init, out);
   SSD_CUDA_CHECK_LAUNCH("sp_prefix_state");
   return SSD_OK;

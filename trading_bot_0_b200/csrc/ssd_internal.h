@@ -7,8 +7,9 @@ namespace ssd {
 enum { SSD_STAGE_ALL = SSD_STAGE_LOCAL | SSD_STAGE_FINISH };
 
 // `tc` selects the tensor-core stages where they exist (caller has checked tensor_supported).
+// `for_backward`: the workspace can hold a backward, which reads the final state there; p.final_state gets it either way.
 int run_forward(const Geo& g, int dtype, bool tc, const SsdFwdPtrs& p, char* ws, const WsLayout& w, cudaStream_t s,
-                int stages);
+                int stages, bool for_backward);
 int run_backward(const Geo& g, int dtype, bool tc, const SsdBwdPtrs& p, char* ws, const WsLayout& w, cudaStream_t s,
                  int stages);
 
@@ -17,14 +18,14 @@ int run_backward(const Geo& g, int dtype, bool tc, const SsdBwdPtrs& p, char* ws
 bool tensor_supported(const Geo& g, int dtype, const char** why);
 int tensor_chunk_state(const Geo& g, int mode, const void* xdy, long long sb, long long sl, const void* bc,
                        long long bsb, long long bsl, const float* tab, float* out, int* status, cudaStream_t s);
-int tensor_state_passing(const Geo& g, float* st, const float* cs, const float* init, float* last, void* st_bf,
+int tensor_state_passing(const Geo& g, float* st, const float* cs, const float* init, float* last, float* last2, void* st_bf,
                          int reverse, bool write, const float* fwd_prev, const void* fwd_prev_bf, const float* fwd_fin,
                          float* sdot, int* sdot_nw,
                          cudaStream_t s);
 // both in one launch where it applies (dstate 64, full pass): fp32 `st` optional, bf16 `st_bf` always
 bool tensor_state_fused_applies(const Geo& g);
 int tensor_state_fused(const Geo& g, int mode, const void* xdy, long long sb, long long sl, const void* bc, long long bsb,
-                       long long bsl, const float* tab, float* st, void* st_bf, const float* init, float* last,
+                       long long bsl, const float* tab, float* st, void* st_bf, const float* init, float* last, float* last2,
                        const void* fwd_prev_bf, const float* fwd_fin, float* sdot, int* sdot_nw, int* status, cudaStream_t s);
 int tensor_chunk_scan(const Geo& g, const SsdFwdPtrs& p, const float* tab, const void* prev_bf, int* status,
                       cudaStream_t s);

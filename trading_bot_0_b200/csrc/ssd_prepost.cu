@@ -139,6 +139,7 @@ template <typename T, int K, int NC>
 __global__ void __launch_bounds__(CONV_THREADS) k_conv_fwd(SsdConvDims d, const T* __restrict__ in,
                                                            const float* __restrict__ weight, const float* __restrict__ bias,
                                                            T* __restrict__ out) {
+  pdl_wait();
   const int CV = d.channels / NC, ntile = (d.seqlen + CONV_TL - 1) / CONV_TL;
   const long long item = (long long)blockIdx.x * CONV_THREADS + threadIdx.x;
   if (item >= (long long)d.batch * ntile * CV) return;
@@ -226,6 +227,7 @@ template <typename T, int K>
 __global__ void __launch_bounds__(CONVS_THREADS, CONVS_CTAS_PER_SM)
 k_conv_fwd_sm(SsdConvDims d, const T* __restrict__ in, const float* __restrict__ weight, const float* __restrict__ bias,
               T* __restrict__ out, int ntt) {
+  pdl_wait();
   constexpr int NC = 16 / (int)sizeof(T);            // channels per 16-byte copy piece
   constexpr int NP = 8 / (int)sizeof(T);             // channels per thread in the arithmetic (8 bytes: half the weights in
                                                      // registers of a 16-byte mapping, so a fourth block fits an SM)
@@ -344,6 +346,7 @@ __global__ void __launch_bounds__(CONV_THREADS, CONV_BWD_MINB) k_conv_bwd(SsdCon
                                                            const float* __restrict__ weight, const float* __restrict__ bias,
                                                            ConvSegs segs, T* __restrict__ din, long long din_stride_b,
                                                            long long din_stride_l, float* __restrict__ partial) {
+  pdl_wait();
   constexpr int CH = CONV_BWD_CH;
   const int CV = d.channels / NC;
   const long long item = (long long)blockIdx.x * CONV_THREADS + threadIdx.x;
@@ -469,6 +472,7 @@ __global__ void __launch_bounds__(CONVS_THREADS, CONVB_CTAS_PER_SM)
 k_conv_bwd_sm(SsdConvDims d, const T* __restrict__ in, const float* __restrict__ weight, const float* __restrict__ bias,
               ConvSegs segs, T* __restrict__ din, long long din_stride_b, long long din_stride_l,
               float* __restrict__ partial, int ntt) {
+  pdl_wait();
   constexpr int NC = 16 / (int)sizeof(T);            // channels per 16-byte copy piece
   constexpr int NP = 8 / (int)sizeof(T);             // channels per thread in the arithmetic phases
   constexpr int CB = CONVS_ROWB / (int)sizeof(T);    // channels per tile
@@ -663,13 +667,35 @@ k_conv_bwd_sm(SsdConvDims d, const T* __restrict__ in, const float* __restrict__
   }
 }
 
-// dweight[c,k] / dbias[c] = sum over blocks of the partials, in block order
-__global__ void k_conv_reduce(int nblk, int channels, int K, const float* __restrict__ partial, float* __restrict__ dweight,
-                              float* __restrict__ dbias) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= channels * (K + 1)) return;
+// Column sums of the per-block partial rows.  A block takes 32 columns with 32 row groups: every group adds its rows in
+// order, then the groups are added in order (the same sum for the same grid, whatever the timing).  The kernel is one chain
+// of memory round trips per thread, so the rows are spread wide and four loads of a group are in flight (one thread walking
+// all 148 conv rows of a column took 14 us, this 7 with its launch).
+constexpr int RED_GROUPS = 32;
+__device__ __forceinline__ float column_sum(const float* __restrict__ partial, int nblk, int width, int i) {
+  __shared__ float red[RED_GROUPS][33];
   float a = 0.f;
-  for (int r = 0; r < nblk; ++r) a += partial[(size_t)r * channels * (K + 1) + i];
+  if (i < width) {
+#pragma unroll 4
+    for (int r = threadIdx.y; r < nblk; r += RED_GROUPS) a += partial[(size_t)r * width + i];
+  }
+  red[threadIdx.y][threadIdx.x] = a;
+  __syncthreads();
+  float t = 0.f;
+  if (threadIdx.y == 0) {
+#pragma unroll
+    for (int q = 0; q < RED_GROUPS; ++q) t += red[q][threadIdx.x];
+  }
+  return t;   // in row group 0
+}
+
+// dweight[c,k] / dbias[c] from rows of [channels][K + 1]
+__global__ void __launch_bounds__(32 * RED_GROUPS) k_conv_reduce(int nblk, int channels, int K, const float* __restrict__ partial,
+                                                                 float* __restrict__ dweight, float* __restrict__ dbias) {
+  pdl_wait();
+  const int i = blockIdx.x * 32 + threadIdx.x, width = channels * (K + 1);
+  const float a = column_sum(partial, nblk, width, i);
+  if (threadIdx.y || i >= width) return;
   const int c = i / (K + 1), k = i - c * (K + 1);
   if (k < K) dweight[(size_t)c * K + k] = a;
   else if (dbias) dbias[c] = a;
@@ -683,6 +709,7 @@ template <typename T, int NV>
 __global__ void __launch_bounds__(NORM_THREADS) k_rmsnorm_fwd(SsdNormDims d, const T* __restrict__ in,
                                                               const float* __restrict__ weight, T* __restrict__ out,
                                                               float* __restrict__ rstd) {
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const long long row = (long long)blockIdx.x * (NORM_THREADS / 32) + (threadIdx.x >> 5);
   if (row >= d.rows) return;
@@ -726,6 +753,7 @@ __global__ void __launch_bounds__(NORM_THREADS) k_rmsnorm_bwd(SsdNormDims d, con
                                                               const T* __restrict__ dout, long long dout_stride_row,
                                                               T* __restrict__ din, long long din_stride_row,
                                                               float* __restrict__ partial) {
+  pdl_wait();
   constexpr int RU = NV == 1 ? 4 : (NV == 2 ? 2 : 1);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nv = d.width / 8;
@@ -827,6 +855,7 @@ __global__ void __launch_bounds__(NORM_THREADS, 8) k_rmsnorm_bwd_ring(SsdNormDim
                                                                       const T* __restrict__ dout, long long dout_stride_row,
                                                                       T* __restrict__ din, long long din_stride_row,
                                                                       float* __restrict__ partial) {
+  pdl_wait();
   constexpr int ES = (int)sizeof(T), RW = NORMR_ROWS, S = NORMR_STAGES;
   extern __shared__ __align__(16) unsigned char norm_ring[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -947,22 +976,13 @@ __global__ void __launch_bounds__(NORM_THREADS, 8) k_rmsnorm_bwd_ring(SsdNormDim
   }
 }
 
-// dweight[i] = sum over blocks of the partials: eight row groups per column add their rows in order, then the groups
-// are added in order (the same sum for the same grid, whatever the timing)
-__global__ void k_norm_reduce(int nblk, int width, const float* __restrict__ partial, float* __restrict__ dweight) {
-  __shared__ float red[8][32];
-  const int i = blockIdx.x * 32 + threadIdx.x, g = threadIdx.y;
-  float a = 0.f;
-  if (i < width)
-    for (int r = g; r < nblk; r += 8) a += partial[(size_t)r * width + i];
-  red[g][threadIdx.x] = a;
-  __syncthreads();
-  if (g == 0 && i < width) {
-    float t = 0.f;
-#pragma unroll
-    for (int q = 0; q < 8; ++q) t += red[q][threadIdx.x];
-    dweight[i] = t;
-  }
+// dweight[i] from rows of [width]
+__global__ void __launch_bounds__(32 * RED_GROUPS) k_norm_reduce(int nblk, int width, const float* __restrict__ partial,
+                                                                 float* __restrict__ dweight) {
+  pdl_wait();
+  const int i = blockIdx.x * 32 + threadIdx.x;
+  const float a = column_sum(partial, nblk, width, i);
+  if (threadIdx.y == 0 && i < width) dweight[i] = a;
 }
 
 int conv_rows(const SsdConvDims* d) {   // thread rows of the backward kernel = partial sums to add
@@ -1016,9 +1036,7 @@ int32_t ssd_conv1d_forward(const SsdConvDims* dims, const void* in, const float*
     // shared-memory staged kernel: tiles of 64 tokens x 256 bytes of channels, persistent CTAs
     const int ntt = (dims->seqlen + CONVS_TT - 1) / CONVS_TT;
     const int ncb = (dims->channels * esz + CONVS_ROWB - 1) / CONVS_ROWB;
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int sms = sm_count();
     const long long pairs = (long long)dims->batch * ntt;
     if (pairs > 0x7fffffffLL) { set_error("conv1d: batch x token tiles exceeds 2^31"); return SSD_ERR_UNSUPPORTED; }
     long long gx = ((long long)sms * CONVS_CTAS_PER_SM) / ncb;
@@ -1028,8 +1046,7 @@ int32_t ssd_conv1d_forward(const SsdConvDims* dims, const void* in, const float*
     const dim3 grid((unsigned)gx, (unsigned)ncb);
 #define CONV_FWD_SM(T, K) do { \
       constexpr int smem = (CONVS_TT + K - 1) * CONVS_ROWB * CONVS_STAGES; \
-      cudaFuncSetAttribute(k_conv_fwd_sm<T, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); \
-      k_conv_fwd_sm<T, K><<<grid, CONVS_THREADS, smem, s>>>(*dims, (const T*)in, weight, bias, (T*)out, ntt); } while (0)
+      launch<k_conv_fwd_sm<T, K>>(grid, CONVS_THREADS, smem, s, *dims, (const T*)in, weight, bias, (T*)out, ntt); } while (0)
     if (dims->dtype == SSD_BF16) {
       if (dims->width == 4) CONV_FWD_SM(__nv_bfloat16, 4); else if (dims->width == 3) CONV_FWD_SM(__nv_bfloat16, 3); else CONV_FWD_SM(__nv_bfloat16, 2);
     } else {
@@ -1042,7 +1059,7 @@ int32_t ssd_conv1d_forward(const SsdConvDims* dims, const void* in, const float*
   constexpr int NCF = 8;   // channels per thread, forward
   const long long items = (long long)dims->batch * ((dims->seqlen + CONV_TL - 1) / CONV_TL) * (dims->channels / NCF);
   const unsigned grid = (unsigned)((items + CONV_THREADS - 1) / CONV_THREADS);
-#define CONV_FWD(T, K) k_conv_fwd<T, K, NCF><<<grid, CONV_THREADS, 0, s>>>(*dims, (const T*)in, weight, bias, (T*)out)
+#define CONV_FWD(T, K) launch<k_conv_fwd<T, K, NCF>>(grid, CONV_THREADS, 0, s, *dims, (const T*)in, weight, bias, (T*)out)
   if (dims->dtype == SSD_BF16) {
     if (dims->width == 4) CONV_FWD(__nv_bfloat16, 4); else if (dims->width == 3) CONV_FWD(__nv_bfloat16, 3); else CONV_FWD(__nv_bfloat16, 2);
   } else {
@@ -1092,9 +1109,7 @@ int32_t ssd_conv1d_backward(const SsdConvDims* dims, const void* in, const float
   if ((long long)dims->channels * es >= CONVS_ROWB / 2) {
     const int ntt = (dims->seqlen + CONVB_TT - 1) / CONVB_TT;
     const int ncb = (dims->channels * es + CONVS_ROWB - 1) / CONVS_ROWB;
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int sms = sm_count();
     long long nx = ((long long)sms * CONVB_CTAS_PER_SM + ncb - 1) / ncb;
     const long long pairs = (long long)dims->batch * ntt;
     if (pairs > 0x7fffffffLL || ncb > 65535) { set_error("conv1d backward: batch x token tiles exceeds 2^31"); return SSD_ERR_UNSUPPORTED; }
@@ -1103,8 +1118,7 @@ int32_t ssd_conv1d_backward(const SsdConvDims* dims, const void* in, const float
     const dim3 grid((unsigned)nx, (unsigned)ncb);
 #define CONV_BWD_SM(T, K) do { \
       constexpr int smem = CONVB_STAGES * (2 * CONVB_TT + 3 * (K - 1)) * CONVS_ROWB + (CONVB_TT + K - 1) * (CONVS_ROWB / (int)sizeof(T)) * 4; \
-      cudaFuncSetAttribute(k_conv_bwd_sm<T, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); \
-      k_conv_bwd_sm<T, K><<<grid, CONVS_THREADS, smem, s>>>(*dims, (const T*)in, weight, bias, segs, (T*)din, din_stride_b, din_stride_l, partial, ntt); } while (0)
+      launch<k_conv_bwd_sm<T, K>>(grid, CONVS_THREADS, smem, s, *dims, (const T*)in, weight, bias, segs, (T*)din, din_stride_b, din_stride_l, partial, ntt); } while (0)
     if (dims->dtype == SSD_BF16) {
       if (dims->width == 4) CONV_BWD_SM(__nv_bfloat16, 4); else if (dims->width == 3) CONV_BWD_SM(__nv_bfloat16, 3); else CONV_BWD_SM(__nv_bfloat16, 2);
     } else {
@@ -1113,13 +1127,13 @@ int32_t ssd_conv1d_backward(const SsdConvDims* dims, const void* in, const float
 #undef CONV_BWD_SM
     SSD_CUDA_CHECK_LAUNCH("conv1d_bwd");
     const int n = dims->channels * (dims->width + 1);
-    k_conv_reduce<<<(n + 255) / 256, 256, 0, s>>>((int)nx, dims->channels, dims->width, partial, dweight, dbias);
+    launch<k_conv_reduce>((n + 31) / 32, dim3(32, RED_GROUPS), 0, s, (int)nx, dims->channels, dims->width, partial, dweight, dbias);
     SSD_CUDA_CHECK_LAUNCH("conv1d_reduce");
     return SSD_OK;
   }
   constexpr int NCB = 4;   // channels per thread, backward (half the registers of 8: twice the resident warps)
   const unsigned grid = (unsigned)(((long long)nblk * (dims->channels / NCB) + CONV_THREADS - 1) / CONV_THREADS);
-#define CONV_BWD(T, K) k_conv_bwd<T, K, NCB><<<grid, CONV_THREADS, 0, s>>>(*dims, nblk, (const T*)in, weight, bias, segs, (T*)din, din_stride_b, din_stride_l, partial)
+#define CONV_BWD(T, K) launch<k_conv_bwd<T, K, NCB>>(grid, CONV_THREADS, 0, s, *dims, nblk, (const T*)in, weight, bias, segs, (T*)din, din_stride_b, din_stride_l, partial)
   if (dims->dtype == SSD_BF16) {
     if (dims->width == 4) CONV_BWD(__nv_bfloat16, 4); else if (dims->width == 3) CONV_BWD(__nv_bfloat16, 3); else CONV_BWD(__nv_bfloat16, 2);
   } else {
@@ -1128,7 +1142,7 @@ int32_t ssd_conv1d_backward(const SsdConvDims* dims, const void* in, const float
 #undef CONV_BWD
   SSD_CUDA_CHECK_LAUNCH("conv1d_bwd");
   const int n = dims->channels * (dims->width + 1);
-  k_conv_reduce<<<(n + 255) / 256, 256, 0, s>>>(nblk, dims->channels, dims->width, partial, dweight, dbias);
+  launch<k_conv_reduce>((n + 31) / 32, dim3(32, RED_GROUPS), 0, s, nblk, dims->channels, dims->width, partial, dweight, dbias);
   SSD_CUDA_CHECK_LAUNCH("conv1d_reduce");
   return SSD_OK;
 }
@@ -1162,7 +1176,7 @@ int32_t ssd_rmsnorm_forward(const SsdNormDims* dims, const void* in, const float
   cudaStream_t s = (cudaStream_t)cuda_stream;
   const long long nb = (dims->rows + NORM_THREADS / 32 - 1) / (NORM_THREADS / 32);
   const int nvl = (dims->width / 8 + 31) / 32;   // vectors per lane
-#define NORM_FWD(T, NV) k_rmsnorm_fwd<T, NV><<<(unsigned)nb, NORM_THREADS, 0, s>>>(*dims, (const T*)in, weight, (T*)out, rstd)
+#define NORM_FWD(T, NV) launch<k_rmsnorm_fwd<T, NV>>((unsigned)nb, NORM_THREADS, 0, s, *dims, (const T*)in, weight, (T*)out, rstd)
 #define NORM_FWD_T(T) do { if (nvl <= 1) NORM_FWD(T, 1); else if (nvl <= 2) NORM_FWD(T, 2); else if (nvl <= 4) NORM_FWD(T, 4); else NORM_FWD(T, 8); } while (0)
   if (dims->dtype == SSD_BF16) NORM_FWD_T(__nv_bfloat16); else NORM_FWD_T(float);
 #undef NORM_FWD_T
@@ -1194,15 +1208,14 @@ int32_t ssd_rmsnorm_backward(const SsdNormDims* dims, const void* in, const floa
   }
   cudaStream_t s = (cudaStream_t)cuda_stream;
   const int nvl = (dims->width / 8 + 31) / 32;
-#define NORM_BWD(T, NV) k_rmsnorm_bwd<T, NV><<<nblk, NORM_THREADS, 0, s>>>(*dims, (const T*)in, weight, rstd, (const T*)dout, dout_stride_row, (T*)din, din_stride_row, partial)
+#define NORM_BWD(T, NV) launch<k_rmsnorm_bwd<T, NV>>(nblk, NORM_THREADS, 0, s, *dims, (const T*)in, weight, rstd, (const T*)dout, dout_stride_row, (T*)din, din_stride_row, partial)
 #define NORM_BWD_T(T) do { if (nvl <= 1) NORM_BWD(T, 1); else if (nvl <= 2) NORM_BWD(T, 2); else if (nvl <= 4) NORM_BWD(T, 4); else NORM_BWD(T, 8); } while (0)
   const int row_bytes = dims->width * es;
   const int ring_smem = (NORM_THREADS / 32) * NORMR_STAGES * 2 * NORMR_ROWS * row_bytes;
   const bool ring = nvl <= 1 && (row_bytes % 16) == 0 && ring_smem <= 96 * 1024 && (dims->in_stride_row * es) % 16 == 0;
   if (ring) {
 #define NORM_BWD_RING(T, NV) do { \
-      cudaFuncSetAttribute(k_rmsnorm_bwd_ring<T, NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, ring_smem); \
-      k_rmsnorm_bwd_ring<T, NV><<<nblk, NORM_THREADS, ring_smem, s>>>(*dims, (const T*)in, weight, rstd, (const T*)dout, dout_stride_row, (T*)din, din_stride_row, partial); } while (0)
+      launch<k_rmsnorm_bwd_ring<T, NV>>(nblk, NORM_THREADS, ring_smem, s, *dims, (const T*)in, weight, rstd, (const T*)dout, dout_stride_row, (T*)din, din_stride_row, partial); } while (0)
     if (dims->dtype == SSD_BF16) NORM_BWD_RING(__nv_bfloat16, 1); else NORM_BWD_RING(float, 1);
 #undef NORM_BWD_RING
   } else if (dims->dtype == SSD_BF16) NORM_BWD_T(__nv_bfloat16); else NORM_BWD_T(float);
@@ -1210,7 +1223,7 @@ int32_t ssd_rmsnorm_backward(const SsdNormDims* dims, const void* in, const floa
 #undef NORM_BWD
   SSD_CUDA_CHECK_LAUNCH("rmsnorm_bwd");
   if (dweight) {
-    k_norm_reduce<<<(dims->width + 31) / 32, dim3(32, 8), 0, s>>>(nblk, dims->width, partial, dweight);
+    launch<k_norm_reduce>((dims->width + 31) / 32, dim3(32, RED_GROUPS), 0, s, nblk, dims->width, partial, dweight);
     SSD_CUDA_CHECK_LAUNCH("rmsnorm_reduce");
   }
   return SSD_OK;

@@ -92,12 +92,16 @@ template <typename T>
 __global__ void __launch_bounds__(NT) k_cumsum(Geo g, const T* __restrict__ dt, const float* __restrict__ dt_bias,
                                                const float* __restrict__ A, float* __restrict__ cs,
                                                float* __restrict__ dtf, float* __restrict__ tab, int* __restrict__ hmax,
-                                               int tag) {
+                                               int tag, int* __restrict__ status) {
+  pdl_wait();
   constexpr int HG = 8;
   const int c = blockIdx.x, b = blockIdx.y, q = threadIdx.x;
   __shared__ float wsum[NT / 32][HG];
   const int t = c * g.Q + q;
-  if (hmax && c == 0 && b == 0 && q == 0) hmax[g.H] = tag;
+  if (c == 0 && b == 0 && q == 0) {   // first kernel of a pass: the status word and the tag of this launch
+    *status = 0;
+    if (hmax) hmax[g.H] = tag;
+  }
   const bool live = (q < g.Q) && (t < g.L);
   const int lane = q & 31, w = q >> 5;
   const T* row = dt + b * g.dtsb + (long long)t * g.dtsl;
@@ -168,6 +172,7 @@ __global__ void __launch_bounds__(NT) k_chunk_state(Geo g, const T* __restrict__
                                                     DySrc<T> dys, const T* __restrict__ Y, long long ysb,
                                                     long long ysl, const float* __restrict__ cs,
                                                     const float* __restrict__ dtf, float* __restrict__ out) {
+  pdl_wait();
   __shared__ __align__(16) float As[TK * LDS];
   __shared__ __align__(16) float Bs[TK * LDS];
   __shared__ float wl[256];
@@ -216,7 +221,8 @@ __global__ void __launch_bounds__(NT) k_chunk_state(Geo g, const T* __restrict__
 template <bool WRITE>
 __global__ void __launch_bounds__(NT) k_state_passing(Geo g, float* __restrict__ st, const float* __restrict__ cs,
                                                       const float* __restrict__ init, float* __restrict__ last,
-                                                      int reverse) {
+                                                      float* __restrict__ last2, int reverse) {
+  pdl_wait();
   const int e = blockIdx.x * NT + threadIdx.x, h = blockIdx.y, b = blockIdx.z;
   const int PN = g.P * g.N;
   if (e >= PN) return;
@@ -229,6 +235,7 @@ __global__ void __launch_bounds__(NT) k_state_passing(Geo g, float* __restrict__
     run = expf(cs[cs_idx(g, b, h, c) + g.Q - 1]) * run + v;
   }
   if (last) last[((size_t)(b * g.H + h)) * PN + e] = run;
+  if (last2) last2[((size_t)(b * g.H + h)) * PN + e] = run;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -236,6 +243,7 @@ __global__ void __launch_bounds__(NT) k_state_passing(Geo g, float* __restrict__
 template <typename T>
 __global__ void __launch_bounds__(NT) k_cb(Geo g, const T* __restrict__ Bm, const T* __restrict__ Cm,
                                            float* __restrict__ cb) {
+  pdl_wait();
   __shared__ __align__(16) float As[TK * LDS];
   __shared__ __align__(16) float Bs[TK * LDS];
   const int nt = (g.Q + TM - 1) / TM;
@@ -285,6 +293,7 @@ __global__ void __launch_bounds__(NT) k_chunk_scan(Geo g, const T* __restrict__ 
                                                    T* __restrict__ y, const T* __restrict__ dy,
                                                    float* __restrict__ dyp, T* __restrict__ dz,
                                                    float* __restrict__ dcsp, float* __restrict__ ddot) {
+  pdl_wait();
   __shared__ __align__(16) float As[TK * LDS];
   __shared__ __align__(16) float Bs[TK * LDS];
   __shared__ float css[256], dts[256];
@@ -380,6 +389,7 @@ __global__ void __launch_bounds__(NT) k_dx(Geo g, const T* __restrict__ x, const
                                            const float* __restrict__ cs, const float* __restrict__ dtf,
                                            const float* __restrict__ cb, const float* __restrict__ dS,
                                            T* __restrict__ dx, float* __restrict__ ddtd) {
+  pdl_wait();
   __shared__ __align__(16) float As[TK * LDS];
   __shared__ __align__(16) float Bs[TK * LDS];
   __shared__ float css[256];
@@ -450,6 +460,7 @@ template <typename T>
 __global__ void __launch_bounds__(NT) k_dw(Geo g, const T* __restrict__ x, DySrc<T> dys,
                                            const float* __restrict__ cs, const float* __restrict__ dtf,
                                            float* __restrict__ wsum) {
+  pdl_wait();
   __shared__ __align__(16) float As[TK * LDS];
   __shared__ __align__(16) float Bs[TK * LDS];
   const int nt = (g.Q + TM - 1) / TM;
@@ -512,6 +523,7 @@ __global__ void __launch_bounds__(NT) k_dbc(Geo g, const T* __restrict__ x, cons
                                             const float* __restrict__ cs, const float* __restrict__ dtf,
                                             const float* __restrict__ wsum, const float* __restrict__ st,
                                             T* __restrict__ out) {
+  pdl_wait();
   __shared__ __align__(16) float As[TK * LDS];
   __shared__ __align__(16) float Bs[TK * LDS];
   const int ntn = (g.N + TN - 1) / TN;
@@ -572,6 +584,7 @@ __global__ void __launch_bounds__(NT) k_dbc(Geo g, const T* __restrict__ x, cons
 // Backward: sdot[b,c,h] = <dS_end_c, S_end_c>, with S_end_c = state entering chunk c+1 (or final).
 __global__ void __launch_bounds__(NT) k_sdot(Geo g, const float* __restrict__ dS, const float* __restrict__ prev,
                                              const float* __restrict__ fin, float* __restrict__ sdot) {
+  pdl_wait();
   const int c = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
   const int PN = g.P * g.N;
   const float* a = dS + st_idx(g, b, c, h);
@@ -599,10 +612,11 @@ __global__ void __launch_bounds__(NT) k_ddt(Geo g, const float* __restrict__ A, 
                                             const float* __restrict__ dcsp, const float* __restrict__ ddtd,
                                             const float* __restrict__ ddot, const float* __restrict__ sdot, int nw,
                                             float* __restrict__ ddt, float* __restrict__ dapart,
-                                            float* __restrict__ ddpart) {
+                                            float* __restrict__ ddpart, float* __restrict__ dbpart) {
+  pdl_wait();
   constexpr int HG = 8;
   const int c = blockIdx.x, b = blockIdx.y, q = threadIdx.x;
-  __shared__ float wsum[NT / 32][HG], red1[NT / 32][HG], red2[NT / 32][HG], ssd[HG];
+  __shared__ float wsum[NT / 32][HG], red1[NT / 32][HG], red2[NT / 32][HG], red3[NT / 32][HG], ssd[HG];
   const int qr = g.Q - 1 - q;   // reversed position: an inclusive prefix scan over q is a suffix sum over qr
   const bool ok = (q < g.Q);
   const int lane = q & 31, w = q >> 5, nwarp = blockDim.x >> 5;   // launched with 128 threads when the chunk is <= 128 long
@@ -672,6 +686,15 @@ __global__ void __launch_bounds__(NT) k_ddt(Geo g, const float* __restrict__ A, 
         s2[k] += __shfl_xor_sync(0xffffffffu, s2[k], o);
       }
     }
+    if (dbpart) {   // the chunk's share of the step-size bias gradient
+#pragma unroll
+      for (int k = 0; k < HG; ++k) {
+        float s3 = (ok && t < g.L) ? v[k] : 0.f;
+#pragma unroll
+        for (int o = 16; o; o >>= 1) s3 += __shfl_xor_sync(0xffffffffu, s3, o);
+        if (lane == 0) red3[w][k] = s3;
+      }
+    }
     if (lane == 0) {
 #pragma unroll
       for (int k = 0; k < HG; ++k) { red1[w][k] = s1[k]; red2[w][k] = s2[k]; }
@@ -680,6 +703,11 @@ __global__ void __launch_bounds__(NT) k_ddt(Geo g, const float* __restrict__ A, 
     if (q < HG && h0 + q < g.H) {
       float a1 = 0.f, a2 = 0.f;
       for (int i = 0; i < nwarp; ++i) { a1 += red1[i][q]; a2 += red2[i][q]; }
+      if (dbpart) {
+        float a3 = 0.f;
+        for (int i = 0; i < nwarp; ++i) a3 += red3[i][q];
+        dbpart[(size_t)(b * g.nc + c) * g.H + h0 + q] = a3;
+      }
       dapart[(size_t)(b * g.nc + c) * g.H + h0 + q] = a1;
       ddpart[(size_t)(b * g.nc + c) * g.H + h0 + q] = a2;
     }
@@ -687,46 +715,37 @@ __global__ void __launch_bounds__(NT) k_ddt(Geo g, const float* __restrict__ A, 
   }
 }
 
-// ddt_bias[h] = sum over (b,t) of ddt[b,t,h].  One block per head, fixed summation order.
-__global__ void __launch_bounds__(NT) k_sum_ddt(long long rows, int H, const float* __restrict__ ddt, float* __restrict__ out) {
+// dA[h] = sum over (b,c) of dapart; dD, ddt_bias likewise.  One block per head, fixed summation order.  The block is as large
+// as it gets because the kernel is a chain of dependent memory round trips: rows / 1024 of them.
+constexpr int RH_THREADS = 1024;
+__global__ void __launch_bounds__(RH_THREADS) k_reduce_heads(int rows, int H, const float* __restrict__ dapart,
+                                                             const float* __restrict__ ddpart, const float* __restrict__ dbpart,
+                                                             float* __restrict__ dA, float* __restrict__ dD, float* __restrict__ dbias) {
+  pdl_wait();
   const int h = blockIdx.x;
-  float a = 0.f;
-  for (long long r = threadIdx.x; r < rows; r += NT) a += ddt[r * H + h];
-  __shared__ float r1[NT / 32];
-#pragma unroll
-  for (int o = 16; o; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-  if ((threadIdx.x & 31) == 0) r1[threadIdx.x >> 5] = a;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float t = 0.f;
-    for (int i = 0; i < NT / 32; ++i) t += r1[i];
-    out[h] = t;
-  }
-}
-
-// dA[h] = sum over (b,c) of dapart ; dD likewise.  One block per head, fixed summation order.
-__global__ void __launch_bounds__(NT) k_reduce_heads(int rows, int H, const float* __restrict__ dapart,
-                                                     const float* __restrict__ ddpart, float* __restrict__ dA,
-                                                     float* __restrict__ dD) {
-  const int h = blockIdx.x;
-  float a = 0.f, d = 0.f;
-  for (int r = threadIdx.x; r < rows; r += NT) {
+  float a = 0.f, d = 0.f, e = 0.f;
+#pragma unroll 4
+  for (int r = threadIdx.x; r < rows; r += RH_THREADS) {
     a += dapart[(size_t)r * H + h];
     d += ddpart[(size_t)r * H + h];
+    if (dbpart) e += dbpart[(size_t)r * H + h];
   }
-  __shared__ float r1[NT / 32], r2[NT / 32];
+  __shared__ float red[3][RH_THREADS / 32];
 #pragma unroll
   for (int o = 16; o; o >>= 1) {
     a += __shfl_xor_sync(0xffffffffu, a, o);
     d += __shfl_xor_sync(0xffffffffu, d, o);
+    e += __shfl_xor_sync(0xffffffffu, e, o);
   }
-  if ((threadIdx.x & 31) == 0) { r1[threadIdx.x >> 5] = a; r2[threadIdx.x >> 5] = d; }
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if (lane == 0) { red[0][w] = a; red[1][w] = d; red[2][w] = e; }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    float ta = 0.f, td = 0.f;
-    for (int i = 0; i < NT / 32; ++i) { ta += r1[i]; td += r2[i]; }
-    dA[h] = ta;
-    if (dD) dD[h] = td;
+  if (w < 3) {
+    float t = red[w][lane];
+#pragma unroll
+    for (int o = 16; o; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    float* out = w == 0 ? dA : w == 1 ? dD : dbias;
+    if (lane == 0 && out) out[h] = t;
   }
 }
 
@@ -737,13 +756,15 @@ __global__ void __launch_bounds__(NT) k_reduce_heads(int rows, int H, const floa
 // =============================================================================================
 template <typename T>
 static int fwd_stages_t(const Geo& g, bool tc, const SsdFwdPtrs& p, char* ws, const WsLayout& w, cudaStream_t s,
-                        int stages, bool need_cb) {
+                        int stages, bool keep_fin) {
   int* status = (int*)(ws + w.status);
   float* cs = (float*)(ws + w.cs);
   float* dtf = (float*)(ws + w.dtf);
   float* states = (float*)(ws + w.states);
   float* cb = (float*)(ws + w.cb);
-  float* fin = p.final_state ? p.final_state : (float*)(ws + w.fin);
+  // the final state: the workspace's copy is the backward's, the other the caller's; both are written where it is formed
+  float* fin = keep_fin ? (float*)(ws + w.fin) : p.final_state;
+  float* fin2 = keep_fin ? p.final_state : nullptr;
   float* tab = (float*)(ws + w.tab);
   void* prev_bf = ws + w.prev_bf;
   const T* x = (const T*)p.x;
@@ -751,12 +772,12 @@ static int fwd_stages_t(const Geo& g, bool tc, const SsdFwdPtrs& p, char* ws, co
   // a full pass (no sequence-parallel staging) computes the chunk states inside the scan over chunks where that kernel applies
   const bool fused = tc && stages == (SSD_STAGE_LOCAL | SSD_STAGE_FINISH) && tensor_state_fused_applies(g);
   if (stages & (SSD_STAGE_LOCAL | SSD_STAGE_LOCAL_STATES)) {
-    cudaMemsetAsync(status, 0, 256, s);
     int* hmax = tc ? (int*)(ws + w.hmax) : nullptr;
     static std::atomic<int> launch_tag{1};
     int tag = launch_tag.fetch_add(1, std::memory_order_relaxed);
     if (tag == 0) tag = launch_tag.fetch_add(1, std::memory_order_relaxed);
-    k_cumsum<T><<<dim3(g.nc, g.B), g.Q <= 128 ? 128 : NT, 0, s>>>(g, (const T*)p.dt, p.dt_bias, p.A, cs, dtf, tc ? tab : nullptr, hmax, tag);
+    launch<k_cumsum<T>>(dim3(g.nc, g.B), g.Q <= 128 ? 128 : NT, 0, s, g, (const T*)p.dt, p.dt_bias, p.A, cs, dtf, tc ? tab : nullptr,
+                        hmax, tag, status);
     SSD_CUDA_CHECK_LAUNCH("cumsum");
     if (tc && fused) {
       // chunk states and the scan over chunks run as one kernel in the FINISH stage
@@ -765,17 +786,16 @@ static int fwd_stages_t(const Geo& g, bool tc, const SsdFwdPtrs& p, char* ws, co
       if (rc) return rc;
     } else {
       DySrc<T> none{nullptr, nullptr, 0, 0};
-      k_chunk_state<T, 0><<<dim3(tp * tn, g.nc * g.H, g.B), NT, 0, s>>>(g, x, g.xsb, g.xsl, none, (const T*)p.Bm,
-                                                                         g.bsb, g.bsl, cs, dtf, states);
+      launch<k_chunk_state<T, 0>>(dim3(tp * tn, g.nc * g.H, g.B), NT, 0, s, g, x, g.xsb, g.xsl, none, (const T*)p.Bm, g.bsb, g.bsl, cs, dtf, states);
       SSD_CUDA_CHECK_LAUNCH("chunk_state");
     }
   }
   if (stages & SSD_STAGE_TOTAL) {
     if (tc) {
-      int rc = tensor_state_passing(g, states, cs, nullptr, fin, nullptr, 0, false, nullptr, nullptr, nullptr, nullptr, nullptr, s);
+      int rc = tensor_state_passing(g, states, cs, nullptr, fin, fin2, nullptr, 0, false, nullptr, nullptr, nullptr, nullptr, nullptr, s);
       if (rc) return rc;
     } else {
-      k_state_passing<false><<<dim3(cdiv(g.P * g.N, NT), g.H, g.B), NT, 0, s>>>(g, states, cs, nullptr, fin, 0);
+      launch<k_state_passing<false>>(dim3(cdiv(g.P * g.N, NT), g.H, g.B), NT, 0, s, g, states, cs, nullptr, fin, fin2, 0);
       SSD_CUDA_CHECK_LAUNCH("state_total");
     }
   }
@@ -783,26 +803,25 @@ static int fwd_stages_t(const Geo& g, bool tc, const SsdFwdPtrs& p, char* ws, co
     if (tc && fused) {
       // no fp32 copy of the chunk-entry states: every reader in this family takes the bf16 one
       int rc = tensor_state_fused(g, 0, p.x, g.xsb, g.xsl, p.Bm, g.bsb, g.bsl, tab, nullptr, prev_bf,
-                                  p.init_state, fin, nullptr, nullptr, nullptr, nullptr, status, s);
+                                  p.init_state, fin, fin2, nullptr, nullptr, nullptr, nullptr, status, s);
       if (rc) return rc;
     } else if (tc) {
-      int rc = tensor_state_passing(g, states, cs, p.init_state, fin, prev_bf, 0, true, nullptr, nullptr, nullptr, nullptr, nullptr, s);
+      int rc = tensor_state_passing(g, states, cs, p.init_state, fin, fin2, prev_bf, 0, true, nullptr, nullptr, nullptr, nullptr, nullptr, s);
       if (rc) return rc;
     } else {
-      k_state_passing<true><<<dim3(cdiv(g.P * g.N, NT), g.H, g.B), NT, 0, s>>>(g, states, cs, p.init_state, fin, 0);
+      launch<k_state_passing<true>>(dim3(cdiv(g.P * g.N, NT), g.H, g.B), NT, 0, s, g, states, cs, p.init_state, fin, fin2, 0);
       SSD_CUDA_CHECK_LAUNCH("state_passing");
     }
     if (!tc) {
-      k_cb<T><<<dim3(tq * tq, g.nc * g.G, g.B), NT, 0, s>>>(g, (const T*)p.Bm, (const T*)p.Cm, cb);
+      launch<k_cb<T>>(dim3(tq * tq, g.nc * g.G, g.B), NT, 0, s, g, (const T*)p.Bm, (const T*)p.Cm, cb);
       SSD_CUDA_CHECK_LAUNCH("cb");
     }
     if (p.y && tc) {
       int rc = tensor_chunk_scan(g, p, tab, prev_bf, status, s);
       if (rc) return rc;
     } else if (p.y) {
-      k_chunk_scan<T, 0><<<dim3(tq * tp, g.nc * g.H, g.B), NT, 0, s>>>(
-          g, x, (const T*)p.Cm, p.D, (const T*)p.z, cs, dtf, cb, states, (T*)p.y, nullptr, nullptr, nullptr,
-          nullptr, nullptr);
+      launch<k_chunk_scan<T, 0>>(dim3(tq * tp, g.nc * g.H, g.B), NT, 0, s, g, x, (const T*)p.Cm, p.D, (const T*)p.z, cs, dtf, cb, states,
+                                 (T*)p.y, nullptr, nullptr, nullptr, nullptr, nullptr);
       SSD_CUDA_CHECK_LAUNCH("chunk_scan");
     }
   }
@@ -810,9 +829,9 @@ static int fwd_stages_t(const Geo& g, bool tc, const SsdFwdPtrs& p, char* ws, co
 }
 
 int run_forward(const Geo& g, int dtype, bool tc, const SsdFwdPtrs& p, char* ws, const WsLayout& w, cudaStream_t s,
-                int stages) {
-  return dtype == SSD_BF16 ? fwd_stages_t<__nv_bfloat16>(g, tc, p, ws, w, s, stages, false)
-                           : fwd_stages_t<float>(g, false, p, ws, w, s, stages, false);
+                int stages, bool for_backward) {
+  return dtype == SSD_BF16 ? fwd_stages_t<__nv_bfloat16>(g, tc, p, ws, w, s, stages, for_backward)
+                           : fwd_stages_t<float>(g, false, p, ws, w, s, stages, for_backward);
 }
 
 template <typename T>
@@ -853,8 +872,8 @@ static int bwd_stages_t(const Geo& g, bool tc, const SsdBwdPtrs& p, char* ws, co
     if (!p.fwd_saved) {
       SsdFwdPtrs f{};
       f.x = p.x; f.dt = p.dt; f.A = p.A; f.Bm = p.Bm; f.Cm = p.Cm; f.D = p.D; f.z = p.z; f.dt_bias = p.dt_bias;
-      f.init_state = p.init_state; f.y = nullptr; f.final_state = fin;
-      int rc = fwd_stages_t<T>(g, tc, f, ws, w, s, SSD_STAGE_LOCAL | SSD_STAGE_FINISH, false);
+      f.init_state = p.init_state; f.y = nullptr; f.final_state = nullptr;
+      int rc = fwd_stages_t<T>(g, tc, f, ws, w, s, SSD_STAGE_LOCAL | SSD_STAGE_FINISH, true);
       if (rc) return rc;
     }
     if (!tc) {  // the CUDA-core kernels accumulate these row sums with atomics; the tensor-core ones store them
@@ -871,9 +890,8 @@ static int bwd_stages_t(const Geo& g, bool tc, const SsdBwdPtrs& p, char* ws, co
       if (rc) return rc;
     } else {
       // forward recompute with the backward epilogue: dz, pre-gate dy, dcsp, ddot
-      k_chunk_scan<T, 1><<<dim3(tq * tp, g.nc * g.H, g.B), NT, 0, s>>>(
-          g, x, (const T*)p.Cm, p.D, (const T*)p.z, cs, dtf, cb, states, nullptr, (const T*)p.dy, dyp, (T*)p.dz,
-          dcsp, ddot);
+      launch<k_chunk_scan<T, 1>>(dim3(tq * tp, g.nc * g.H, g.B), NT, 0, s, g, x, (const T*)p.Cm, p.D, (const T*)p.z, cs, dtf, cb, states,
+                                 nullptr, (const T*)p.dy, dyp, (T*)p.dz, dcsp, ddot);
       SSD_CUDA_CHECK_LAUNCH("chunk_scan_bwd_epilogue");
     }
   }
@@ -885,17 +903,16 @@ static int bwd_stages_t(const Geo& g, bool tc, const SsdBwdPtrs& p, char* ws, co
         if (rc) return rc;
       }
     } else {
-      k_chunk_state<T, 1><<<dim3(tp * tn, g.nc * g.H, g.B), NT, 0, s>>>(g, x, g.xsb, g.xsl, dys, (const T*)p.Cm,
-                                                                         g.csb, g.csl, cs, dtf, dst);
+      launch<k_chunk_state<T, 1>>(dim3(tp * tn, g.nc * g.H, g.B), NT, 0, s, g, x, g.xsb, g.xsl, dys, (const T*)p.Cm, g.csb, g.csl, cs, dtf, dst);
       SSD_CUDA_CHECK_LAUNCH("dstates_local");
     }
   }
   if (stages & SSD_STAGE_TOTAL) {
     if (tc) {
-      int rc = tensor_state_passing(g, dst, cs, nullptr, dini, nullptr, 1, false, nullptr, nullptr, nullptr, nullptr, nullptr, s);
+      int rc = tensor_state_passing(g, dst, cs, nullptr, dini, nullptr, nullptr, 1, false, nullptr, nullptr, nullptr, nullptr, nullptr, s);
       if (rc) return rc;
     } else {
-      k_state_passing<false><<<dim3(cdiv(g.P * g.N, NT), g.H, g.B), NT, 0, s>>>(g, dst, cs, nullptr, dini, 1);
+      launch<k_state_passing<false>>(dim3(cdiv(g.P * g.N, NT), g.H, g.B), NT, 0, s, g, dst, cs, nullptr, dini, nullptr, 1);
       SSD_CUDA_CHECK_LAUNCH("dstate_total");
     }
   }
@@ -905,16 +922,16 @@ static int bwd_stages_t(const Geo& g, bool tc, const SsdBwdPtrs& p, char* ws, co
       // local state gradients, the reverse scan and the <dS_end, S_end> partial sums in one kernel (no fp32 copy is kept)
       int rc = tensor_state_fused(g, 1, tc_dy, tc_dense ? (long long)g.L * g.H * g.P : g.ysb,
                                   tc_dense ? (long long)g.H * g.P : g.ysl, p.Cm, g.csb, g.csl, tab, nullptr, ds_bf,
-                                  p.dfinal_state, dini, prev_bf, fin, sdot, &sdot_nw, status, s);
+                                  p.dfinal_state, dini, nullptr, prev_bf, fin, sdot, &sdot_nw, status, s);
       if (rc) return rc;
     } else if (tc) {
       // the reverse scan also leaves the warp-partial sums of <dS_end, S_end> per chunk
-      int rc = tensor_state_passing(g, dst, cs, p.dfinal_state, dini, ds_bf, 1, true, states, prev_bf, fin, sdot, &sdot_nw, s);
+      int rc = tensor_state_passing(g, dst, cs, p.dfinal_state, dini, nullptr, ds_bf, 1, true, states, prev_bf, fin, sdot, &sdot_nw, s);
       if (rc) return rc;
     } else {
-      k_state_passing<true><<<dim3(cdiv(g.P * g.N, NT), g.H, g.B), NT, 0, s>>>(g, dst, cs, p.dfinal_state, dini, 1);
+      launch<k_state_passing<true>>(dim3(cdiv(g.P * g.N, NT), g.H, g.B), NT, 0, s, g, dst, cs, p.dfinal_state, dini, nullptr, 1);
       SSD_CUDA_CHECK_LAUNCH("dstate_passing");
-      k_sdot<<<dim3(g.nc, g.H, g.B), NT, 0, s>>>(g, dst, states, fin, sdot);
+      launch<k_sdot>(dim3(g.nc, g.H, g.B), NT, 0, s, g, dst, states, fin, sdot);
       SSD_CUDA_CHECK_LAUNCH("sdot");
     }
     if (tc) {
@@ -924,26 +941,20 @@ static int bwd_stages_t(const Geo& g, bool tc, const SsdBwdPtrs& p, char* ws, co
       rc = tensor_dbc(g, p, tc_dy, tc_dense, tab, (const float*)(ws + w.hmax), prev_bf, ds_bf, status, s);
       if (rc) return rc;
     } else {
-      k_dx<T><<<dim3(tq * tp, g.nc * g.H, g.B), NT, 0, s>>>(g, x, (const T*)p.Bm, p.D, dys, cs, dtf, cb, dst,
-                                                             (T*)p.dx, ddtd);
+      launch<k_dx<T>>(dim3(tq * tp, g.nc * g.H, g.B), NT, 0, s, g, x, (const T*)p.Bm, p.D, dys, cs, dtf, cb, dst, (T*)p.dx, ddtd);
       SSD_CUDA_CHECK_LAUNCH("dx");
-      k_dw<T><<<dim3(tq * tq, g.nc * g.G, g.B), NT, 0, s>>>(g, x, dys, cs, dtf, wsum);
+      launch<k_dw<T>>(dim3(tq * tq, g.nc * g.G, g.B), NT, 0, s, g, x, dys, cs, dtf, wsum);
       SSD_CUDA_CHECK_LAUNCH("dw");
-      k_dbc<T, 0><<<dim3(tq * tn, g.nc * g.G, g.B), NT, 0, s>>>(g, x, (const T*)p.Bm, g.bsb, g.bsl, dys, cs, dtf,
-                                                                 wsum, states, (T*)p.dC);
+      launch<k_dbc<T, 0>>(dim3(tq * tn, g.nc * g.G, g.B), NT, 0, s, g, x, (const T*)p.Bm, g.bsb, g.bsl, dys, cs, dtf, wsum, states, (T*)p.dC);
       SSD_CUDA_CHECK_LAUNCH("dC");
-      k_dbc<T, 1><<<dim3(tq * tn, g.nc * g.G, g.B), NT, 0, s>>>(g, x, (const T*)p.Cm, g.csb, g.csl, dys, cs, dtf,
-                                                                 wsum, dst, (T*)p.dB);
+      launch<k_dbc<T, 1>>(dim3(tq * tn, g.nc * g.G, g.B), NT, 0, s, g, x, (const T*)p.Cm, g.csb, g.csl, dys, cs, dtf, wsum, dst, (T*)p.dB);
       SSD_CUDA_CHECK_LAUNCH("dB");
     }
-    k_ddt<<<dim3(g.nc, g.B), g.Q <= 128 ? 128 : NT, 0, s>>>(g, p.A, dtf, dcsp, ddtd, ddot, sdot, sdot_nw, p.ddt, dapart, ddpart);
+    float* dbpart = p.ddt_bias ? (float*)(ws + w.dbpart) : nullptr;
+    launch<k_ddt>(dim3(g.nc, g.B), g.Q <= 128 ? 128 : NT, 0, s, g, p.A, dtf, dcsp, ddtd, ddot, sdot, sdot_nw, p.ddt, dapart, ddpart, dbpart);
     SSD_CUDA_CHECK_LAUNCH("ddt");
-    k_reduce_heads<<<g.H, NT, 0, s>>>(g.B * g.nc, g.H, dapart, ddpart, p.dA, p.dD);
+    launch<k_reduce_heads>(g.H, RH_THREADS, 0, s, g.B * g.nc, g.H, dapart, ddpart, dbpart, p.dA, p.dD, p.ddt_bias);
     SSD_CUDA_CHECK_LAUNCH("reduce_heads");
-    if (p.ddt_bias) {
-      k_sum_ddt<<<g.H, NT, 0, s>>>((long long)g.B * g.L, g.H, p.ddt, p.ddt_bias);
-      SSD_CUDA_CHECK_LAUNCH("sum_ddt");
-    }
   }
   return SSD_OK;
 }

@@ -533,9 +533,6 @@ __global__ void __launch_bounds__(PsCfg<P, N_>::THREADS, 1) k_state_ps(Geo g, co
   __shared__ int s_abort;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (tid == 0) s_abort = *(volatile int*)status;
-  __syncthreads();
-  if (s_abort) return;
   if (tid == 0) {
     for (int i = 0; i < NX; ++i) { mbar_init(&x_full[i], 1); mbar_init(&x_free[i], 1); }
     for (int i = 0; i < 2; ++i) {
@@ -546,10 +543,16 @@ __global__ void __launch_bounds__(PsCfg<P, N_>::THREADS, 1) k_state_ps(Geo g, co
     mbar_fence_init();
   }
   if (warp == 1) tmem_alloc(&tmem_slot, 2 * N);
+  pdl_wait();
+  if (tid == 0) s_abort = *(volatile int*)status;   // an earlier kernel gave up
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tm = tmem_slot;
+  if (s_abort) {
+    if (warp == 1) tmem_dealloc(tm, 2 * N);
+    return;
+  }
   Waiter w{status, false};
 
   const int MT = g.hpg * P / 128;
@@ -728,7 +731,7 @@ struct StateScanArgs {
   float* st;            // [B,nc,H,P,N] fp32 out, optional
   void* st_bf;          // [B,nc,H,P,N] bf16 out
   const float* init;    // [B,H,P,N] fp32, optional
-  float* last;          // [B,H,P,N] fp32 out, optional
+  float *last, *last2;  // [B,H,P,N] fp32 out, both optional
   const void* fwd_prev_bf;  // MODE 1: bf16 copy of the forward pass's chunk-entry states (read through a tensor map)
   const float* fwd_fin;   // MODE 1: forward final state
   float* sdot;            // MODE 1: [B,nc,H,SDOT_NW]
@@ -755,9 +758,6 @@ __global__ void __launch_bounds__(PfCfg<P, MODE>::THREADS, 1) k_state_scan_ps(Ge
   __shared__ int s_abort;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (tid == 0) s_abort = *(volatile int*)status;
-  __syncthreads();
-  if (s_abort) return;
   if (tid == 0) {
     for (int i = 0; i < NX; ++i) { mbar_init(&x_full[i], 1); mbar_init(&x_free[i], 1); }
     for (int i = 0; i < NB; ++i) { mbar_init(&b_full[i], 1); mbar_init(&b_free[i], 1); }
@@ -767,10 +767,16 @@ __global__ void __launch_bounds__(PfCfg<P, MODE>::THREADS, 1) k_state_scan_ps(Ge
     mbar_fence_init();
   }
   if (warp == 1) tmem_alloc(&tmem_slot, 128);
+  pdl_wait();
+  if (tid == 0) s_abort = *(volatile int*)status;   // an earlier kernel gave up
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tm = tmem_slot;
+  if (s_abort) {
+    if (warp == 1) tmem_dealloc(tm, 128);
+    return;
+  }
   Waiter w{status, false};
   const bool want_sdot = MODE == 1 && a.sdot != nullptr;
 
@@ -960,11 +966,15 @@ __global__ void __launch_bounds__(PfCfg<P, MODE>::THREADS, 1) k_state_scan_ps(Ge
       }
 #pragma unroll
       for (int j = 0; j < 16; ++j) run[j] = fmaf(dec, run[j], v[j]);
-      if (t.s == g.nc - 1 && a.last) {
+      if (t.s == g.nc - 1) {
+        auto put = [&](float* to) {
 #pragma unroll
-        for (int j = 0; j < 16; j += 8)
-          st_global_32B(a.last + bstate + e + j, make_uint4(__float_as_uint(run[j]), __float_as_uint(run[j + 1]), __float_as_uint(run[j + 2]), __float_as_uint(run[j + 3])),
-                        make_uint4(__float_as_uint(run[j + 4]), __float_as_uint(run[j + 5]), __float_as_uint(run[j + 6]), __float_as_uint(run[j + 7])));
+          for (int j = 0; j < 16; j += 8)
+            st_global_32B(to + bstate + e + j, make_uint4(__float_as_uint(run[j]), __float_as_uint(run[j + 1]), __float_as_uint(run[j + 2]), __float_as_uint(run[j + 3])),
+                          make_uint4(__float_as_uint(run[j + 4]), __float_as_uint(run[j + 5]), __float_as_uint(run[j + 6]), __float_as_uint(run[j + 7])));
+        };
+        if (a.last) put(a.last);
+        if (a.last2) put(a.last2);
       }
     };
     Tile cur{0, 0, 0, 0}, prev{0, 0, 0, 0};
@@ -1501,6 +1511,7 @@ k_dbc_tc(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant__
   __shared__ int s_abort;
 
   const int tid = threadIdx.x, warp = tid >> 5;
+  pdl_wait();
   if (tid == 0) s_abort = *(volatile int*)status;
   __syncthreads();
   if (s_abort) return;
@@ -1828,9 +1839,6 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
   __shared__ int s_abort;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (tid == 0) s_abort = *(volatile int*)status;
-  __syncthreads();
-  if (s_abort) return;
   if (tid == 0) {
     for (int i = 0; i < 2; ++i) {
       mbar_init(&bars.cb_full[i], 1); mbar_init(&bars.cb_empty[i], Cfg::NI);
@@ -1853,10 +1861,16 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
     for (int i = 0; i < NM; ++i) zero_upper_blocks(tid & 127, tid >> 7, warp, smem_u32(sM + i * 2 * BOX_BYTES));
     fence_async_smem();
   }
+  pdl_wait();
+  if (tid == 0) s_abort = *(volatile int*)status;   // an earlier kernel gave up
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tm = tmem_slot;
+  if (s_abort) {
+    if (warp == Cfg::W_MMA) tmem_dealloc(tm, 512);
+    return;
+  }
   Waiter w{status, false};
 
   const int nblk = g.hpg / HB;
@@ -2263,9 +2277,6 @@ k_bwd_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant__
   __shared__ int s_abort;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (tid == 0) s_abort = *(volatile int*)status;
-  __syncthreads();
-  if (s_abort) return;
   if (tid == 0) {
     for (int i = 0; i < 2; ++i) {
       mbar_init(&bars.cb_full[i], 1); mbar_init(&bars.cb_empty[i], SPLIT ? 2 : 1);
@@ -2285,10 +2296,16 @@ k_bwd_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant__
     for (int i = 0; i < NM; ++i) zero_upper_blocks(tid & 127, tid >> 7, warp, smem_u32(sM + i * 2 * BOX_BYTES));
     fence_async_smem();
   }
+  pdl_wait();
+  if (tid == 0) s_abort = *(volatile int*)status;   // an earlier kernel gave up
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tm = tmem_slot;
+  if (s_abort) {
+    if (warp == 17) tmem_dealloc(tm, 512);
+    return;
+  }
   const uint32_t tmYd = tm + 256, tmYo = tm + 320, tmUd = tm + 384, tmUo = tm + 448;
   Waiter w{status, false};
 
@@ -2653,9 +2670,6 @@ k_dbc_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant__
   __shared__ int s_abort;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (tid == 0) s_abort = *(volatile int*)status;
-  __syncthreads();
-  if (s_abort) return;
   if (tid == 0) {
     // two MMA issuer lanes (dC side, dB side): tcgen05.commit tracks the MMAs of its own thread only, so every barrier that
     // releases something both of them read expects one commit from each
@@ -2678,10 +2692,16 @@ k_dbc_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant__
     zero_upper_blocks(tid & 127, tid >> 7, warp, smem_u32(sM));
     fence_async_smem();
   }
+  pdl_wait();
+  if (tid == 0) s_abort = *(volatile int*)status;   // an earlier kernel gave up
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tm = tmem_slot;
+  if (s_abort) {
+    if (warp == 17) tmem_dealloc(tm, 512);
+    return;
+  }
   const uint32_t tmDC = tm + 256, tmDB = tm + 320, tmWsep = tm + 384;
   Waiter w{status, false};
   // which heads take the separable path: one bit per head, the same in every role (up to 64 heads; beyond that none)
@@ -3007,11 +3027,12 @@ k_dbc_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant__
 template <bool WRITE, bool BFDOT = false>
 __global__ void __launch_bounds__(256, BFDOT ? 3 : 1) k_state_passing_v4(Geo g, float* __restrict__ st, const float* __restrict__ cs,
                                                           const float* __restrict__ init, float* __restrict__ last,
-                                                          bf16* __restrict__ st_bf, int reverse,
+                                                          float* __restrict__ last2, bf16* __restrict__ st_bf, int reverse,
                                                           const float* __restrict__ fwd_prev,
                                                           const bf16* __restrict__ fwd_prev_bf,
                                                           const float* __restrict__ fwd_fin, float* __restrict__ sdot) {
   extern __shared__ float sdec[];  // [nc]
+  pdl_wait();
   // fp32 chunk-entry states have no reader in this family: the reverse scans form <dS_end, S_end> from the bf16 copy (here
   // given as `fwd_prev_bf`), so a scan that writes the copy leaves the fp32 values unwritten: 2 of its 5 bytes per element
   const int h = blockIdx.y, b = blockIdx.z;
@@ -3094,6 +3115,7 @@ __global__ void __launch_bounds__(256, BFDOT ? 3 : 1) k_state_passing_v4(Geo g, 
     }
   }
   if (last && valid) *reinterpret_cast<float4*>(last + ((size_t)(b * g.H + h)) * PN + eo) = run;
+  if (last2 && valid) *reinterpret_cast<float4*>(last2 + ((size_t)(b * g.H + h)) * PN + eo) = run;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -3166,18 +3188,13 @@ constexpr size_t dbc_smem() {
   return 1024 + 2 * (N / 64) * BOX_BYTES + 2 * BOX_BYTES + (N > 64 ? 2 : 1) * (2 * BOX_BYTES + (64 / P) * TAB_BYTES);
 }
 
-int sm_count();
-
 template <int P, int N, int MODE>
 int launch_state(const Geo& g, const CUtensorMap& tx, const CUtensorMap& tb, const float* tab, float* out, int* status,
                  cudaStream_t s) {
   if (!g.onetile) {   // persistent, ring-fed version
-    auto kp = k_state_ps<P, N, MODE>;
-    constexpr size_t sm = PsCfg<P, N>::SMEM;
-    cudaFuncSetAttribute(kp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     const int nitems = g.B * g.G * g.nc;
     const int grid = nitems < sm_count() ? nitems : sm_count();
-    kp<<<grid, PsCfg<P, N>::THREADS, sm, s>>>(g, tx, tb, tab, out, status);
+    launch<k_state_ps<P, N, MODE>>(grid, PsCfg<P, N>::THREADS, PsCfg<P, N>::SMEM, s, g, tx, tb, tab, out, status);
     SSD_CUDA_CHECK_LAUNCH(MODE == 0 ? "chunk_state_ps" : "dstates_local_ps");
     return SSD_OK;
   }
@@ -3200,27 +3217,16 @@ struct SeqMaps {
   CUtensorMap z;       // the gate (forward of the persistent scan kernel)
 };
 
-int sm_count() {
-  static int n[64] = {0};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64) return 132;
-  if (!n[dev]) cudaDeviceGetAttribute(&n[dev], cudaDevAttrMultiProcessorCount, dev);
-  return n[dev] > 0 ? n[dev] : 132;
-}
-
 template <int P, int MODE, int N, bool GATED = false>
 int launch_scan_ws(const Geo& g, const SeqMaps& m, const CUtensorMap& ts, const ScanArgs& a, int* status, cudaStream_t s) {
   if constexpr (!GATED && MODE != 2) {
     if (a.z) return launch_scan_ws<P, MODE, N, true>(g, m, ts, a, status, s);
   }
-  auto k = k_scan_ws<P, MODE, N, GATED>;
-  constexpr size_t sm = WsCfg<P, MODE, N, GATED>::SMEM;
-  cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  using Cfg = WsCfg<P, MODE, N, GATED>;
   const int ntiles = g.B * g.G * g.nc;
   const int grid = ntiles < sm_count() ? ntiles : sm_count();
-  k<<<grid, WsCfg<P, MODE, N, GATED>::THREADS, sm, s>>>(g, m.x, m.dy, m.b, m.c, ts, m.out, m.z, a.tab, a.D, (const bf16*)a.z, (bf16*)a.y, (bf16*)a.dypb,
-                                 (bf16*)a.dz, (bf16*)a.dx, a.rs0, a.rs1, status);
+  launch<k_scan_ws<P, MODE, N, GATED>>(grid, Cfg::THREADS, Cfg::SMEM, s, g, m.x, m.dy, m.b, m.c, ts, m.out, m.z, a.tab, a.D,
+                                       (const bf16*)a.z, (bf16*)a.y, (bf16*)a.dypb, (bf16*)a.dz, (bf16*)a.dx, a.rs0, a.rs1, status);
   SSD_CUDA_CHECK_LAUNCH(MODE == 0 ? "chunk_scan_ws" : (MODE == 1 ? "chunk_scan_bwd_ws" : "dx_ws"));
   return SSD_OK;
 }
@@ -3241,12 +3247,10 @@ int launch_scan(const Geo& g, const SeqMaps& m, const CUtensorMap& ts, const Sca
 template <int P, int N = 64>
 int launch_bwd_ws(const Geo& g, const SeqMaps& m, const float* tab, const float* D, void* dx, float* dcsp, float* ddot,
                   float* ddtd, int* status, cudaStream_t s) {
-  auto k = k_bwd_ws<P, N>;
-  constexpr size_t sm = BwCfg<P, N>::SMEM;
-  cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   const int ntiles = g.B * g.G * g.nc;
   const int grid = ntiles < sm_count() ? ntiles : sm_count();
-  k<<<grid, WS_THREADS, sm, s>>>(g, m.x, m.dy, m.b, m.c, m.s, m.ds, tab, D, (bf16*)dx, dcsp, ddot, ddtd, status);
+  launch<k_bwd_ws<P, N>>(grid, WS_THREADS, BwCfg<P, N>::SMEM, s, g, m.x, m.dy, m.b, m.c, m.s, m.ds, tab, D, (bf16*)dx, dcsp, ddot, ddtd,
+                         status);
   SSD_CUDA_CHECK_LAUNCH("scan_bwd_dx_ws");
   return SSD_OK;
 }
@@ -3269,12 +3273,9 @@ int launch_bwd_tc(const Geo& g, const SeqMaps& m, const float* tab, const float*
 
 template <int P>
 int launch_dbc_ws(const Geo& g, const SeqMaps& m, const float* tab, const float* hmax, void* dB, void* dC, int* status, cudaStream_t s) {
-  auto k = k_dbc_ws<P>;
-  constexpr size_t sm = DbCfg<P>::SMEM;
-  cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   const int ntiles = g.B * g.G * g.nc;
   const int grid = ntiles < sm_count() ? ntiles : sm_count();
-  k<<<grid, WS_THREADS, sm, s>>>(g, m.x, m.dy, m.b, m.c, m.s, m.ds, tab, hmax, (bf16*)dB, (bf16*)dC, status);
+  launch<k_dbc_ws<P>>(grid, WS_THREADS, DbCfg<P>::SMEM, s, g, m.x, m.dy, m.b, m.c, m.s, m.ds, tab, hmax, (bf16*)dB, (bf16*)dC, status);
   SSD_CUDA_CHECK_LAUNCH("dBdC_ws");
   return SSD_OK;
 }
@@ -3282,10 +3283,8 @@ int launch_dbc_ws(const Geo& g, const SeqMaps& m, const float* tab, const float*
 template <int P, int N>
 int launch_dbc(const Geo& g, const SeqMaps& m, const float* tab, const float* hmax, void* dB, void* dC, int* status, cudaStream_t s) {
   if (N == 64 && !g.onetile) return launch_dbc_ws<P>(g, m, tab, hmax, dB, dC, status, s);
-  auto k = k_dbc_tc<P, N>;
-  cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dbc_smem<P, N>());
-  k<<<dim3(g.nc, g.G, g.B), TC_THREADS, dbc_smem<P, N>(), s>>>(g, m.x, m.dy, m.b, m.c, m.s, m.ds, tab, (bf16*)dB, (bf16*)dC,
-                                                               status);
+  launch<k_dbc_tc<P, N>>(dim3(g.nc, g.G, g.B), TC_THREADS, dbc_smem<P, N>(), s, g, m.x, m.dy, m.b, m.c, m.s, m.ds, tab, (bf16*)dB,
+                         (bf16*)dC, status);
   SSD_CUDA_CHECK_LAUNCH("dBdC_tc");
   return SSD_OK;
 }
@@ -3339,7 +3338,7 @@ bool tensor_supported(const Geo& g, int dtype, const char** why) {
   return true;
 }
 
-int tensor_state_passing(const Geo& g, float* st, const float* cs, const float* init, float* last, void* st_bf,
+int tensor_state_passing(const Geo& g, float* st, const float* cs, const float* init, float* last, float* last2, void* st_bf,
                          int reverse, bool write, const float* fwd_prev, const void* fwd_prev_bf, const float* fwd_fin,
                          float* sdot, int* sdot_nw, cudaStream_t s) {
   const int PN = g.P * g.N;
@@ -3349,9 +3348,12 @@ int tensor_state_passing(const Geo& g, float* st, const float* cs, const float* 
   // the bf16 copy stands in for the fp32 chunk-entry states wherever the forward scan no longer writes those
   const bf16* prev_bf = (const bf16*)fwd_prev_bf;
   if (write && prev_bf && sdot)
-    k_state_passing_v4<true, true><<<grid, 256, sm, s>>>(g, st, cs, init, last, (bf16*)st_bf, reverse, nullptr, prev_bf, fwd_fin, sdot);
-  else if (write) k_state_passing_v4<true><<<grid, 256, sm, s>>>(g, st, cs, init, last, (bf16*)st_bf, reverse, fwd_prev, nullptr, fwd_fin, sdot);
-  else k_state_passing_v4<false><<<grid, 256, sm, s>>>(g, st, cs, init, last, nullptr, reverse, nullptr, nullptr, nullptr, nullptr);
+    launch<k_state_passing_v4<true, true>>(grid, 256, sm, s, g, st, cs, init, last, last2, (bf16*)st_bf, reverse, nullptr, prev_bf, fwd_fin,
+                                           sdot);
+  else if (write)
+    launch<k_state_passing_v4<true>>(grid, 256, sm, s, g, st, cs, init, last, last2, (bf16*)st_bf, reverse, fwd_prev, nullptr, fwd_fin, sdot);
+  else
+    launch<k_state_passing_v4<false>>(grid, 256, sm, s, g, st, cs, init, last, last2, nullptr, reverse, nullptr, nullptr, nullptr, nullptr);
   SSD_CUDA_CHECK_LAUNCH(reverse ? (write ? "dstate_passing" : "dstate_total") : (write ? "state_passing" : "state_total"));
   return SSD_OK;
 }
@@ -3382,25 +3384,22 @@ bool tensor_state_fused_applies(const Geo& g) { return g.N == 64 && !g.onetile; 
 template <int P, int MODE>
 static int launch_state_scan(const Geo& g, const CUtensorMap& tx, const CUtensorMap& tb, const CUtensorMap& ts, const CUtensorMap& tf,
                              const StateScanArgs& a, int* status, cudaStream_t s) {
-  auto k = k_state_scan_ps<P, MODE>;
-  constexpr size_t sm = PfCfg<P, MODE>::SMEM;
-  cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   const int nunits = g.B * g.G * (g.hpg * P / 128);
   const int grid = nunits < sm_count() ? nunits : sm_count();
-  k<<<grid, PfCfg<P, MODE>::THREADS, sm, s>>>(g, tx, tb, ts, tf, a, status);
+  launch<k_state_scan_ps<P, MODE>>(grid, PfCfg<P, MODE>::THREADS, PfCfg<P, MODE>::SMEM, s, g, tx, tb, ts, tf, a, status);
   SSD_CUDA_CHECK_LAUNCH(MODE == 0 ? "chunk_state_scan" : "dstate_scan");
   return SSD_OK;
 }
 
 int tensor_state_fused(const Geo& g, int mode, const void* xdy, long long sb, long long sl, const void* bc, long long bsb,
-                       long long bsl, const float* tab, float* st, void* st_bf, const float* init, float* last,
+                       long long bsl, const float* tab, float* st, void* st_bf, const float* init, float* last, float* last2,
                        const void* fwd_prev_bf, const float* fwd_fin, float* sdot, int* sdot_nw, int* status, cudaStream_t s) {
   CUtensorMap tx, tb;
   int rc = make_seq_map(&tx, xdy, (long long)g.H * g.P, g.L, g.B, sl, sb, "x/dy");
   if (rc) return rc;
   rc = make_seq_map(&tb, bc, (long long)g.G * g.N, g.L, g.B, bsl, bsb, "B/C");
   if (rc) return rc;
-  StateScanArgs a{tab, st, st_bf, init, last, fwd_prev_bf, fwd_fin, sdot};
+  StateScanArgs a{tab, st, st_bf, init, last, last2, fwd_prev_bf, fwd_fin, sdot};
   if (sdot_nw) *sdot_nw = 4 * (g.P / 32);
   CUtensorMap ts = tx, tf = tx;   // placeholders unless the backward kernel reads the forward states
   if (mode == 1 && sdot) {
