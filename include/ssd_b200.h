@@ -175,6 +175,14 @@ SSD_API int32_t ssd_backward(const SsdDims* dims, const SsdBwdPtrs* p, void* wor
  * (trading_bots/src/torch/train/rollout.rs:209-235). */
 SSD_API int32_t ssd_state_update(const SsdStepDims* dims, const SsdStepPtrs* p, void* cuda_stream);
 
+/* The same timestep for a host that keeps the step's vectors itself: x, dt, B and C point to pinned host memory that the
+ * device can address, the result goes to `y_host` (pinned, y_stride_s between streams) and, if p->y is given, to that device
+ * buffer too.  One kernel, no copies: it reads every byte of a stream's vectors over PCIe while it updates the state.
+ * Segments of 16-byte pieces (per stream at most 4 KB in all), dstate 64 or 128, no gate; SSD_ERR_UNSUPPORTED otherwise and
+ * for pageable memory.  The reference copies views in and results out around its step instead
+ * (trading_bots/src/torch/train/rollout.rs:67,85-141). */
+SSD_API int32_t ssd_state_update_host(const SsdStepDims* dims, const SsdStepPtrs* p, void* y_host, void* cuda_stream);
+
 /* Zero the state rows of the streams listed in `stream_idx` (device int64 indices, `count` of
  * them) without a host sync: the per-environment reset of the reference
  * (trading_bots/src/torch/model/stream/live.rs:114-158, which avoids a sync at :155-157). */

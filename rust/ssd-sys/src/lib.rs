@@ -211,6 +211,7 @@ extern "C" {
         cuda_stream: *mut c_void,
     ) -> i32;
     pub fn ssd_state_update(dims: *const SsdStepDims, p: *const SsdStepPtrs, cuda_stream: *mut c_void) -> i32;
+    pub fn ssd_state_update_host(dims: *const SsdStepDims, p: *const SsdStepPtrs, y_host: *mut c_void, cuda_stream: *mut c_void) -> i32;
     pub fn ssd_state_reset_rows(
         state: *mut f32,
         row_elems: i64,

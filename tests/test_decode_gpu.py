@@ -117,3 +117,48 @@ def test_host_step_groups_match_oracle(lib, groups, graph):
         ys.append(hs.hy.clone())
     assert_close("y", torch.stack(ys).to(DEV), ref_y, "bf16")
     assert_close("state", state, ref_S, "bf16")
+
+
+@pytest.mark.parametrize("S,H,P,N,G,dtype", [(1, 8, 32, 64, 1, "bf16"), (33, 8, 32, 64, 1, "fp32"), (1201, 8, 32, 64, 2, "bf16"),
+                                             (5, 24, 64, 128, 1, "bf16"), (70, 8, 32, 128, 2, "bf16"), (9, 4, 64, 64, 2, "fp32"),
+                                             (3, 6, 24, 40, 3, "bf16")])
+def test_host_memory_step_matches_oracle(lib, S, H, P, N, G, dtype):
+    """The one-kernel host-memory step (and, for the last shape, the copies it leaves to): one stream, fewer and more units than
+    resident blocks, several groups, several tiles per head, rows of one and two pieces per thread."""
+    from trading_bot_0_b200.host import HostStep
+    cfg = O.SsdConfig("dec", S, 1, H, P, N, G, 1, dtype)
+    inp = O.make_decode_inputs(cfg, 3)
+    ref_y, ref_S = oracle_steps(inp, 3)
+    d = to_dev(inp, DEV)
+    state = d["state"].clone()
+    hs = HostStep(state, G, O.torch_dtype(dtype))
+    ys = []
+    for t in range(3):
+        hs.load_inputs(inp["x"][t], inp["dt"][t], inp["B"][t], inp["C"][t])
+        hs.step(d["A"], d["D"])
+        torch.cuda.synchronize()
+        ys.append(hs.hy.clone())
+        assert torch.equal(hs.y.cpu(), hs.hy)
+    assert hs._in_place == (N != 40)
+    assert_close("y", torch.stack(ys).to(DEV), ref_y, dtype)
+    assert_close("state", state, ref_S, dtype)
+
+
+@pytest.mark.parametrize("P,N,dtype", [(64, 64, "bf16"), (16, 128, "fp32"), (32, 256, "bf16"), (8, 256, "fp32"), (16, 64, "bf16"), (24, 128, "bf16")])
+@pytest.mark.parametrize("S", [1, 401])
+def test_state_tiles_of_every_width(lib, S, P, N, dtype):
+    """Heads of one, several and half tiles of the ring kernel, a single stream and more tiles than the grid has blocks, with
+    the gate and the fused step-size activation."""
+    import trading_bot_0_b200 as T
+    cfg = O.SsdConfig("dec", S, 1, 6, P, N, 2, 1, dtype)
+    inp = O.make_decode_inputs(cfg, 1)
+    g = torch.Generator().manual_seed(5)
+    z = torch.randn(S, 6, P, generator=g).to(O.torch_dtype(dtype))
+    bias = torch.full((6,), -1.0)
+    d = to_dev(inp, DEV)
+    state = d["state"].clone()
+    y = T.state_update(state, d["x"][0], d["dt"][0], d["A"], d["B"][0], d["C"][0], d["D"], z.to(DEV), dt_bias=bias.to(DEV), dt_softplus=True)
+    dt = torch.nn.functional.softplus(inp["dt"][0].double() + bias.double())
+    yr, Sr = O.state_update(inp["state"].double(), inp["x"][0], dt, inp["A"], inp["B"][0], inp["C"][0], inp["D"], z)
+    assert_close("y", y, yr, dtype)
+    assert_close("state", state, Sr, dtype)

@@ -28,7 +28,7 @@ SP_UNIQUE_ID_BYTES = 128
 
 EXPORTS = [
     "ssd_workspace_bytes", "ssd_forward", "ssd_backward", "ssd_forward_staged", "ssd_backward_staged",
-    "ssd_state_update", "ssd_state_reset_rows", "ssd_sp_total_logdecay", "ssd_sp_prefix_state",
+    "ssd_state_update", "ssd_state_update_host", "ssd_state_reset_rows", "ssd_sp_total_logdecay", "ssd_sp_prefix_state",
     "ssd_last_error", "ssd_version", "ssd_compiled_arch", "ssd_launch_count", "ssd_profile_begin",
     "ssd_profile_end", "ssd_forward_noalloc", "ssd_noalloc_max_bytes",
     "ssd_conv1d_workspace_bytes", "ssd_conv1d_forward", "ssd_conv1d_backward",
@@ -119,6 +119,8 @@ def load() -> C.CDLL:
     lib.ssd_backward_staged.argtypes = [C.POINTER(SsdDims), C.POINTER(SsdBwdPtrs), vp, sz, vp, i32]
     lib.ssd_state_update.restype = i32
     lib.ssd_state_update.argtypes = [C.POINTER(SsdStepDims), C.POINTER(SsdStepPtrs), vp]
+    lib.ssd_state_update_host.restype = i32
+    lib.ssd_state_update_host.argtypes = [C.POINTER(SsdStepDims), C.POINTER(SsdStepPtrs), vp, vp]
     lib.ssd_state_reset_rows.restype = i32
     lib.ssd_state_reset_rows.argtypes = [vp, i64, vp, i64, i64, vp]
     lib.ssd_sp_total_logdecay.restype = i32
@@ -199,7 +201,8 @@ def host():
     loader = importlib.machinery.ExtensionFileLoader("_ssd_host", str(HOST_PATH))
     mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("_ssd_host", loader))
     loader.exec_module(mod)
-    names = ("ssd_workspace_bytes", "ssd_forward_staged", "ssd_backward_staged", "ssd_state_update", "ssd_last_error",
+    names = ("ssd_workspace_bytes", "ssd_forward_staged", "ssd_backward_staged", "ssd_state_update", "ssd_state_update_host",
+             "ssd_last_error",
              "ssd_conv1d_workspace_bytes", "ssd_conv1d_forward", "ssd_conv1d_backward", "ssd_rmsnorm_workspace_bytes",
              "ssd_rmsnorm_forward", "ssd_rmsnorm_backward")
     mod.bind(tuple(C.cast(getattr(lib, n), C.c_void_p).value for n in names), SsdError, torch.OutOfMemoryError)

@@ -203,6 +203,43 @@ static int check_ws(const void* ws, size_t have, size_t need) {
   return SSD_OK;
 }
 
+// Checks one step and fills in the strides left at 0.
+static int check_step(const SsdStepDims* d, const SsdStepPtrs* p, const void* y, SsdStepDims* out) {
+  if (!d || !p) { set_error("dims/ptrs is NULL"); return SSD_ERR_NULL_POINTER; }
+  if (d->streams <= 0 || d->nheads <= 0 || d->headdim <= 0 || d->dstate <= 0 || d->ngroups <= 0) {
+    set_error("streams/nheads/headdim/dstate/ngroups must be positive"); return SSD_ERR_BAD_SHAPE;
+  }
+  if (d->nheads % d->ngroups) { set_error("nheads (%d) must be a multiple of ngroups (%d)", d->nheads, d->ngroups); return SSD_ERR_BAD_SHAPE; }
+  if (d->dtype != SSD_F32 && d->dtype != SSD_BF16) { set_error("unknown dtype %d", d->dtype); return SSD_ERR_UNSUPPORTED; }
+  if (!p->state || !p->x || !p->dt || !p->A || !p->Bm || !p->Cm || !y) { set_error("state, x, dt, A, B, C, y must be non-NULL"); return SSD_ERR_NULL_POINTER; }
+  if ((long long)d->streams * d->nheads > 2147483647LL) { set_error("streams*nheads exceeds the grid limit"); return SSD_ERR_UNSUPPORTED; }
+  SsdStepDims& e = *out;
+  e = *d;
+  const long long HP = (long long)d->nheads * d->headdim, GN = (long long)d->ngroups * d->dstate;
+  if (!e.x_stride_s) e.x_stride_s = HP;
+  if (!e.z_stride_s) e.z_stride_s = HP;
+  if (!e.y_stride_s) e.y_stride_s = HP;
+  if (!e.dt_stride_s) e.dt_stride_s = d->nheads;
+  if (!e.b_stride_s) e.b_stride_s = GN;
+  if (!e.c_stride_s) e.c_stride_s = GN;
+  const int N = d->dstate;
+  const bool vec = (N == 16 || N == 32 || N == 64 || N == 128 || N == 256);
+  if (vec) {
+    const size_t es = d->dtype == SSD_BF16 ? 2 : 4;
+    if (((uintptr_t)p->state & 15) || ((uintptr_t)p->Bm % (4 * es)) || ((uintptr_t)p->Cm % (4 * es)) ||
+        (e.b_stride_s % 4) || (e.c_stride_s % 4)) {
+      set_error("state must be 16-byte aligned and B/C rows aligned to 4 elements"); return SSD_ERR_BAD_ALIGNMENT;
+    }
+  }
+  if (d->device >= 0) {
+    int cur = -1;
+    if (cudaGetDevice(&cur) != cudaSuccess || cur != d->device) {
+      set_error("current CUDA device is %d but dims.device is %d", cur, d->device); return SSD_ERR_CUDA;
+    }
+  }
+  return SSD_OK;
+}
+
 int status_code_to_rc(int32_t code, const char* where) {
   if (code == 0) return SSD_OK;
   set_error("%s: a bounded wait inside a pipelined kernel ran out (wait-site code %d); the results of that call are invalid, "
@@ -354,38 +391,26 @@ int32_t ssd_backward(const SsdDims* dims, const SsdBwdPtrs* p, void* workspace, 
 
 int32_t ssd_state_update(const SsdStepDims* d, const SsdStepPtrs* p, void* cuda_stream) {
   clear_error();
-  if (!d || !p) { set_error("dims/ptrs is NULL"); return SSD_ERR_NULL_POINTER; }
-  if (d->streams <= 0 || d->nheads <= 0 || d->headdim <= 0 || d->dstate <= 0 || d->ngroups <= 0) {
-    set_error("streams/nheads/headdim/dstate/ngroups must be positive"); return SSD_ERR_BAD_SHAPE;
-  }
-  if (d->nheads % d->ngroups) { set_error("nheads (%d) must be a multiple of ngroups (%d)", d->nheads, d->ngroups); return SSD_ERR_BAD_SHAPE; }
-  if (d->dtype != SSD_F32 && d->dtype != SSD_BF16) { set_error("unknown dtype %d", d->dtype); return SSD_ERR_UNSUPPORTED; }
-  if (!p->state || !p->x || !p->dt || !p->A || !p->Bm || !p->Cm || !p->y) { set_error("state, x, dt, A, B, C, y must be non-NULL"); return SSD_ERR_NULL_POINTER; }
-  if ((long long)d->streams * d->nheads > 2147483647LL) { set_error("streams*nheads exceeds the grid limit"); return SSD_ERR_UNSUPPORTED; }
-  SsdStepDims e = *d;
-  const long long HP = (long long)d->nheads * d->headdim, GN = (long long)d->ngroups * d->dstate;
-  if (!e.x_stride_s) e.x_stride_s = HP;
-  if (!e.z_stride_s) e.z_stride_s = HP;
-  if (!e.y_stride_s) e.y_stride_s = HP;
-  if (!e.dt_stride_s) e.dt_stride_s = d->nheads;
-  if (!e.b_stride_s) e.b_stride_s = GN;
-  if (!e.c_stride_s) e.c_stride_s = GN;
-  const int N = d->dstate;
-  const bool vec = (N == 16 || N == 32 || N == 64 || N == 128 || N == 256);
-  if (vec) {
-    const size_t es = d->dtype == SSD_BF16 ? 2 : 4;
-    if (((uintptr_t)p->state & 15) || ((uintptr_t)p->Bm % (4 * es)) || ((uintptr_t)p->Cm % (4 * es)) ||
-        (e.b_stride_s % 4) || (e.c_stride_s % 4)) {
-      set_error("state must be 16-byte aligned and B/C rows aligned to 4 elements"); return SSD_ERR_BAD_ALIGNMENT;
+  SsdStepDims e;
+  const int rc = check_step(d, p, p ? p->y : nullptr, &e);
+  return rc ? rc : decode_step(e, *p, (cudaStream_t)cuda_stream);
+}
+
+int32_t ssd_state_update_host(const SsdStepDims* d, const SsdStepPtrs* p, void* y_host, void* cuda_stream) {
+  clear_error();
+  SsdStepDims e;
+  const int rc = check_step(d, p, y_host, &e);
+  if (rc) return rc;
+  const void* host[] = {p->x, p->dt, p->Bm, p->Cm, y_host};
+  for (const void* q : host) {   // pageable memory must not reach the kernel
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, q) != cudaSuccess || at.devicePointer != q) {
+      cudaGetLastError();
+      set_error("state_update_host: x, dt, B, C and y_host must be pinned host memory (or device memory) the device can address");
+      return SSD_ERR_UNSUPPORTED;
     }
   }
-  if (d->device >= 0) {
-    int cur = -1;
-    if (cudaGetDevice(&cur) != cudaSuccess || cur != d->device) {
-      set_error("current CUDA device is %d but dims.device is %d", cur, d->device); return SSD_ERR_CUDA;
-    }
-  }
-  return decode_step(e, *p, (cudaStream_t)cuda_stream);
+  return decode_step_host(e, *p, y_host, (cudaStream_t)cuda_stream);
 }
 
 // ---- status word ----------------------------------------------------------------------------------

@@ -36,6 +36,7 @@ struct Api {
   decltype(&::ssd_forward_staged) forward_staged;
   decltype(&::ssd_backward_staged) backward_staged;
   decltype(&::ssd_state_update) state_update;
+  decltype(&::ssd_state_update_host) state_update_host;
   decltype(&::ssd_last_error) last_error;
   decltype(&::ssd_conv1d_workspace_bytes) conv1d_workspace_bytes;
   decltype(&::ssd_conv1d_forward) conv1d_forward;
@@ -468,46 +469,82 @@ PyObject* triple(const Tensor& a, const Tensor& b, const Tensor& c) {
   return r;
 }
 
+// One step's operands: `where` is the device of the per-stream vectors (the state's, or the CPU).
+struct Step {
+  SsdStepDims d;
+  SsdStepPtrs p;
+  int64_t S, H, P;
+};
+Step step_of(const Tensor& state, const Tensor& x, const Tensor& dt, const Tensor& A, const Tensor& Bm, const Tensor& Cm, const Tensor* D,
+             const Tensor* z, const Tensor* bias, bool softplus, const at::Device& where) {
+  const at::Device dev = state.device();
+  if (state.dim() != 4 || state.scalar_type() != at::kFloat || !state.is_contiguous())
+    fail("state must be a contiguous float32 [streams, nheads, headdim, dstate] tensor");
+  const int64_t S = state.size(0), H = state.size(1), P = state.size(2), N = state.size(3);
+  Step s;
+  std::memset(&s, 0, sizeof s);
+  SsdStepDims& d = s.d;
+  d.dtype = storage_type(x);
+  if (Bm.dim() != 3 || Bm.size(0) != S || Bm.size(2) != N) fail("B must be [streams, ngroups, dstate]");
+  const int64_t G = Bm.size(1);
+  if (G <= 0 || H % G) fail("nheads (", H, ") must be a multiple of ngroups (", G, ")");
+  auto vec = [&](const char* name, const Tensor& t, const Shape& shape) {
+    if (!same(t, shape) || t.scalar_type() != x.scalar_type() || t.device() != where)
+      fail(name, ": expected ", at::IntArrayRef(shape), " ", x.scalar_type(), " on ", where);
+    if (t.stride(-1) != 1 || (t.dim() >= 3 && t.stride(1) != t.size(2))) fail(name, ": inner dims must be dense");
+  };
+  vec("x", x, Shape(S, H, P)); vec("dt", dt, Shape(S, H)); vec("B", Bm, Shape(S, G, N)); vec("C", Cm, Shape(S, G, N));
+  check_dense_f32("A", &A, Shape(H), dev);
+  check_dense_f32("D", D, Shape(H), dev);
+  check_dense_f32("dt_bias", bias, Shape(H), dev);
+  if (z) vec("z", *z, Shape(S, H, P));
+  d.streams = (int32_t)S; d.nheads = (int32_t)H; d.headdim = (int32_t)P; d.dstate = (int32_t)N; d.ngroups = (int32_t)G;
+  d.device = dev.index(); d.dt_softplus = softplus ? 1 : 0;
+  d.x_stride_s = x.stride(0); d.dt_stride_s = dt.stride(0); d.b_stride_s = Bm.stride(0); d.c_stride_s = Cm.stride(0);
+  d.z_stride_s = z ? z->stride(0) : 0;
+  SsdStepPtrs& p = s.p;
+  p.state = fptr(&state); p.x = ptr(&x); p.dt = ptr(&dt); p.A = fptr(&A); p.Bm = ptr(&Bm); p.Cm = ptr(&Cm); p.D = fptr(D); p.z = ptr(z);
+  p.dt_bias = fptr(bias);
+  s.S = S; s.H = H; s.P = P;
+  return s;
+}
+
 // state, x, dt, A, B, C, D, z, y, dt_bias, dt_softplus -> y
 PyObject* py_state_update(PyObject*, PyObject* const* argv, Py_ssize_t argc) {
   return guarded([&]() -> PyObject* {
     const Args a(argv, argc, 11);
-    const Tensor &state = a.tensor(0, "state"), &x = a.tensor(1, "x"), &dt = a.tensor(2, "dt"), &A = a.tensor(3, "A"),
-                 &Bm = a.tensor(4, "B"), &Cm = a.tensor(5, "C");
-    const Tensor *D = a.opt(6, "D"), *z = a.opt(7, "z"), *y_in = a.opt(8, "y"), *bias = a.opt(9, "dt_bias");
+    const Tensor &state = a.tensor(0, "state"), &x = a.tensor(1, "x");
     if (!state.is_cuda()) fail("state must be a CUDA tensor (there is no CPU path)");
     const at::Device dev = state.device();
-    if (state.dim() != 4 || state.scalar_type() != at::kFloat || !state.is_contiguous())
-      fail("state must be a contiguous float32 [streams, nheads, headdim, dstate] tensor");
-    const int64_t S = state.size(0), H = state.size(1), P = state.size(2), N = state.size(3);
-    SsdStepDims d;
-    std::memset(&d, 0, sizeof d);
-    d.dtype = storage_type(x);
-    if (Bm.dim() != 3 || Bm.size(0) != S || Bm.size(2) != N) fail("B must be [streams, ngroups, dstate]");
-    const int64_t G = Bm.size(1);
-    if (G <= 0 || H % G) fail("nheads (", H, ") must be a multiple of ngroups (", G, ")");
-    auto vec = [&](const char* name, const Tensor& t, const Shape& shape) {
-      if (!same(t, shape) || t.scalar_type() != x.scalar_type() || t.device() != dev)
-        fail(name, ": expected ", at::IntArrayRef(shape), " ", x.scalar_type(), " on ", dev);
-      if (t.stride(-1) != 1 || (t.dim() >= 3 && t.stride(1) != t.size(2))) fail(name, ": inner dims must be dense");
-    };
-    vec("x", x, Shape(S, H, P)); vec("dt", dt, Shape(S, H)); vec("B", Bm, Shape(S, G, N)); vec("C", Cm, Shape(S, G, N));
-    check_dense_f32("A", &A, Shape(H), dev);
-    check_dense_f32("D", D, Shape(H), dev);
-    check_dense_f32("dt_bias", bias, Shape(H), dev);
-    Tensor y = y_in ? *y_in : empty(Shape(S, H, P), x.scalar_type(), dev);
-    if (z) vec("z", *z, Shape(S, H, P));
-    d.streams = (int32_t)S; d.nheads = (int32_t)H; d.headdim = (int32_t)P; d.dstate = (int32_t)N; d.ngroups = (int32_t)G;
-    d.device = dev.index(); d.dt_softplus = a.flag(10) ? 1 : 0;
-    d.x_stride_s = x.stride(0); d.dt_stride_s = dt.stride(0); d.b_stride_s = Bm.stride(0); d.c_stride_s = Cm.stride(0);
-    d.z_stride_s = z ? z->stride(0) : 0; d.y_stride_s = y.stride(0);
-    SsdStepPtrs p;
-    std::memset(&p, 0, sizeof p);
-    p.state = fptr(&state); p.x = ptr(&x); p.dt = ptr(&dt); p.A = fptr(&A); p.Bm = ptr(&Bm); p.Cm = ptr(&Cm); p.D = fptr(D); p.z = ptr(z);
-    p.y = ptr(&y); p.dt_bias = fptr(bias);
+    Step s = step_of(state, x, a.tensor(2, "dt"), a.tensor(3, "A"), a.tensor(4, "B"), a.tensor(5, "C"), a.opt(6, "D"), a.opt(7, "z"),
+                     a.opt(9, "dt_bias"), a.flag(10), dev);
+    const Tensor* y_in = a.opt(8, "y");
+    Tensor y = y_in ? *y_in : empty(Shape(s.S, s.H, s.P), x.scalar_type(), dev);
+    s.d.y_stride_s = y.stride(0);
+    s.p.y = ptr(&y);
     const c10::cuda::CUDAGuard guard(dev);
-    check_rc(api.state_update(&d, &p, stream_of(dev)));
+    check_rc(api.state_update(&s.d, &s.p, stream_of(dev)));
     return wrap(y);
+  });
+}
+
+// state, x, dt, A, B, C, D, y, y_host: the vectors and y_host in pinned host memory -> None
+PyObject* py_state_update_host(PyObject*, PyObject* const* argv, Py_ssize_t argc) {
+  return guarded([&]() -> PyObject* {
+    const Args a(argv, argc, 9);
+    const Tensor &state = a.tensor(0, "state"), &y = a.tensor(7, "y"), &yh = a.tensor(8, "y_host");
+    if (!state.is_cuda()) fail("state must be a CUDA tensor (there is no CPU path)");
+    const at::Device dev = state.device();
+    Step s = step_of(state, a.tensor(1, "x"), a.tensor(2, "dt"), a.tensor(3, "A"), a.tensor(4, "B"), a.tensor(5, "C"), a.opt(6, "D"), nullptr,
+                     nullptr, false, at::Device(at::kCPU));
+    for (const Tensor* t : {&y, &yh})
+      if (!same(*t, Shape(s.S, s.H, s.P)) || t->scalar_type() != a.tensor(1, "x").scalar_type() || !t->is_contiguous())
+        fail("y: expected a contiguous ", at::IntArrayRef(Shape(s.S, s.H, s.P)), " tensor");
+    s.d.y_stride_s = s.H * s.P;
+    s.p.y = ptr(&y);
+    const c10::cuda::CUDAGuard guard(dev);
+    check_rc(api.state_update_host(&s.d, &s.p, ptr(&yh), stream_of(dev)));
+    Py_RETURN_NONE;
   });
 }
 
@@ -656,7 +693,7 @@ PyObject* py_bind(PyObject*, PyObject* const* argv, Py_ssize_t argc) {
 }
 
 #define FAST(name, fn) {name, (PyCFunction)(void (*)(void))fn, METH_FASTCALL, nullptr}
-PyMethodDef methods[] = {FAST("bind", py_bind), FAST("state_update", py_state_update), FAST("forward", py_forward),
+PyMethodDef methods[] = {FAST("bind", py_bind), FAST("state_update", py_state_update), FAST("state_update_host", py_state_update_host), FAST("forward", py_forward),
                          FAST("backward", py_backward), FAST("scan", py_scan), FAST("mixer", py_mixer),
                          FAST("conv1d_forward", py_conv_forward), FAST("conv1d_backward", py_conv_backward),
                          FAST("rmsnorm_forward", py_norm_forward), FAST("rmsnorm_backward", py_norm_backward), {nullptr, nullptr, 0, nullptr}};

@@ -47,6 +47,7 @@ int read_status_sync(const void* word, void* cuda_stream, int32_t* code_out, con
 
 int tensor_selftest_wait(int* status, long long max_cycles, cudaStream_t s);
 int decode_step(const SsdStepDims& d, const SsdStepPtrs& p, cudaStream_t s);
+int decode_step_host(const SsdStepDims& d, const SsdStepPtrs& p, void* y_host, cudaStream_t s);
 int reset_rows(float* state, long long row_elems, const long long* idx, long long count, long long streams,
                cudaStream_t s);
 int sp_total_logdecay(const Geo& g, const float* cs, float* out, cudaStream_t s);

@@ -12,7 +12,10 @@ from typing import Dict, Optional
 
 import torch
 
+from . import _lib as L
 from . import ssd
+
+SSD_ERR_UNSUPPORTED = -3
 
 _SEQ_IN = ("x", "dt", "B", "C", "dy", "z")
 _SEQ_OUT = ("y", "dx", "ddt", "dB", "dC", "dz")
@@ -114,8 +117,9 @@ class HostStep:
     the device: one call copies x, dt, B, C in, runs the state update and copies y out.
 
     The object owns the pinned staging buffers: the caller writes the step's vectors into `hx`, `hdt`,
-    `hB`, `hC` (views of ONE packed pinned buffer, one packed row per stream, so a group of streams moves
-    with a single copy) and reads the result from `hy`.  The streams (environments) are cut into `groups`
+    `hB`, `hC` (views of ONE packed pinned buffer, one packed row per stream) and reads the result from `hy`.
+    Where the library's host-memory step covers the shape, a step is one kernel that reads the packed rows and writes
+    `hy` over PCIe itself.  Other shapes copy: the streams (environments) are cut into `groups`
     row ranges that flow through three CUDA streams (host->device copies, kernels, device->host copies),
     the way a rollout double-buffers groups of environments: while one group's kernel runs, the next
     group's inputs arrive and the previous group's outputs leave.  After one eager step the whole step is
@@ -146,6 +150,7 @@ class HostStep:
         self.s_in, self.s_run, self.s_out = (torch.cuda.Stream(dev) for _ in range(3))
         self.ev_in = [torch.cuda.Event() for _ in self.ranges]
         self.ev_run = [torch.cuda.Event() for _ in self.ranges]
+        self._in_place = True
         self.use_graph, self._graph, self._calls, self._params = graph, None, 0, None
 
     def bytes_per_call(self):
@@ -177,7 +182,19 @@ class HostStep:
         for s in (self.s_in, self.s_run, self.s_out):
             root.wait_stream(s)
 
+    def _step_in_place(self, A, D) -> bool:
+        """One host-memory step; False (and never asked again) where the library does not cover the shape."""
+        try:
+            L.host().state_update_host(self.state, self.hx, self.hdt, A, self.hB, self.hC, D, self.y, self.hy)
+        except L.SsdError as e:
+            if e.code != SSD_ERR_UNSUPPORTED:
+                raise
+            self._in_place = False
+        return self._in_place
+
     def step(self, A, D) -> None:
+        if self._in_place and self._step_in_place(A, D):
+            return
         cur = torch.cuda.current_stream(self.dev)
         self._calls += 1
         if not self.use_graph or self._calls == 1:          # first step eagerly (also warms everything up)
