@@ -131,8 +131,9 @@ static void make_layout(const Geo& g, bool has_z, bool tcfam, WsLayout* w) {
   w->ds_bf = take(tcfam ? nst / 2 : 0);
   w->wsum = take(tcfam ? 0 : ncb);
   w->dyp = take(has_z ? (size_t)g.B * g.L * g.H * g.P * f : 0);
-  w->dcsp = take(nq); w->ddtd = take(nq); w->ddot = take(nq);
-  w->sdot = take(nbh * (tcfam ? 64 : 1));   // tensor family: up to 64 warp-partial sums per entry
+  // CUDA-core family: dcsp in one part per 32 chunk positions and per 32 state columns, ddtd in one per 32 features
+  w->dcsp = take(nq * (tcfam ? 1 : (g.Q + 31) / 32 + (g.N + 31) / 32)); w->ddtd = take(nq * (tcfam ? 1 : (g.P + 31) / 32)); w->ddot = take(nq);
+  w->sdot = take(nbh * 8 * ((g.P * g.N / 4 + 255) / 256 + 1));   // warp-partial sums of the reverse scan
   w->dapart = take(nbh); w->ddpart = take(nbh); w->dbpart = take(nbh);
   w->dini = take(nfin);
   w->total_bwd = o;
@@ -169,10 +170,11 @@ static size_t forward_bytes(const SsdDims* d) {
   return any.total_fwd > fwd.total_fwd ? any.total_fwd : fwd.total_fwd;
 }
 
-// The CUDA-core kernels put (chunk, head) on one grid axis.
+// The CUDA-core kernels have a block per output tile on one grid axis.
 static int check_core_grid(const Geo& g) {
-  if ((long long)g.nc * g.H > 65535) {
-    set_error("CUDA-core family: nchunks*nheads (%lld) must be <= 65535 (grid limit)", (long long)g.nc * g.H);
+  const long long most = (long long)g.B * g.nc * g.H * ((g.Q + 31) / 32) * ((g.N + 31) / 32 + (g.P + 31) / 32) * 2;
+  if (most > 0x7fffffffLL) {
+    set_error("CUDA-core family: too many output tiles for one grid (%lld)", most);
     return SSD_ERR_UNSUPPORTED;
   }
   return 0;

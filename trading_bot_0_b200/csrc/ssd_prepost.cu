@@ -95,25 +95,6 @@ template <> __device__ __forceinline__ float sig_<__nv_bfloat16>(float a) {
 }
 template <> __device__ __forceinline__ float sig_<float>(float a) { return __fdividef(1.f, 1.f + __expf(-a)); }
 
-// Packed pairs of fp32 (one 64-bit register): sm_100 executes fma / add on both halves in one instruction, with the same
-// rounding as the scalar forms.
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
-  f32x2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ void unpack2(f32x2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-  f32x2 d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
-  f32x2 d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
 // NC storage elements -> NC/2 packed pairs
 __device__ __forceinline__ void unpack_pairs(const RawN<__nv_bfloat16, 8>& r, f32x2 (&v)[4]) {
   const uint32_t w[4] = {r.v.x, r.v.y, r.v.z, r.v.w};
