@@ -4,7 +4,7 @@ import pytest
 import torch
 
 from oracle import ssd_oracle as O
-from tests._util import assert_close, mean_rel, oracle_all, to_dev
+from tests._util import assert_close, assert_close_dA_few_rows, mean_rel, oracle_all, to_dev
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -185,3 +185,51 @@ def test_ragged_forward_runs_on_the_tensor_family(lib, L, H, P, N, G, has_z):
     assert_close("y", y, y_ref, "bf16")
     assert_close("final_state", fin, fin_ref, "bf16")
     assert (buf[:, L:] == 7.0).all()
+
+
+@pytest.mark.parametrize("L", [1, 100, 129, 383])
+@pytest.mark.parametrize("H,P,N,G,has_z", [(8, 32, 64, 1, False), (4, 64, 64, 2, True), (24, 64, 128, 1, True), (8, 32, 128, 2, False)])
+def test_ragged_training_runs_on_the_tensor_family(lib, L, H, P, N, G, has_z):
+    """Forward and backward of any sequence length: outputs of one batch row stop at its end, padded positions add nothing."""
+    import trading_bot_0_b200 as T
+    cfg = O.SsdConfig("rag", 3, L, H, P, N, G, 128, "bf16", has_z)
+    inp = O.make_inputs(cfg, with_init_state=True)
+    ref = oracle_all(inp)
+    d = to_dev(inp, DEV)
+    a = (d["x"], d["dt"], d["A"], d["B"], d["C"], d["D"], d.get("z"), d["init_state"])
+    y, fin, ws = T.forward(*a, chunk=128, algo="tensor", for_backward=True)
+    g = T.backward(d["dy"], *a, chunk=128, algo="tensor", workspace=ws, fwd_saved=True, want_dinit=True)
+    torch.cuda.synchronize()
+    assert status_word(ws) == 0
+    assert_close("y", y, ref["y"], "bf16")
+    for k in ("dx", "ddt", "dB", "dC", "dD", "dinit") + (("dz",) if has_z else ()):
+        assert_close(k, g[k], ref[k], "bf16")
+    assert_close_dA_few_rows("dA", g["dA"], ref["dA"])
+
+
+@pytest.mark.parametrize("which", ["y", "dy", "both", "x"])
+@pytest.mark.parametrize("N", [64, 128])
+def test_ragged_operands_of_any_alignment(lib, which, N):
+    """algo = auto on a ragged sequence takes pointers that TMA cannot address: y goes through the workspace, a backward with
+    such a dy recomputes on the CUDA cores, a shared operand moves both passes there."""
+    import trading_bot_0_b200 as T
+    cfg = O.SsdConfig("al", 2, 200, 8, 32, N, 1, 128, "bf16")
+    inp = O.make_inputs(cfg, with_init_state=True)
+    ref = oracle_all(inp)
+    d = to_dev(inp, DEV)
+
+    def off(t):
+        v = torch.zeros(t.numel() + 8, dtype=t.dtype, device=DEV)[3:3 + t.numel()].view_as(t)
+        v.copy_(t)
+        return v
+
+    x = off(d["x"]) if which == "x" else d["x"]
+    a = (x, d["dt"], d["A"], d["B"], d["C"], d["D"], None, d["init_state"])
+    y_out = off(torch.zeros_like(d["x"])) if which in ("y", "both") else None
+    y, fin, ws = T.forward(*a, chunk=128, for_backward=True, y=y_out)
+    dy = off(d["dy"]) if which in ("dy", "both") else d["dy"]
+    g = T.backward(dy, *a, chunk=128, workspace=ws, fwd_saved=True, want_dinit=True)
+    assert_close("y", y, ref["y"], "bf16")
+    assert_close("final_state", fin, ref["final_state"], "bf16")
+    for k in ("dx", "ddt", "dB", "dC", "dD", "dinit"):
+        assert_close(k, g[k], ref[k], "bf16")

@@ -20,7 +20,7 @@ struct Geo {
   int B, L, H, P, N, G, Q, nc, hpg;  // hpg = heads per group
   long long xsb, xsl, dtsb, dtsl, bsb, bsl, csb, csl, zsb, zsl, ysb, ysl;
   int dt_softplus;                     // step size = softplus(dt + dt_bias) instead of dt + dt_bias
-  int fwd_only;                        // the workspace is too small for a backward: none will follow in it (see forward_geo)
+  int any_y;                           // y / dy need not suit TMA: the caller takes care of them (see Plan in ssd_api.cu)
   int onetile;                         // tensor family: the one-tile-per-CTA kernels for every shape (SSD_ALGO_TENSOR_ONETILE)
 };
 

@@ -1,5 +1,6 @@
 // extern "C" entry points: argument validation, workspace layout, kernel-family dispatch.
 #include <atomic>
+#include <initializer_list>
 #include <stdarg.h>
 #include <stdio.h>
 #include <string.h>
@@ -58,7 +59,7 @@ int sm_count() {
 static size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
 
 // Returns 0 or a negative status (error string set).
-static int make_geo(const SsdDims* d, Geo* g, bool fwd_only = false) {
+static int make_geo(const SsdDims* d, Geo* g) {
   if (!d) { set_error("dims is NULL"); return SSD_ERR_NULL_POINTER; }
   if (d->batch <= 0 || d->seqlen <= 0 || d->nheads <= 0 || d->headdim <= 0 || d->dstate <= 0 || d->ngroups <= 0 ||
       d->chunk <= 0) {
@@ -76,7 +77,7 @@ static int make_geo(const SsdDims* d, Geo* g, bool fwd_only = false) {
   g->B = d->batch; g->L = d->seqlen; g->H = d->nheads; g->P = d->headdim; g->N = d->dstate; g->G = d->ngroups;
   g->Q = d->chunk; g->nc = (d->seqlen + d->chunk - 1) / d->chunk; g->hpg = d->nheads / d->ngroups;
   g->dt_softplus = d->dt_softplus != 0;
-  g->fwd_only = fwd_only;
+  g->any_y = d->algo == SSD_ALGO_AUTO && d->seqlen % 128 != 0;
   g->onetile = d->algo == SSD_ALGO_TENSOR_ONETILE;
   if (g->B > 65535) { set_error("batch (%d) must be <= 65535 (grid limit)", g->B); return SSD_ERR_UNSUPPORTED; }
   const long long HP = (long long)g->H * g->P, GN = (long long)g->G * g->N;
@@ -105,8 +106,7 @@ static int make_geo(const SsdDims* d, Geo* g, bool fwd_only = false) {
     Geo t = *g;
     t.Q = 128;
     t.nc = (t.L + 127) / 128;
-    t.fwd_only = 1;   // also where only the forward will: both families then cut a sequence into the same chunks
-    if (tensor_supported(t, d->dtype, nullptr)) { t.fwd_only = fwd_only; *g = t; }
+    if (tensor_supported(t, d->dtype, nullptr)) *g = t;
   }
   return SSD_OK;
 }
@@ -143,31 +143,29 @@ static bool family_is_tensor(const Geo& g, const SsdDims* d) {
   return d->algo != SSD_ALGO_FP32_CORES && tensor_supported(g, d->dtype, nullptr);
 }
 
-// Geometry and layout of a forward (or of a call on a forward's workspace).  The tensor family's forward takes any sequence
-// length, its backward multiples of 128 only, and a backward with fwd_saved has to find the workspace as its own family
-// lays it out.  The size of the workspace tells the two apart: one that could not hold a backward's layout belongs to a
-// forward on its own.  `whole` = a full pass on pointers that suit the tensor family; anything else that is ragged stays on
-// the CUDA cores, whose layout fits as well (forward_bytes).
-static int forward_geo(const SsdDims* d, size_t workspace_bytes, bool whole, Geo* g, WsLayout* w) {
-  int rc = make_geo(d, g);
-  if (rc) return rc;
-  const bool has_z = d->has_z != 0;
-  make_layout(*g, has_z, family_is_tensor(*g, d), w);
-  if (g->L % 128 && whole && workspace_bytes < w->total_bwd) {
-    Geo t;
-    make_geo(d, &t, true);
-    if (family_is_tensor(t, d)) {
-      *g = t;
-      make_layout(t, has_z, true, w);
-    }
-  }
-  return SSD_OK;
-}
-static size_t forward_bytes(const SsdDims* d) {
+// Geometry, family and workspace layout of a call.  Whole chunks: the tensor family where it covers the dims, and operands it
+// cannot address are an error.  A sequence with a ragged tail and algo = AUTO takes any operands, so there the family goes
+// by what a forward and its backward share: x, B, C and z suit TMA or not.  With them a forward whose y does not suit writes
+// it dense into the workspace (the fp32 chunk states are dead by then, and as large at least) and copies it out; a
+// backward whose own operands do not suit runs on the CUDA cores and recomputes the forward in their layout, for which
+// ssd_workspace_bytes leaves room.
+struct Plan {
   Geo g;
-  WsLayout any, fwd;
-  if (forward_geo(d, SIZE_MAX, true, &g, &any) || forward_geo(d, 0, true, &g, &fwd)) return 0;
-  return any.total_fwd > fwd.total_fwd ? any.total_fwd : fwd.total_fwd;
+  WsLayout w;
+  bool tensor;
+};
+static bool unaligned(std::initializer_list<const void*> ps) {
+  uintptr_t low = 0;
+  for (const void* p : ps) low |= (uintptr_t)p;
+  return (low & 15) != 0;
+}
+static bool y_suits(const Geo& g, const void* y) { return !unaligned({y}) && g.ysl % 8 == 0 && g.ysb % 8 == 0; }
+static int make_plan(const SsdDims* d, std::initializer_list<const void*> shared, Plan* p) {
+  const int rc = make_geo(d, &p->g);
+  if (rc) return rc;
+  p->tensor = family_is_tensor(p->g, d) && !(p->g.any_y && unaligned(shared));
+  make_layout(p->g, d->has_z != 0, p->tensor, &p->w);
+  return SSD_OK;
 }
 
 // The CUDA-core kernels have a block per output tile on one grid axis.
@@ -317,20 +315,26 @@ size_t ssd_workspace_bytes(const SsdDims* dims, int32_t pass) {
   SsdDims d2;
   if (dims) { d2 = *dims; d2.device = -1; }
   if (make_geo(dims ? &d2 : nullptr, &g)) return 0;
-  if (pass != SSD_PASS_BWD) return forward_bytes(&d2);
+  const bool bwd = pass == SSD_PASS_BWD, tensor = family_is_tensor(g, dims);
   WsLayout w;
-  make_layout(g, dims->has_z != 0, family_is_tensor(g, dims), &w);
-  return w.total_bwd;
+  make_layout(g, dims->has_z != 0, tensor, &w);
+  size_t n = bwd ? w.total_bwd : w.total_fwd;
+  if (tensor && g.any_y) {   // either family may run (see Plan)
+    make_layout(g, dims->has_z != 0, false, &w);
+    const size_t m = bwd ? w.total_bwd : w.total_fwd;
+    if (m > n) n = m;
+  }
+  return n;
 }
 
 int32_t ssd_forward_staged(const SsdDims* dims, const SsdFwdPtrs* p, void* workspace, size_t workspace_bytes,
                            void* cuda_stream, int32_t stages) {
   clear_error();
-  Geo g;
-  WsLayout w;
-  const uintptr_t low = p ? ((uintptr_t)p->x | (uintptr_t)p->Bm | (uintptr_t)p->Cm | (uintptr_t)p->z | (uintptr_t)p->y) & 15 : 0;
-  int rc = forward_geo(dims, workspace_bytes, low == 0 && stages == SSD_STAGE_ALL, &g, &w);
+  Plan plan;
+  int rc = p ? make_plan(dims, {p->x, p->Bm, p->Cm, p->z}, &plan) : make_plan(dims, {}, &plan);
   if (rc) return rc;
+  Geo& g = plan.g;
+  const WsLayout& w = plan.w;
   if (!p) { set_error("ptrs is NULL"); return SSD_ERR_NULL_POINTER; }
   if (!p->x || !p->dt || !p->A || !p->Bm || !p->Cm) { set_error("x, dt, A, B, C must be non-NULL"); return SSD_ERR_NULL_POINTER; }
   if ((stages & SSD_STAGE_FINISH) && !p->y) { set_error("y must be non-NULL"); return SSD_ERR_NULL_POINTER; }
@@ -339,15 +343,23 @@ int32_t ssd_forward_staged(const SsdDims* dims, const SsdFwdPtrs* p, void* works
   rc = check_ws(workspace, workspace_bytes, w.total_fwd);
   if (rc) return rc;
   cudaStream_t s = (cudaStream_t)cuda_stream;
-  const int fam = pick_family(g, dims);
-  if (fam < 0) return fam;
-  if (fam == 1) {
-    const void* ptrs[] = {p->x, p->Bm, p->Cm, p->z, p->y};
-    const char* names[] = {"x", "B", "C", "z", "y"};
-    for (int i = 0; i < 5; ++i)
-      if ((rc = check_align16(names[i], ptrs[i]))) return rc;
-  }
-  return run_forward(g, dims->dtype, fam == 1, *p, (char*)workspace, w, s, stages, workspace_bytes >= w.total_bwd);
+  if (!plan.tensor && (rc = g.any_y ? check_core_grid(g) : pick_family(g, dims)) < 0) return rc;
+  const bool keep_fin = workspace_bytes >= w.total_bwd;
+  if (!plan.tensor) return run_forward(g, dims->dtype, false, *p, (char*)workspace, w, s, stages, keep_fin);
+  const bool bounce = g.any_y && p->y && !y_suits(g, p->y);
+  const void* ptrs[] = {p->x, p->Bm, p->Cm, p->z, bounce ? nullptr : p->y};
+  const char* names[] = {"x", "B", "C", "z", "y"};
+  for (int i = 0; i < 5; ++i)
+    if ((rc = check_align16(names[i], ptrs[i]))) return rc;
+  if (!bounce) return run_forward(g, dims->dtype, true, *p, (char*)workspace, w, s, stages, keep_fin);
+  Geo dense = g;
+  dense.ysl = (long long)g.H * g.P;
+  dense.ysb = dense.ysl * g.L;
+  SsdFwdPtrs q = *p;
+  q.y = (char*)workspace + w.states;
+  rc = run_forward(dense, dims->dtype, true, q, (char*)workspace, w, s, stages, keep_fin);
+  if (rc || !(stages & SSD_STAGE_FINISH)) return rc;
+  return tensor_copy_y(g, q.y, p->y, s);
 }
 
 int32_t ssd_forward(const SsdDims* dims, const SsdFwdPtrs* p, void* workspace, size_t workspace_bytes,
@@ -358,9 +370,10 @@ int32_t ssd_forward(const SsdDims* dims, const SsdFwdPtrs* p, void* workspace, s
 int32_t ssd_backward_staged(const SsdDims* dims, const SsdBwdPtrs* p, void* workspace, size_t workspace_bytes,
                             void* cuda_stream, int32_t stages) {
   clear_error();
-  Geo g;
-  int rc = make_geo(dims, &g);
+  Plan plan;
+  int rc = p ? make_plan(dims, {p->x, p->Bm, p->Cm, p->z}, &plan) : make_plan(dims, {}, &plan);
   if (rc) return rc;
+  const Geo& g = plan.g;
   if (!p) { set_error("ptrs is NULL"); return SSD_ERR_NULL_POINTER; }
   if (!p->x || !p->dt || !p->A || !p->Bm || !p->Cm || !p->dy) { set_error("x, dt, A, B, C, dy must be non-NULL"); return SSD_ERR_NULL_POINTER; }
   if (stages & SSD_STAGE_FINISH) {
@@ -371,19 +384,25 @@ int32_t ssd_backward_staged(const SsdDims* dims, const SsdBwdPtrs* p, void* work
   if ((p->z != nullptr) != (dims->has_z != 0)) { set_error("dims.has_z (%d) does not match the z pointer", dims->has_z); return SSD_ERR_BAD_SHAPE; }
   if (p->z && !p->dz) { set_error("dz must be non-NULL when z is given"); return SSD_ERR_NULL_POINTER; }
   if (stages == 0 || (stages & ~(SSD_STAGE_LOCAL | SSD_STAGE_TOTAL | SSD_STAGE_FINISH | SSD_STAGE_LOCAL_STATES | SSD_STAGE_LOCAL_REST))) { set_error("bad stage mask %d", stages); return SSD_ERR_BAD_SHAPE; }
-  WsLayout w;
-  make_layout(g, dims->has_z != 0, family_is_tensor(g, dims), &w);
+  SsdBwdPtrs q = *p;
+  if (plan.tensor && g.any_y && (!y_suits(g, p->dy) || unaligned({p->dx, p->dz, p->dB, p->dC}))) {
+    plan.tensor = false;
+    make_layout(g, dims->has_z != 0, false, &plan.w);
+    q.fwd_saved = 0;
+  }
+  const WsLayout& w = plan.w;
   rc = check_ws(workspace, workspace_bytes, w.total_bwd);
   if (rc) return rc;
-  const int fam = pick_family(g, dims);
-  if (fam < 0) return fam;
-  if (fam == 1) {
+  if (!plan.tensor) {
+    rc = g.any_y ? check_core_grid(g) : pick_family(g, dims);
+    if (rc < 0) return rc;
+  } else {
     const void* ptrs[] = {p->x, p->Bm, p->Cm, p->z, p->dy, p->dx, p->dz, p->dB, p->dC};
     const char* names[] = {"x", "B", "C", "z", "dy", "dx", "dz", "dB", "dC"};
     for (int i = 0; i < 9; ++i)
       if ((rc = check_align16(names[i], ptrs[i]))) return rc;
   }
-  return run_backward(g, dims->dtype, fam == 1, *p, (char*)workspace, w, (cudaStream_t)cuda_stream, stages);
+  return run_backward(g, dims->dtype, plan.tensor, q, (char*)workspace, w, (cudaStream_t)cuda_stream, stages);
 }
 
 int32_t ssd_backward(const SsdDims* dims, const SsdBwdPtrs* p, void* workspace, size_t workspace_bytes,

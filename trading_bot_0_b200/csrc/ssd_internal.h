@@ -45,6 +45,8 @@ int tensor_dbc(const Geo& g, const SsdBwdPtrs& p, const void* dyp, bool dy_dense
 int status_code_to_rc(int32_t code, const char* where);
 int read_status_sync(const void* word, void* cuda_stream, int32_t* code_out, const char* where);
 
+// y = src, src dense [B,L,H,P] bf16, y with the geometry's strides
+int tensor_copy_y(const Geo& g, const void* src, void* y, cudaStream_t s);
 int tensor_selftest_wait(int* status, long long max_cycles, cudaStream_t s);
 int decode_step(const SsdStepDims& d, const SsdStepPtrs& p, cudaStream_t s);
 int decode_step_host(const SsdStepDims& d, const SsdStepPtrs& p, void* y_host, cudaStream_t s);

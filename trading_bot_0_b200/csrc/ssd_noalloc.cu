@@ -59,7 +59,7 @@ extern "C" int32_t ssd_forward_noalloc(const SsdDims* dims, const SsdFwdPtrs* p,
   void* scratch = nullptr;
   const int rc = scratch_address("ssd_forward_noalloc", &scratch);
   if (rc) return rc;
-  return ssd_forward(dims, p, scratch, need, cuda_stream);   // the size tells the forward that no backward will follow
+  return ssd_forward(dims, p, scratch, kScratchBytes, cuda_stream);
 }
 
 // The status word of the built-in scratch (its first four bytes, like any workspace): the only way a caller of

@@ -953,8 +953,7 @@ __global__ void __launch_bounds__(PfCfg<P, MODE>::THREADS, 1) k_state_scan_ps(Ge
               d += run[8 * j + 2 * i] * __uint_as_float(q[i] << 16) + run[8 * j + 2 * i + 1] * __uint_as_float(q[i] & 0xffff0000u);
           }
         }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&se_free);
+        if (reads_done(__float_as_uint(d), lane)) mbar_arrive(&se_free);
 #pragma unroll
         for (int off = 16; off; off >>= 1) d += __shfl_xor_sync(0xffffffffu, d, off);
         if (lane == 0) {
@@ -1716,12 +1715,15 @@ k_dbc_tc(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant__
       float vc[16], vb[16];
       tmem_ld16(tmem_addr(tmDC, (warp & 3) * 32, part * (N / PARTS) + q * 16), vc);
       tmem_ld16(tmem_addr(tmDB, (warp & 3) * 32, part * (N / PARTS) + q * 16), vb);
-      st_global_32B(dC + o + q * 16,
-                    make_uint4(pack_bf16(vc[0], vc[1]), pack_bf16(vc[2], vc[3]), pack_bf16(vc[4], vc[5]), pack_bf16(vc[6], vc[7])),
-                    make_uint4(pack_bf16(vc[8], vc[9]), pack_bf16(vc[10], vc[11]), pack_bf16(vc[12], vc[13]), pack_bf16(vc[14], vc[15])));
-      st_global_32B(dB + o + q * 16,
-                    make_uint4(pack_bf16(vb[0], vb[1]), pack_bf16(vb[2], vb[3]), pack_bf16(vb[4], vb[5]), pack_bf16(vb[6], vb[7])),
-                    make_uint4(pack_bf16(vb[8], vb[9]), pack_bf16(vb[10], vb[11]), pack_bf16(vb[12], vb[13]), pack_bf16(vb[14], vb[15])));
+      if (c * QT + row < g.L) {   // a ragged sequence ends inside its last tile
+        st_global_32B(dC + o + q * 16,
+                      make_uint4(pack_bf16(vc[0], vc[1]), pack_bf16(vc[2], vc[3]), pack_bf16(vc[4], vc[5]), pack_bf16(vc[6], vc[7])),
+                      make_uint4(pack_bf16(vc[8], vc[9]), pack_bf16(vc[10], vc[11]), pack_bf16(vc[12], vc[13]), pack_bf16(vc[14], vc[15])));
+        st_global_32B(dB + o + q * 16,
+                      make_uint4(pack_bf16(vb[0], vb[1]), pack_bf16(vb[2], vb[3]), pack_bf16(vb[4], vb[5]), pack_bf16(vb[6], vb[7])),
+                      make_uint4(pack_bf16(vb[8], vb[9]), pack_bf16(vb[10], vb[11]), pack_bf16(vb[12], vb[13]), pack_bf16(vb[14], vb[15])));
+      }
+      __syncwarp();
     }
   }
   tc_fence_before();
@@ -2087,6 +2089,11 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         if (t_ >= my_tiles) return;
         int b_, grp_, c_;
         tile_coords(t_, b_, grp_, c_);
+        if (c_ * QT + row >= g.L) {   // past the end of a ragged sequence
+#pragma unroll
+          for (int q = 0; q < 4; ++q) dst[q] = make_uint4(0u, 0u, 0u, 0u);
+          return;
+        }
         const bf16* zp_ = z + b_ * g.zsb + (long long)(c_ * QT + row) * g.zsl + (long long)(grp_ * g.hpg + blk_ * HB) * P + half * 32;
         ld_global_32B(zp_, dst[0], dst[1]);
         ld_global_32B(zp_ + 16, dst[2], dst[3]);
@@ -2110,8 +2117,7 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         const uint32_t tbs = smem_u32(tb);
         const float cs_r = lds_f32(tbs + 4 * (T_CS + row)), dt_r = lds_f32(tbs + 4 * (T_DT + row));
         const float osc = (MODE == 2) ? dt_r * ex2(lds_f32(tbs + 4 * (T_CS + 127)) - cs_r) : ex2(cs_r);
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&bars.tab_empty[ts]);
+        if (reads_done(__float_as_uint(cs_r) ^ __float_as_uint(dt_r) ^ __float_as_uint(osc), lane)) mbar_arrive(&bars.tab_empty[ts]);
         w.wait(&bars.in_full[ib], (kb >> 1) & 1, 54);
         w.wait(&bars.acc_full[ab], (kb >> 1) & 1, 55);
         tc_fence_after();
@@ -2139,8 +2145,13 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
           }
           if (h16 == 1) {
             tc_fence_before();
-            __syncwarp();
-            if (lane == 0) { mbar_arrive(&bars.acc_empty[ab]); if (!TSTORE) mbar_arrive(&bars.in_empty[ib]); }
+            if (TSTORE) {
+              __syncwarp();
+              if (lane == 0) mbar_arrive(&bars.acc_empty[ab]);
+            } else if (reads_done(xv[0].x ^ xv[1].x ^ dv[0].x ^ dv[1].x, lane)) {
+              mbar_arrive(&bars.acc_empty[ab]);
+              mbar_arrive(&bars.in_empty[ib]);
+            }
           }
           uint4 ov[2], dpk[2];
 #pragma unroll
@@ -2183,10 +2194,11 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
               ov[q] = pack8(o);
             }
           }
-          if (MODE == 1 && GATED) {
+          if (MODE == 1 && GATED && t_row < g.L) {
             st_global_32B(dz + dense + h16 * 16, ov[0], ov[1]);
             st_global_32B(dypb + dense + h16 * 16, dpk[0], dpk[1]);
           }
+          if (MODE == 1 && GATED) __syncwarp();
           if (TSTORE) {   // over the chunks of the x (dy) box this thread has just read
 #pragma unroll
             for (int q = 0; q < 2; ++q)
@@ -2533,8 +2545,7 @@ k_bwd_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant__
         const uint32_t tbs = smem_u32(tb);
         const float cs_r = lds_f32(tbs + 4 * (T_CS + row)), dt_r = lds_f32(tbs + 4 * (T_DT + row));
         const float osc_y = ex2(cs_r), osc_u = dt_r * ex2(lds_f32(tbs + 4 * (T_CS + 127)) - cs_r);
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&bars.tab_empty[ts]);
+        if (reads_done(__float_as_uint(cs_r) ^ __float_as_uint(osc_u), lane)) mbar_arrive(&bars.tab_empty[ts]);
         w.wait(&bars.in_full[ib], (kb >> 1) & 1, 54);
         w.wait(&bars.acc_full, kb & 1, 55);
         tc_fence_after();
@@ -2561,8 +2572,7 @@ k_bwd_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant__
           }
           if (ph == 3) {   // everything read: hand the accumulators and the input slot back
             tc_fence_before();
-            __syncwarp();
-            if (lane == 0) { mbar_arrive(&bars.acc_empty); mbar_arrive(&bars.in_empty[ib]); }
+            if (reads_done(xv[0].x ^ xv[1].x ^ dv[0].x ^ dv[1].x, lane)) { mbar_arrive(&bars.acc_empty); mbar_arrive(&bars.in_empty[ib]); }
           }
           const float osc = upass ? osc_u : osc_y;
           uint4 ov[2];
@@ -2589,7 +2599,8 @@ k_bwd_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant__
               ov[q] = pack8(o);
             }
           }
-          if (upass) st_global_32B(dx + dense + h16 * 16, ov[0], ov[1]);
+          if (upass && t_row < g.L) st_global_32B(dx + dense + h16 * 16, ov[0], ov[1]);
+          __syncwarp();
         }
         if (P == 64) {   // the two column halves of a row belong to one head: combine through shared memory
           asm volatile("bar.sync 1, 256;" ::: "memory");
@@ -3004,12 +3015,15 @@ k_dbc_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant__
           __syncwarp();
           if (lane == 0) mbar_arrive(&bars.acc_empty);
         }
-        st_global_32B(dC + o + j,
-                      make_uint4(pack_bf16(vc[0], vc[1]), pack_bf16(vc[2], vc[3]), pack_bf16(vc[4], vc[5]), pack_bf16(vc[6], vc[7])),
-                      make_uint4(pack_bf16(vc[8], vc[9]), pack_bf16(vc[10], vc[11]), pack_bf16(vc[12], vc[13]), pack_bf16(vc[14], vc[15])));
-        st_global_32B(dB + o + j,
-                      make_uint4(pack_bf16(vb[0], vb[1]), pack_bf16(vb[2], vb[3]), pack_bf16(vb[4], vb[5]), pack_bf16(vb[6], vb[7])),
-                      make_uint4(pack_bf16(vb[8], vb[9]), pack_bf16(vb[10], vb[11]), pack_bf16(vb[12], vb[13]), pack_bf16(vb[14], vb[15])));
+        if (c * QT + row < g.L) {   // a ragged sequence ends inside its last tile
+          st_global_32B(dC + o + j,
+                        make_uint4(pack_bf16(vc[0], vc[1]), pack_bf16(vc[2], vc[3]), pack_bf16(vc[4], vc[5]), pack_bf16(vc[6], vc[7])),
+                        make_uint4(pack_bf16(vc[8], vc[9]), pack_bf16(vc[10], vc[11]), pack_bf16(vc[12], vc[13]), pack_bf16(vc[14], vc[15])));
+          st_global_32B(dB + o + j,
+                        make_uint4(pack_bf16(vb[0], vb[1]), pack_bf16(vb[2], vb[3]), pack_bf16(vb[4], vb[5]), pack_bf16(vb[6], vb[7])),
+                        make_uint4(pack_bf16(vb[8], vb[9]), pack_bf16(vb[10], vb[11]), pack_bf16(vb[12], vb[13]), pack_bf16(vb[14], vb[15])));
+        }
+        __syncwarp();
       }
     }
   }
@@ -3327,12 +3341,12 @@ bool tensor_supported(const Geo& g, int dtype, const char** why) {
   auto no = [&](const char* m) { if (why) *why = m; return false; };
   if (dtype != SSD_BF16) return no("tensor-core kernels need bf16 storage");
   if (g.Q != QT) return no("tensor-core kernels need chunk == 128 (or a multiple of it)");
-  // A ragged tail costs the forward nothing: its loads zero-fill and its stores drop the rows past the end, and the cumsum
-  // kernel gives those positions a step size of zero.  The backward kernels store rows of their own.
-  if (g.L % QT && (!g.fwd_only || g.onetile)) return no("tensor-core kernels need seqlen % 128 == 0, except in a forward without a backward");
+  // A ragged tail costs nothing: loads zero-fill, stores drop the rows past the end, and the cumsum kernel gives those
+  // positions a step size of zero.  The one-tile kernels store unguarded rows.
+  if (g.L % QT && g.onetile) return no("the one-tile kernels need seqlen % 128 == 0");
   if (!((g.P == 32 || g.P == 64) && (g.N == 64 || g.N == 128))) return no("tensor-core kernels cover headdim in {32,64}, dstate in {64,128}");
   if ((g.hpg * g.P) % 128) return no("heads_per_group * headdim must be a multiple of 128");
-  if ((g.xsl % 8) || (g.xsb % 8) || (g.bsl % 8) || (g.bsb % 8) || (g.csl % 8) || (g.csb % 8) || (g.ysl % 8) || (g.ysb % 8) ||
+  if ((g.xsl % 8) || (g.xsb % 8) || (g.bsl % 8) || (g.bsb % 8) || (g.csl % 8) || (g.csb % 8) || (!g.any_y && ((g.ysl % 8) || (g.ysb % 8))) ||
       (g.zsl % 8) || (g.zsb % 8))
     return no("strides must be multiples of 8 elements (16 bytes) for TMA");
   return true;
@@ -3493,6 +3507,19 @@ int tensor_dbc(const Geo& g, const SsdBwdPtrs& p, const void* dyp, bool dy_dense
 #define CALL(PP, NN) return launch_dbc<PP, NN>(g, m, tab, hmax, p.dB, p.dC, status, s);
   DISPATCH_PN(CALL)
 #undef CALL
+}
+
+// y between the caller's strides and a dense buffer, for pointers or strides TMA cannot take (any alignment).
+__global__ void k_copy_y(Geo g, const bf16* __restrict__ src, bf16* __restrict__ dst) {
+  pdl_wait();
+  const int HP = g.H * g.P;
+  const size_t r = blockIdx.x, b = r / g.L, t = r - b * g.L;
+  for (int e = threadIdx.x; e < HP; e += blockDim.x) dst[b * g.ysb + t * g.ysl + e] = src[r * HP + e];
+}
+int tensor_copy_y(const Geo& g, const void* src, void* y, cudaStream_t s) {
+  launch<k_copy_y>((unsigned)((size_t)g.B * g.L), 128, 0, s, g, (const bf16*)src, (bf16*)y);
+  SSD_CUDA_CHECK_LAUNCH("copy_y");
+  return SSD_OK;
 }
 
 int tensor_selftest_wait(int* status, long long max_cycles, cudaStream_t s) {

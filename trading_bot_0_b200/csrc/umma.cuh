@@ -286,6 +286,18 @@ __device__ __forceinline__ float4 lds_v4f32(uint32_t addr) {
   asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
   return v;
 }
+// Warp-wide: every lane's shared-memory reads that `bits` depends on have returned; lane 0 gets true, the others false.  A
+// warp that hands a buffer back with an mbarrier arrive has to know that: the reads queue behind earlier stores to global
+// memory in the load/store pipe, the arrive does not.  With stores held up by address translation (freshly allocated
+// outputs) an arrive overtook reads by the whole time the producer took to refill the box, and four-row groups of the next
+// block's x were used (ddt of a few positions wrong in one call of a hundred).  The vote needs every lane's value, so it
+// cannot issue before the reads are back.
+__device__ __forceinline__ bool reads_done(uint32_t bits, int lane) {
+  uint32_t t;
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.u32 p, %1, 1;\n\tvote.sync.ballot.b32 %0, p, 0xffffffff;\n\t}"
+               : "=r"(t) : "r"(lane == 0 ? (bits & 0xfffffffeu) : bits) : "memory");
+  return lane == 0 && (t & 1u) == 0;   // bit 0 is clear: lane 0 votes on an even number
+}
 __device__ __forceinline__ uint4 ld_shared_v4(uint32_t addr) {
   uint4 v;
   asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
