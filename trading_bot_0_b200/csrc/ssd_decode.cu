@@ -152,29 +152,6 @@ __device__ __forceinline__ void tile_request(unsigned char* sm, const float* gst
     }
 }
 
-// The sums of R values over groups of LPR lanes, R values at a time: every exchange folds two values into one, so a tile row
-// set costs R - 1 + log2(LPR / R) shuffles instead of R log2(LPR).  Lane `lir` ends up with the sum of value `u` (returned);
-// all lanes whose lir agrees in its log2(R) top bits hold the same one.
-template <int LPR, int R>
-__device__ __forceinline__ float fold_rows(float (&v)[R], int lir, int& u) {
-  u = 0;
-  int o = LPR / 2;
-#pragma unroll
-  for (int n = R; n > 1; n >>= 1, o >>= 1) {
-    const bool up = lir & o;
-#pragma unroll
-    for (int i = 0; i < n / 2; ++i) {
-      const float keep = up ? v[n / 2 + i] : v[i], give = up ? v[i] : v[n / 2 + i];
-      v[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
-    }
-    u += up ? n / 2 : 0;
-  }
-  float t = v[0];
-#pragma unroll
-  for (; o; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-  return t;
-}
-
 // One tile: new state to global memory, `out(row, y)` called by one lane of every row.  sx: the tile's x, sB / sC: the group's
 // vectors, all in shared memory; a: the step's decay.
 template <class Tl, typename T, int N, class Out>

@@ -220,24 +220,24 @@ __device__ __forceinline__ size_t cb_idx(const Geo& g, int b, int c, int grp) {
 // step size after the optional bias / softplus, which every later stage reads from dtf or the decay tables.
 // One block per (chunk, batch): thread q reads the H contiguous dt values of position q once and
 // the block scans 8 heads at a time with warp shuffles.
-template <typename T>
+// HG heads at a time, as in k_ddt.
+template <typename T, int HG>
 __global__ void __launch_bounds__(256) k_cumsum(Geo g, const T* __restrict__ dt, const float* __restrict__ dt_bias,
                                                const float* __restrict__ A, float* __restrict__ cs,
                                                float* __restrict__ dtf, float* __restrict__ tab, int* __restrict__ hmax,
                                                int tag, int* __restrict__ status) {
   pdl_wait();
-  constexpr int HG = 8;
   const int c = blockIdx.x, b = blockIdx.y, q = threadIdx.x;
   __shared__ float wsum[8][HG];
   const int t = c * g.Q + q;
-  if (c == 0 && b == 0 && q == 0) {   // first kernel of a pass: the status word and the tag of this launch
+  if (c == 0 && b == 0 && blockIdx.z == 0 && q == 0) {   // first kernel of a pass: the status word and the tag of this launch
     *status = 0;
     if (hmax) hmax[g.H] = tag;
   }
   const bool live = (q < g.Q) && (t < g.L);
   const int lane = q & 31, w = q >> 5;
   const T* row = dt + b * g.dtsb + (long long)t * g.dtsl;
-  for (int h0 = 0; h0 < g.H; h0 += HG) {
+  for (int h0 = blockIdx.z * HG; h0 < g.H; h0 += HG * gridDim.z) {
     float d[HG], v[HG];
 #pragma unroll
     for (int k = 0; k < HG; ++k) {
@@ -819,20 +819,23 @@ __global__ void __launch_bounds__(ST) k_sdot(Geo g, const float* __restrict__ dS
 // 32-column strip of the chunk (strips; only those up to the position's own hold anything), one per 32 state columns, and one
 // part of ddtd per 32 features, `stride` elements apart.
 struct DdtParts { int strips, columns, features; size_t stride; };
+// HG heads at a time: 8 fill the sectors of a [B,L,H] row; 2 give a short batch four times the blocks (its time is one chain
+// of loads and scans).  PARTS: the CUDA-core family's partial sums (their loops cost the other family 30 of 60 us at 512 x
+// 1024 tokens of 8 heads).  The two sums over the chunk fold 2 HG values across the warp together: 16 shuffles instead of 80.
+template <int HG, bool PARTS>
 __global__ void __launch_bounds__(ST) k_ddt(Geo g, const float* __restrict__ A, const float* __restrict__ dtf,
                                             DdtParts parts, const float* __restrict__ dcsp,
                                             const float* __restrict__ ddtd, const float* __restrict__ ddot, const float* __restrict__ sdot, int nw,
                                             float* __restrict__ ddt, float* __restrict__ dapart,
                                             float* __restrict__ ddpart, float* __restrict__ dbpart) {
   pdl_wait();
-  constexpr int HG = 8;
   const int c = blockIdx.x, b = blockIdx.y, q = threadIdx.x;
-  __shared__ float wsum[ST / 32][HG], red1[ST / 32][HG], red2[ST / 32][HG], red3[ST / 32][HG], ssd[HG];
+  __shared__ float wsum[ST / 32][HG], red[ST / 32][2 * HG], red3[ST / 32][HG], ssd[HG];
   const int qr = g.Q - 1 - q;   // reversed position: an inclusive prefix scan over q is a suffix sum over qr
   const bool ok = (q < g.Q);
   const int lane = q & 31, w = q >> 5, nwarp = blockDim.x >> 5;   // launched with 128 threads when the chunk is <= 128 long
   const int t = c * g.Q + qr;
-  for (int h0 = 0; h0 < g.H; h0 += HG) {
+  for (int h0 = blockIdx.z * HG; h0 < g.H; h0 += HG * gridDim.z) {
     for (int hh = w; hh < HG; hh += nwarp) {   // a warp adds the partial sums of head h0 + hh (fixed order: lane-strided, then a butterfly)
       float s = 0.f;
       if (h0 + hh < g.H) {
@@ -843,7 +846,7 @@ __global__ void __launch_bounds__(ST) k_ddt(Geo g, const float* __restrict__ A, 
       for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
       if (lane == 0) ssd[hh] = s;
     }
-    float d[HG], dd[HG], v[HG], s2[HG];
+    float d[HG], dd[HG], v[HG], s12[2 * HG];   // s12: the dA terms, then the dD terms
 #pragma unroll
     for (int k = 0; k < HG; ++k) {
       const int h = h0 + k;
@@ -852,7 +855,7 @@ __global__ void __launch_bounds__(ST) k_ddt(Geo g, const float* __restrict__ A, 
       d[k] = live ? dtf[o] : 0.f;
       dd[k] = live ? ddtd[o] : 0.f;
       float dc = live ? dcsp[o] : 0.f;
-      if (live) {   // further parts, in a fixed order
+      if (PARTS && live) {   // further parts, in a fixed order
 #pragma unroll 4
         for (int s = 1; s < parts.features; ++s) dd[k] += ddtd[s * parts.stride + o];
         const int strips = min(parts.strips - 1, qr / TN);
@@ -862,7 +865,7 @@ __global__ void __launch_bounds__(ST) k_ddt(Geo g, const float* __restrict__ A, 
         for (int s = 0; s < parts.columns; ++s) dc += dcsp[(parts.strips + s) * parts.stride + o];
       }
       v[k] = live ? dc - d[k] * dd[k] : 0.f;
-      s2[k] = live ? ddot[o] : 0.f;
+      s12[HG + k] = live ? ddot[o] : 0.f;
     }
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -877,53 +880,42 @@ __global__ void __launch_bounds__(ST) k_ddt(Geo g, const float* __restrict__ A, 
       for (int k = 0; k < HG; ++k) wsum[w][k] = v[k];
     }
     __syncthreads();
-    float s1[HG];
 #pragma unroll
     for (int k = 0; k < HG; ++k) {
       float base = 0.f;
       for (int i = 0; i < w; ++i) base += wsum[i][k];
       const float da = v[k] + base + ssd[k];
-      s1[k] = ok ? d[k] * da : 0.f;
+      s12[k] = ok ? d[k] * da : 0.f;
       v[k] = dd[k] + ((h0 + k < g.H) ? A[h0 + k] : 0.f) * da;   // gradient w.r.t. the step size of this position
       // ... and through softplus to the dt that was passed in: softplus'(r) = sigmoid(r) = 1 - exp(-softplus(r))
       if (g.dt_softplus) v[k] *= 1.f - __expf(-d[k]);
     }
     if (ok && t < g.L) {
       float* o = ddt + ((size_t)b * g.L + t) * g.H + h0;
-      if (h0 + HG <= g.H && (reinterpret_cast<uintptr_t>(o) & 15) == 0) {
-        reinterpret_cast<float4*>(o)[0] = make_float4(v[0], v[1], v[2], v[3]);
-        reinterpret_cast<float4*>(o)[1] = make_float4(v[4], v[5], v[6], v[7]);
+      if (HG % 4 == 0 && h0 + HG <= g.H && (reinterpret_cast<uintptr_t>(o) & 15) == 0) {
+#pragma unroll
+        for (int k = 0; k + 3 < HG; k += 4) *reinterpret_cast<float4*>(o + k) = make_float4(v[k], v[k + 1], v[k + 2], v[k + 3]);
       } else {
 #pragma unroll
         for (int k = 0; k < HG; ++k)
           if (h0 + k < g.H) o[k] = v[k];
       }
     }
-#pragma unroll
-    for (int o = 16; o; o >>= 1) {
-#pragma unroll
-      for (int k = 0; k < HG; ++k) {
-        s1[k] += __shfl_xor_sync(0xffffffffu, s1[k], o);
-        s2[k] += __shfl_xor_sync(0xffffffffu, s2[k], o);
-      }
-    }
+    int which;
+    const float s = fold_rows<32, 2 * HG>(s12, lane, which);
+    if (lane % (32 / (2 * HG)) == 0) red[w][which] = s;
     if (dbpart) {   // the chunk's share of the step-size bias gradient
+      if (!(ok && t < g.L)) {
 #pragma unroll
-      for (int k = 0; k < HG; ++k) {
-        float s3 = (ok && t < g.L) ? v[k] : 0.f;
-#pragma unroll
-        for (int o = 16; o; o >>= 1) s3 += __shfl_xor_sync(0xffffffffu, s3, o);
-        if (lane == 0) red3[w][k] = s3;
+        for (int k = 0; k < HG; ++k) v[k] = 0.f;
       }
-    }
-    if (lane == 0) {
-#pragma unroll
-      for (int k = 0; k < HG; ++k) { red1[w][k] = s1[k]; red2[w][k] = s2[k]; }
+      const float s3 = fold_rows<32, HG>(v, lane, which);
+      if (lane % (32 / HG) == 0) red3[w][which] = s3;
     }
     __syncthreads();
     if (q < HG && h0 + q < g.H) {
       float a1 = 0.f, a2 = 0.f;
-      for (int i = 0; i < nwarp; ++i) { a1 += red1[i][q]; a2 += red2[i][q]; }
+      for (int i = 0; i < nwarp; ++i) { a1 += red[i][q]; a2 += red[i][HG + q]; }
       if (dbpart) {
         float a3 = 0.f;
         for (int i = 0; i < nwarp; ++i) a3 += red3[i][q];
@@ -975,6 +967,8 @@ __global__ void __launch_bounds__(RH_THREADS) k_reduce_heads(int rows, int H, co
 // =============================================================================================
 // Host launchers
 // =============================================================================================
+template <auto K> struct Fn { static constexpr auto value = K; };   // a kernel as a value of its own type
+
 // Blocks of the CUDA-core kernels (one tile each); pick_family has checked that they fit a grid.
 struct Tiles {
   unsigned state, cb, scan, bc;
@@ -1033,8 +1027,12 @@ static int fwd_stages_t(const Geo& g, bool tc, const SsdFwdPtrs& p, char* ws, co
     static std::atomic<int> launch_tag{1};
     int tag = launch_tag.fetch_add(1, std::memory_order_relaxed);
     if (tag == 0) tag = launch_tag.fetch_add(1, std::memory_order_relaxed);
-    launch<k_cumsum<T>>(dim3(g.nc, g.B), g.Q <= 128 ? 128 : 256, 0, s, g, (const T*)p.dt, p.dt_bias, p.A, cs, dtf, tc ? tab : nullptr,
-                        hmax, tag, status);
+    const bool wide = (long long)g.nc * g.B >= 2LL * sm_count();
+    auto cumsum = [&](auto kernel) {
+      launch<kernel.value>(dim3(g.nc, g.B, wide ? 1 : cdiv(g.H, 2)), g.Q <= 128 ? 128 : 256, 0, s, g, (const T*)p.dt, p.dt_bias, p.A, cs, dtf,
+                           tc ? tab : nullptr, hmax, tag, status);
+    };
+    wide ? cumsum(Fn<k_cumsum<T, 8>>()) : cumsum(Fn<k_cumsum<T, 2>>());
     SSD_CUDA_CHECK_LAUNCH("cumsum");
     if (tc && fused) {
       // chunk states and the scan over chunks run as one kernel in the FINISH stage
@@ -1200,7 +1198,13 @@ static int bwd_stages_t(const Geo& g, bool tc, const SsdBwdPtrs& p, char* ws, co
     }
     const DdtParts parts = tc ? DdtParts{1, 0, 1, 0} : DdtParts{n.strips, cdiv(g.N, TN), cdiv(g.P, TN), n.nq};
     float* dbpart = p.ddt_bias ? (float*)(ws + w.dbpart) : nullptr;
-    launch<k_ddt>(dim3(g.nc, g.B), g.Q <= 128 ? 128 : 256, 0, s, g, p.A, dtf, parts, dcsp, ddtd, ddot, sdot, sdot_nw, p.ddt, dapart, ddpart, dbpart);
+    const bool wide = (long long)g.nc * g.B >= 2LL * sm_count();   // eight heads per block fill the SMs twice
+    auto ddt = [&](auto kernel) {
+      launch<kernel.value>(dim3(g.nc, g.B, wide ? 1 : cdiv(g.H, 2)), g.Q <= 128 ? 128 : 256, 0, s, g, p.A, dtf, parts, dcsp, ddtd, ddot, sdot,
+                           sdot_nw, p.ddt, dapart, ddpart, dbpart);
+    };
+    if (tc) wide ? ddt(Fn<k_ddt<8, false>>()) : ddt(Fn<k_ddt<2, false>>());
+    else wide ? ddt(Fn<k_ddt<8, true>>()) : ddt(Fn<k_ddt<2, true>>());
     SSD_CUDA_CHECK_LAUNCH("ddt");
     launch<k_reduce_heads>(g.H, RH_THREADS, 0, s, g.B * g.nc, g.H, dapart, ddpart, dbpart, p.dA, p.dD, p.ddt_bias);
     SSD_CUDA_CHECK_LAUNCH("reduce_heads");
