@@ -699,58 +699,62 @@ __global__ void __launch_bounds__(PsCfg<P, N_>::THREADS, 1) k_state_ps(Geo g, co
 }
 
 // ---------------------------------------------------------------------------------------------
-// Chunk states AND the scan over chunks in one persistent kernel (dstate 64): k_state_ps with the work ordered so that
-// one CTA walks the chunks of a (batch, group, 128-row tile) unit in scan order and keeps the running state of its
-// 128 x 64 tile in registers (16 floats per thread).  The fp32 per-chunk states then never travel to memory and back
-// between two kernels: the epilogue of chunk c writes the state ENTERING the chunk (fp32 for the backward pass, bf16 for
-// the tensor-core scan kernels), then folds the chunk's own contribution in:  run = exp(sum of dt*A over c) * run + local_c.
+// Chunk states AND the scan over chunks in one persistent kernel: k_state_ps with the work ordered so that one CTA walks the
+// chunks of a (batch, group, 128-row tile) unit in scan order and keeps the running state of its 128 x N tile in registers
+// (N / 4 floats per thread).  The fp32 per-chunk states then never travel to memory and back between two kernels: the epilogue
+// of chunk c writes the state ENTERING the chunk (bf16, what the scan kernels load), then folds the chunk's own contribution
+// in:  run = exp(sum of dt*A over c) * run + local_c.
 //   MODE 0  forward:  units scan c = 0 .. nc-1 from `init` (or zero); `last` receives the final state.
 //   MODE 1  backward: c = nc-1 .. 0 from `init` = the gradient w.r.t. the final state (or zero); the value written for
-//           chunk c is the gradient w.r.t. the state LEAVING it (bf16 only: nothing reads an fp32 copy), and the epilogue
-//           also emits per-warp partial sums of <dS_end_c, S_end_c> (the per-chunk term of the dt*A gradient, S_end_c read
-//           from the forward pass's bf16 copy of the chunk-entry states, the fp32 final state for the last chunk), `nw` =
-//           4 * P / 32 partials per (batch, chunk, head) in `sdot`;
-//           `last` receives the gradient w.r.t. the initial state.
-// Pipeline and barriers as in k_state_ps; the B (or C) tile now changes with every tile, so it has a ring of its own.
-template <int P, int MODE>
+//           chunk c is the gradient w.r.t. the state LEAVING it, and the epilogue also emits per-warp partial sums of
+//           <dS_end_c, S_end_c> (the per-chunk term of the dt*A gradient, S_end_c read from the forward pass's bf16 copy of
+//           the chunk-entry states, the fp32 final state for the last chunk), `nw` = 4 * P / 32 partials per (batch, chunk,
+//           head) in `sdot`; `last` receives the gradient w.r.t. the initial state.
+// Where there are too few units to fill the SMs, the sequence is cut into `nseg` segments of `seglen` chunks: a first launch
+// (TOT) walks every segment but the last from a zero state and leaves its total and its decay, the second folds the totals
+// before its segment into the state it starts from.  x and B are then read twice; fp32 states per chunk, written and read
+// back by a kernel of their own, would be twice that again (dstate 128) and leave the scan to a few hundred warps.
+// Pipeline and barriers as in k_state_ps; the B (or C) tile changes with every tile, so it has a ring of its own.
+template <int P, int N_, int MODE, bool TOT>
 struct PfCfg {
-  // the backward kernel gives one slot of the x ring to the S_end tile (128 rows x 64: one 16 KB bf16 box, or for the last
-  // chunk the fp32 final state as two swizzled 16 KB boxes)
-  static constexpr int N = 64, HT = 128 / P, NX = MODE == 1 ? 3 : 4, NB = 3;
-  static constexpr int X_BYTES = 2 * BOX_BYTES;
+  // the backward kernel gives a slot of the x ring to the S_end tile (128 rows x N bf16: one or two 16 KB boxes)
+  static constexpr bool SE = MODE == 1 && !TOT;
+  static constexpr int N = N_, HT = 128 / P, NBX = N / 64, NX = (N == 64 ? 4 : 3) - (SE ? 1 : 0), NB = N == 64 ? 3 : 2;
+  static constexpr int X_BYTES = 2 * BOX_BYTES, B_BYTES = NBX * BOX_BYTES;
   static constexpr int TBH = 256;
   static constexpr int TB_BYTES = HT * TBH * 4;
-  static constexpr int SE_BYTES = MODE == 1 ? 2 * BOX_BYTES : 0;
-  static constexpr int W_MMA = 16, W_PROD = 17, W_PROD2 = 18, THREADS = (MODE == 1 ? 19 : 18) * 32;
+  static constexpr int SE_BYTES = SE ? B_BYTES : 0;
+  static constexpr int W_MMA = 16, W_PROD = 17, W_PROD2 = 18, THREADS = (SE ? 19 : 18) * 32;
   static constexpr int SDOT_NW = 4 * (P / 32);
-  static constexpr size_t SMEM = 1024 + NX * X_BYTES + X_BYTES + NB * BOX_BYTES + SE_BYTES + NX * TB_BYTES;
+  static constexpr int NQ = N / 64;   // 16-column slices per thread
+  static constexpr size_t SMEM = 1024 + NX * X_BYTES + X_BYTES + NB * B_BYTES + SE_BYTES + NX * TB_BYTES;
+  static_assert(SMEM <= 232448, "shared-memory plan exceeds the 227 KB a CTA can have");
 };
 
 struct StateScanArgs {
   const float* tab;
-  float* st;            // [B,nc,H,P,N] fp32 out, optional
   void* st_bf;          // [B,nc,H,P,N] bf16 out
   const float* init;    // [B,H,P,N] fp32, optional
   float *last, *last2;  // [B,H,P,N] fp32 out, both optional
   const void* fwd_prev_bf;  // MODE 1: bf16 copy of the forward pass's chunk-entry states (read through a tensor map)
   const float* fwd_fin;   // MODE 1: forward final state
   float* sdot;            // MODE 1: [B,nc,H,SDOT_NW]
+  int nseg, seglen;       // segments of the sequence, chunks in each (the last may be shorter)
+  float *tot, *tdec;      // [B,nseg,H,P,N] totals and [B,nseg,H] decays of the segments (nseg > 1)
 };
 
-template <int P, int MODE>
-__global__ void __launch_bounds__(PfCfg<P, MODE>::THREADS, 1) k_state_scan_ps(Geo g, const __grid_constant__ CUtensorMap tmX,
-                                                                              const __grid_constant__ CUtensorMap tmB,
-                                                                              const __grid_constant__ CUtensorMap tmS,
-                                                                              const __grid_constant__ CUtensorMap tmF,
-                                                                              StateScanArgs a, int* __restrict__ status) {
-  using Cfg = PfCfg<P, MODE>;
-  constexpr int N = Cfg::N, HT = Cfg::HT, NX = Cfg::NX, NB = Cfg::NB;
+template <int P, int N_, int MODE, bool TOT>
+__global__ void __launch_bounds__(PfCfg<P, N_, MODE, TOT>::THREADS, 1)
+k_state_scan_ps(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmB,
+                const __grid_constant__ CUtensorMap tmS, StateScanArgs a, int* __restrict__ status) {
+  using Cfg = PfCfg<P, N_, MODE, TOT>;
+  constexpr int N = Cfg::N, HT = Cfg::HT, NX = Cfg::NX, NB = Cfg::NB, NQ = Cfg::NQ;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);   // 1 KB aligned, still known to be shared memory
   uint8_t* sX = smem;                                  // NX x {two 64-column boxes}: the tile, scaled in place (high part)
   uint8_t* sL = sX + NX * Cfg::X_BYTES;                // low bf16 part of the tile being multiplied
   uint8_t* sB = sL + Cfg::X_BYTES;                     // NB x B (or C) tile
-  uint8_t* sSE = sB + NB * BOX_BYTES;                  // MODE 1: S_end of the tile whose epilogue comes next (128B swizzle)
+  uint8_t* sSE = sB + NB * Cfg::B_BYTES;               // S_end of the tile whose epilogue comes next (128B swizzle)
   uint8_t* sTabs = sSE + Cfg::SE_BYTES;                // NX x the table sections of a tile's heads
   __shared__ __align__(8) uint64_t x_full[NX], x_free[NX], b_full[NB], b_free[NB], half_ready[2], h0_done, mma_done[2], acc_empty[2],
       se_full, se_free;
@@ -766,7 +770,7 @@ __global__ void __launch_bounds__(PfCfg<P, MODE>::THREADS, 1) k_state_scan_ps(Ge
     mbar_init(&se_full, 1); mbar_init(&se_free, 16);
     mbar_fence_init();
   }
-  if (warp == 1) tmem_alloc(&tmem_slot, 128);
+  if (warp == 1) tmem_alloc(&tmem_slot, 2 * N);
   pdl_wait();
   if (tid == 0) s_abort = *(volatile int*)status;   // an earlier kernel gave up
   tc_fence_before();
@@ -774,67 +778,72 @@ __global__ void __launch_bounds__(PfCfg<P, MODE>::THREADS, 1) k_state_scan_ps(Ge
   tc_fence_after();
   const uint32_t tm = tmem_slot;
   if (s_abort) {
-    if (warp == 1) tmem_dealloc(tm, 128);
+    if (warp == 1) tmem_dealloc(tm, 2 * N);
     return;
   }
   Waiter w{status, false};
-  const bool want_sdot = MODE == 1 && a.sdot != nullptr;
+  const bool want_sdot = Cfg::SE && a.sdot != nullptr;
 
   const int MT = g.hpg * P / 128;
-  const int nunits = g.B * g.G * MT;
-  const int my_units = (nunits - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
-  const int total = my_units * g.nc;
-  auto coords = [&](int n, int& b, int& grp, int& mt) {   // this CTA's n-th unit; neighbouring units share a B/C tile
-    const int u = blockIdx.x + n * gridDim.x;
-    mt = u % MT;
-    const int r = u / MT;
-    grp = r % g.G;
-    b = r / g.G;
+  const int nunits = g.B * g.G * MT * (TOT ? a.nseg - 1 : a.nseg);
+  // This CTA's tiles in order: the chunks of a unit in scan order, unit after unit; neighbouring units share a B/C tile.
+  struct Walk {
+    const Geo& g;
+    int MT, nunits, seglen, u, b, grp, mt, seg, s, s1;
+    __device__ __forceinline__ Walk(const Geo& g_, int MT_, int nunits_, int seglen_)
+        : g(g_), MT(MT_), nunits(nunits_), seglen(seglen_), u(blockIdx.x) { place(); }
+    __device__ __forceinline__ void place() {
+      mt = u % MT;
+      int r = u / MT;
+      grp = r % g.G; r /= g.G;
+      b = r % g.B;
+      seg = r / g.B;
+      s = seg * seglen;
+      s1 = min(s + seglen, g.nc);
+    }
+    __device__ __forceinline__ bool more() const { return u < nunits; }
+    __device__ __forceinline__ void next() {
+      if (++s == s1) { u += gridDim.x; place(); }
+    }
+    __device__ __forceinline__ bool begins() const { return s == seg * seglen; }
+    __device__ __forceinline__ bool ends() const { return s + 1 == s1; }
+    __device__ __forceinline__ int chunk() const { return MODE == 0 ? s : g.nc - 1 - s; }
   };
-  auto chunk_of = [&](int s) { return MODE == 0 ? s : g.nc - 1 - s; };
 
   if (warp == Cfg::W_PROD) {
     if (lane == 0) {
-      int n = 0, sidx = 0, b = 0, grp = 0, mt = 0;
-      for (int k = 0; k < total; ++k) {
-        if (sidx == 0) coords(n, b, grp, mt);
-        const int c = chunk_of(sidx);
-        const int slot = k % NX, bs = k % NB;
+      Walk t(g, MT, nunits, a.seglen);
+      for (int k = 0; t.more(); ++k, t.next()) {
+        const int c = t.chunk(), slot = k % NX, bs = k % NB;
         if (k >= NX) w.wait(&x_free[slot], ((k / NX) - 1) & 1, 14);
-        const int col = grp * g.hpg * P + mt * 128;
+        const int col = t.grp * g.hpg * P + t.mt * 128;
         mbar_expect_tx(&x_full[slot], Cfg::X_BYTES + Cfg::TB_BYTES);
-        tma_load_3d(sX + slot * Cfg::X_BYTES, &tmX, col, c * QT, b, &x_full[slot]);
-        tma_load_3d(sX + slot * Cfg::X_BYTES + BOX_BYTES, &tmX, col + 64, c * QT, b, &x_full[slot]);
-        const float* t0 = a.tab + ((size_t)(b * g.nc + c) * g.H + grp * g.hpg + mt * HT) * TAB;
+        tma_load_3d(sX + slot * Cfg::X_BYTES, &tmX, col, c * QT, t.b, &x_full[slot]);
+        tma_load_3d(sX + slot * Cfg::X_BYTES + BOX_BYTES, &tmX, col + 64, c * QT, t.b, &x_full[slot]);
+        const float* t0 = a.tab + ((size_t)(t.b * g.nc + c) * g.H + t.grp * g.hpg + t.mt * HT) * TAB;
         for (int hl = 0; hl < HT; ++hl)
           bulk_load(sTabs + slot * Cfg::TB_BYTES + hl * Cfg::TBH * 4, t0 + (size_t)hl * TAB, Cfg::TBH * 4, &x_full[slot]);
         if (k >= NB) w.wait(&b_free[bs], ((k / NB) - 1) & 1, 15);
-        mbar_expect_tx(&b_full[bs], BOX_BYTES);
-        tma_load_3d(sB + bs * BOX_BYTES, &tmB, grp * N, c * QT, b, &b_full[bs]);
-        if (++sidx == g.nc) { sidx = 0; ++n; }
+        mbar_expect_tx(&b_full[bs], Cfg::B_BYTES);
+        for (int j = 0; j < Cfg::NBX; ++j)
+          tma_load_3d(sB + bs * Cfg::B_BYTES + j * BOX_BYTES, &tmB, t.grp * N + 64 * j, c * QT, t.b, &b_full[bs]);
       }
     }
     __syncwarp();
-  } else if (MODE == 1 && warp == Cfg::W_PROD2) {
-    // second producer lane: the forward state leaving chunk c (= entering chunk c+1, or the final state), one tile ahead of
-    // the epilogue that multiplies it with the running gradient
+  } else if (Cfg::SE && warp == Cfg::W_PROD2) {
+    // second producer lane: the forward state leaving chunk c = the bf16 copy of the state entering chunk c + 1, one tile
+    // ahead of the epilogue that multiplies it with the running gradient (the last chunk's is the fp32 final state, which
+    // the epilogue reads itself)
     if (lane == 0 && want_sdot) {
-      int n = 0, sidx = 0, b = 0, grp = 0, mt = 0;
-      for (int k = 0; k < total; ++k) {
-        if (sidx == 0) coords(n, b, grp, mt);
-        const int c = chunk_of(sidx);
-        const int h0 = grp * g.hpg + mt * HT;
+      int k = 0;
+      for (Walk t(g, MT, nunits, a.seglen); t.more(); t.next()) {
+        const int c = t.chunk();
+        if (c + 1 >= g.nc) continue;
         if (k >= 1) w.wait(&se_free, (k - 1) & 1, 20);
-        if (c + 1 >= g.nc) {   // the forward's final state: fp32, two boxes of 32 columns
-          const int row0 = (b * g.H + h0) * P;
-          mbar_expect_tx(&se_full, 2 * BOX_BYTES);
-          tma_load_3d(sSE, &tmF, 0, row0, 0, &se_full);
-          tma_load_3d(sSE + BOX_BYTES, &tmF, 32, row0, 0, &se_full);
-        } else {               // the bf16 copy of the state entering chunk c + 1: one box of 64 columns
-          mbar_expect_tx(&se_full, BOX_BYTES);
-          tma_load_3d(sSE, &tmS, 0, ((b * g.nc + c + 1) * g.H + h0) * P, 0, &se_full);
-        }
-        if (++sidx == g.nc) { sidx = 0; ++n; }
+        mbar_expect_tx(&se_full, Cfg::SE_BYTES);
+        for (int j = 0; j < Cfg::NBX; ++j)
+          tma_load_3d(sSE + j * BOX_BYTES, &tmS, 64 * j, ((t.b * g.nc + c + 1) * g.H + t.grp * g.hpg + t.mt * HT) * P, 0, &se_full);
+        ++k;
       }
     }
     __syncwarp();
@@ -842,11 +851,12 @@ __global__ void __launch_bounds__(PfCfg<P, MODE>::THREADS, 1) k_state_scan_ps(Ge
     if (lane == 0) {
       const uint32_t idesc = make_idesc(128, N, 1, 1);
       const uint64_t dL0 = desc_sw128_mn(smem_u32(sL), 0, 0, BOX_BYTES);
-      for (int k = 0; k < total; ++k) {
+      Walk t(g, MT, nunits, a.seglen);
+      for (int k = 0; t.more(); ++k, t.next()) {
         const int slot = k % NX, bs = k % NB;
         const uint64_t dX0 = desc_sw128_mn(smem_u32(sX + slot * Cfg::X_BYTES), 0, 0, BOX_BYTES),
-                       dB0 = desc_sw128_mn(smem_u32(sB + bs * BOX_BYTES), 0, 0, BOX_BYTES);
-        const uint32_t acc = tm + (k & 1) * 64;
+                       dB0 = desc_sw128_mn(smem_u32(sB + bs * Cfg::B_BYTES), 0, 0, BOX_BYTES);
+        const uint32_t acc = tm + (k & 1) * N;
         w.wait(&b_full[bs], (k / NB) & 1, 12);
         if (k >= 2) w.wait(&acc_empty[k & 1], ((k >> 1) - 1) & 1, 16);
         w.wait(&half_ready[0], k & 1, 17);
@@ -897,90 +907,110 @@ __global__ void __launch_bounds__(PfCfg<P, MODE>::THREADS, 1) k_state_scan_ps(Ge
       __syncwarp();
       if (lane == 0) mbar_arrive(&half_ready[h]);
     };
-    float run[16];          // running state of this thread's (row, 16 columns)
-    struct Tile { int b, grp, mt, s; };
-    auto elem = [&](const Tile& t) {   // offset of this thread's 16 columns inside a [.., H, P, N] state
-      return ((size_t)(t.grp * g.hpg + t.mt * HT) * P + row) * N + part * 16;
+    float run[16 * NQ];          // running state of this thread's (row, N / 4 columns)
+    float pdec = 1.f;            // TOT: decay of the row's head over the chunks of the segment so far
+    int kse = 0;
+    auto put = [&](float* to) {
+#pragma unroll
+      for (int j = 0; j < 16 * NQ; j += 8)
+        st_global_32B(to + j, make_uint4(__float_as_uint(run[j]), __float_as_uint(run[j + 1]), __float_as_uint(run[j + 2]), __float_as_uint(run[j + 3])),
+                      make_uint4(__float_as_uint(run[j + 4]), __float_as_uint(run[j + 5]), __float_as_uint(run[j + 6]), __float_as_uint(run[j + 7])));
     };
-    auto epilogue = [&](int k, const Tile& t, float dec) {
-      const int c = chunk_of(t.s);
-      const size_t e = elem(t), bstate = (size_t)t.b * g.H * P * N;
-      if (t.s == 0) {
-        if (a.init) {
+    auto epilogue = [&](int k, const Walk& t, float dec) {
+      const int c = t.chunk(), h = t.grp * g.hpg + t.mt * HT + row / P;
+      const size_t PNH = (size_t)g.H * P * N;
+      const size_t e = ((size_t)(t.grp * g.hpg + t.mt * HT) * P + row) * N + part * (N / PARTS);   // inside a [.., H, P, N] state
+      float acc[16 * NQ];
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const float4 v4 = *reinterpret_cast<const float4*>(a.init + bstate + e + 4 * j);
-            run[4 * j] = v4.x; run[4 * j + 1] = v4.y; run[4 * j + 2] = v4.z; run[4 * j + 3] = v4.w;
-          }
-        } else {
+      for (int q = 0; q < NQ; ++q) {
+        float v[16];
+        tmem_ld16(tmem_addr(tm + (k & 1) * N, (warp & 3) * 32, part * (N / PARTS) + 16 * q), v);
 #pragma unroll
-          for (int j = 0; j < 16; ++j) run[j] = 0.f;
-        }
+        for (int j = 0; j < 16; ++j) acc[16 * q + j] = v[j];
       }
-      float v[16];
-      tmem_ld16(tmem_addr(tm + (k & 1) * 64, (warp & 3) * 32, part * 16), v);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&acc_empty[k & 1]);
-      const size_t o = (size_t)(t.b * g.nc + c) * g.H * P * N + e;
-      if (a.st) {
+      if (t.begins()) {
+        if (!TOT && a.init) {
 #pragma unroll
-        for (int j = 0; j < 16; j += 8)
-          st_global_32B(a.st + o + j, make_uint4(__float_as_uint(run[j]), __float_as_uint(run[j + 1]), __float_as_uint(run[j + 2]), __float_as_uint(run[j + 3])),
-                        make_uint4(__float_as_uint(run[j + 4]), __float_as_uint(run[j + 5]), __float_as_uint(run[j + 6]), __float_as_uint(run[j + 7])));
+          for (int j = 0; j < 16 * NQ; j += 4) {
+            const float4 v = *reinterpret_cast<const float4*>(a.init + t.b * PNH + e + j);
+            run[j] = v.x; run[j + 1] = v.y; run[j + 2] = v.z; run[j + 3] = v.w;
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < 16 * NQ; ++j) run[j] = 0.f;
+        }
+        pdec = 1.f;
+        if constexpr (!TOT) {
+          for (int sg = 0; sg < t.seg; ++sg) {   // the segments before this one
+            const size_t i = (size_t)t.b * a.nseg + sg;
+            const float d = a.tdec[i * g.H + h];
+#pragma unroll
+            for (int j = 0; j < 16 * NQ; j += 4) {
+              const float4 v = *reinterpret_cast<const float4*>(a.tot + i * PNH + e + j);
+              run[j] = fmaf(d, run[j], v.x); run[j + 1] = fmaf(d, run[j + 1], v.y);
+              run[j + 2] = fmaf(d, run[j + 2], v.z); run[j + 3] = fmaf(d, run[j + 3], v.w);
+            }
+          }
+        }
       }
-      st_global_32B((bf16*)a.st_bf + o,
-                    make_uint4(pack_bf16(run[0], run[1]), pack_bf16(run[2], run[3]), pack_bf16(run[4], run[5]), pack_bf16(run[6], run[7])),
-                    make_uint4(pack_bf16(run[8], run[9]), pack_bf16(run[10], run[11]), pack_bf16(run[12], run[13]), pack_bf16(run[14], run[15])));
+      if constexpr (!TOT) {
+        bf16* o = (bf16*)a.st_bf + (size_t)(t.b * g.nc + c) * PNH + e;
+#pragma unroll
+        for (int j = 0; j < 16 * NQ; j += 16)
+          st_global_32B(o + j,
+                        make_uint4(pack_bf16(run[j], run[j + 1]), pack_bf16(run[j + 2], run[j + 3]), pack_bf16(run[j + 4], run[j + 5]), pack_bf16(run[j + 6], run[j + 7])),
+                        make_uint4(pack_bf16(run[j + 8], run[j + 9]), pack_bf16(run[j + 10], run[j + 11]), pack_bf16(run[j + 12], run[j + 13]), pack_bf16(run[j + 14], run[j + 15])));
+      }
       if (want_sdot) {
-        w.wait(&se_full, k & 1, 21);
         float d = 0.f;
         if (c + 1 >= g.nc) {   // block-uniform: the final state, fp32
-          const uint32_t sb = smem_u32(sSE) + (part >> 1) * BOX_BYTES;
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const uint4 u = ld_shared_v4(sb + sw128_off(row, (part & 1) * 4 + j));
-            d += run[4 * j] * __uint_as_float(u.x) + run[4 * j + 1] * __uint_as_float(u.y) + run[4 * j + 2] * __uint_as_float(u.z) +
-                 run[4 * j + 3] * __uint_as_float(u.w);
+          for (int j = 0; j < 16 * NQ; j += 4) {
+            const float4 f = *reinterpret_cast<const float4*>(a.fwd_fin + t.b * PNH + e + j);
+            d += run[j] * f.x + run[j + 1] * f.y + run[j + 2] * f.z + run[j + 3] * f.w;
           }
-        } else {               // the bf16 copy: this thread's 16 columns are two 16-byte pieces of its row
+        } else {               // the bf16 copy: this thread's columns are 16-byte pieces of its row
+          w.wait(&se_full, kse & 1, 21);
+          ++kse;
+          const uint32_t sb = smem_u32(sSE) + ((part * (N / PARTS)) / 64) * BOX_BYTES;
 #pragma unroll
-          for (int j = 0; j < 2; ++j) {
-            const uint4 u = ld_shared_v4(smem_u32(sSE) + sw128_off(row, part * 2 + j));
+          for (int j = 0; j < 2 * NQ; ++j) {
+            const uint4 u = ld_shared_v4(sb + sw128_off(row, ((part * (N / PARTS)) % 64) / 8 + j));
             const uint32_t q[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
             for (int i = 0; i < 4; ++i)
               d += run[8 * j + 2 * i] * __uint_as_float(q[i] << 16) + run[8 * j + 2 * i + 1] * __uint_as_float(q[i] & 0xffff0000u);
           }
+          if (reads_done(__float_as_uint(d), lane)) mbar_arrive(&se_free);
         }
-        if (reads_done(__float_as_uint(d), lane)) mbar_arrive(&se_free);
 #pragma unroll
         for (int off = 16; off; off >>= 1) d += __shfl_xor_sync(0xffffffffu, d, off);
-        if (lane == 0) {
-          const int q = warp & 3;                                  // 32-row quarter of the tile
-          const int h = t.grp * g.hpg + t.mt * HT + (q * 32) / P;
-          const int slot = part * (P / 32) + q % (P / 32);
+        if (lane == 0) {   // the warp's 32 rows belong to one head
+          const int slot = part * (P / 32) + (warp & 3) % (P / 32);
           a.sdot[((size_t)(t.b * g.nc + c) * g.H + h) * Cfg::SDOT_NW + slot] = d;
         }
       }
 #pragma unroll
-      for (int j = 0; j < 16; ++j) run[j] = fmaf(dec, run[j], v[j]);
-      if (t.s == g.nc - 1) {
-        auto put = [&](float* to) {
-#pragma unroll
-          for (int j = 0; j < 16; j += 8)
-            st_global_32B(to + bstate + e + j, make_uint4(__float_as_uint(run[j]), __float_as_uint(run[j + 1]), __float_as_uint(run[j + 2]), __float_as_uint(run[j + 3])),
-                          make_uint4(__float_as_uint(run[j + 4]), __float_as_uint(run[j + 5]), __float_as_uint(run[j + 6]), __float_as_uint(run[j + 7])));
-        };
-        if (a.last) put(a.last);
-        if (a.last2) put(a.last2);
+      for (int j = 0; j < 16 * NQ; ++j) run[j] = fmaf(dec, run[j], acc[j]);
+      if (TOT) pdec *= dec;
+      if (t.ends()) {
+        if constexpr (TOT) {
+          const size_t i = (size_t)t.b * a.nseg + t.seg;
+          put(a.tot + i * PNH + e);
+          if (part == 0 && row % P == 0) a.tdec[i * g.H + h] = pdec;
+        } else if (t.seg == a.nseg - 1) {
+          if (a.last) put(a.last + t.b * PNH + e);
+          if (a.last2) put(a.last2 + t.b * PNH + e);
+        }
       }
     };
-    Tile cur{0, 0, 0, 0}, prev{0, 0, 0, 0};
-    int n = 0;
+    Walk cur(g, MT, nunits, a.seglen), prev = cur;
     float dec_prev = 0.f;
-    for (int k = 0; k < total; ++k) {
-      if (cur.s == 0) coords(n, cur.b, cur.grp, cur.mt);
+    int k = 0;
+    for (; cur.more(); ++k) {
       const int slot = k % NX;
       const uint32_t xs = smem_u32(sX + slot * Cfg::X_BYTES);
       const float* tb = (const float*)(sTabs + slot * Cfg::TB_BYTES);
@@ -993,18 +1023,20 @@ __global__ void __launch_bounds__(PfCfg<P, MODE>::THREADS, 1) k_state_scan_ps(Ge
         tc_fence_after();
       }
       scale_half(1, xs, tb);
-      if (k > 0) epilogue(k - 1, prev, dec_prev);
-      prev = cur;
+      if (k > 0) {
+        epilogue(k - 1, prev, dec_prev);
+        prev.next();
+      }
       dec_prev = dec;
-      if (++cur.s == g.nc) { cur.s = 0; ++n; }
+      cur.next();
     }
-    w.wait(&mma_done[(total - 1) & 1], ((total - 1) >> 1) & 1, 13);
+    w.wait(&mma_done[(k - 1) & 1], ((k - 1) >> 1) & 1, 13);
     tc_fence_after();
-    epilogue(total - 1, prev, dec_prev);
+    epilogue(k - 1, prev, dec_prev);
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 1) tmem_dealloc(tm, 128);
+  if (warp == 1) tmem_dealloc(tm, 2 * N);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -3165,20 +3197,6 @@ int make_map3(CUtensorMap* m, const void* ptr, long long d0, long long d1, long 
   if (r != CUDA_SUCCESS) { set_error("cuTensorMapEncodeTiled(%s) failed with CUresult %d", what, (int)r); return SSD_ERR_CUDA; }
   return SSD_OK;
 }
-// fp32 [rows, 64] state rows (dstate 64), 128B swizzle: box = 32 columns (128 bytes) x 128 rows
-int make_f32_rows_map(CUtensorMap* m, const float* ptr, long long rows, const char* what) {
-  EncodeFn enc = get_encode();
-  if (!enc) { set_error("cuTensorMapEncodeTiled is not available from the driver"); return SSD_ERR_CUDA; }
-  cuuint64_t dims[3] = {64, (cuuint64_t)rows, 1};
-  cuuint64_t strides[2] = {64 * 4, (cuuint64_t)rows * 64 * 4};
-  cuuint32_t box[3] = {32, 128, 1};
-  cuuint32_t es[3] = {1, 1, 1};
-  CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(ptr), dims, strides, box, es,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) { set_error("cuTensorMapEncodeTiled(%s) failed with CUresult %d", what, (int)r); return SSD_ERR_CUDA; }
-  return SSD_OK;
-}
 // [batch, seqlen, cols] sequence tensor: box = 64 cols x 128 rows
 int make_seq_map(CUtensorMap* m, const void* ptr, long long cols, long long L, long long B, long long stride_l,
                  long long stride_b, const char* what) {
@@ -3392,41 +3410,63 @@ int tensor_chunk_state(const Geo& g, int mode, const void* xdy, long long sb, lo
 #undef CALL
 }
 
-// Chunk states and the scan over chunks in one launch (see k_state_scan_ps): dstate 64, persistent family.
-bool tensor_state_fused_applies(const Geo& g) { return g.N == 64 && !g.onetile; }
+// Chunk states and the scan over chunks together (see k_state_scan_ps): the persistent family, unstaged passes.
+bool tensor_state_fused_applies(const Geo& g) { return !g.onetile; }
 
-template <int P, int MODE>
-static int launch_state_scan(const Geo& g, const CUtensorMap& tx, const CUtensorMap& tb, const CUtensorMap& ts, const CUtensorMap& tf,
-                             const StateScanArgs& a, int* status, cudaStream_t s) {
-  const int nunits = g.B * g.G * (g.hpg * P / 128);
-  const int grid = nunits < sm_count() ? nunits : sm_count();
-  launch<k_state_scan_ps<P, MODE>>(grid, PfCfg<P, MODE>::THREADS, PfCfg<P, MODE>::SMEM, s, g, tx, tb, ts, tf, a, status);
+// Segments of the sequence.  A launch takes (units per CTA, rounded up) x (chunks of a segment) steps; cutting costs a second
+// launch over all segments but the last, whose steps are 0.7 of the others' (nothing is written), the launch itself (about
+// three steps) and a fold per segment.  Many units: one segment.  Fewer than 16 chunks: one segment as well, the second launch
+// would cost what it saves, and a row's result then does not depend on how many rows the call has.
+static int state_segments(const Geo& g, int units) {
+  const int sms = sm_count();
+  if (g.nc < 16) return 1;
+  int best = 1;
+  double least = 1e30;
+  for (int n = 1; n <= g.nc / 2; ++n) {
+    const int len = cdiv(g.nc, n), seg = cdiv(g.nc, len);
+    const double t = (double)cdiv(units * seg, sms) * len + (seg > 1 ? 0.7 * cdiv(units * (seg - 1), sms) * len + 3 + 0.3 * seg : 0.);
+    if (t < least) { least = t; best = n; }
+    if ((long long)units * n > 4LL * sms) break;
+  }
+  return best;
+}
+
+template <int P, int N, int MODE>
+static int launch_state_scan(const Geo& g, const CUtensorMap& tx, const CUtensorMap& tb, const CUtensorMap& ts, const StateScanArgs& a,
+                             int* status, cudaStream_t s) {
+  const int units = g.B * g.G * (g.hpg * P / 128), n1 = units * (a.nseg - 1), n2 = units * a.nseg;
+  if (n1) {
+    using C1 = PfCfg<P, N, MODE, true>;
+    launch<k_state_scan_ps<P, N, MODE, true>>(n1 < sm_count() ? n1 : sm_count(), C1::THREADS, C1::SMEM, s, g, tx, tb, ts, a, status);
+    SSD_CUDA_CHECK_LAUNCH(MODE == 0 ? "chunk_state_totals" : "dstate_totals");
+  }
+  using C2 = PfCfg<P, N, MODE, false>;
+  launch<k_state_scan_ps<P, N, MODE, false>>(n2 < sm_count() ? n2 : sm_count(), C2::THREADS, C2::SMEM, s, g, tx, tb, ts, a, status);
   SSD_CUDA_CHECK_LAUNCH(MODE == 0 ? "chunk_state_scan" : "dstate_scan");
   return SSD_OK;
 }
 
 int tensor_state_fused(const Geo& g, int mode, const void* xdy, long long sb, long long sl, const void* bc, long long bsb,
-                       long long bsl, const float* tab, float* st, void* st_bf, const float* init, float* last, float* last2,
+                       long long bsl, const float* tab, float* scratch, void* st_bf, const float* init, float* last, float* last2,
                        const void* fwd_prev_bf, const float* fwd_fin, float* sdot, int* sdot_nw, int* status, cudaStream_t s) {
   CUtensorMap tx, tb;
   int rc = make_seq_map(&tx, xdy, (long long)g.H * g.P, g.L, g.B, sl, sb, "x/dy");
   if (rc) return rc;
   rc = make_seq_map(&tb, bc, (long long)g.G * g.N, g.L, g.B, bsl, bsb, "B/C");
   if (rc) return rc;
-  StateScanArgs a{tab, st, st_bf, init, last, last2, fwd_prev_bf, fwd_fin, sdot};
+  const int seglen = cdiv(g.nc, state_segments(g, g.B * g.G * (g.hpg * g.P / 128))), nseg = cdiv(g.nc, seglen);
+  const size_t PNH = (size_t)g.H * g.P * g.N;
+  StateScanArgs a{tab, st_bf, init, last, last2, fwd_prev_bf, fwd_fin, sdot, nseg, seglen, scratch, scratch + (size_t)g.B * nseg * PNH};
   if (sdot_nw) *sdot_nw = 4 * (g.P / 32);
-  CUtensorMap ts = tx, tf = tx;   // placeholders unless the backward kernel reads the forward states
+  CUtensorMap ts = tx;   // a placeholder unless the backward kernel reads the forward states
   if (mode == 1 && sdot) {
-    const long long rows = (long long)g.B * g.nc * g.H * g.P;   // bf16 [rows, 64]: boxes of 128 rows x 64 columns
-    rc = make_map3(&ts, fwd_prev_bf, 64, rows, 1, 64, rows * 64, 128, "forward chunk-entry states (bf16 copy)");
-    if (rc) return rc;
-    rc = make_f32_rows_map(&tf, fwd_fin, (long long)g.B * g.H * g.P, "forward final state");
+    const long long rows = (long long)g.B * g.nc * g.H * g.P;   // bf16 [rows, N]: boxes of 128 rows x 64 columns
+    rc = make_map3(&ts, fwd_prev_bf, g.N, rows, 1, g.N, rows * g.N, 128, "forward chunk-entry states (bf16 copy)");
     if (rc) return rc;
   }
-  if (g.P == 32) return mode == 0 ? launch_state_scan<32, 0>(g, tx, tb, ts, tf, a, status, s) : launch_state_scan<32, 1>(g, tx, tb, ts, tf, a, status, s);
-  if (g.P == 64) return mode == 0 ? launch_state_scan<64, 0>(g, tx, tb, ts, tf, a, status, s) : launch_state_scan<64, 1>(g, tx, tb, ts, tf, a, status, s);
-  set_error("tensor_state_fused: unsupported headdim %d", g.P);
-  return SSD_ERR_UNSUPPORTED;
+#define CALL(PP, NN) return mode == 0 ? launch_state_scan<PP, NN, 0>(g, tx, tb, ts, a, status, s) : launch_state_scan<PP, NN, 1>(g, tx, tb, ts, a, status, s);
+  DISPATCH_PN(CALL)
+#undef CALL
 }
 
 int tensor_chunk_scan(const Geo& g, const SsdFwdPtrs& p, const float* tab, const void* prev_bf, int* status,
