@@ -233,3 +233,28 @@ def test_ragged_operands_of_any_alignment(lib, which, N):
     assert_close("final_state", fin, ref["final_state"], "bf16")
     for k in ("dx", "ddt", "dB", "dC", "dD", "dinit"):
         assert_close(k, g[k], ref[k], "bf16")
+
+
+@pytest.mark.parametrize("L", [1921, 2304, 4200])
+@pytest.mark.parametrize("H,P,N,G", [(8, 32, 64, 1), (4, 64, 128, 2), (12, 64, 128, 1)])
+def test_segmented_state_scan_matches_oracle(lib, L, H, P, N, G):
+    """Few units and many chunks: the state scans run in segments (a shorter last segment, a last chunk of one token)."""
+    import trading_bot_0_b200 as T
+    Bn = 2
+    cfg = O.SsdConfig("seg", Bn, L, H, P, N, G, 128, "bf16", False)
+    inp = O.make_inputs(cfg, with_init_state=True)
+    dfinal = 0.1 * torch.randn(Bn, H, P, N, generator=torch.Generator().manual_seed(4))
+    ref = oracle_all(inp, dfinal)
+    d = to_dev(inp, DEV)
+    y, fin, ws = T.forward(d["x"], d["dt"], d["A"], d["B"], d["C"], d.get("D"), None, d["init_state"], chunk=128, for_backward=True)
+    g = T.backward(d["dy"], d["x"], d["dt"], d["A"], d["B"], d["C"], d.get("D"), None, d["init_state"], dfinal.to(DEV),
+                   chunk=128, workspace=ws, fwd_saved=True, want_dinit=True)
+    torch.cuda.synchronize()
+    assert status_word(ws) == 0
+    assert_close("y", y, ref["y"], "bf16")
+    assert_close("final_state", fin, ref["final_state"], "bf16")
+    for k in GRADS + ("dinit",):
+        if k == "dA":
+            assert_close_dA_few_rows(k, g[k], ref[k])
+        else:
+            assert_close(k, g[k], ref[k], "bf16")

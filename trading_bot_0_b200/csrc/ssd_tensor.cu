@@ -717,17 +717,17 @@ __global__ void __launch_bounds__(PsCfg<P, N_>::THREADS, 1) k_state_ps(Geo g, co
 // Pipeline and barriers as in k_state_ps; the B (or C) tile changes with every tile, so it has a ring of its own.
 template <int P, int N_, int MODE, bool TOT>
 struct PfCfg {
-  // the backward kernel gives a slot of the x ring to the S_end tile (128 rows x N bf16: one or two 16 KB boxes)
+  // the backward kernel gives a slot of the x ring to the S_end tiles (128 rows x N bf16: one or two 16 KB boxes each)
   static constexpr bool SE = MODE == 1 && !TOT;
   static constexpr int N = N_, HT = 128 / P, NBX = N / 64, NX = (N == 64 ? 4 : 3) - (SE ? 1 : 0), NB = N == 64 ? 3 : 2;
   static constexpr int X_BYTES = 2 * BOX_BYTES, B_BYTES = NBX * BOX_BYTES;
   static constexpr int TBH = 256;
   static constexpr int TB_BYTES = HT * TBH * 4;
-  static constexpr int SE_BYTES = SE ? B_BYTES : 0;
+  static constexpr int SE_BYTES = SE ? B_BYTES : 0, NSE = N == 64 ? 2 : 1;   // S_end tiles in flight
   static constexpr int W_MMA = 16, W_PROD = 17, W_PROD2 = 18, THREADS = (SE ? 19 : 18) * 32;
   static constexpr int SDOT_NW = 4 * (P / 32);
   static constexpr int NQ = N / 64;   // 16-column slices per thread
-  static constexpr size_t SMEM = 1024 + NX * X_BYTES + X_BYTES + NB * B_BYTES + SE_BYTES + NX * TB_BYTES;
+  static constexpr size_t SMEM = 1024 + NX * X_BYTES + X_BYTES + NB * B_BYTES + NSE * SE_BYTES + NX * TB_BYTES;
   static_assert(SMEM <= 232448, "shared-memory plan exceeds the 227 KB a CTA can have");
 };
 
@@ -748,16 +748,16 @@ __global__ void __launch_bounds__(PfCfg<P, N_, MODE, TOT>::THREADS, 1)
 k_state_scan_ps(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmB,
                 const __grid_constant__ CUtensorMap tmS, StateScanArgs a, int* __restrict__ status) {
   using Cfg = PfCfg<P, N_, MODE, TOT>;
-  constexpr int N = Cfg::N, HT = Cfg::HT, NX = Cfg::NX, NB = Cfg::NB, NQ = Cfg::NQ;
+  constexpr int N = Cfg::N, HT = Cfg::HT, NX = Cfg::NX, NB = Cfg::NB, NQ = Cfg::NQ, NSE = Cfg::NSE;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);   // 1 KB aligned, still known to be shared memory
   uint8_t* sX = smem;                                  // NX x {two 64-column boxes}: the tile, scaled in place (high part)
   uint8_t* sL = sX + NX * Cfg::X_BYTES;                // low bf16 part of the tile being multiplied
   uint8_t* sB = sL + Cfg::X_BYTES;                     // NB x B (or C) tile
-  uint8_t* sSE = sB + NB * Cfg::B_BYTES;               // S_end of the tile whose epilogue comes next (128B swizzle)
-  uint8_t* sTabs = sSE + Cfg::SE_BYTES;                // NX x the table sections of a tile's heads
+  uint8_t* sSE = sB + NB * Cfg::B_BYTES;               // NSE x S_end tile (128B swizzle), one per epilogue
+  uint8_t* sTabs = sSE + NSE * Cfg::SE_BYTES;                // NX x the table sections of a tile's heads
   __shared__ __align__(8) uint64_t x_full[NX], x_free[NX], b_full[NB], b_free[NB], half_ready[2], h0_done, mma_done[2], acc_empty[2],
-      se_full, se_free;
+      se_full[NSE], se_free[NSE];
   __shared__ uint32_t tmem_slot;
   __shared__ int s_abort;
 
@@ -767,7 +767,7 @@ k_state_scan_ps(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_con
     for (int i = 0; i < NB; ++i) { mbar_init(&b_full[i], 1); mbar_init(&b_free[i], 1); }
     for (int i = 0; i < 2; ++i) { mbar_init(&half_ready[i], 16); mbar_init(&mma_done[i], 1); mbar_init(&acc_empty[i], 16); }
     mbar_init(&h0_done, 1);
-    mbar_init(&se_full, 1); mbar_init(&se_free, 16);
+    for (int i = 0; i < NSE; ++i) { mbar_init(&se_full[i], 1); mbar_init(&se_free[i], 16); }
     mbar_fence_init();
   }
   if (warp == 1) tmem_alloc(&tmem_slot, 2 * N);
@@ -784,43 +784,45 @@ k_state_scan_ps(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_con
   Waiter w{status, false};
   const bool want_sdot = Cfg::SE && a.sdot != nullptr;
 
-  const int MT = g.hpg * P / 128;
-  const int nunits = g.B * g.G * MT * (TOT ? a.nseg - 1 : a.nseg);
   // This CTA's tiles in order: the chunks of a unit in scan order, unit after unit; neighbouring units share a B/C tile.
+  // (Few members: the consumers hold one beside the running state.)
+  const int nunits = g.B * g.G * (g.hpg * P / 128) * (TOT ? a.nseg - 1 : a.nseg);
   struct Walk {
-    const Geo& g;
-    int MT, nunits, seglen, u, b, grp, mt, seg, s, s1;
-    __device__ __forceinline__ Walk(const Geo& g_, int MT_, int nunits_, int seglen_)
-        : g(g_), MT(MT_), nunits(nunits_), seglen(seglen_), u(blockIdx.x) { place(); }
-    __device__ __forceinline__ void place() {
-      mt = u % MT;
+    int u, b, h0, grp, seg, s, s1;
+    __device__ __forceinline__ Walk(const Geo& g, const StateScanArgs& a) : u(blockIdx.x) { place(g, a); }
+    __device__ __forceinline__ void place(const Geo& g, const StateScanArgs& a) {
+      const int MT = g.hpg * P / 128;
       int r = u / MT;
+      h0 = (u - r * MT) * HT;
       grp = r % g.G; r /= g.G;
+      h0 += grp * g.hpg;
       b = r % g.B;
       seg = r / g.B;
-      s = seg * seglen;
-      s1 = min(s + seglen, g.nc);
+      s = seg * a.seglen;
+      s1 = min(s + a.seglen, g.nc);
     }
-    __device__ __forceinline__ bool more() const { return u < nunits; }
-    __device__ __forceinline__ void next() {
-      if (++s == s1) { u += gridDim.x; place(); }
+    __device__ __forceinline__ void next(const Geo& g, const StateScanArgs& a) {
+      if (++s == s1) { u += gridDim.x; place(g, a); }
     }
-    __device__ __forceinline__ bool begins() const { return s == seg * seglen; }
-    __device__ __forceinline__ bool ends() const { return s + 1 == s1; }
-    __device__ __forceinline__ int chunk() const { return MODE == 0 ? s : g.nc - 1 - s; }
+    __device__ __forceinline__ int chunk(const Geo& g) const { return MODE == 0 ? s : g.nc - 1 - s; }
   };
+  int total = 0;   // tiles of this CTA
+  for (int u = blockIdx.x; u < nunits; u += gridDim.x) {
+    const int s0 = u / (nunits / (TOT ? a.nseg - 1 : a.nseg)) * a.seglen;
+    total += min(a.seglen, g.nc - s0);
+  }
 
   if (warp == Cfg::W_PROD) {
     if (lane == 0) {
-      Walk t(g, MT, nunits, a.seglen);
-      for (int k = 0; t.more(); ++k, t.next()) {
-        const int c = t.chunk(), slot = k % NX, bs = k % NB;
+      Walk t(g, a);
+      for (int k = 0; k < total; ++k, t.next(g, a)) {
+        const int c = t.chunk(g), slot = k % NX, bs = k % NB;
         if (k >= NX) w.wait(&x_free[slot], ((k / NX) - 1) & 1, 14);
-        const int col = t.grp * g.hpg * P + t.mt * 128;
+        const int col = t.h0 * P;
         mbar_expect_tx(&x_full[slot], Cfg::X_BYTES + Cfg::TB_BYTES);
         tma_load_3d(sX + slot * Cfg::X_BYTES, &tmX, col, c * QT, t.b, &x_full[slot]);
         tma_load_3d(sX + slot * Cfg::X_BYTES + BOX_BYTES, &tmX, col + 64, c * QT, t.b, &x_full[slot]);
-        const float* t0 = a.tab + ((size_t)(t.b * g.nc + c) * g.H + t.grp * g.hpg + t.mt * HT) * TAB;
+        const float* t0 = a.tab + ((size_t)(t.b * g.nc + c) * g.H + t.h0) * TAB;
         for (int hl = 0; hl < HT; ++hl)
           bulk_load(sTabs + slot * Cfg::TB_BYTES + hl * Cfg::TBH * 4, t0 + (size_t)hl * TAB, Cfg::TBH * 4, &x_full[slot]);
         if (k >= NB) w.wait(&b_free[bs], ((k / NB) - 1) & 1, 15);
@@ -836,13 +838,15 @@ k_state_scan_ps(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_con
     // the epilogue reads itself)
     if (lane == 0 && want_sdot) {
       int k = 0;
-      for (Walk t(g, MT, nunits, a.seglen); t.more(); t.next()) {
-        const int c = t.chunk();
+      Walk t(g, a);
+      for (int n = 0; n < total; ++n, t.next(g, a)) {
+        const int c = t.chunk(g);
         if (c + 1 >= g.nc) continue;
-        if (k >= 1) w.wait(&se_free, (k - 1) & 1, 20);
-        mbar_expect_tx(&se_full, Cfg::SE_BYTES);
+        const int slot = k % NSE;
+        if (k >= NSE) w.wait(&se_free[slot], ((k / NSE) - 1) & 1, 20);
+        mbar_expect_tx(&se_full[slot], Cfg::SE_BYTES);
         for (int j = 0; j < Cfg::NBX; ++j)
-          tma_load_3d(sSE + j * BOX_BYTES, &tmS, 64 * j, ((t.b * g.nc + c + 1) * g.H + t.grp * g.hpg + t.mt * HT) * P, 0, &se_full);
+          tma_load_3d(sSE + slot * Cfg::SE_BYTES + j * BOX_BYTES, &tmS, 64 * j, ((t.b * g.nc + c + 1) * g.H + t.h0) * P, 0, &se_full[slot]);
         ++k;
       }
     }
@@ -851,8 +855,7 @@ k_state_scan_ps(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_con
     if (lane == 0) {
       const uint32_t idesc = make_idesc(128, N, 1, 1);
       const uint64_t dL0 = desc_sw128_mn(smem_u32(sL), 0, 0, BOX_BYTES);
-      Walk t(g, MT, nunits, a.seglen);
-      for (int k = 0; t.more(); ++k, t.next()) {
+      for (int k = 0; k < total; ++k) {
         const int slot = k % NX, bs = k % NB;
         const uint64_t dX0 = desc_sw128_mn(smem_u32(sX + slot * Cfg::X_BYTES), 0, 0, BOX_BYTES),
                        dB0 = desc_sw128_mn(smem_u32(sB + bs * Cfg::B_BYTES), 0, 0, BOX_BYTES);
@@ -917,21 +920,10 @@ k_state_scan_ps(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_con
                       make_uint4(__float_as_uint(run[j + 4]), __float_as_uint(run[j + 5]), __float_as_uint(run[j + 6]), __float_as_uint(run[j + 7])));
     };
     auto epilogue = [&](int k, const Walk& t, float dec) {
-      const int c = t.chunk(), h = t.grp * g.hpg + t.mt * HT + row / P;
+      const int c = t.chunk(g);
       const size_t PNH = (size_t)g.H * P * N;
-      const size_t e = ((size_t)(t.grp * g.hpg + t.mt * HT) * P + row) * N + part * (N / PARTS);   // inside a [.., H, P, N] state
-      float acc[16 * NQ];
-#pragma unroll
-      for (int q = 0; q < NQ; ++q) {
-        float v[16];
-        tmem_ld16(tmem_addr(tm + (k & 1) * N, (warp & 3) * 32, part * (N / PARTS) + 16 * q), v);
-#pragma unroll
-        for (int j = 0; j < 16; ++j) acc[16 * q + j] = v[j];
-      }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&acc_empty[k & 1]);
-      if (t.begins()) {
+      const size_t e = ((size_t)t.h0 * P + row) * N + part * (N / PARTS);   // this thread's columns inside a [.., H, P, N] state
+      if (t.s == t.seg * a.seglen) {
         if (!TOT && a.init) {
 #pragma unroll
           for (int j = 0; j < 16 * NQ; j += 4) {
@@ -946,7 +938,7 @@ k_state_scan_ps(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_con
         if constexpr (!TOT) {
           for (int sg = 0; sg < t.seg; ++sg) {   // the segments before this one
             const size_t i = (size_t)t.b * a.nseg + sg;
-            const float d = a.tdec[i * g.H + h];
+            const float d = a.tdec[i * g.H + t.h0 + row / P];
 #pragma unroll
             for (int j = 0; j < 16 * NQ; j += 4) {
               const float4 v = *reinterpret_cast<const float4*>(a.tot + i * PNH + e + j);
@@ -956,61 +948,74 @@ k_state_scan_ps(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_con
           }
         }
       }
-      if constexpr (!TOT) {
-        bf16* o = (bf16*)a.st_bf + (size_t)(t.b * g.nc + c) * PNH + e;
+      const bool tail = c + 1 >= g.nc;   // MODE 1: this chunk's S_end is the final state, fp32
+      float d = 0.f;
 #pragma unroll
-        for (int j = 0; j < 16 * NQ; j += 16)
-          st_global_32B(o + j,
-                        make_uint4(pack_bf16(run[j], run[j + 1]), pack_bf16(run[j + 2], run[j + 3]), pack_bf16(run[j + 4], run[j + 5]), pack_bf16(run[j + 6], run[j + 7])),
-                        make_uint4(pack_bf16(run[j + 8], run[j + 9]), pack_bf16(run[j + 10], run[j + 11]), pack_bf16(run[j + 12], run[j + 13]), pack_bf16(run[j + 14], run[j + 15])));
+      for (int q = 0; q < NQ; ++q) {     // 16 columns at a time: one slice of the accumulator in registers
+        float* r = run + 16 * q;
+        float v[16];
+        tmem_ld16(tmem_addr(tm + (k & 1) * N, (warp & 3) * 32, part * (N / PARTS) + 16 * q), v);
+        if (q + 1 == NQ) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&acc_empty[k & 1]);
+        }
+        if constexpr (!TOT)
+          st_global_32B((bf16*)a.st_bf + (size_t)(t.b * g.nc + c) * PNH + e + 16 * q,
+                        make_uint4(pack_bf16(r[0], r[1]), pack_bf16(r[2], r[3]), pack_bf16(r[4], r[5]), pack_bf16(r[6], r[7])),
+                        make_uint4(pack_bf16(r[8], r[9]), pack_bf16(r[10], r[11]), pack_bf16(r[12], r[13]), pack_bf16(r[14], r[15])));
+        if (want_sdot) {
+          if (q == 0 && !tail) w.wait(&se_full[kse % NSE], (kse / NSE) & 1, 21);
+          if (tail) {
+            if (a.init) {   // else the running gradient is still zero, and the reads (nothing fetched them ahead) are not needed
+#pragma unroll
+              for (int j = 0; j < 16; j += 4) {
+                const float4 f = *reinterpret_cast<const float4*>(a.fwd_fin + t.b * PNH + e + 16 * q + j);
+                d += r[j] * f.x + r[j + 1] * f.y + r[j + 2] * f.z + r[j + 3] * f.w;
+              }
+            }
+          } else {   // the bf16 copy: this thread's columns are 16-byte pieces of its row
+            const uint32_t sb = smem_u32(sSE) + (kse % NSE) * Cfg::SE_BYTES + ((part * (N / PARTS)) / 64) * BOX_BYTES;
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+              const uint4 u = ld_shared_v4(sb + sw128_off(row, ((part * (N / PARTS)) % 64) / 8 + 2 * q + j));
+              const uint32_t uw[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+              for (int i = 0; i < 4; ++i)
+                d += r[8 * j + 2 * i] * __uint_as_float(uw[i] << 16) + r[8 * j + 2 * i + 1] * __uint_as_float(uw[i] & 0xffff0000u);
+            }
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < 16; ++j) r[j] = fmaf(dec, r[j], v[j]);
       }
       if (want_sdot) {
-        float d = 0.f;
-        if (c + 1 >= g.nc) {   // block-uniform: the final state, fp32
-#pragma unroll
-          for (int j = 0; j < 16 * NQ; j += 4) {
-            const float4 f = *reinterpret_cast<const float4*>(a.fwd_fin + t.b * PNH + e + j);
-            d += run[j] * f.x + run[j + 1] * f.y + run[j + 2] * f.z + run[j + 3] * f.w;
-          }
-        } else {               // the bf16 copy: this thread's columns are 16-byte pieces of its row
-          w.wait(&se_full, kse & 1, 21);
+        if (!tail) {
+          if (reads_done(__float_as_uint(d), lane)) mbar_arrive(&se_free[kse % NSE]);
           ++kse;
-          const uint32_t sb = smem_u32(sSE) + ((part * (N / PARTS)) / 64) * BOX_BYTES;
-#pragma unroll
-          for (int j = 0; j < 2 * NQ; ++j) {
-            const uint4 u = ld_shared_v4(sb + sw128_off(row, ((part * (N / PARTS)) % 64) / 8 + j));
-            const uint32_t q[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-              d += run[8 * j + 2 * i] * __uint_as_float(q[i] << 16) + run[8 * j + 2 * i + 1] * __uint_as_float(q[i] & 0xffff0000u);
-          }
-          if (reads_done(__float_as_uint(d), lane)) mbar_arrive(&se_free);
         }
 #pragma unroll
         for (int off = 16; off; off >>= 1) d += __shfl_xor_sync(0xffffffffu, d, off);
         if (lane == 0) {   // the warp's 32 rows belong to one head
           const int slot = part * (P / 32) + (warp & 3) % (P / 32);
-          a.sdot[((size_t)(t.b * g.nc + c) * g.H + h) * Cfg::SDOT_NW + slot] = d;
+          a.sdot[((size_t)(t.b * g.nc + c) * g.H + t.h0 + row / P) * Cfg::SDOT_NW + slot] = d;
         }
       }
-#pragma unroll
-      for (int j = 0; j < 16 * NQ; ++j) run[j] = fmaf(dec, run[j], acc[j]);
       if (TOT) pdec *= dec;
-      if (t.ends()) {
+      if (t.s + 1 == t.s1) {
         if constexpr (TOT) {
           const size_t i = (size_t)t.b * a.nseg + t.seg;
           put(a.tot + i * PNH + e);
-          if (part == 0 && row % P == 0) a.tdec[i * g.H + h] = pdec;
+          if (part == 0 && row % P == 0) a.tdec[i * g.H + t.h0 + row / P] = pdec;
         } else if (t.seg == a.nseg - 1) {
           if (a.last) put(a.last + t.b * PNH + e);
           if (a.last2) put(a.last2 + t.b * PNH + e);
         }
       }
     };
-    Walk cur(g, MT, nunits, a.seglen), prev = cur;
+    Walk prev(g, a);
     float dec_prev = 0.f;
-    int k = 0;
-    for (; cur.more(); ++k) {
+    for (int k = 0; k < total; ++k) {
       const int slot = k % NX;
       const uint32_t xs = smem_u32(sX + slot * Cfg::X_BYTES);
       const float* tb = (const float*)(sTabs + slot * Cfg::TB_BYTES);
@@ -1025,14 +1030,13 @@ k_state_scan_ps(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_con
       scale_half(1, xs, tb);
       if (k > 0) {
         epilogue(k - 1, prev, dec_prev);
-        prev.next();
+        prev.next(g, a);
       }
       dec_prev = dec;
-      cur.next();
     }
-    w.wait(&mma_done[(k - 1) & 1], ((k - 1) >> 1) & 1, 13);
+    w.wait(&mma_done[(total - 1) & 1], ((total - 1) >> 1) & 1, 13);
     tc_fence_after();
-    epilogue(k - 1, prev, dec_prev);
+    epilogue(total - 1, prev, dec_prev);
   }
   tc_fence_before();
   __syncthreads();
