@@ -258,3 +258,28 @@ def test_segmented_state_scan_matches_oracle(lib, L, H, P, N, G):
             assert_close_dA_few_rows(k, g[k], ref[k])
         else:
             assert_close(k, g[k], ref[k], "bf16")
+
+
+@pytest.mark.parametrize("H,P,N,G,Bn", [(6, 64, 64, 1, 35), (18, 64, 128, 1, 40), (12, 32, 64, 1, 60)])
+@pytest.mark.parametrize("has_z", [False, True])
+def test_split_heads_are_the_same_bits(lib, H, P, N, G, Bn, has_z):
+    """The scan kernels cut a group's heads into parts by the number of tiles: a few rows alone (many parts) match the oracle,
+    and the rows of a larger batch (fewer parts, an odd number of head blocks in each) match them bit for bit."""
+    import trading_bot_0_b200 as T
+    inp = O.make_inputs(O.SsdConfig("split", Bn, 256, H, P, N, G, 128, "bf16", has_z))
+    per_row = ("x", "dt", "B", "C", "z", "dy")
+
+    def run(v):
+        d = to_dev(v, DEV)
+        a = (d["x"], d["dt"], d["A"], d["B"], d["C"], d["D"], d.get("z"))
+        y, _, ws = T.forward(*a, chunk=128, algo="tensor", for_backward=True)
+        g = T.backward(d["dy"], *a, chunk=128, algo="tensor", workspace=ws, fwd_saved=True)
+        torch.cuda.synchronize()
+        assert status_word(ws) == 0
+        return {"y": y, **g}
+
+    few = {k: (v[:2].contiguous() if k in per_row and v is not None else v) for k, v in inp.items()}
+    got, ref, whole = run(few), oracle_all(few), run(inp)
+    for k in ("y", "dx", "ddt", "dB", "dC") + (("dz",) if has_z else ()):
+        assert_close(k, got[k], ref[k], "bf16")
+        assert torch.equal(got[k], whole[k][:2]), k

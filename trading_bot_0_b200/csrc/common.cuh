@@ -22,6 +22,7 @@ struct Geo {
   int dt_softplus;                     // step size = softplus(dt + dt_bias) instead of dt + dt_bias
   int any_y;                           // y / dy need not suit TMA: the caller takes care of them (see Plan in ssd_api.cu)
   int onetile;                         // tensor family: the one-tile-per-CTA kernels for every shape (SSD_ALGO_TENSOR_ONETILE)
+  int hsplit = 1;                      // scan kernels: G and hpg describe parts of a group, `hsplit` to the group (see split_heads)
 };
 
 // The step-size pre-activation of a Mamba-2 layer, fused where dt is first read.  Above 20 softplus is the

@@ -1935,8 +1935,8 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         mbar_expect_tx(&bars.cb_full[cs_], Cfg::CB_BYTES);
 #pragma unroll
         for (int j = 0; j < NB64; ++j) {
-          tma_load_3d(keep + j * BOX_BYTES, (MODE == 2) ? &tmB : &tmC, grp * N + 64 * j, c * QT, b, &bars.cb_full[cs_]);
-          tma_load_3d(keep + (NB64 + j) * BOX_BYTES, (MODE == 2) ? &tmC : &tmB, grp * N + 64 * j, c * QT, b, &bars.cb_full[cs_]);
+          tma_load_3d(keep + j * BOX_BYTES, (MODE == 2) ? &tmB : &tmC, grp / g.hsplit * N + 64 * j, c * QT, b, &bars.cb_full[cs_]);
+          tma_load_3d(keep + (NB64 + j) * BOX_BYTES, (MODE == 2) ? &tmC : &tmB, grp / g.hsplit * N + 64 * j, c * QT, b, &bars.cb_full[cs_]);
         }
       };
       const int total_blocks = my_tiles * nblk;
@@ -2381,8 +2381,8 @@ k_bwd_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant__
         mbar_expect_tx(&bars.cb_full[cs_], Cfg::CB_BYTES);
 #pragma unroll
         for (int j = 0; j < NB64; ++j) {
-          tma_load_3d(dst + j * BOX_BYTES, &tmC, grp * N + 64 * j, c * QT, b, &bars.cb_full[cs_]);
-          tma_load_3d(dst + (NB64 + j) * BOX_BYTES, &tmB, grp * N + 64 * j, c * QT, b, &bars.cb_full[cs_]);
+          tma_load_3d(dst + j * BOX_BYTES, &tmC, grp / g.hsplit * N + 64 * j, c * QT, b, &bars.cb_full[cs_]);
+          tma_load_3d(dst + (NB64 + j) * BOX_BYTES, &tmB, grp / g.hsplit * N + 64 * j, c * QT, b, &bars.cb_full[cs_]);
         }
       };
       const int total_blocks = my_tiles * nblk;
@@ -3253,12 +3253,35 @@ struct SeqMaps {
   CUtensorMap z;       // the gate (forward of the persistent scan kernel)
 };
 
+// The persistent scan kernels walk tiles of (batch, group, chunk), a tile's heads in blocks of HB.  Where the tiles do not divide
+// evenly over the SMs, or are fewer, the heads of a group are cut into parts and a tile is (batch, part, chunk): the part's C/B
+// load and its G = C B^T (about one block's time) are repeated, which a better-filled last wave or the otherwise idle SMs repay.
+// A part keeps at least two blocks, so that its products still overlap.  Heads do not interact: results are the same bits.
+// 16x4096, 24 heads: 512 tiles = 3.46 waves of 148 become 1024 half tiles = 6.92.
+template <int HB>
+Geo split_heads(const Geo& g) {
+  const int nblk = g.hpg / HB, tiles = g.B * g.G * g.nc, sms = sm_count();
+  int best = 1;
+  if (tiles < 32 * sms) {   // beyond, the last wave is no more than a thirtieth of the time
+    int least = cdiv(tiles, sms) * (nblk + 1);
+    for (int n = 2; nblk / n >= 2; ++n) {
+      if (nblk % n) continue;
+      const int t = cdiv(tiles * n, sms) * (nblk / n + 1);
+      if (t < least) { least = t; best = n; }
+    }
+  }
+  Geo s = g;
+  s.G *= best; s.hpg /= best; s.hsplit = best;
+  return s;
+}
+
 template <int P, int MODE, int N, bool GATED = false>
-int launch_scan_ws(const Geo& g, const SeqMaps& m, const CUtensorMap& ts, const ScanArgs& a, int* status, cudaStream_t s) {
+int launch_scan_ws(const Geo& geo, const SeqMaps& m, const CUtensorMap& ts, const ScanArgs& a, int* status, cudaStream_t s) {
   if constexpr (!GATED && MODE != 2) {
-    if (a.z) return launch_scan_ws<P, MODE, N, true>(g, m, ts, a, status, s);
+    if (a.z) return launch_scan_ws<P, MODE, N, true>(geo, m, ts, a, status, s);
   }
   using Cfg = WsCfg<P, MODE, N, GATED>;
+  const Geo g = split_heads<64 / P>(geo);
   const int ntiles = g.B * g.G * g.nc;
   const int grid = ntiles < sm_count() ? ntiles : sm_count();
   launch<k_scan_ws<P, MODE, N, GATED>>(grid, Cfg::THREADS, Cfg::SMEM, s, g, m.x, m.dy, m.b, m.c, ts, m.out, m.z, a.tab, a.D,
@@ -3281,8 +3304,9 @@ int launch_scan(const Geo& g, const SeqMaps& m, const CUtensorMap& ts, const Sca
 }
 
 template <int P, int N = 64>
-int launch_bwd_ws(const Geo& g, const SeqMaps& m, const float* tab, const float* D, void* dx, float* dcsp, float* ddot,
+int launch_bwd_ws(const Geo& geo, const SeqMaps& m, const float* tab, const float* D, void* dx, float* dcsp, float* ddot,
                   float* ddtd, int* status, cudaStream_t s) {
+  const Geo g = split_heads<64 / P>(geo);
   const int ntiles = g.B * g.G * g.nc;
   const int grid = ntiles < sm_count() ? ntiles : sm_count();
   launch<k_bwd_ws<P, N>>(grid, WS_THREADS, BwCfg<P, N>::SMEM, s, g, m.x, m.dy, m.b, m.c, m.s, m.ds, tab, D, (bf16*)dx, dcsp, ddot, ddtd,
