@@ -3069,6 +3069,295 @@ k_dbc_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant__
 }
 
 // ---------------------------------------------------------------------------------------------
+// dB, dC at dstate 128, persistent and warp-specialised; the arithmetic of k_dbc_tc with SUMW (the decayed tiles W'_h of a
+// group's heads are summed in registers, the sum is multiplied with B and C once per tile).  k_dbc_tc walks the heads with all
+// of its warps in one phase after another (product, decay, scaling, state products: 2.6 us per head where the operands of a
+// head need 1.5 us of memory time); here the phases of neighbouring heads overlap:
+//   * warp 16: TMA.  A ring of three 32 KB slots holds {x box, dy box} of a head block, and after a tile's last block its C
+//     tile and its B tile (needed once, at the end of the tile: a buffer of their own would cost a slot); a ring of two for the
+//     {S_prev, dS_end} boxes, one of four for the decay tables;
+//   * warp 17: MMA issue.  W products one block ahead into two accumulators, state products, and the tile's two products;
+//   * warps 0-15: W -> decay -> register sum (thread = row x 32 columns) -> the M tile;
+//   * warps 20-27: scale the boxes in place for the state products, and drain dC / dB of a finished tile.
+// TMEM: two W accumulators, dC, dB = 512 columns.  2x131072, 24 heads: 0.97 -> 0.64 ms = 5.1 TB/s, what a pure TMA stream of
+// boxes reaches; 16x4096: 0.27 -> 0.19 ms (3.46 waves of tiles take the time of four).
+template <int P>
+struct DsCfg {
+  static constexpr int N = 128, HB = 64 / P, NT = 4, NIN = 3, NST = 2;
+  static constexpr int IN_BYTES = 2 * BOX_BYTES;             // x box, dy box; or the C (B) tile
+  static constexpr int ST_BYTES = 4 * SBOX_BYTES;            // S_prev, dS_end: two boxes each
+  static constexpr int TB_BYTES = HB * TAB_BYTES;
+  static constexpr int W_SCALE = 20, NSCALE = 8;
+  static constexpr size_t SMEM = 1024 + 2 * BOX_BYTES + NIN * IN_BYTES + NST * ST_BYTES + NT * TB_BYTES;
+  static_assert(SMEM <= 232448 - 512, "shared-memory plan exceeds the 227 KB a CTA can have");
+};
+
+template <int P>
+__global__ void __launch_bounds__(WS_THREADS, 1)
+k_dbc_sum_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmDY,
+             const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmC,
+             const __grid_constant__ CUtensorMap tmS, const __grid_constant__ CUtensorMap tmDS,
+             const float* __restrict__ tab, bf16* __restrict__ dB, bf16* __restrict__ dC, int* __restrict__ status) {
+  using Cfg = DsCfg<P>;
+  constexpr int N = Cfg::N, HB = Cfg::HB, NIN = Cfg::NIN, NST = Cfg::NST, NT = Cfg::NT;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);   // 1 KB aligned, still known to be shared memory
+  uint8_t* sM = smem;                                    // the masked sum of a tile's W'_h
+  uint8_t* sIn = sM + 2 * BOX_BYTES;                     // NIN x {x box, dy box} or {C tile} or {B tile}
+  uint8_t* sSt = sIn + NIN * Cfg::IN_BYTES;              // NST x {S_prev, dS_end}
+  uint8_t* sTab = sSt + NST * Cfg::ST_BYTES;             // NT x decay tables of a head block
+  __shared__ __align__(8) uint64_t in_full[NIN], in_empty[NIN], raw_done[NIN], sc_full[NIN], st_full[NST], st_empty[NST], tab_full[NT],
+      tab_empty[NT], w_full[2], w_empty[2], m_full, m_empty, acc_full, acc_empty;
+  __shared__ uint32_t tmem_slot;
+  __shared__ int s_abort;
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (tid == 0) {
+    for (int i = 0; i < NIN; ++i) {
+      mbar_init(&in_full[i], 1); mbar_init(&in_empty[i], 1);
+      mbar_init(&raw_done[i], 1); mbar_init(&sc_full[i], Cfg::NSCALE);
+    }
+    for (int i = 0; i < NST; ++i) { mbar_init(&st_full[i], 1); mbar_init(&st_empty[i], 1); }
+    for (int i = 0; i < NT; ++i) { mbar_init(&tab_full[i], 1); mbar_init(&tab_empty[i], 16 + Cfg::NSCALE); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&w_full[i], 1); mbar_init(&w_empty[i], 16); }
+    mbar_init(&m_full, 16); mbar_init(&m_empty, 1);
+    mbar_init(&acc_full, 1); mbar_init(&acc_empty, Cfg::NSCALE);
+    mbar_fence_init();
+  }
+  if (warp == 17) tmem_alloc(&tmem_slot, 512);
+  if (tid < 512) {   // the blocks above the diagonal stay zero for the whole kernel
+    zero_upper_block(tid & 127, tid >> 7, warp, smem_u32(sM));
+    fence_async_smem();
+  }
+  pdl_wait();
+  if (tid == 0) s_abort = *(volatile int*)status;   // an earlier kernel gave up
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tm = tmem_slot;
+  if (s_abort) {
+    if (warp == 17) tmem_dealloc(tm, 512);
+    return;
+  }
+  const uint32_t tmDC = tm + 256, tmDB = tm + 384;
+  Waiter w{status, false};
+
+  const int nblk = g.hpg / HB;
+  const int ntiles = g.B * g.G * g.nc;
+  const int my_tiles = (ntiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;   // >= 1 by launch
+  auto tile_coords = [&](int t, int& b, int& grp, int& c) {
+    const int u = blockIdx.x + t * gridDim.x;
+    c = u % g.nc;
+    const int r = u / g.nc;
+    grp = r % g.G;
+    b = r / g.G;
+  };
+  // use n (0, 1, 2, ...) of a ring of depth D sits in slot n % D; its `full` wait has parity (n / D) & 1, its `empty` wait the
+  // opposite (a fresh barrier passes a wait on parity 1).  kb counts head blocks, ki the uses of the input ring: nblk + 2 per
+  // tile.  raw_done and sc_full go by kb: block kb + NIN is loaded only after block kb's state products.
+  auto par = [](int n, int depth) { return (uint32_t)((n / depth) & 1); };
+
+  // registers: 80 * 512 + 64 * 128 + 56 * 256 <= the launch-time 72 * 896
+  if (warp >= 16 && warp < 20) reg_dec<64>();
+  if (warp == 16) {
+    // ------------------------------------------------------------------ TMA producer
+    if (lane == 0) {
+      int kb = 0, ki = 0;
+      for (int t = 0; t < my_tiles; ++t) {
+        int b, grp, c;
+        tile_coords(t, b, grp, c);
+        for (int blk = 0; blk < nblk; ++blk, ++kb, ++ki) {
+          const int ib = ki % NIN, sb = kb % NST, ts = kb % NT;
+          const int h0 = grp * g.hpg + blk * HB, col = h0 * P;
+          w.wait(&in_empty[ib], par(ki, NIN) ^ 1, 42);
+          uint8_t* dst = sIn + ib * Cfg::IN_BYTES;
+          mbar_expect_tx(&in_full[ib], Cfg::IN_BYTES);
+          tma_load_3d(dst, &tmX, col, c * QT, b, &in_full[ib]);
+          tma_load_3d(dst + BOX_BYTES, &tmDY, col, c * QT, b, &in_full[ib]);
+          w.wait(&tab_empty[ts], par(kb, NT) ^ 1, 49);
+          mbar_expect_tx(&tab_full[ts], Cfg::TB_BYTES);
+          bulk_load(sTab + ts * Cfg::TB_BYTES, tab + ((size_t)(b * g.nc + c) * g.H + h0) * TAB, Cfg::TB_BYTES, &tab_full[ts]);
+          w.wait(&st_empty[sb], par(kb, NST) ^ 1, 50);
+          uint8_t* sd = sSt + sb * Cfg::ST_BYTES;
+          mbar_expect_tx(&st_full[sb], Cfg::ST_BYTES);
+          for (int j = 0; j < 2; ++j) {
+            tma_load_3d(sd + j * SBOX_BYTES, &tmS, 64 * j, h0 * P, b * g.nc + c, &st_full[sb]);
+            tma_load_3d(sd + (2 + j) * SBOX_BYTES, &tmDS, 64 * j, h0 * P, b * g.nc + c, &st_full[sb]);
+          }
+        }
+        for (int side = 0; side < 2; ++side, ++ki) {   // C, then B
+          const int ib = ki % NIN;
+          uint8_t* dst = sIn + ib * Cfg::IN_BYTES;
+          w.wait(&in_empty[ib], par(ki, NIN) ^ 1, 41);
+          mbar_expect_tx(&in_full[ib], Cfg::IN_BYTES);
+          for (int j = 0; j < 2; ++j)
+            tma_load_3d(dst + j * BOX_BYTES, side ? &tmB : &tmC, grp * N + 64 * j, c * QT, b, &in_full[ib]);
+        }
+      }
+    }
+  } else if (warp == 17) {
+    // ------------------------------------------------------------------ MMA issuer
+    if (lane == 0) {
+      const uint32_t idW = make_idesc(128, 128, 0, 0), idC = make_idesc(128, N, 0, 1), idB = make_idesc(128, N, 1, 1);
+      const uint64_t dMk = desc_plain_k(smem_u32(sM), 128, 0), dMt = desc_plain_mn(smem_u32(sM), 128, 0, 0);
+      int kb = 0, ki = 0, kw = 0;
+      auto issue_w = [&](int kbn, int kin) {   // the W products of block kbn, whose boxes are use kin of the input ring
+        const int ib = kin % NIN;
+        w.wait(&in_full[ib], par(kin, NIN), 45);
+        const uint32_t inb = smem_u32(sIn + ib * Cfg::IN_BYTES);
+        const uint64_t dX0 = desc_sw128_k(inb, 0), dDY0 = desc_sw128_k(inb + BOX_BYTES, 0);
+        for (int hl = 0; hl < HB; ++hl, ++kw) {
+          w.wait(&w_empty[kw & 1], par(kw, 2) ^ 1, 58);
+          tc_fence_after();
+#pragma unroll
+          for (int ks = 0; ks < P / 16; ++ks)
+            mma_bf16(tm + (kw & 1) * 128, desc_adv(dDY0, hl * P * 2 + ks * 32), desc_adv(dX0, hl * P * 2 + ks * 32), idW, ks > 0);
+          mma_commit(&w_full[kw & 1]);
+        }
+        mma_commit(&raw_done[kbn % NIN]);
+      };
+      for (int t = 0; t < my_tiles; ++t) {
+        issue_w(kb, ki);   // after the previous tile's last products: its first box reuses the slot of that tile's last block
+        w.wait(&acc_empty, (t & 1) ^ 1, 46);
+        for (int blk = 0; blk < nblk; ++blk, ++kb, ++ki) {
+          if (blk + 1 < nblk) issue_w(kb + 1, ki + 1);
+          const int ib = ki % NIN, sb = kb % NST;
+          const uint32_t inb = smem_u32(sIn + ib * Cfg::IN_BYTES), stb = smem_u32(sSt + sb * Cfg::ST_BYTES);
+          const uint64_t dXk = desc_sw128_k(inb, 0), dDYk = desc_sw128_k(inb + BOX_BYTES, 0);
+          const uint64_t dSm0 = desc_sw128_mn(stb, 0, 0, SBOX_BYTES), dDSm0 = desc_sw128_mn(stb + 2 * SBOX_BYTES, 0, 0, SBOX_BYTES);
+          w.wait(&st_full[sb], par(kb, NST), 57);
+          w.wait(&sc_full[kb % NIN], par(kb, NIN), 59);
+          tc_fence_after();
+#pragma unroll
+          for (int ks = 0; ks < 4; ++ks) {
+            mma_bf16(tmDC, desc_adv(dDYk, ks * 32), desc_adv(dSm0, ks * 2048), idC, blk > 0 || ks > 0);
+            mma_bf16(tmDB, desc_adv(dXk, ks * 32), desc_adv(dDSm0, ks * 2048), idC, blk > 0 || ks > 0);
+          }
+          mma_commit(&in_empty[ib]);
+          mma_commit(&st_empty[sb]);
+        }
+        const int ic = ki % NIN, ibb = (ki + 1) % NIN;
+        w.wait(&in_full[ic], par(ki, NIN), 43);
+        w.wait(&in_full[ibb], par(ki + 1, NIN), 44);
+        w.wait(&m_full, t & 1, 47);
+        tc_fence_after();
+        const uint64_t dCm0 = desc_sw128_mn(smem_u32(sIn + ic * Cfg::IN_BYTES), 0, 0, BOX_BYTES),
+                       dBm0 = desc_sw128_mn(smem_u32(sIn + ibb * Cfg::IN_BYTES), 0, 0, BOX_BYTES);
+#pragma unroll
+        for (int ks = 0; ks < 8; ++ks) {
+          mma_bf16(tmDC, desc_adv(dMk, ks * 4096), desc_adv(dBm0, ks * 2048), idC, true);
+          mma_bf16(tmDB, desc_adv(dMt, ks * 256), desc_adv(dCm0, ks * 2048), idB, true);
+        }
+        mma_commit(&in_empty[ic]);
+        mma_commit(&in_empty[ibb]);
+        mma_commit(&m_empty);
+        mma_commit(&acc_full);
+        ki += 2;
+      }
+    }
+  } else if (warp < 16) {
+    // ------------------------------------------------------------------ decay warps
+    reg_inc<80>();
+    const int row = tid & 127, part = tid >> 7;
+    int kb = 0, kw = 0;
+    for (int t = 0; t < my_tiles; ++t) {
+      float acc[32];
+#pragma unroll
+      for (int k = 0; k < 32; ++k) acc[k] = 0.f;
+      for (int blk = 0; blk < nblk; ++blk, ++kb) {
+        const int ts = kb % NT;
+        const float* tb = (const float*)(sTab + ts * Cfg::TB_BYTES);
+        w.wait(&tab_full[ts], par(kb, NT), 52);
+        for (int hl = 0; hl < HB; ++hl, ++kw) {
+          w.wait(&w_full[kw & 1], par(kw, 2), 51);
+          tc_fence_after();
+          decay_acc_block(tm + (kw & 1) * 128, tb + hl * TAB, row, part, warp, acc);
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&w_empty[kw & 1]);
+        }
+        if (reads_done(__float_as_uint(acc[0]) ^ __float_as_uint(acc[15]) ^ __float_as_uint(acc[16]) ^ __float_as_uint(acc[31]), lane))
+          mbar_arrive(&tab_empty[ts]);
+      }
+      w.wait(&m_empty, (t & 1) ^ 1, 53);
+      store_acc_block(acc, row, part, warp, smem_u32(sM));
+      fence_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&m_full);
+    }
+  } else if (warp >= Cfg::W_SCALE) {
+    // ------------------------------------------------------------------ scaling warps, and the drain of a finished tile
+    reg_dec<56>();
+    const int sid = tid - Cfg::W_SCALE * 32, ew = warp - Cfg::W_SCALE;
+    const int row = (ew & 3) * 32 + lane, half = ew >> 2;     // 64 of the 128 columns
+    int kb = 0, ki = 0;
+    for (int t = 0; t < my_tiles; ++t) {
+      for (int blk = 0; blk < nblk; ++blk, ++kb, ++ki) {
+        const int ts = kb % NT, ib = ki % NIN;
+        const uint32_t tbs = smem_u32(sTab + ts * Cfg::TB_BYTES), xb = smem_u32(sIn + ib * Cfg::IN_BYTES);
+        w.wait(&tab_full[ts], par(kb, NT), 55);
+        w.wait(&in_full[ib], par(ki, NIN), 54);
+        w.wait(&raw_done[kb % NIN], par(kb, NIN), 60);
+        // dy by exp(cs_i), x by exp(cs_end - cs_j) dt_j: eight 16-byte pieces per thread, four loads in flight
+#pragma unroll
+        for (int box = 0; box < 2; ++box) {
+          uint4 raw[4];
+          float fac[4];
+#pragma unroll
+          for (int r = 0; r < 4; ++r) raw[r] = ld_shared_v4(xb + box * BOX_BYTES + (sid + r * 256) * 16);
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            const int l = (sid + r * 256) >> 3, pc = sid & 7;
+            const uint32_t tt = tbs + ((((pc ^ l) & 7) * 8) / P) * TAB_BYTES;
+            const float csl = lds_f32(tt + 4 * (T_CS + l));
+            fac[r] = box ? ex2(csl) : ex2(lds_f32(tt + 4 * (T_CS + 127)) - csl) * lds_f32(tt + 4 * (T_DT + l));
+          }
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            float v[8];
+            unpack8(raw[r], v);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v[k] *= fac[r];
+            const uint4 o = pack8(v);
+            st_shared_v4(xb + box * BOX_BYTES + (sid + r * 256) * 16, o.x, o.y, o.z, o.w);
+          }
+        }
+        fence_async_smem();
+        __syncwarp();
+        if (lane == 0) { mbar_arrive(&sc_full[kb % NIN]); mbar_arrive(&tab_empty[ts]); }
+      }
+      ki += 2;
+      int b, grp, c;
+      tile_coords(t, b, grp, c);
+      w.wait(&acc_full, t & 1, 56);
+      tc_fence_after();
+      const size_t o = (((size_t)b * g.L + c * QT + row) * g.G + grp) * N + half * 64;
+#pragma unroll
+      for (int j = 0; j < 64; j += 16) {
+#pragma unroll
+        for (int side = 0; side < 2; ++side) {
+          float v[16];
+          tmem_ld16(tmem_addr(side ? tmDB : tmDC, (ew & 3) * 32, half * 64 + j), v);
+          if (j == 48 && side == 1) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&acc_empty);
+          }
+          if (c * QT + row < g.L)   // a ragged sequence ends inside its last tile
+            st_global_32B((side ? dB : dC) + o + j,
+                          make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7])),
+                          make_uint4(pack_bf16(v[8], v[9]), pack_bf16(v[10], v[11]), pack_bf16(v[12], v[13]), pack_bf16(v[14], v[15])));
+          __syncwarp();
+        }
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 17) tmem_dealloc(tm, 512);
+}
+
+// ---------------------------------------------------------------------------------------------
 // Exclusive scan over chunks, 4 state elements per thread, decays staged in shared memory.
 // Optionally also writes the bf16 copy of the chunk-entry states that the tensor kernels load.
 // The reverse scan (state gradient) can also emit, per chunk, this block's warp-partial sums of
@@ -3343,6 +3632,13 @@ int launch_dbc_ws(const Geo& g, const SeqMaps& m, const float* tab, const float*
 template <int P, int N>
 int launch_dbc(const Geo& g, const SeqMaps& m, const float* tab, const float* hmax, void* dB, void* dC, int* status, cudaStream_t s) {
   if (N == 64 && !g.onetile) return launch_dbc_ws<P>(g, m, tab, hmax, dB, dC, status, s);
+  if (N == 128 && !g.onetile) {
+    const int ntiles = g.B * g.G * g.nc;
+    launch<k_dbc_sum_ws<P>>(ntiles < sm_count() ? ntiles : sm_count(), WS_THREADS, DsCfg<P>::SMEM, s, g, m.x, m.dy, m.b, m.c, m.s, m.ds,
+                            tab, (bf16*)dB, (bf16*)dC, status);
+    SSD_CUDA_CHECK_LAUNCH("dBdC_sum_ws");
+    return SSD_OK;
+  }
   launch<k_dbc_tc<P, N>>(dim3(g.nc, g.G, g.B), TC_THREADS, dbc_smem<P, N>(), s, g, m.x, m.dy, m.b, m.c, m.s, m.ds, tab, (bf16*)dB,
                          (bf16*)dC, status);
   SSD_CUDA_CHECK_LAUNCH("dBdC_tc");
