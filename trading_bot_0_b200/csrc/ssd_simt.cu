@@ -224,16 +224,12 @@ __device__ __forceinline__ size_t cb_idx(const Geo& g, int b, int c, int grp) {
 template <typename T, int HG>
 __global__ void __launch_bounds__(256) k_cumsum(Geo g, const T* __restrict__ dt, const float* __restrict__ dt_bias,
                                                const float* __restrict__ A, float* __restrict__ cs,
-                                               float* __restrict__ dtf, float* __restrict__ tab, int* __restrict__ hmax,
-                                               int tag, int* __restrict__ status) {
+                                               float* __restrict__ dtf, float* __restrict__ tab, int* __restrict__ status) {
   pdl_wait();
   const int c = blockIdx.x, b = blockIdx.y, q = threadIdx.x;
   __shared__ float wsum[8][HG];
   const int t = c * g.Q + q;
-  if (c == 0 && b == 0 && blockIdx.z == 0 && q == 0) {   // first kernel of a pass: the status word and the tag of this launch
-    *status = 0;
-    if (hmax) hmax[g.H] = tag;
-  }
+  if (c == 0 && b == 0 && blockIdx.z == 0 && q == 0) *status = 0;   // first kernel of a pass
   const bool live = (q < g.Q) && (t < g.L);
   const int lane = q & 31, w = q >> 5;
   const T* row = dt + b * g.dtsb + (long long)t * g.dtsl;
@@ -276,10 +272,6 @@ __global__ void __launch_bounds__(256) k_cumsum(Geo g, const T* __restrict__ dt,
         // tensor-core family (chunk 128 only): the per-head decay table [cs*log2e | dt | exp(cs_r - cs) dt |
         // exp(dt_{l+1} A)], r = last position of the 32-block (lane 31 of this warp)
         const float vend = __shfl_sync(0xffffffffu, v[k], 31);
-        // per head: does any chunk of the call accumulate a decay exponent beyond the range inside which dB/dC may carry the
-        // decay on the operands?  Only then this launch's tag is written to the head's word (plain store), so the usual case
-        // costs nothing and nothing has to be zeroed.
-        if (hmax && h < g.H && q == g.Q - 1 && fabsf(v[k]) > SSD_SEP_LOG_RANGE) hmax[h] = tag;
         if (tab && h < g.H && q < g.Q) {
           const float L2E = 1.4426950408889634f;
           float* t = tab + ((size_t)(b * g.nc + c) * g.H + h) * SSD_TAB_FLOATS + q;
@@ -1023,14 +1015,10 @@ static int fwd_stages_t(const Geo& g, bool tc, const SsdFwdPtrs& p, char* ws, co
   // a full pass (no sequence-parallel staging) computes the chunk states inside the scan over chunks where that kernel applies
   const bool fused = tc && stages == (SSD_STAGE_LOCAL | SSD_STAGE_FINISH) && tensor_state_fused_applies(g);
   if (stages & (SSD_STAGE_LOCAL | SSD_STAGE_LOCAL_STATES)) {
-    int* hmax = tc ? (int*)(ws + w.hmax) : nullptr;
-    static std::atomic<int> launch_tag{1};
-    int tag = launch_tag.fetch_add(1, std::memory_order_relaxed);
-    if (tag == 0) tag = launch_tag.fetch_add(1, std::memory_order_relaxed);
     const bool wide = (long long)g.nc * g.B >= 2LL * sm_count();
     auto cumsum = [&](auto kernel) {
       launch<kernel.value>(dim3(g.nc, g.B, wide ? 1 : cdiv(g.H, 2)), g.Q <= 128 ? 128 : 256, 0, s, g, (const T*)p.dt, p.dt_bias, p.A, cs, dtf,
-                           tc ? tab : nullptr, hmax, tag, status);
+                           tc ? tab : nullptr, status);
     };
     wide ? cumsum(Fn<k_cumsum<T, 8>>()) : cumsum(Fn<k_cumsum<T, 2>>());
     SSD_CUDA_CHECK_LAUNCH("cumsum");
@@ -1183,7 +1171,7 @@ static int bwd_stages_t(const Geo& g, bool tc, const SsdBwdPtrs& p, char* ws, co
       int rc = tensor_bwd_merged_applies(g, p) ? tensor_bwd_merged(g, p, tab, prev_bf, ds_bf, dcsp, ddot, ddtd, status, s)
                                                 : tensor_dx(g, p, tc_dy, tc_dense, tab, ds_bf, ddtd, status, s);
       if (rc) return rc;
-      rc = tensor_dbc(g, p, tc_dy, tc_dense, tab, (const float*)(ws + w.hmax), prev_bf, ds_bf, status, s);
+      rc = tensor_dbc(g, p, tc_dy, tc_dense, tab, prev_bf, ds_bf, status, s);
       if (rc) return rc;
     } else {
       float* dcs_cols = dcsp + (size_t)n.strips * n.nq;

@@ -117,27 +117,6 @@ __device__ __forceinline__ void decay_mask_tile(uint32_t tm_src, const float* __
                  pack_bf16(v[6], v[7]));
   }
 }
-// Lower-triangular mask only: source = a 128x128 fp32 accumulator in TMEM that already carries the decay (separable heads,
-// see k_dbc_ws), result = src[i,j] for j <= i as bf16 in a plain 128x128 tile.  Thread mapping of decay_mask_tile; blocks
-// above the diagonal are never written (they are zero in every ring tile for the whole kernel).
-__device__ __forceinline__ void mask_tril_tile(uint32_t tm_src, int row, int part, int warp, uint32_t mtile) {
-  const int rb = warp & 3;
-  uint32_t raw[4][8];
-#pragma unroll
-  for (int cb = 0; cb < 4; ++cb)
-    if (cb <= rb) tmem_ld8_issue(tmem_addr(tm_src, rb * 32, cb * 32 + part * 8), raw[cb]);
-  tmem_ld_wait();
-#pragma unroll
-  for (int cb = 0; cb < 4; ++cb) {
-    if (cb > rb) continue;
-    const int c0 = cb * 32 + part * 8;
-    float v[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) v[k] = (cb < rb || c0 + k <= row) ? __uint_as_float(raw[cb][k]) : 0.f;
-    st_shared_v4(mtile + plain_off(128, row, c0), pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]),
-                 pack_bf16(v[6], v[7]));
-  }
-}
 // zero the 32x32 blocks above the diagonal of a plain 128x128 tile (same thread mapping)
 __device__ __forceinline__ void zero_upper_blocks(int row, int part, int warp, uint32_t mtile) {
 #pragma unroll
@@ -292,7 +271,13 @@ __device__ __forceinline__ void decay_mask_block(uint32_t tm_src, const float* _
     st_shared_v4(mtile + plain_off(128, row, c0 + j8), pack_bf16(v[j8], v[j8 + 1]), pack_bf16(v[j8 + 2], v[j8 + 3]),
                  pack_bf16(v[j8 + 4], v[j8 + 5]), pack_bf16(v[j8 + 6], v[j8 + 7]));
 }
-// Accumulating variant for the one-tile dB / dC kernel: dC = sum_h W'_h B and dB = sum_h W'_h^T C are linear in W'_h, so
+// a0 += x0 * y0, a1 += x1 * y1 as one packed instruction, same rounding as two
+__device__ __forceinline__ void fma2(float& a0, float& a1, float x0, float x1, float y0, float y1) {
+  asm("{\n\t.reg .b64 a, x, y;\n\tmov.b64 a, {%0, %1};\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
+      "fma.rn.f32x2 a, x, y, a;\n\tmov.b64 {%0, %1}, a;\n\t}"
+      : "+f"(a0), "+f"(a1) : "f"(x0), "f"(x1), "f"(y0), "f"(y1));
+}
+// Accumulating variant for dB / dC: dC = sum_h W'_h B and dB = sum_h W'_h^T C are linear in W'_h, so
 // the decayed, masked tiles of all heads of a group are added up in registers (fp32; thread = row x one 32-column block)
 // and only their SUM goes to shared memory, once per tile.
 __device__ __forceinline__ void decay_acc_block(uint32_t tm_src, const float* __restrict__ tab, int row, int part, int warp,
@@ -301,28 +286,36 @@ __device__ __forceinline__ void decay_acc_block(uint32_t tm_src, const float* __
   if (cb > rb) return;
   const int c0 = cb * 32;
   const uint32_t ts = smem_u32(tab);
-  float v[32];
-  tmem_ld32(tmem_addr(tm_src, rb * 32, c0), v);
-  if (cb == rb) {
-    float run = 0.f;
+  // right half first (the chain of the diagonal block runs that way), 16 columns in registers at a time beside the 32 sums
+  const bool diag = cb == rb;
+  const float rf = diag ? 0.f : ex2(lds_f32(ts + 4 * (T_CS + row)) - lds_f32(ts + 4 * (T_CS + c0 + 31)));
+  float run = 0.f;
 #pragma unroll
-    for (int k4 = 28; k4 >= 0; k4 -= 4) {
-      const float4 d = lds_v4f32(ts + 4 * (T_DS + c0 + k4)), t = lds_v4f32(ts + 4 * (T_DT + c0 + k4));
-      const float ds[4] = {d.x, d.y, d.z, d.w}, dt[4] = {t.x, t.y, t.z, t.w};
+  for (int half = 16; half >= 0; half -= 16) {
+    float v[16];
+    tmem_ld16(tmem_addr(tm_src, rb * 32, c0 + half), v);
+    if (diag) {
 #pragma unroll
-      for (int q = 3; q >= 0; --q) {
-        const int j = c0 + k4 + q;
-        run = (j == row) ? 1.f : run * ds[q];
-        acc[k4 + q] = fmaf(v[k4 + q], run * dt[q], acc[k4 + q]);
+      for (int k4 = 12; k4 >= 0; k4 -= 4) {
+        const float4 d = lds_v4f32(ts + 4 * (T_DS + c0 + half + k4)), t = lds_v4f32(ts + 4 * (T_DT + c0 + half + k4));
+        const float ds[4] = {d.x, d.y, d.z, d.w};
+        float r[4], * a = acc + half + k4;
+#pragma unroll
+        for (int q = 3; q >= 0; --q) {
+          run = (c0 + half + k4 + q == row) ? 1.f : run * ds[q];
+          r[q] = run;
+        }
+        fma2(a[0], a[1], v[k4], v[k4 + 1], r[0] * t.x, r[1] * t.y);
+        fma2(a[2], a[3], v[k4 + 2], v[k4 + 3], r[2] * t.z, r[3] * t.w);
       }
-    }
-  } else {
-    const float rf = ex2(lds_f32(ts + 4 * (T_CS + row)) - lds_f32(ts + 4 * (T_CS + c0 + 31)));
+    } else {
 #pragma unroll
-    for (int k4 = 0; k4 < 32; k4 += 4) {
-      const float4 f = lds_v4f32(ts + 4 * (T_CF + c0 + k4));
-      acc[k4] = fmaf(v[k4], rf * f.x, acc[k4]); acc[k4 + 1] = fmaf(v[k4 + 1], rf * f.y, acc[k4 + 1]);
-      acc[k4 + 2] = fmaf(v[k4 + 2], rf * f.z, acc[k4 + 2]); acc[k4 + 3] = fmaf(v[k4 + 3], rf * f.w, acc[k4 + 3]);
+      for (int k4 = 0; k4 < 16; k4 += 4) {
+        const float4 f = lds_v4f32(ts + 4 * (T_CF + c0 + half + k4));
+        float* a = acc + half + k4;
+        fma2(a[0], a[1], v[k4], v[k4 + 1], rf * f.x, rf * f.y);
+        fma2(a[2], a[3], v[k4 + 2], v[k4 + 3], rf * f.z, rf * f.w);
+      }
     }
   }
 }
@@ -2659,447 +2652,43 @@ k_bwd_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant__
 }
 
 // ---------------------------------------------------------------------------------------------
-// Backward dB / dC, dstate 64, persistent and warp-specialised like k_scan_ws.
-//
-// Block path (any head).  Per head W_h = dY_h X_h^T (K = P) into one of two TMEM slots -> decay pass (32x32 blocks, the
-// factorisation of decay_mask_tile) -> W'_h as bf16 in shared memory -> dC += W'_h B, dB += W'_h^T C.
-// Per head block, once its raw x / dy boxes are no longer needed by a W product, the decay warps scale them in place and
-// one K = 64 product each adds the state terms dC += dY' S_prev, dB += X' dS_end.  dC / dB stay in TMEM for the whole tile.
-//
-// Separable heads.  exp(cs_i - cs_j) dt_j = a_i b_j with a_i = exp(cs_i), b_j = exp(-cs_j) dt_j, and dC, dB are linear in
-// W'_h, so for a head whose decay over a chunk stays inside the range of the storage type (|cs_end| <= SSD_SEP_LOG_RANGE for
-// every chunk of the call; the cumsum kernel records the per-head maximum) the decay can ride on the OPERANDS:
-//   sum_h W'_h = tril( sum_h (a_h o dY_h) (b_h o X_h)^T ),
-// one accumulator for all such heads of the tile, filled by the tensor core from the boxes the decay warps scale in place
-// anyway for the state terms (dy by a, x by b; the factor exp(cs_end) that the x-side state term then lacks goes onto the
-// rows of the dS_end box).  Those heads need no per-head pass over a 128x128 tile at all; once per tile the accumulator is
-// masked to its lower triangle and multiplied like one more W'_h.  Heads outside the range (strong decay: a_i or b_j alone
-// would leave the range although every a_i b_j with j <= i is at most dt_j) keep the block path.
-//
-// With the per-head pass gone for most heads a tile is a short chain of scale -> multiply steps, and what bounds the kernel
-// is how far the loads run ahead of it: the x/dy boxes have a ring of three, the state boxes of two, the tables of four;
-// the B/C tiles (read at the END of a tile by the separable path) and the W' tile are single.
-
-template <int P>
-struct DbCfg {
-  static constexpr int N = 64, HB = 64 / P, NT = 4, NIN = 3, NST = 2;
-  static constexpr int CB_BYTES = 2 * BOX_BYTES;             // B tile, C tile
-  static constexpr int IN_BYTES = 2 * BOX_BYTES;             // x box, dy box
-  static constexpr int ST_BYTES = 2 * SBOX_BYTES;            // S_prev box, dS_end box
-  static constexpr int TB_BYTES = HB * TAB_BYTES;
-  static constexpr size_t SMEM = 1024 + CB_BYTES + 2 * BOX_BYTES + NIN * IN_BYTES + NST * ST_BYTES + NT * TB_BYTES;
-};
-
-struct DbBars {
-  uint64_t cb_full, cb_empty, in_full[3], in_empty[3], w_full[2], w_empty[2], m_full, m_empty;
-  uint64_t tab_full[4], tab_empty[4], st_full[2], st_empty[2], wraw_done[3], sc_full[3], acc_full, acc_empty, done;
-  uint64_t wsep_full, wsep_empty;
-};
-
-template <int P>
-__global__ void __launch_bounds__(WS_THREADS, 1)
-k_dbc_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmDY,
-         const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmC,
-         const __grid_constant__ CUtensorMap tmS, const __grid_constant__ CUtensorMap tmDS,
-         const float* __restrict__ tab, const float* __restrict__ hmax, bf16* __restrict__ dB, bf16* __restrict__ dC,
-         int* __restrict__ status) {
-  using Cfg = DbCfg<P>;
-  constexpr int N = Cfg::N, HB = Cfg::HB, NIN = Cfg::NIN, NST = Cfg::NST, NT = Cfg::NT;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);   // 1 KB aligned, still known to be shared memory
-  uint8_t* sCB = smem;                                   // {B tile, C tile} of the current tile
-  uint8_t* sM = sCB + Cfg::CB_BYTES;                     // one 32 KB W' tile
-  uint8_t* sIn = sM + 2 * BOX_BYTES;                     // NIN x {x box, dy box}
-  uint8_t* sSt = sIn + NIN * Cfg::IN_BYTES;              // NST x {S_prev box, dS_end box}
-  uint8_t* sTab = sSt + NST * Cfg::ST_BYTES;             // NT x decay tables of a head block
-  __shared__ __align__(8) DbBars bars;
-  __shared__ uint32_t tmem_slot;
-  __shared__ int s_abort;
-
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (tid == 0) {
-    // two MMA issuer lanes (dC side, dB side): tcgen05.commit tracks the MMAs of its own thread only, so every barrier that
-    // releases something both of them read expects one commit from each
-    mbar_init(&bars.cb_full, 1); mbar_init(&bars.cb_empty, 2);
-    for (int i = 0; i < NIN; ++i) {
-      mbar_init(&bars.in_full[i], 1); mbar_init(&bars.in_empty[i], 2);
-      mbar_init(&bars.wraw_done[i], 1); mbar_init(&bars.sc_full[i], WS_SCALE_WARPS);
-    }
-    for (int i = 0; i < 2; ++i) { mbar_init(&bars.w_full[i], 1); mbar_init(&bars.w_empty[i], WS_SCALE_WARPS); }
-    mbar_init(&bars.m_full, WS_SCALE_WARPS); mbar_init(&bars.m_empty, 2);
-    for (int i = 0; i < NT; ++i) { mbar_init(&bars.tab_full[i], 1); mbar_init(&bars.tab_empty[i], WS_SCALE_WARPS); }
-    for (int i = 0; i < NST; ++i) { mbar_init(&bars.st_full[i], 1); mbar_init(&bars.st_empty[i], 2); }
-    mbar_init(&bars.acc_full, 2); mbar_init(&bars.acc_empty, WS_EPI_WARPS);
-    mbar_init(&bars.done, 2);
-    mbar_init(&bars.wsep_full, 1); mbar_init(&bars.wsep_empty, WS_SCALE_WARPS);
-    mbar_fence_init();
-  }
-  if (warp == 17) tmem_alloc(&tmem_slot, 512);
-  if (tid < 512) {
-    zero_upper_blocks(tid & 127, tid >> 7, warp, smem_u32(sM));
-    fence_async_smem();
-  }
-  pdl_wait();
-  if (tid == 0) s_abort = *(volatile int*)status;   // an earlier kernel gave up
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tm = tmem_slot;
-  if (s_abort) {
-    if (warp == 17) tmem_dealloc(tm, 512);
-    return;
-  }
-  const uint32_t tmDC = tm + 256, tmDB = tm + 320, tmWsep = tm + 384;
-  Waiter w{status, false};
-  // which heads take the separable path: one bit per head, the same in every role (up to 64 heads; beyond that none)
-  unsigned long long sepmask = 0ull;
-  if (hmax && g.H <= 64) {
-    const int* tags = reinterpret_cast<const int*>(hmax);
-    const int cur = __ldg(tags + g.H);
-    for (int h = 0; h < g.H; ++h)
-      if (__ldg(tags + h) != cur) sepmask |= 1ull << h;
-  }
-  auto is_sep = [&](int h) { return ((sepmask >> h) & 1ull) != 0; };
-  auto group_has_sep = [&](int grp) {
-    const unsigned long long gm = (g.hpg >= 64 ? ~0ull : ((1ull << g.hpg) - 1ull)) << (grp * g.hpg);
-    return (sepmask & gm) != 0ull;
-  };
-
-  const int nblk = g.hpg / HB;
-  const int ntiles = g.B * g.G * g.nc;
-  const int my_tiles = (ntiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
-  auto tile_coords = [&](int t, int& b, int& grp, int& c) {
-    const int u = blockIdx.x + t * gridDim.x;
-    c = u % g.nc;
-    const int r = u / g.nc;
-    grp = r % g.G;
-    b = r / g.G;
-  };
-  // use n (0, 1, 2, ...) of a ring of depth D sits in slot n % D; its `full` wait has parity (n / D) & 1, its `empty` wait the
-  // opposite (a fresh barrier passes a wait on parity 1)
-  auto par = [](int n, int depth) { return (uint32_t)((n / depth) & 1); };
-
-  // registers: the single-thread roles (warps 16-19, one aligned group of four) and the epilogue hand some back, the decay
-  // warps take them (80 * 512 + 64 * 128 + 48 * 256 <= the launch-time 72 * 896)
-  if (warp >= 16 && warp < 20) reg_dec<64>();
-  if (warp == 16) {
-    // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
-      const int total_blocks = my_tiles * nblk;
-      auto load_tab = [&](int kg) {
-        if (kg >= total_blocks) return;
-        int b, grp, c;
-        tile_coords(kg / nblk, b, grp, c);
-        const int h0 = grp * g.hpg + (kg % nblk) * HB, ts = kg % NT;
-        w.wait(&bars.tab_empty[ts], par(kg, NT) ^ 1, 49);
-        mbar_expect_tx(&bars.tab_full[ts], Cfg::TB_BYTES);
-        bulk_load(sTab + ts * Cfg::TB_BYTES, tab + ((size_t)(b * g.nc + c) * g.H + h0) * TAB, Cfg::TB_BYTES, &bars.tab_full[ts]);
-      };
-      int kb = 0;
-      load_tab(0);
-      load_tab(1);
-      for (int t = 0; t < my_tiles; ++t) {
-        int b, grp, c;
-        tile_coords(t, b, grp, c);
-        for (int blk = 0; blk < nblk; ++blk, ++kb) {
-          load_tab(kb + 2);
-          const int ib = kb % NIN, sb = kb % NST;
-          const int h0 = grp * g.hpg + blk * HB, col = grp * g.hpg * P + blk * 64;
-          w.wait(&bars.in_empty[ib], par(kb, NIN) ^ 1, 42);
-          uint8_t* dst = sIn + ib * Cfg::IN_BYTES;
-          mbar_expect_tx(&bars.in_full[ib], Cfg::IN_BYTES);
-          tma_load_3d(dst, &tmX, col, c * QT, b, &bars.in_full[ib]);
-          tma_load_3d(dst + BOX_BYTES, &tmDY, col, c * QT, b, &bars.in_full[ib]);
-          w.wait(&bars.st_empty[sb], par(kb, NST) ^ 1, 50);
-          uint8_t* sd = sSt + sb * Cfg::ST_BYTES;
-          mbar_expect_tx(&bars.st_full[sb], Cfg::ST_BYTES);
-          tma_load_3d(sd, &tmS, 0, h0 * P, b * g.nc + c, &bars.st_full[sb]);
-          tma_load_3d(sd + SBOX_BYTES, &tmDS, 0, h0 * P, b * g.nc + c, &bars.st_full[sb]);
-          // this tile's B / C: single buffer, free once the previous tile's last products have completed; requested behind
-          // the tile's first boxes so that this wait does not hold the box stream back
-          if (blk == (nblk > 1 ? 1 : 0)) {
-            w.wait(&bars.cb_empty, (t & 1) ^ 1, 41);
-            mbar_expect_tx(&bars.cb_full, Cfg::CB_BYTES);
-            tma_load_3d(sCB, &tmB, grp * N, c * QT, b, &bars.cb_full);
-            tma_load_3d(sCB + BOX_BYTES, &tmC, grp * N, c * QT, b, &bars.cb_full);
-          }
-        }
-      }
-    }
-  } else if (warp == 17 || warp == 18) {
-    // ------------------------------------------------------------------ MMA issuers.  The products are split by side:
-    // lane A (warp 17) issues every W product and everything that accumulates into dC, lane B (warp 18) everything into dB.
-    if (lane == 0) {
-      const bool side_c = warp == 17;
-      const uint32_t idW = make_idesc(128, 128, 0, 0), idC = make_idesc(128, N, 0, 1), idB = make_idesc(128, N, 1, 1);
-      const int total_blocks = my_tiles * nblk;
-      int kw = 0;   // W products of block-path heads issued so far
-      auto issue_w_block = [&](int kg) {   // the W products of global block kg's heads on the block path (lane A only)
-        if (kg >= total_blocks) return;
-        const int ib = kg % NIN;
-        int bb, gg, cc;
-        tile_coords(kg / nblk, bb, gg, cc);
-        const int h0 = gg * g.hpg + (kg % nblk) * HB;
-        bool any_block_path = false;
-        for (int hl = 0; hl < HB; ++hl) any_block_path |= !is_sep(h0 + hl);
-        if (!any_block_path) {   // nothing reads the raw boxes: release them at once, without waiting for them to land
-          mbar_arrive(&bars.wraw_done[ib]);
-          return;
-        }
-        w.wait(&bars.in_full[ib], par(kg, NIN), 45);
-        tc_fence_after();
-        const uint32_t inb = smem_u32(sIn + ib * Cfg::IN_BYTES);
-        const uint64_t dX0 = desc_sw128_k(inb, 0), dDY0 = desc_sw128_k(inb + BOX_BYTES, 0);
-        for (int hl = 0; hl < HB; ++hl) {
-          if (is_sep(h0 + hl)) continue;
-          const int ws = kw & 1;
-          w.wait(&bars.w_empty[ws], par(kw, 2) ^ 1, 58);
-          tc_fence_after();
-#pragma unroll
-          for (int ks = 0; ks < P / 16; ++ks)
-            mma_bf16(tm + ws * 128, desc_adv(dDY0, hl * P * 2 + ks * 32), desc_adv(dX0, hl * P * 2 + ks * 32), idW, ks > 0);
-          mma_commit(&bars.w_full[ws]);
-          ++kw;
-        }
-        mma_commit(&bars.wraw_done[ib]);   // the raw boxes of this block have been read by every W product
-      };
-      if (side_c) issue_w_block(0);
-      const uint64_t dBm0 = desc_sw128_mn(smem_u32(sCB), 0, 0, BOX_BYTES), dCm0 = desc_sw128_mn(smem_u32(sCB) + BOX_BYTES, 0, 0, BOX_BYTES);
-      const uint32_t mt = smem_u32(sM);
-      const uint64_t dMk = desc_plain_k(mt, 128, 0), dMt = desc_plain_mn(mt, 128, 0, 0);
-      int kb = 0, kh = 0, ksep = 0;   // kh: W' tiles consumed; ksep: tiles with separable heads so far
-      for (int t = 0; t < my_tiles; ++t) {
-        w.wait(&bars.acc_empty, (t & 1) ^ 1, 46);
-        tc_fence_after();
-        int tb_, tg_, tc_;
-        tile_coords(t, tb_, tg_, tc_);
-        const bool anysep = group_has_sep(tg_);
-        bool first = true, firstsep = true, have_cb = false;
-        auto issue_m = [&]() {   // the W' tile -> dC (lane A) or dB (lane B)
-          if (!have_cb) { w.wait(&bars.cb_full, t & 1, 43); have_cb = true; }
-          w.wait(&bars.m_full, kh & 1, 47);
-          tc_fence_after();
-          if (side_c) {
-#pragma unroll
-            for (int ks = 0; ks < 8; ++ks) mma_bf16(tmDC, desc_adv(dMk, ks * 4096), desc_adv(dBm0, ks * 2048), idC, !first || ks > 0);
-          } else {
-#pragma unroll
-            for (int ks = 0; ks < 8; ++ks) mma_bf16(tmDB, desc_adv(dMt, ks * 256), desc_adv(dCm0, ks * 2048), idB, !first || ks > 0);
-          }
-          first = false;
-          mma_commit(&bars.m_empty);
-          ++kh;
-        };
-        for (int blk = 0; blk < nblk; ++blk, ++kb) {
-          const int ib = kb % NIN, sb = kb % NST;
-          const uint32_t inb = smem_u32(sIn + ib * Cfg::IN_BYTES), stb = smem_u32(sSt + sb * Cfg::ST_BYTES);
-          const int h0 = tg_ * g.hpg + blk * HB;
-          for (int hl = 0; hl < HB; ++hl)
-            if (!is_sep(h0 + hl)) issue_m();
-          // the next block's W products go out before this block's state terms, so the decay warps
-          // find their next input ready when they come back from scaling this block's boxes
-          if (side_c) issue_w_block(kb + 1);
-          w.wait(&bars.sc_full[ib], par(kb, NIN), 59);
-          w.wait(&bars.st_full[sb], par(kb, NST), 57);
-          tc_fence_after();
-          if (side_c) {
-            const uint64_t dDYk = desc_sw128_k(inb + BOX_BYTES, 0), dXk = desc_sw128_k(inb, 0);
-            const uint64_t dSm0 = desc_sw128_mn(stb, 0, 0, SBOX_BYTES);
-            // separable heads of this block: their W, decay included, adds up in one accumulator for the whole tile
-            for (int hl = 0; hl < HB; ++hl) {
-              if (!is_sep(h0 + hl)) continue;
-              if (firstsep) w.wait(&bars.wsep_empty, (ksep & 1) ^ 1, 60);   // the decay warps have read the previous tile's sum
-#pragma unroll
-              for (int ks = 0; ks < P / 16; ++ks)
-                mma_bf16(tmWsep, desc_adv(dDYk, hl * P * 2 + ks * 32), desc_adv(dXk, hl * P * 2 + ks * 32), idW, !firstsep || ks > 0);
-              firstsep = false;
-            }
-#pragma unroll
-            for (int ks = 0; ks < 4; ++ks) mma_bf16(tmDC, desc_adv(dDYk, ks * 32), desc_adv(dSm0, ks * 2048), idC, !first || ks > 0);
-          } else {
-            const uint64_t dXk = desc_sw128_k(inb, 0);
-            const uint64_t dDSm0 = desc_sw128_mn(stb + SBOX_BYTES, 0, 0, SBOX_BYTES);
-#pragma unroll
-            for (int ks = 0; ks < 4; ++ks) mma_bf16(tmDB, desc_adv(dXk, ks * 32), desc_adv(dDSm0, ks * 2048), idC, !first || ks > 0);
-          }
-          first = false;
-          mma_commit(&bars.st_empty[sb]);
-          mma_commit(&bars.in_empty[ib]);
-        }
-        if (anysep) {
-          if (side_c) mma_commit(&bars.wsep_full);
-          ++ksep;
-          issue_m();   // the masked sum of the separable heads, handed over by the decay warps like one more W'_h
-        }
-        if (!have_cb) w.wait(&bars.cb_full, t & 1, 43);   // keep the barrier's phases in step even if nothing read the tiles
-        mma_commit(&bars.cb_empty);
-        mma_commit(&bars.acc_full);
-      }
-      mma_commit(&bars.done);
-      w.wait(&bars.done, 0, 48);
-    }
-  } else if (warp < WS_SCALE_WARPS) {
-    // ------------------------------------------------------------------ decay pass warps
-    reg_inc<80>();
-    const int row = tid & 127, part = tid >> 7;
-    int kb = 0, kh = 0, kw = 0, ksep = 0;
-    for (int t = 0; t < my_tiles; ++t) {
-      int tb_, tg_, tc_;
-      tile_coords(t, tb_, tg_, tc_);
-      const bool anysep = group_has_sep(tg_);
-      for (int blk = 0; blk < nblk; ++blk, ++kb) {
-        const int ts = kb % NT, ib = kb % NIN, sb = kb % NST;
-        const int h0 = tg_ * g.hpg + blk * HB;
-        const float* tb = (const float*)(sTab + ts * Cfg::TB_BYTES);
-        const uint32_t tbs = smem_u32(sTab + ts * Cfg::TB_BYTES);
-        w.wait(&bars.tab_full[ts], par(kb, NT), 52);
-        for (int hl = 0; hl < HB; ++hl) {
-          if (is_sep(h0 + hl)) continue;
-          const int ws = kw & 1;
-          w.wait(&bars.w_full[ws], par(kw, 2), 51);
-          w.wait(&bars.m_empty, (kh & 1) ^ 1, 53);
-          tc_fence_after();
-          decay_mask_tile(tm + ws * 128, tb + hl * TAB, row, part, warp, smem_u32(sM));
-          fence_async_smem();
-
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) { mbar_arrive(&bars.m_full); mbar_arrive(&bars.w_empty[ws]); }
-          ++kh;
-          ++kw;
-        }
-        // scale this block's boxes in place for the state terms (x: box 0, dy: box 1).  Block-path heads: x by
-        // exp(cs_end - cs_j) dt_j.  Separable heads: x by b_j = exp(-cs_j) dt_j (the operand of their W product as well),
-        // and the missing exp(cs_end) goes onto their rows of the dS_end box.
-        w.wait(&bars.in_full[ib], par(kb, NIN), 54);
-        w.wait(&bars.wraw_done[ib], par(kb, NIN), 55);
-        uint8_t* xb = sIn + ib * Cfg::IN_BYTES;
-        // four 16-byte pieces per thread (x box: two, dy box: two): all loads first, then the factors, then the arithmetic,
-        // so that one warp has several independent chains in flight (four decay warps share a scheduler)
-        {
-          uint32_t adr[4];
-          uint4 raw[4];
-          float fac[4];
-#pragma unroll
-          for (int r = 0; r < 4; ++r) {
-            const int idx = tid + r * 512;
-            const int box = idx >> 10, l = (idx >> 3) & 127, pc = idx & 7;
-            adr[r] = smem_u32(xb + box * BOX_BYTES + l * 128 + pc * 16);
-            raw[r] = ld_shared_v4(adr[r]);
-          }
-#pragma unroll
-          for (int r = 0; r < 4; ++r) {
-            const int idx = tid + r * 512;
-            const int box = idx >> 10, l = (idx >> 3) & 127, pc = idx & 7;
-            const int hl = (((pc ^ l) & 7) * 8) / P;
-            const uint32_t tt = tbs + hl * TAB_BYTES;
-            const float csl = lds_f32(tt + 4 * (T_CS + l));
-            fac[r] = box ? ex2(csl)
-                         : (is_sep(h0 + hl) ? ex2(-csl) : ex2(lds_f32(tt + 4 * (T_CS + 127)) - csl)) * lds_f32(tt + 4 * (T_DT + l));
-          }
-#pragma unroll
-          for (int r = 0; r < 4; ++r) raw[r] = scale8_bf16(raw[r], fac[r]);
-#pragma unroll
-          for (int r = 0; r < 4; ++r) st_shared_v4(adr[r], raw[r].x, raw[r].y, raw[r].z, raw[r].w);
-        }
-        if (anysep) {
-          w.wait(&bars.st_full[sb], par(kb, NST), 61);
-          const int r = tid >> 3;                      // row (h,p) of the 64 x 64 dS_end box, one 16-byte piece per thread
-          const int hl = r / P;
-          if (is_sep(h0 + hl)) {
-            const float f = ex2(lds_f32(tbs + hl * TAB_BYTES + 4 * (T_CS + 127)));
-            const uint32_t a = smem_u32(sSt + sb * Cfg::ST_BYTES + SBOX_BYTES + r * 128 + (tid & 7) * 16);
-            const uint4 o = scale8_bf16(ld_shared_v4(a), f);
-            st_shared_v4(a, o.x, o.y, o.z, o.w);
-          }
-        }
-        fence_async_smem();
-        __syncwarp();
-        if (lane == 0) { mbar_arrive(&bars.sc_full[ib]); mbar_arrive(&bars.tab_empty[ts]); }
-      }
-      if (anysep) {   // the separable heads' sum: mask to the lower triangle, hand over like one more W'_h
-        w.wait(&bars.wsep_full, ksep & 1, 62);
-        ++ksep;
-        w.wait(&bars.m_empty, (kh & 1) ^ 1, 53);
-        tc_fence_after();
-        mask_tril_tile(tmWsep, row, part, warp, smem_u32(sM));
-        fence_async_smem();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) { mbar_arrive(&bars.m_full); mbar_arrive(&bars.wsep_empty); }
-        ++kh;
-      }
-    }
-  } else if (warp >= 20) {
-    // ------------------------------------------------------------------ epilogue warps: dC, dB of a finished tile
-    reg_dec<48>();
-    const int ew = warp - 20;
-    const int row = (ew & 3) * 32 + lane, half = ew >> 2;     // 32 of the 64 columns
-    for (int t = 0; t < my_tiles; ++t) {
-      int b, grp, c;
-      tile_coords(t, b, grp, c);
-      w.wait(&bars.acc_full, t & 1, 56);
-      tc_fence_after();
-      const size_t o = (((size_t)b * g.L + c * QT + row) * g.G + grp) * N + half * 32;
-#pragma unroll
-      for (int j = 0; j < 32; j += 16) {
-        float vc[16], vb[16];
-        tmem_ld16(tmem_addr(tmDC, (ew & 3) * 32, half * 32 + j), vc);
-        tmem_ld16(tmem_addr(tmDB, (ew & 3) * 32, half * 32 + j), vb);
-        if (j == 16) {   // both accumulators are in registers: hand them back before the stores
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&bars.acc_empty);
-        }
-        if (c * QT + row < g.L) {   // a ragged sequence ends inside its last tile
-          st_global_32B(dC + o + j,
-                        make_uint4(pack_bf16(vc[0], vc[1]), pack_bf16(vc[2], vc[3]), pack_bf16(vc[4], vc[5]), pack_bf16(vc[6], vc[7])),
-                        make_uint4(pack_bf16(vc[8], vc[9]), pack_bf16(vc[10], vc[11]), pack_bf16(vc[12], vc[13]), pack_bf16(vc[14], vc[15])));
-          st_global_32B(dB + o + j,
-                        make_uint4(pack_bf16(vb[0], vb[1]), pack_bf16(vb[2], vb[3]), pack_bf16(vb[4], vb[5]), pack_bf16(vb[6], vb[7])),
-                        make_uint4(pack_bf16(vb[8], vb[9]), pack_bf16(vb[10], vb[11]), pack_bf16(vb[12], vb[13]), pack_bf16(vb[14], vb[15])));
-        }
-        __syncwarp();
-      }
-    }
-  }
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 17) tmem_dealloc(tm, 512);
-}
-
-// ---------------------------------------------------------------------------------------------
-// dB, dC at dstate 128, persistent and warp-specialised; the arithmetic of k_dbc_tc with SUMW (the decayed tiles W'_h of a
-// group's heads are summed in registers, the sum is multiplied with B and C once per tile).  k_dbc_tc walks the heads with all
-// of its warps in one phase after another (product, decay, scaling, state products: 2.6 us per head where the operands of a
-// head need 1.5 us of memory time); here the phases of neighbouring heads overlap:
-//   * warp 16: TMA.  A ring of three 32 KB slots holds {x box, dy box} of a head block, and after a tile's last block its C
-//     tile and its B tile (needed once, at the end of the tile: a buffer of their own would cost a slot); a ring of two for the
-//     {S_prev, dS_end} boxes, one of four for the decay tables;
-//   * warp 17: MMA issue.  W products one block ahead into two accumulators, state products, and the tile's two products;
+// dB, dC, persistent and warp-specialised; the arithmetic of k_dbc_tc with SUMW (the decayed tiles W'_h of a group's heads are
+// summed in registers, the sum is multiplied with B and C once per tile).  k_dbc_tc walks the heads with all of its warps in
+// one phase after another (product, decay, scaling, state products: 2.6 us per head where the operands of a head need 1.5 us
+// of memory time at dstate 128); here the phases of neighbouring heads overlap:
+//   * warp 16: TMA.  A ring of three (dstate 64: four) 32 KB slots holds {x box, dy box} of a head block, and after a tile's
+//     last block its C and B tiles (needed once, at the end of the tile: a buffer of their own would cost slots); a ring for
+//     the {S_prev, dS_end} boxes, one of four for the decay tables;
+//   * warp 17: MMA issue.  W products one block ahead into two (three) accumulators, state products, the tile's two products;
 //   * warps 0-15: W -> decay -> register sum (thread = row x 32 columns) -> the M tile;
 //   * warps 20-27: scale the boxes in place for the state products, and drain dC / dB of a finished tile.
-// TMEM: two W accumulators, dC, dB = 512 columns.  2x131072, 24 heads: 0.97 -> 0.64 ms = 5.1 TB/s, what a pure TMA stream of
-// boxes reaches; 16x4096: 0.27 -> 0.19 ms (3.46 waves of tiles take the time of four).
-template <int P>
-struct DsCfg {
-  static constexpr int N = 128, HB = 64 / P, NT = 4, NIN = 3, NST = 2;
-  static constexpr int IN_BYTES = 2 * BOX_BYTES;             // x box, dy box; or the C (B) tile
-  static constexpr int ST_BYTES = 4 * SBOX_BYTES;            // S_prev, dS_end: two boxes each
+// TMEM: the W accumulators, dC, dB = 512 columns.
+// dstate 128: 2x131072 with 24 heads 0.97 -> 0.64 ms = 5.1 TB/s, what a pure TMA stream of boxes reaches; 16x4096 0.27 -> 0.185
+// ms (3.46 waves of tiles take the time of four).  dstate 64, 512x1024 with 8 heads: 0.278 ms whatever the decay; a kernel that
+// carried the decay on the operands where its range allowed took 0.290, and 0.394 with one head beyond the range.  There the
+// issue slots bound it: 0.339 with 32 columns of W in registers beside the sums (spills), 0.306 with 16, 0.301 with packed
+// scaling of the boxes, 0.278 with packed FMAs and without the six warps whose blocks lie above the diagonal.
+template <int P, int N_>
+struct DbCfg {
+  static constexpr int N = N_, NB64 = N / 64, HB = 64 / P, NT = 4, NIN = N == 64 ? 4 : 3, NST = N == 64 ? 3 : 2;
+  static constexpr int NCB = NB64;                           // uses of the input ring for a tile's C and B (dstate 64: both in one)
+  static constexpr int NW = N == 64 ? 3 : 2;                 // W accumulators
+  static constexpr int IN_BYTES = 2 * BOX_BYTES;             // x box, dy box; or C and B of a tile
+  static constexpr int ST_BYTES = 2 * NB64 * SBOX_BYTES;     // S_prev, dS_end
   static constexpr int TB_BYTES = HB * TAB_BYTES;
-  static constexpr int W_SCALE = 20, NSCALE = 8;
+  static constexpr int W_SCALE = 20, NSCALE = 8, NDECAY = 10;   // decay warps with a block on or below the diagonal
   static constexpr size_t SMEM = 1024 + 2 * BOX_BYTES + NIN * IN_BYTES + NST * ST_BYTES + NT * TB_BYTES;
   static_assert(SMEM <= 232448 - 512, "shared-memory plan exceeds the 227 KB a CTA can have");
 };
 
-template <int P>
+template <int P, int N_>
 __global__ void __launch_bounds__(WS_THREADS, 1)
-k_dbc_sum_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmDY,
-             const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmC,
-             const __grid_constant__ CUtensorMap tmS, const __grid_constant__ CUtensorMap tmDS,
-             const float* __restrict__ tab, bf16* __restrict__ dB, bf16* __restrict__ dC, int* __restrict__ status) {
-  using Cfg = DsCfg<P>;
-  constexpr int N = Cfg::N, HB = Cfg::HB, NIN = Cfg::NIN, NST = Cfg::NST, NT = Cfg::NT;
+k_dbc_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmDY,
+         const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmC,
+         const __grid_constant__ CUtensorMap tmS, const __grid_constant__ CUtensorMap tmDS,
+         const float* __restrict__ tab, bf16* __restrict__ dB, bf16* __restrict__ dC, int* __restrict__ status) {
+  using Cfg = DbCfg<P, N_>;
+  constexpr int N = Cfg::N, HB = Cfg::HB, NIN = Cfg::NIN, NST = Cfg::NST, NT = Cfg::NT, NB64 = Cfg::NB64, NCB = Cfg::NCB, NW = Cfg::NW;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);   // 1 KB aligned, still known to be shared memory
   uint8_t* sM = smem;                                    // the masked sum of a tile's W'_h
@@ -3107,7 +2696,7 @@ k_dbc_sum_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_consta
   uint8_t* sSt = sIn + NIN * Cfg::IN_BYTES;              // NST x {S_prev, dS_end}
   uint8_t* sTab = sSt + NST * Cfg::ST_BYTES;             // NT x decay tables of a head block
   __shared__ __align__(8) uint64_t in_full[NIN], in_empty[NIN], raw_done[NIN], sc_full[NIN], st_full[NST], st_empty[NST], tab_full[NT],
-      tab_empty[NT], w_full[2], w_empty[2], m_full, m_empty, acc_full, acc_empty;
+      tab_empty[NT], w_full[NW], w_empty[NW], m_full, m_empty, acc_full, acc_empty;
   __shared__ uint32_t tmem_slot;
   __shared__ int s_abort;
 
@@ -3118,9 +2707,9 @@ k_dbc_sum_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_consta
       mbar_init(&raw_done[i], 1); mbar_init(&sc_full[i], Cfg::NSCALE);
     }
     for (int i = 0; i < NST; ++i) { mbar_init(&st_full[i], 1); mbar_init(&st_empty[i], 1); }
-    for (int i = 0; i < NT; ++i) { mbar_init(&tab_full[i], 1); mbar_init(&tab_empty[i], 16 + Cfg::NSCALE); }
-    for (int i = 0; i < 2; ++i) { mbar_init(&w_full[i], 1); mbar_init(&w_empty[i], 16); }
-    mbar_init(&m_full, 16); mbar_init(&m_empty, 1);
+    for (int i = 0; i < NT; ++i) { mbar_init(&tab_full[i], 1); mbar_init(&tab_empty[i], Cfg::NDECAY + Cfg::NSCALE); }
+    for (int i = 0; i < NW; ++i) { mbar_init(&w_full[i], 1); mbar_init(&w_empty[i], Cfg::NDECAY); }
+    mbar_init(&m_full, Cfg::NDECAY); mbar_init(&m_empty, 1);
     mbar_init(&acc_full, 1); mbar_init(&acc_empty, Cfg::NSCALE);
     mbar_fence_init();
   }
@@ -3139,7 +2728,7 @@ k_dbc_sum_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_consta
     if (warp == 17) tmem_dealloc(tm, 512);
     return;
   }
-  const uint32_t tmDC = tm + 256, tmDB = tm + 384;
+  const uint32_t tmDC = tm + NW * 128, tmDB = tmDC + N;
   Waiter w{status, false};
 
   const int nblk = g.hpg / HB;
@@ -3153,7 +2742,7 @@ k_dbc_sum_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_consta
     b = r / g.G;
   };
   // use n (0, 1, 2, ...) of a ring of depth D sits in slot n % D; its `full` wait has parity (n / D) & 1, its `empty` wait the
-  // opposite (a fresh barrier passes a wait on parity 1).  kb counts head blocks, ki the uses of the input ring: nblk + 2 per
+  // opposite (a fresh barrier passes a wait on parity 1).  kb counts head blocks, ki the uses of the input ring: nblk + NCB per
   // tile.  raw_done and sc_full go by kb: block kb + NIN is loaded only after block kb's state products.
   auto par = [](int n, int depth) { return (uint32_t)((n / depth) & 1); };
 
@@ -3180,18 +2769,19 @@ k_dbc_sum_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_consta
           w.wait(&st_empty[sb], par(kb, NST) ^ 1, 50);
           uint8_t* sd = sSt + sb * Cfg::ST_BYTES;
           mbar_expect_tx(&st_full[sb], Cfg::ST_BYTES);
-          for (int j = 0; j < 2; ++j) {
+          for (int j = 0; j < NB64; ++j) {
             tma_load_3d(sd + j * SBOX_BYTES, &tmS, 64 * j, h0 * P, b * g.nc + c, &st_full[sb]);
-            tma_load_3d(sd + (2 + j) * SBOX_BYTES, &tmDS, 64 * j, h0 * P, b * g.nc + c, &st_full[sb]);
+            tma_load_3d(sd + (NB64 + j) * SBOX_BYTES, &tmDS, 64 * j, h0 * P, b * g.nc + c, &st_full[sb]);
           }
         }
-        for (int side = 0; side < 2; ++side, ++ki) {   // C, then B
+        for (int n = 0; n < NCB; ++n, ++ki) {   // C, then B: NB64 boxes each, two boxes to a slot
           const int ib = ki % NIN;
-          uint8_t* dst = sIn + ib * Cfg::IN_BYTES;
           w.wait(&in_empty[ib], par(ki, NIN) ^ 1, 41);
           mbar_expect_tx(&in_full[ib], Cfg::IN_BYTES);
-          for (int j = 0; j < 2; ++j)
-            tma_load_3d(dst + j * BOX_BYTES, side ? &tmB : &tmC, grp * N + 64 * j, c * QT, b, &in_full[ib]);
+          for (int j = 0; j < 2; ++j) {
+            const int box = 2 * n + j;
+            tma_load_3d(sIn + ib * Cfg::IN_BYTES + j * BOX_BYTES, box >= NB64 ? &tmB : &tmC, grp * N + 64 * (box % NB64), c * QT, b, &in_full[ib]);
+          }
         }
       }
     }
@@ -3207,12 +2797,12 @@ k_dbc_sum_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_consta
         const uint32_t inb = smem_u32(sIn + ib * Cfg::IN_BYTES);
         const uint64_t dX0 = desc_sw128_k(inb, 0), dDY0 = desc_sw128_k(inb + BOX_BYTES, 0);
         for (int hl = 0; hl < HB; ++hl, ++kw) {
-          w.wait(&w_empty[kw & 1], par(kw, 2) ^ 1, 58);
+          w.wait(&w_empty[kw % NW], par(kw, NW) ^ 1, 58);
           tc_fence_after();
 #pragma unroll
           for (int ks = 0; ks < P / 16; ++ks)
-            mma_bf16(tm + (kw & 1) * 128, desc_adv(dDY0, hl * P * 2 + ks * 32), desc_adv(dX0, hl * P * 2 + ks * 32), idW, ks > 0);
-          mma_commit(&w_full[kw & 1]);
+            mma_bf16(tm + (kw % NW) * 128, desc_adv(dDY0, hl * P * 2 + ks * 32), desc_adv(dX0, hl * P * 2 + ks * 32), idW, ks > 0);
+          mma_commit(&w_full[kw % NW]);
         }
         mma_commit(&raw_done[kbn % NIN]);
       };
@@ -3224,7 +2814,7 @@ k_dbc_sum_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_consta
           const int ib = ki % NIN, sb = kb % NST;
           const uint32_t inb = smem_u32(sIn + ib * Cfg::IN_BYTES), stb = smem_u32(sSt + sb * Cfg::ST_BYTES);
           const uint64_t dXk = desc_sw128_k(inb, 0), dDYk = desc_sw128_k(inb + BOX_BYTES, 0);
-          const uint64_t dSm0 = desc_sw128_mn(stb, 0, 0, SBOX_BYTES), dDSm0 = desc_sw128_mn(stb + 2 * SBOX_BYTES, 0, 0, SBOX_BYTES);
+          const uint64_t dSm0 = desc_sw128_mn(stb, 0, 0, SBOX_BYTES), dDSm0 = desc_sw128_mn(stb + NB64 * SBOX_BYTES, 0, 0, SBOX_BYTES);
           w.wait(&st_full[sb], par(kb, NST), 57);
           w.wait(&sc_full[kb % NIN], par(kb, NIN), 59);
           tc_fence_after();
@@ -3236,23 +2826,21 @@ k_dbc_sum_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_consta
           mma_commit(&in_empty[ib]);
           mma_commit(&st_empty[sb]);
         }
-        const int ic = ki % NIN, ibb = (ki + 1) % NIN;
-        w.wait(&in_full[ic], par(ki, NIN), 43);
-        w.wait(&in_full[ibb], par(ki + 1, NIN), 44);
+        for (int n = 0; n < NCB; ++n) w.wait(&in_full[(ki + n) % NIN], par(ki + n, NIN), 43);
         w.wait(&m_full, t & 1, 47);
         tc_fence_after();
-        const uint64_t dCm0 = desc_sw128_mn(smem_u32(sIn + ic * Cfg::IN_BYTES), 0, 0, BOX_BYTES),
-                       dBm0 = desc_sw128_mn(smem_u32(sIn + ibb * Cfg::IN_BYTES), 0, 0, BOX_BYTES);
+        const uint32_t ct = smem_u32(sIn + (ki % NIN) * Cfg::IN_BYTES),
+                       bt = NCB == 2 ? smem_u32(sIn + ((ki + 1) % NIN) * Cfg::IN_BYTES) : ct + BOX_BYTES;
+        const uint64_t dCm0 = desc_sw128_mn(ct, 0, 0, BOX_BYTES), dBm0 = desc_sw128_mn(bt, 0, 0, BOX_BYTES);
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks) {
           mma_bf16(tmDC, desc_adv(dMk, ks * 4096), desc_adv(dBm0, ks * 2048), idC, true);
           mma_bf16(tmDB, desc_adv(dMt, ks * 256), desc_adv(dCm0, ks * 2048), idB, true);
         }
-        mma_commit(&in_empty[ic]);
-        mma_commit(&in_empty[ibb]);
+        for (int n = 0; n < NCB; ++n) mma_commit(&in_empty[(ki + n) % NIN]);
         mma_commit(&m_empty);
         mma_commit(&acc_full);
-        ki += 2;
+        ki += NCB;
       }
     }
   } else if (warp < 16) {
@@ -3260,7 +2848,7 @@ k_dbc_sum_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_consta
     reg_inc<80>();
     const int row = tid & 127, part = tid >> 7;
     int kb = 0, kw = 0;
-    for (int t = 0; t < my_tiles; ++t) {
+    for (int t = part <= (warp & 3) ? 0 : my_tiles; t < my_tiles; ++t) {   // the blocks above the diagonal have no work
       float acc[32];
 #pragma unroll
       for (int k = 0; k < 32; ++k) acc[k] = 0.f;
@@ -3269,12 +2857,12 @@ k_dbc_sum_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_consta
         const float* tb = (const float*)(sTab + ts * Cfg::TB_BYTES);
         w.wait(&tab_full[ts], par(kb, NT), 52);
         for (int hl = 0; hl < HB; ++hl, ++kw) {
-          w.wait(&w_full[kw & 1], par(kw, 2), 51);
+          w.wait(&w_full[kw % NW], par(kw, NW), 51);
           tc_fence_after();
-          decay_acc_block(tm + (kw & 1) * 128, tb + hl * TAB, row, part, warp, acc);
+          decay_acc_block(tm + (kw % NW) * 128, tb + hl * TAB, row, part, warp, acc);
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive(&w_empty[kw & 1]);
+          if (lane == 0) mbar_arrive(&w_empty[kw % NW]);
         }
         if (reads_done(__float_as_uint(acc[0]) ^ __float_as_uint(acc[15]) ^ __float_as_uint(acc[16]) ^ __float_as_uint(acc[31]), lane))
           mbar_arrive(&tab_empty[ts]);
@@ -3289,7 +2877,7 @@ k_dbc_sum_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_consta
     // ------------------------------------------------------------------ scaling warps, and the drain of a finished tile
     reg_dec<56>();
     const int sid = tid - Cfg::W_SCALE * 32, ew = warp - Cfg::W_SCALE;
-    const int row = (ew & 3) * 32 + lane, half = ew >> 2;     // 64 of the 128 columns
+    const int row = (ew & 3) * 32 + lane, half = ew >> 2;     // half of the columns
     int kb = 0, ki = 0;
     for (int t = 0; t < my_tiles; ++t) {
       for (int blk = 0; blk < nblk; ++blk, ++kb, ++ki) {
@@ -3314,11 +2902,16 @@ k_dbc_sum_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_consta
           }
 #pragma unroll
           for (int r = 0; r < 4; ++r) {
-            float v[8];
-            unpack8(raw[r], v);
+            uint4 o;
+            if constexpr (N == 64) {
+              o = scale8_bf16(raw[r], fac[r]);
+            } else {
+              float v[8];
+              unpack8(raw[r], v);
 #pragma unroll
-            for (int k = 0; k < 8; ++k) v[k] *= fac[r];
-            const uint4 o = pack8(v);
+              for (int k = 0; k < 8; ++k) v[k] *= fac[r];
+              o = pack8(v);
+            }
             st_shared_v4(xb + box * BOX_BYTES + (sid + r * 256) * 16, o.x, o.y, o.z, o.w);
           }
         }
@@ -3326,19 +2919,19 @@ k_dbc_sum_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_consta
         __syncwarp();
         if (lane == 0) { mbar_arrive(&sc_full[kb % NIN]); mbar_arrive(&tab_empty[ts]); }
       }
-      ki += 2;
+      ki += NCB;
       int b, grp, c;
       tile_coords(t, b, grp, c);
       w.wait(&acc_full, t & 1, 56);
       tc_fence_after();
-      const size_t o = (((size_t)b * g.L + c * QT + row) * g.G + grp) * N + half * 64;
+      const size_t o = (((size_t)b * g.L + c * QT + row) * g.G + grp) * N + half * (N / 2);
 #pragma unroll
-      for (int j = 0; j < 64; j += 16) {
+      for (int j = 0; j < N / 2; j += 16) {
 #pragma unroll
         for (int side = 0; side < 2; ++side) {
           float v[16];
-          tmem_ld16(tmem_addr(side ? tmDB : tmDC, (ew & 3) * 32, half * 64 + j), v);
-          if (j == 48 && side == 1) {
+          tmem_ld16(tmem_addr(side ? tmDB : tmDC, (ew & 3) * 32, half * (N / 2) + j), v);
+          if (j + 16 == N / 2 && side == 1) {
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&acc_empty);
@@ -3620,23 +3213,13 @@ int launch_bwd_tc(const Geo& g, const SeqMaps& m, const float* tab, const float*
   return SSD_OK;
 }
 
-template <int P>
-int launch_dbc_ws(const Geo& g, const SeqMaps& m, const float* tab, const float* hmax, void* dB, void* dC, int* status, cudaStream_t s) {
-  const int ntiles = g.B * g.G * g.nc;
-  const int grid = ntiles < sm_count() ? ntiles : sm_count();
-  launch<k_dbc_ws<P>>(grid, WS_THREADS, DbCfg<P>::SMEM, s, g, m.x, m.dy, m.b, m.c, m.s, m.ds, tab, hmax, (bf16*)dB, (bf16*)dC, status);
-  SSD_CUDA_CHECK_LAUNCH("dBdC_ws");
-  return SSD_OK;
-}
-
 template <int P, int N>
-int launch_dbc(const Geo& g, const SeqMaps& m, const float* tab, const float* hmax, void* dB, void* dC, int* status, cudaStream_t s) {
-  if (N == 64 && !g.onetile) return launch_dbc_ws<P>(g, m, tab, hmax, dB, dC, status, s);
-  if (N == 128 && !g.onetile) {
+int launch_dbc(const Geo& g, const SeqMaps& m, const float* tab, void* dB, void* dC, int* status, cudaStream_t s) {
+  if (!g.onetile) {
     const int ntiles = g.B * g.G * g.nc;
-    launch<k_dbc_sum_ws<P>>(ntiles < sm_count() ? ntiles : sm_count(), WS_THREADS, DsCfg<P>::SMEM, s, g, m.x, m.dy, m.b, m.c, m.s, m.ds,
-                            tab, (bf16*)dB, (bf16*)dC, status);
-    SSD_CUDA_CHECK_LAUNCH("dBdC_sum_ws");
+    launch<k_dbc_ws<P, N>>(ntiles < sm_count() ? ntiles : sm_count(), WS_THREADS, DbCfg<P, N>::SMEM, s, g, m.x, m.dy, m.b, m.c, m.s, m.ds,
+                           tab, (bf16*)dB, (bf16*)dC, status);
+    SSD_CUDA_CHECK_LAUNCH("dBdC_ws");
     return SSD_OK;
   }
   launch<k_dbc_tc<P, N>>(dim3(g.nc, g.G, g.B), TC_THREADS, dbc_smem<P, N>(), s, g, m.x, m.dy, m.b, m.c, m.s, m.ds, tab, (bf16*)dB,
@@ -3863,12 +3446,12 @@ int tensor_bwd_merged(const Geo& g, const SsdBwdPtrs& p, const float* tab, const
   return launch_bwd_ws<64>(g, m, tab, p.D, p.dx, dcsp, ddot, ddtd, status, s);
 }
 
-int tensor_dbc(const Geo& g, const SsdBwdPtrs& p, const void* dyp, bool dy_dense, const float* tab, const float* hmax,
+int tensor_dbc(const Geo& g, const SsdBwdPtrs& p, const void* dyp, bool dy_dense, const float* tab,
                const void* prev_bf, const void* ds_bf, int* status, cudaStream_t s) {
   SeqMaps m;
   int rc = make_maps(g, p.x, dyp, dy_dense, p.Bm, p.Cm, prev_bf, ds_bf, &m);
   if (rc) return rc;
-#define CALL(PP, NN) return launch_dbc<PP, NN>(g, m, tab, hmax, p.dB, p.dC, status, s);
+#define CALL(PP, NN) return launch_dbc<PP, NN>(g, m, tab, p.dB, p.dC, status, s);
   DISPATCH_PN(CALL)
 #undef CALL
 }
