@@ -283,3 +283,29 @@ def test_split_heads_are_the_same_bits(lib, H, P, N, G, Bn, has_z):
     for k in ("y", "dx", "ddt", "dB", "dC") + (("dz",) if has_z else ()):
         assert_close(k, got[k], ref[k], "bf16")
         assert torch.equal(got[k], whole[k][:2]), k
+
+
+@pytest.mark.parametrize("H,P,N,Bn,L", [(24, 64, 128, 14, 1100), (8, 32, 64, 80, 1700)])
+def test_balanced_state_scan_is_the_same_bits(lib, H, P, N, Bn, L):
+    """More units than SMs and a last wave far from full: units are cut between neighbouring blocks, which hand the running
+    state over.  A row's results are those of the row in a small batch, again and again over one forward."""
+    import trading_bot_0_b200 as T
+    inp = O.make_inputs(O.SsdConfig("bal", Bn, L, H, P, N, 1, 128, "bf16", False), with_init_state=True)
+    dfinal = 0.1 * torch.randn(Bn, H, P, N, generator=torch.Generator().manual_seed(4))
+    d = to_dev(inp, DEV)
+
+    def run(rows, times):
+        a = (d["x"][rows], d["dt"][rows], d["A"], d["B"][rows], d["C"][rows], d["D"], None, d["init_state"][rows])
+        y, fin, ws = T.forward(*a, chunk=128, algo="tensor", for_backward=True)
+        for _ in range(times):
+            g = T.backward(d["dy"][rows], *a, dfinal[rows].to(DEV), chunk=128, algo="tensor", workspace=ws, fwd_saved=True,
+                           want_dinit=True)
+        torch.cuda.synchronize()
+        assert status_word(ws) == 0
+        return {"y": y, "final_state": fin, **g}
+
+    whole = run(slice(0, Bn), 3)
+    for r in range(0, Bn, max(1, Bn // 10)):
+        row = run(slice(r, r + 1), 1)
+        for k in ("y", "final_state", "dx", "ddt", "dB", "dC", "dinit"):
+            assert torch.equal(whole[k][r:r + 1], row[k]), (k, r)

@@ -224,12 +224,17 @@ __device__ __forceinline__ size_t cb_idx(const Geo& g, int b, int c, int grp) {
 template <typename T, int HG>
 __global__ void __launch_bounds__(256) k_cumsum(Geo g, const T* __restrict__ dt, const float* __restrict__ dt_bias,
                                                const float* __restrict__ A, float* __restrict__ cs,
-                                               float* __restrict__ dtf, float* __restrict__ tab, int* __restrict__ status) {
+                                               float* __restrict__ dtf, float* __restrict__ tab, int* __restrict__ hand,
+                                               int* __restrict__ status) {
   pdl_wait();
   const int c = blockIdx.x, b = blockIdx.y, q = threadIdx.x;
   __shared__ float wsum[8][HG];
   const int t = c * g.Q + q;
-  if (c == 0 && b == 0 && blockIdx.z == 0 && q == 0) *status = 0;   // first kernel of a pass
+  if (c == 0 && blockIdx.z == 0) {   // first kernel of a pass: the status word, the counters of the state scan
+    if (b == 0 && q == 0) *status = 0;
+    if (hand)
+      for (int i = q, n = g.H * g.P / 128; i < n; i += blockDim.x) hand[b * n + i] = 0;
+  }
   const bool live = (q < g.Q) && (t < g.L);
   const int lane = q & 31, w = q >> 5;
   const T* row = dt + b * g.dtsb + (long long)t * g.dtsl;
@@ -1018,7 +1023,7 @@ static int fwd_stages_t(const Geo& g, bool tc, const SsdFwdPtrs& p, char* ws, co
     const bool wide = (long long)g.nc * g.B >= 2LL * sm_count();
     auto cumsum = [&](auto kernel) {
       launch<kernel.value>(dim3(g.nc, g.B, wide ? 1 : cdiv(g.H, 2)), g.Q <= 128 ? 128 : 256, 0, s, g, (const T*)p.dt, p.dt_bias, p.A, cs, dtf,
-                           tc ? tab : nullptr, status);
+                           tc ? tab : nullptr, tc ? (int*)(ws + w.hand) : nullptr, status);
     };
     wide ? cumsum(Fn<k_cumsum<T, 8>>()) : cumsum(Fn<k_cumsum<T, 2>>());
     SSD_CUDA_CHECK_LAUNCH("cumsum");
@@ -1045,7 +1050,7 @@ static int fwd_stages_t(const Geo& g, bool tc, const SsdFwdPtrs& p, char* ws, co
   if (stages & SSD_STAGE_FINISH) {
     if (tc && fused) {
       // no fp32 copy of the chunk-entry states: every reader in this family takes the bf16 one
-      int rc = tensor_state_fused(g, 0, p.x, g.xsb, g.xsl, p.Bm, g.bsb, g.bsl, tab, states, prev_bf,
+      int rc = tensor_state_fused(g, 0, p.x, g.xsb, g.xsl, p.Bm, g.bsb, g.bsl, tab, states, (int*)(ws + w.hand), prev_bf,
                                   p.init_state, fin, fin2, nullptr, nullptr, nullptr, nullptr, status, s);
       if (rc) return rc;
     } else if (tc) {
@@ -1156,7 +1161,7 @@ static int bwd_stages_t(const Geo& g, bool tc, const SsdBwdPtrs& p, char* ws, co
     if (tc && fused) {
       // local state gradients, the reverse scan and the <dS_end, S_end> partial sums in one kernel (no fp32 copy is kept)
       int rc = tensor_state_fused(g, 1, tc_dy, tc_dense ? (long long)g.L * g.H * g.P : g.ysb,
-                                  tc_dense ? (long long)g.H * g.P : g.ysl, p.Cm, g.csb, g.csl, tab, dst, ds_bf,
+                                  tc_dense ? (long long)g.H * g.P : g.ysl, p.Cm, g.csb, g.csl, tab, dst, (int*)(ws + w.hand), ds_bf,
                                   p.dfinal_state, dini, nullptr, prev_bf, fin, sdot, &sdot_nw, status, s);
       if (rc) return rc;
     } else if (tc) {

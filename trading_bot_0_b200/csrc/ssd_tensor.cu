@@ -52,6 +52,20 @@ struct Waiter {
       atomicExch(status, code);
     }
   }
+  // bounded wait for a count in global memory that warps of another block of the grid add to
+  __device__ __forceinline__ void wait_count(const int* p, int n, int code) {
+    if (dead) return;
+    const long long t0 = clock64();
+    for (;;) {
+      int v;
+      asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+      if (v >= n) return;
+      if (clock64() - t0 > 4000000000LL) break;
+      __nanosleep(64);
+    }
+    dead = true;
+    atomicExch(status, code);
+  }
 };
 
 // Self-test of the bounded wait: one warp waits on an mbarrier that nothing ever arrives on.  The wait gives up after
@@ -707,9 +721,16 @@ __global__ void __launch_bounds__(PsCfg<P, N_>::THREADS, 1) k_state_ps(Geo g, co
 // (TOT) walks every segment but the last from a zero state and leaves its total and its decay, the second folds the totals
 // before its segment into the state it starts from.  x and B are then read twice; fp32 states per chunk, written and read
 // back by a kernel of their own, would be twice that again (dstate 128) and leave the scan to a few hundred warps.
+// Where there are more units than SMs but the last wave is far from full (192 units on 148 SMs took the time of 296), every CTA
+// gets the same number of chunks instead (BAL): unit after unit, a unit that crosses the end of a CTA's share is continued by
+// the next CTA.  A CTA starts with that cut unit and publishes its state, then walks its whole units, and ends with the one it
+// takes over - by then long published, a share being longer than a unit.  CTA i waits only for CTA i - 1 and only for what that
+// one does first, so blocks placed in index order always get on; the wait is bounded all the same.  Same order of operations on
+// every unit: same bits.  16x4096, 24 heads: 154 -> 122 us forward, 210 -> 167 us backward.
 // Pipeline and barriers as in k_state_ps; the B (or C) tile changes with every tile, so it has a ring of its own.
-template <int P, int N_, int MODE, bool TOT>
+template <int P, int N_, int MODE, int KIND>
 struct PfCfg {
+  static constexpr bool TOT = KIND == 1, BAL = KIND == 2;
   // the backward kernel gives a slot of the x ring to the S_end tiles (128 rows x N bf16: one or two 16 KB boxes each)
   static constexpr bool SE = MODE == 1 && !TOT;
   static constexpr int N = N_, HT = 128 / P, NBX = N / 64, NX = (N == 64 ? 4 : 3) - (SE ? 1 : 0), NB = N == 64 ? 3 : 2;
@@ -733,14 +754,16 @@ struct StateScanArgs {
   const float* fwd_fin;   // MODE 1: forward final state
   float* sdot;            // MODE 1: [B,nc,H,SDOT_NW]
   int nseg, seglen;       // segments of the sequence, chunks in each (the last may be shorter)
-  float *tot, *tdec;      // [B,nseg,H,P,N] totals and [B,nseg,H] decays of the segments (nseg > 1)
+  float *tot, *tdec;      // [B,nseg,H,P,N] totals and [B,nseg,H] decays of the segments (nseg > 1); BAL: [B,H,P,N] states handed over
+  int* hand;              // BAL: per unit, warps that have written (16), then read, its state; zero before and after the launch
 };
 
-template <int P, int N_, int MODE, bool TOT>
-__global__ void __launch_bounds__(PfCfg<P, N_, MODE, TOT>::THREADS, 1)
+template <int P, int N_, int MODE, int KIND>
+__global__ void __launch_bounds__(PfCfg<P, N_, MODE, KIND>::THREADS, 1)
 k_state_scan_ps(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmB,
                 const __grid_constant__ CUtensorMap tmS, StateScanArgs a, int* __restrict__ status) {
-  using Cfg = PfCfg<P, N_, MODE, TOT>;
+  using Cfg = PfCfg<P, N_, MODE, KIND>;
+  constexpr bool TOT = Cfg::TOT, BAL = Cfg::BAL;
   constexpr int N = Cfg::N, HT = Cfg::HT, NX = Cfg::NX, NB = Cfg::NB, NQ = Cfg::NQ, NSE = Cfg::NSE;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);   // 1 KB aligned, still known to be shared memory
@@ -781,8 +804,18 @@ k_state_scan_ps(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_con
   // (Few members: the consumers hold one beside the running state.)
   const int nunits = g.B * g.G * (g.hpg * P / 128) * (TOT ? a.nseg - 1 : a.nseg);
   struct Walk {
-    int u, b, h0, grp, seg, s, s1;
-    __device__ __forceinline__ Walk(const Geo& g, const StateScanArgs& a) : u(blockIdx.x) { place(g, a); }
+    int u, b, h0, grp, seg, s, s0, s1;
+    __device__ __forceinline__ Walk(const Geo& g, const StateScanArgs& a, int nunits) {
+      if constexpr (BAL) {
+        const long long a1 = (long long)(blockIdx.x + 1) * nunits * g.nc / gridDim.x;
+        u = (int)(a1 / g.nc);
+        piece(g, a, 0, (int)(a1 - (long long)u * g.nc));   // the unit cut at the end of the share, first
+        if (s == s1) next_unit(g, a, nunits);
+      } else {
+        u = blockIdx.x;
+        place(g, a);
+      }
+    }
     __device__ __forceinline__ void place(const Geo& g, const StateScanArgs& a) {
       const int MT = g.hpg * P / 128;
       int r = u / MT;
@@ -790,25 +823,51 @@ k_state_scan_ps(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_con
       grp = r % g.G; r /= g.G;
       h0 += grp * g.hpg;
       b = r % g.B;
-      seg = r / g.B;
-      s = seg * a.seglen;
+      seg = BAL ? 0 : r / g.B;
+      s = s0 = seg * a.seglen;
       s1 = min(s + a.seglen, g.nc);
     }
-    __device__ __forceinline__ void next(const Geo& g, const StateScanArgs& a) {
-      if (++s == s1) { u += gridDim.x; place(g, a); }
+    __device__ __forceinline__ void piece(const Geo& g, const StateScanArgs& a, int from, int to) {
+      place(g, a);
+      s = s0 = from;
+      s1 = to;
+    }
+    __device__ __forceinline__ void next_unit(const Geo& g, const StateScanArgs& a, int nunits) {
+      if constexpr (BAL) {
+        const long long T = (long long)nunits * g.nc, a0 = blockIdx.x * T / gridDim.x, a1 = (blockIdx.x + 1) * T / gridDim.x;
+        const int first = (int)(a0 / g.nc), off = (int)(a0 - (long long)first * g.nc), last = (int)(a1 / g.nc);
+        u = u == last ? first + (off > 0) : u + 1;
+        if (u < last) {
+          piece(g, a, 0, g.nc);
+        } else {   // whole units done: the rest of the unit that the CTA before cut
+          u = first;
+          piece(g, a, off, g.nc);
+        }
+      } else {
+        u += gridDim.x;
+        place(g, a);
+      }
+    }
+    __device__ __forceinline__ void next(const Geo& g, const StateScanArgs& a, int nunits) {
+      if (++s == s1) next_unit(g, a, nunits);
     }
     __device__ __forceinline__ int chunk(const Geo& g) const { return MODE == 0 ? s : g.nc - 1 - s; }
   };
   int total = 0;   // tiles of this CTA
-  for (int u = blockIdx.x; u < nunits; u += gridDim.x) {
-    const int s0 = u / (nunits / (TOT ? a.nseg - 1 : a.nseg)) * a.seglen;
-    total += min(a.seglen, g.nc - s0);
+  if constexpr (BAL) {
+    const long long T = (long long)nunits * g.nc;
+    total = (int)((blockIdx.x + 1) * T / gridDim.x - blockIdx.x * T / gridDim.x);
+  } else {
+    for (int u = blockIdx.x; u < nunits; u += gridDim.x) {
+      const int s0 = u / (nunits / (TOT ? a.nseg - 1 : a.nseg)) * a.seglen;
+      total += min(a.seglen, g.nc - s0);
+    }
   }
 
   if (warp == Cfg::W_PROD) {
     if (lane == 0) {
-      Walk t(g, a);
-      for (int k = 0; k < total; ++k, t.next(g, a)) {
+      Walk t(g, a, nunits);
+      for (int k = 0; k < total; ++k, t.next(g, a, nunits)) {
         const int c = t.chunk(g), slot = k % NX, bs = k % NB;
         if (k >= NX) w.wait(&x_free[slot], ((k / NX) - 1) & 1, 14);
         const int col = t.h0 * P;
@@ -831,8 +890,8 @@ k_state_scan_ps(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_con
     // the epilogue reads itself)
     if (lane == 0 && want_sdot) {
       int k = 0;
-      Walk t(g, a);
-      for (int n = 0; n < total; ++n, t.next(g, a)) {
+      Walk t(g, a, nunits);
+      for (int n = 0; n < total; ++n, t.next(g, a, nunits)) {
         const int c = t.chunk(g);
         if (c + 1 >= g.nc) continue;
         const int slot = k % NSE;
@@ -916,7 +975,17 @@ k_state_scan_ps(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_con
       const int c = t.chunk(g);
       const size_t PNH = (size_t)g.H * P * N;
       const size_t e = ((size_t)t.h0 * P + row) * N + part * (N / PARTS);   // this thread's columns inside a [.., H, P, N] state
-      if (t.s == t.seg * a.seglen) {
+      if (BAL && t.s == t.s0 && t.s0 > 0) {   // the state the CTA before has published
+        if (lane == 0) w.wait_count(a.hand + t.u, 16, 63);
+        __syncwarp();
+        __threadfence();
+#pragma unroll
+        for (int j = 0; j < 16 * NQ; j += 4) {
+          const float4 v = __ldcg(reinterpret_cast<const float4*>(a.tot + t.b * PNH + e + j));
+          run[j] = v.x; run[j + 1] = v.y; run[j + 2] = v.z; run[j + 3] = v.w;
+        }
+        if (lane == 0 && atomicAdd(a.hand + t.u, 1) == 31) *(volatile int*)(a.hand + t.u) = 0;   // every warp has seen the count
+      } else if (t.s == t.s0) {
         if (!TOT && a.init) {
 #pragma unroll
           for (int j = 0; j < 16 * NQ; j += 4) {
@@ -1000,13 +1069,18 @@ k_state_scan_ps(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_con
           const size_t i = (size_t)t.b * a.nseg + t.seg;
           put(a.tot + i * PNH + e);
           if (part == 0 && row % P == 0) a.tdec[i * g.H + t.h0 + row / P] = pdec;
+        } else if (BAL && t.s1 < g.nc) {
+          put(a.tot + t.b * PNH + e);
+          __threadfence();
+          __syncwarp();
+          if (lane == 0) atomicAdd(a.hand + t.u, 1);
         } else if (t.seg == a.nseg - 1) {
           if (a.last) put(a.last + t.b * PNH + e);
           if (a.last2) put(a.last2 + t.b * PNH + e);
         }
       }
     };
-    Walk prev(g, a);
+    Walk prev(g, a, nunits);
     float dec_prev = 0.f;
     for (int k = 0; k < total; ++k) {
       const int slot = k % NX;
@@ -1023,7 +1097,7 @@ k_state_scan_ps(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_con
       scale_half(1, xs, tb);
       if (k > 0) {
         epilogue(k - 1, prev, dec_prev);
-        prev.next(g, a);
+        prev.next(g, a, nunits);
       }
       dec_prev = dec;
     }
@@ -3343,18 +3417,26 @@ static int launch_state_scan(const Geo& g, const CUtensorMap& tx, const CUtensor
                              int* status, cudaStream_t s) {
   const int units = g.B * g.G * (g.hpg * P / 128), n1 = units * (a.nseg - 1), n2 = units * a.nseg;
   if (n1) {
-    using C1 = PfCfg<P, N, MODE, true>;
-    launch<k_state_scan_ps<P, N, MODE, true>>(n1 < sm_count() ? n1 : sm_count(), C1::THREADS, C1::SMEM, s, g, tx, tb, ts, a, status);
+    using C1 = PfCfg<P, N, MODE, 1>;
+    launch<k_state_scan_ps<P, N, MODE, 1>>(n1 < sm_count() ? n1 : sm_count(), C1::THREADS, C1::SMEM, s, g, tx, tb, ts, a, status);
     SSD_CUDA_CHECK_LAUNCH(MODE == 0 ? "chunk_state_totals" : "dstate_totals");
   }
-  using C2 = PfCfg<P, N, MODE, false>;
-  launch<k_state_scan_ps<P, N, MODE, false>>(n2 < sm_count() ? n2 : sm_count(), C2::THREADS, C2::SMEM, s, g, tx, tb, ts, a, status);
+  // even shares where they save more than a twentieth (a hand-over costs a state's write and read per CTA); a share has to be
+  // longer than a unit
+  const int sms = sm_count();
+  if (units > sms && cdiv(units, sms) * sms > units + units / 20 && (long long)units * g.nc / sms > g.nc) {
+    using C3 = PfCfg<P, N, MODE, 2>;
+    launch<k_state_scan_ps<P, N, MODE, 2>>(sms, C3::THREADS, C3::SMEM, s, g, tx, tb, ts, a, status);
+  } else {
+    using C2 = PfCfg<P, N, MODE, 0>;
+    launch<k_state_scan_ps<P, N, MODE, 0>>(n2 < sms ? n2 : sms, C2::THREADS, C2::SMEM, s, g, tx, tb, ts, a, status);
+  }
   SSD_CUDA_CHECK_LAUNCH(MODE == 0 ? "chunk_state_scan" : "dstate_scan");
   return SSD_OK;
 }
 
 int tensor_state_fused(const Geo& g, int mode, const void* xdy, long long sb, long long sl, const void* bc, long long bsb,
-                       long long bsl, const float* tab, float* scratch, void* st_bf, const float* init, float* last, float* last2,
+                       long long bsl, const float* tab, float* scratch, int* hand, void* st_bf, const float* init, float* last, float* last2,
                        const void* fwd_prev_bf, const float* fwd_fin, float* sdot, int* sdot_nw, int* status, cudaStream_t s) {
   CUtensorMap tx, tb;
   int rc = make_seq_map(&tx, xdy, (long long)g.H * g.P, g.L, g.B, sl, sb, "x/dy");
@@ -3363,7 +3445,7 @@ int tensor_state_fused(const Geo& g, int mode, const void* xdy, long long sb, lo
   if (rc) return rc;
   const int seglen = cdiv(g.nc, state_segments(g, g.B * g.G * (g.hpg * g.P / 128))), nseg = cdiv(g.nc, seglen);
   const size_t PNH = (size_t)g.H * g.P * g.N;
-  StateScanArgs a{tab, st_bf, init, last, last2, fwd_prev_bf, fwd_fin, sdot, nseg, seglen, scratch, scratch + (size_t)g.B * nseg * PNH};
+  StateScanArgs a{tab, st_bf, init, last, last2, fwd_prev_bf, fwd_fin, sdot, nseg, seglen, scratch, scratch + (size_t)g.B * nseg * PNH, hand};
   if (sdot_nw) *sdot_nw = 4 * (g.P / 32);
   CUtensorMap ts = tx;   // a placeholder unless the backward kernel reads the forward states
   if (mode == 1 && sdot) {
