@@ -77,6 +77,12 @@ __global__ void k_selftest_wait(int* status, long long max_cycles) {
   if (!mbar_wait(&bar, 0, max_cycles) && threadIdx.x == 0) atomicExch(status, 99);
 }
 
+// a0 *= y0, a1 *= y1 as one packed instruction, same rounding as two (the decay passes are bound by issue slots)
+__device__ __forceinline__ void mul2(float& a0, float& a1, float y0, float y1) {
+  asm("{\n\t.reg .b64 a, y;\n\tmov.b64 a, {%0, %1};\n\tmov.b64 y, {%2, %3};\n\tmul.rn.f32x2 a, a, y;\n\tmov.b64 {%0, %1}, a;\n\t}"
+      : "+f"(a0), "+f"(a1) : "f"(y0), "f"(y1));
+}
+
 // ---------------------------------------------------------------------------------------------
 // Decayed lower-triangular tile.  Source: a 128x128 fp32 accumulator in TMEM (C B^T or dY X^T).
 // Result: out[i,j] = src[i,j] * exp(cs_i - cs_j) * dt_j for j <= i, written as bf16 into a plain
@@ -111,20 +117,25 @@ __device__ __forceinline__ void decay_mask_tile(uint32_t tm_src, const float* __
     if (cb < rb) {
       const float rf = ex2(csi - lds_f32(ts + 4 * (T_CS + cb * 32 + 31)));
       const float4 f0 = lds_v4f32(ts + 4 * (T_CF + c0)), f1 = lds_v4f32(ts + 4 * (T_CF + c0 + 4));
-      v[0] *= rf * f0.x; v[1] *= rf * f0.y; v[2] *= rf * f0.z; v[3] *= rf * f0.w;
-      v[4] *= rf * f1.x; v[5] *= rf * f1.y; v[6] *= rf * f1.z; v[7] *= rf * f1.w;
+      float f[8] = {f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, f1.z, f1.w};
+#pragma unroll
+      for (int k = 0; k < 8; k += 2) {
+        mul2(f[k], f[k + 1], rf, rf);
+        mul2(v[k], v[k + 1], f[k], f[k + 1]);
+      }
     } else {
       const int je = c0 + 7;
       const float4 d0 = lds_v4f32(ts + 4 * (T_DS + c0)), d1 = lds_v4f32(ts + 4 * (T_DS + c0 + 4));
       const float4 t0 = lds_v4f32(ts + 4 * (T_DT + c0)), t1 = lds_v4f32(ts + 4 * (T_DT + c0 + 4));
       const float ds[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};   // ds[k] = decay of step c0+k+1
-      const float dt[8] = {t0.x, t0.y, t0.z, t0.w, t1.x, t1.y, t1.z, t1.w};
-      float run = (row >= je) ? ex2(csi - lds_f32(ts + 4 * (T_CS + je))) : 0.f;
-      v[7] *= run * dt[7];
+      float dt[8] = {t0.x, t0.y, t0.z, t0.w, t1.x, t1.y, t1.z, t1.w}, run[8];
+      run[7] = (row >= je) ? ex2(csi - lds_f32(ts + 4 * (T_CS + je))) : 0.f;
 #pragma unroll
-      for (int k = 6; k >= 0; --k) {
-        run = (c0 + k == row) ? 1.f : run * ds[k];
-        v[k] *= run * dt[k];
+      for (int k = 6; k >= 0; --k) run[k] = (c0 + k == row) ? 1.f : run[k + 1] * ds[k];
+#pragma unroll
+      for (int k = 0; k < 8; k += 2) {
+        mul2(dt[k], dt[k + 1], run[k], run[k + 1]);
+        mul2(v[k], v[k + 1], dt[k], dt[k + 1]);
       }
     }
     st_shared_v4(mtile + plain_off(128, row, c0), pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]),
@@ -165,11 +176,15 @@ __device__ __forceinline__ void decay_off_half(const uint32_t (&raw)[16], float 
 #pragma unroll
   for (int j8 = 0; j8 < 16; j8 += 8) {
     const float4 f0 = lds_v4f32(cf + 4 * j8), f1 = lds_v4f32(cf + 4 * (j8 + 4));
-    const float v0 = __uint_as_float(raw[j8]) * f0.x * rf, v1 = __uint_as_float(raw[j8 + 1]) * f0.y * rf;
-    const float v2 = __uint_as_float(raw[j8 + 2]) * f0.z * rf, v3 = __uint_as_float(raw[j8 + 3]) * f0.w * rf;
-    const float v4 = __uint_as_float(raw[j8 + 4]) * f1.x * rf, v5 = __uint_as_float(raw[j8 + 5]) * f1.y * rf;
-    const float v6 = __uint_as_float(raw[j8 + 6]) * f1.z * rf, v7 = __uint_as_float(raw[j8 + 7]) * f1.w * rf;
-    st_shared_v4(dst + (j8 >> 3) * 2048, pack_bf16(v0, v1), pack_bf16(v2, v3), pack_bf16(v4, v5), pack_bf16(v6, v7));
+    const float f[8] = {f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, f1.z, f1.w};
+    float v[8];
+#pragma unroll
+    for (int k = 0; k < 8; k += 2) {
+      v[k] = __uint_as_float(raw[j8 + k]); v[k + 1] = __uint_as_float(raw[j8 + k + 1]);
+      mul2(v[k], v[k + 1], f[k], f[k + 1]);
+      mul2(v[k], v[k + 1], rf, rf);
+    }
+    st_shared_v4(dst + (j8 >> 3) * 2048, pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
   }
 }
 // 16 columns (starting at column c0) of the diagonal block: two independent 8-column walks; `ts` = shared-memory address
@@ -181,14 +196,14 @@ __device__ __forceinline__ void decay_diag_half(const uint32_t (&raw)[16], uint3
     const float4 d0 = lds_v4f32(ts + 4 * (T_DS + cs0)), d1 = lds_v4f32(ts + 4 * (T_DS + cs0 + 4));
     const float4 t0 = lds_v4f32(ts + 4 * (T_DT + cs0)), t1 = lds_v4f32(ts + 4 * (T_DT + cs0 + 4));
     const float ds[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};   // ds[k] = decay of step cs0+k+1
-    const float dt[8] = {t0.x, t0.y, t0.z, t0.w, t1.x, t1.y, t1.z, t1.w};
-    float v[8];
-    float run = (row >= je) ? ex2(csi - lds_f32(ts + 4 * (T_CS + je))) : 0.f;
-    v[7] = __uint_as_float(raw[8 * s + 7]) * (run * dt[7]);
+    float v[8] = {t0.x, t0.y, t0.z, t0.w, t1.x, t1.y, t1.z, t1.w}, run[8];
+    run[7] = (row >= je) ? ex2(csi - lds_f32(ts + 4 * (T_CS + je))) : 0.f;
 #pragma unroll
-    for (int k = 6; k >= 0; --k) {
-      run = (cs0 + k == row) ? 1.f : run * ds[k];
-      v[k] = __uint_as_float(raw[8 * s + k]) * (run * dt[k]);
+    for (int k = 6; k >= 0; --k) run[k] = (cs0 + k == row) ? 1.f : run[k + 1] * ds[k];
+#pragma unroll
+    for (int k = 0; k < 8; k += 2) {
+      mul2(v[k], v[k + 1], run[k], run[k + 1]);
+      mul2(v[k], v[k + 1], __uint_as_float(raw[8 * s + k]), __uint_as_float(raw[8 * s + k + 1]));
     }
     st_shared_v4(dst + s * 2048, pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
   }
