@@ -661,10 +661,12 @@ __global__ void __launch_bounds__(PsCfg<P, N_>::THREADS, 1) k_state_ps(Geo g, co
         uint32_t hi[4], lo[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-          const float f0 = f[2 * q] * wv, f1 = f[2 * q + 1] * wv;
+          float f0 = f[2 * q], f1 = f[2 * q + 1];
+          mul2(f0, f1, wv, wv);
           hi[q] = pack_bf16(f0, f1);
           const float2 hf = unpack_bf16(hi[q]);
-          lo[q] = pack_bf16(f0 - hf.x, f1 - hf.y);
+          fma2(f0, f1, hf.x, hf.y, -1.f, -1.f);
+          lo[q] = pack_bf16(f0, f1);
         }
         st_shared_v4(xs + off, hi[0], hi[1], hi[2], hi[3]);
         st_shared_v4(ls + off, lo[0], lo[1], lo[2], lo[3]);
@@ -965,10 +967,12 @@ k_state_scan_ps(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_con
         uint32_t hi[4], lo[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-          const float f0 = f[2 * q] * wv, f1 = f[2 * q + 1] * wv;
+          float f0 = f[2 * q], f1 = f[2 * q + 1];
+          mul2(f0, f1, wv, wv);
           hi[q] = pack_bf16(f0, f1);
           const float2 hf = unpack_bf16(hi[q]);
-          lo[q] = pack_bf16(f0 - hf.x, f1 - hf.y);
+          fma2(f0, f1, hf.x, hf.y, -1.f, -1.f);
+          lo[q] = pack_bf16(f0, f1);
         }
         st_shared_v4(xs + off, hi[0], hi[1], hi[2], hi[3]);
         st_shared_v4(ls + off, lo[0], lo[1], lo[2], lo[3]);
@@ -1064,7 +1068,10 @@ k_state_scan_ps(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_con
           }
         }
 #pragma unroll
-        for (int j = 0; j < 16; ++j) r[j] = fmaf(dec, r[j], v[j]);
+        for (int j = 0; j < 16; j += 2) {
+          fma2(v[j], v[j + 1], dec, dec, r[j], r[j + 1]);
+          r[j] = v[j]; r[j + 1] = v[j + 1];
+        }
       }
       if (want_sdot) {
         if (!tail) {
