@@ -309,3 +309,24 @@ def test_balanced_state_scan_is_the_same_bits(lib, H, P, N, Bn, L):
         row = run(slice(r, r + 1), 1)
         for k in ("y", "final_state", "dx", "ddt", "dB", "dC", "dinit"):
             assert torch.equal(whole[k][r:r + 1], row[k]), (k, r)
+
+
+@pytest.mark.parametrize("H,P,N,G,Bn", [(8, 32, 64, 1, 75), (8, 32, 128, 2, 92)])
+def test_more_units_than_sms_and_many_chunks(lib, H, P, N, G, Bn):
+    """150 and 184 units of 88 chunks (a last chunk of 64 tokens): even shares and no segments.  The first and the last row
+    against the oracle, final state and the gradients of both states included."""
+    import trading_bot_0_b200 as T
+    L = 87 * 128 + 64
+    inp = O.make_inputs(O.SsdConfig("many", Bn, L, H, P, N, G, 128, "bf16", False), with_init_state=True)
+    dfinal = 0.1 * torch.randn(Bn, H, P, N, generator=torch.Generator().manual_seed(4))
+    d = to_dev(inp, DEV)
+    a = (d["x"], d["dt"], d["A"], d["B"], d["C"], d["D"], None, d["init_state"])
+    y, fin, ws = T.forward(*a, chunk=128, algo="tensor", for_backward=True)
+    g = T.backward(d["dy"], *a, dfinal.to(DEV), chunk=128, algo="tensor", workspace=ws, fwd_saved=True, want_dinit=True)
+    torch.cuda.synchronize()
+    assert status_word(ws) == 0
+    for r in (0, Bn - 1):
+        row = {k: (v[r:r + 1] if k in ("x", "dt", "B", "C", "dy", "init_state") else v) for k, v in inp.items()}
+        ref = oracle_all(row, dfinal[r:r + 1])
+        for k, v in (("y", y), ("final_state", fin), *((k, g[k]) for k in ("dx", "ddt", "dB", "dC", "dinit"))):
+            assert_close(k, v[r:r + 1], ref[k], "bf16")

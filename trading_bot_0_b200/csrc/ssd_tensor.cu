@@ -23,6 +23,7 @@
 
 #include "common.cuh"
 #include "ssd_internal.h"
+#include "state_plan.h"
 #include "umma.cuh"
 
 namespace ssd {
@@ -817,75 +818,17 @@ k_state_scan_ps(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_con
   Waiter w{status, false};
   const bool want_sdot = Cfg::SE && a.sdot != nullptr;
 
-  // This CTA's tiles in order: the chunks of a unit in scan order, unit after unit; neighbouring units share a B/C tile.
-  // (Few members: the consumers hold one beside the running state.)
-  const int nunits = g.B * g.G * (g.hpg * P / 128) * (TOT ? a.nseg - 1 : a.nseg);
-  struct Walk {
-    int u, b, h0, grp, seg, s, s0, s1;
-    __device__ __forceinline__ Walk(const Geo& g, const StateScanArgs& a, int nunits) {
-      if constexpr (BAL) {
-        const long long a1 = (long long)(blockIdx.x + 1) * nunits * g.nc / gridDim.x;
-        u = (int)(a1 / g.nc);
-        piece(g, a, 0, (int)(a1 - (long long)u * g.nc));   // the unit cut at the end of the share, first
-        if (s == s1) next_unit(g, a, nunits);
-      } else {
-        u = blockIdx.x;
-        place(g, a);
-      }
-    }
-    __device__ __forceinline__ void place(const Geo& g, const StateScanArgs& a) {
-      const int MT = g.hpg * P / 128;
-      int r = u / MT;
-      h0 = (u - r * MT) * HT;
-      grp = r % g.G; r /= g.G;
-      h0 += grp * g.hpg;
-      b = r % g.B;
-      seg = BAL ? 0 : r / g.B;
-      s = s0 = seg * a.seglen;
-      s1 = min(s + a.seglen, g.nc);
-    }
-    __device__ __forceinline__ void piece(const Geo& g, const StateScanArgs& a, int from, int to) {
-      place(g, a);
-      s = s0 = from;
-      s1 = to;
-    }
-    __device__ __forceinline__ void next_unit(const Geo& g, const StateScanArgs& a, int nunits) {
-      if constexpr (BAL) {
-        const long long T = (long long)nunits * g.nc, a0 = blockIdx.x * T / gridDim.x, a1 = (blockIdx.x + 1) * T / gridDim.x;
-        const int first = (int)(a0 / g.nc), off = (int)(a0 - (long long)first * g.nc), last = (int)(a1 / g.nc);
-        u = u == last ? first + (off > 0) : u + 1;
-        if (u < last) {
-          piece(g, a, 0, g.nc);
-        } else {   // whole units done: the rest of the unit that the CTA before cut
-          u = first;
-          piece(g, a, off, g.nc);
-        }
-      } else {
-        u += gridDim.x;
-        place(g, a);
-      }
-    }
-    __device__ __forceinline__ void next(const Geo& g, const StateScanArgs& a, int nunits) {
-      if (++s == s1) next_unit(g, a, nunits);
-    }
-    __device__ __forceinline__ int chunk(const Geo& g) const { return MODE == 0 ? s : g.nc - 1 - s; }
-  };
-  int total = 0;   // tiles of this CTA
-  if constexpr (BAL) {
-    const long long T = (long long)nunits * g.nc;
-    total = (int)((blockIdx.x + 1) * T / gridDim.x - blockIdx.x * T / gridDim.x);
-  } else {
-    for (int u = blockIdx.x; u < nunits; u += gridDim.x) {
-      const int s0 = u / (nunits / (TOT ? a.nseg - 1 : a.nseg)) * a.seglen;
-      total += min(a.seglen, g.nc - s0);
-    }
-  }
+  using Walk = StateWalk<P, BAL>;
+  const int segs = TOT ? a.nseg - 1 : a.nseg, nunits = g.B * g.G * (g.hpg * P / 128) * segs;
+  const int blk = blockIdx.x, grid = gridDim.x;
+  auto chunk = [&](const Walk& t) { return MODE == 0 ? t.s : g.nc - 1 - t.s; };
+  const int total = Walk::total(g, a.seglen, nunits, segs, blk, grid);
 
   if (warp == Cfg::W_PROD) {
     if (lane == 0) {
-      Walk t(g, a, nunits);
-      for (int k = 0; k < total; ++k, t.next(g, a, nunits)) {
-        const int c = t.chunk(g), slot = k % NX, bs = k % NB;
+      Walk t(g, a.seglen, nunits, blk, grid);
+      for (int k = 0; k < total; ++k, t.next(g, a.seglen, nunits, blk, grid)) {
+        const int c = chunk(t), slot = k % NX, bs = k % NB;
         if (k >= NX) w.wait(&x_free[slot], ((k / NX) - 1) & 1, 14);
         const int col = t.h0 * P;
         mbar_expect_tx(&x_full[slot], Cfg::X_BYTES + Cfg::TB_BYTES);
@@ -907,9 +850,9 @@ k_state_scan_ps(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_con
     // the epilogue reads itself)
     if (lane == 0 && want_sdot) {
       int k = 0;
-      Walk t(g, a, nunits);
-      for (int n = 0; n < total; ++n, t.next(g, a, nunits)) {
-        const int c = t.chunk(g);
+      Walk t(g, a.seglen, nunits, blk, grid);
+      for (int n = 0; n < total; ++n, t.next(g, a.seglen, nunits, blk, grid)) {
+        const int c = chunk(t);
         if (c + 1 >= g.nc) continue;
         const int slot = k % NSE;
         if (k >= NSE) w.wait(&se_free[slot], ((k / NSE) - 1) & 1, 20);
@@ -991,7 +934,7 @@ k_state_scan_ps(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_con
                       make_uint4(__float_as_uint(run[j + 4]), __float_as_uint(run[j + 5]), __float_as_uint(run[j + 6]), __float_as_uint(run[j + 7])));
     };
     auto epilogue = [&](int k, const Walk& t, float dec) {
-      const int c = t.chunk(g);
+      const int c = chunk(t);
       const size_t PNH = (size_t)g.H * P * N;
       const size_t e = ((size_t)t.h0 * P + row) * N + part * (N / PARTS);   // this thread's columns inside a [.., H, P, N] state
       if (BAL && t.s == t.s0 && t.s0 > 0) {   // the state the CTA before has published
@@ -1102,7 +1045,7 @@ k_state_scan_ps(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_con
         }
       }
     };
-    Walk prev(g, a, nunits);
+    Walk prev(g, a.seglen, nunits, blk, grid);
     float dec_prev = 0.f;
     for (int k = 0; k < total; ++k) {
       const int slot = k % NX;
@@ -1119,7 +1062,7 @@ k_state_scan_ps(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_con
       scale_half(1, xs, tb);
       if (k > 0) {
         epilogue(k - 1, prev, dec_prev);
-        prev.next(g, a, nunits);
+        prev.next(g, a.seglen, nunits, blk, grid);
       }
       dec_prev = dec;
     }
@@ -3416,37 +3359,17 @@ int tensor_chunk_state(const Geo& g, int mode, const void* xdy, long long sb, lo
 // Chunk states and the scan over chunks together (see k_state_scan_ps): the persistent family, unstaged passes.
 bool tensor_state_fused_applies(const Geo& g) { return !g.onetile; }
 
-// Segments of the sequence.  A launch takes (units per CTA, rounded up) x (chunks of a segment) steps; cutting costs a second
-// launch over all segments but the last, whose steps are 0.7 of the others' (nothing is written), the launch itself (about
-// three steps) and a fold per segment.  Many units: one segment.  Fewer than 16 chunks: one segment as well, the second launch
-// would cost what it saves, and a row's result then does not depend on how many rows the call has.
-static int state_segments(const Geo& g, int units) {
-  const int sms = sm_count();
-  if (g.nc < 16) return 1;
-  int best = 1;
-  double least = 1e30;
-  for (int n = 1; n <= g.nc / 2; ++n) {
-    const int len = cdiv(g.nc, n), seg = cdiv(g.nc, len);
-    const double t = (double)cdiv(units * seg, sms) * len + (seg > 1 ? 0.7 * cdiv(units * (seg - 1), sms) * len + 3 + 0.3 * seg : 0.);
-    if (t < least) { least = t; best = n; }
-    if ((long long)units * n > 4LL * sms) break;
-  }
-  return best;
-}
-
 template <int P, int N, int MODE>
 static int launch_state_scan(const Geo& g, const CUtensorMap& tx, const CUtensorMap& tb, const CUtensorMap& ts, const StateScanArgs& a,
-                             int* status, cudaStream_t s) {
-  const int units = g.B * g.G * (g.hpg * P / 128), n1 = units * (a.nseg - 1), n2 = units * a.nseg;
+                             bool shares, int* status, cudaStream_t s) {
+  const int units = g.B * g.G * (g.hpg * P / 128), n1 = units * (a.nseg - 1), n2 = units * a.nseg, sms = sm_count();
+  if (shares && n1) { set_error("state scan: even shares of a sequence in segments"); return SSD_ERR_UNSUPPORTED; }
   if (n1) {
     using C1 = PfCfg<P, N, MODE, 1>;
-    launch<k_state_scan_ps<P, N, MODE, 1>>(n1 < sm_count() ? n1 : sm_count(), C1::THREADS, C1::SMEM, s, g, tx, tb, ts, a, status);
+    launch<k_state_scan_ps<P, N, MODE, 1>>(n1 < sms ? n1 : sms, C1::THREADS, C1::SMEM, s, g, tx, tb, ts, a, status);
     SSD_CUDA_CHECK_LAUNCH(MODE == 0 ? "chunk_state_totals" : "dstate_totals");
   }
-  // even shares where they save more than a twentieth (a hand-over costs a state's write and read per CTA); a share has to be
-  // longer than a unit
-  const int sms = sm_count();
-  if (units > sms && cdiv(units, sms) * sms > units + units / 20 && (long long)units * g.nc / sms > g.nc) {
+  if (shares) {
     using C3 = PfCfg<P, N, MODE, 2>;
     launch<k_state_scan_ps<P, N, MODE, 2>>(sms, C3::THREADS, C3::SMEM, s, g, tx, tb, ts, a, status);
   } else {
@@ -3465,9 +3388,9 @@ int tensor_state_fused(const Geo& g, int mode, const void* xdy, long long sb, lo
   if (rc) return rc;
   rc = make_seq_map(&tb, bc, (long long)g.G * g.N, g.L, g.B, bsl, bsb, "B/C");
   if (rc) return rc;
-  const int seglen = cdiv(g.nc, state_segments(g, g.B * g.G * (g.hpg * g.P / 128))), nseg = cdiv(g.nc, seglen);
+  const StatePlan plan = state_plan(g.nc, g.B * g.G * (g.hpg * g.P / 128), sm_count());
   const size_t PNH = (size_t)g.H * g.P * g.N;
-  StateScanArgs a{tab, st_bf, init, last, last2, fwd_prev_bf, fwd_fin, sdot, nseg, seglen, scratch, scratch + (size_t)g.B * nseg * PNH, hand};
+  StateScanArgs a{tab, st_bf, init, last, last2, fwd_prev_bf, fwd_fin, sdot, plan.nseg, plan.seglen, scratch, scratch + (size_t)g.B * plan.nseg * PNH, hand};
   if (sdot_nw) *sdot_nw = 4 * (g.P / 32);
   CUtensorMap ts = tx;   // a placeholder unless the backward kernel reads the forward states
   if (mode == 1 && sdot) {
@@ -3475,7 +3398,8 @@ int tensor_state_fused(const Geo& g, int mode, const void* xdy, long long sb, lo
     rc = make_map3(&ts, fwd_prev_bf, g.N, rows, 1, g.N, rows * g.N, 128, "forward chunk-entry states (bf16 copy)");
     if (rc) return rc;
   }
-#define CALL(PP, NN) return mode == 0 ? launch_state_scan<PP, NN, 0>(g, tx, tb, ts, a, status, s) : launch_state_scan<PP, NN, 1>(g, tx, tb, ts, a, status, s);
+#define CALL(PP, NN) return mode == 0 ? launch_state_scan<PP, NN, 0>(g, tx, tb, ts, a, plan.shares, status, s) \
+                                      : launch_state_scan<PP, NN, 1>(g, tx, tb, ts, a, plan.shares, status, s);
   DISPATCH_PN(CALL)
 #undef CALL
 }
