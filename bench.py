@@ -91,7 +91,7 @@ def kernel_bytes_per_token(name, c, e=2):
         "chunk_state_ps": (hp + gn) * e, "dstates_local_ps": (hp + gn) * e,
         # chunk states fused with the scan over chunks: the operator's inputs on the way in; the states stay on chip
         "chunk_state_scan": (hp + gn) * e, "dstate_scan": (hp + gn) * e,
-        "chunk_state_totals": (hp + gn) * e, "dstate_totals": (hp + gn) * e,   # first launch of a scan cut into segments
+        "state_fold": 0.75 * st, "dstate_fold": st,   # few units: after chunk_state_ps / dstates_local_ps, as state_passing
         "chunk_scan_tc": (2 * hp + 2 * gn) * e + zb, "chunk_scan_bwd_tc": (2 * hp + 2 * gn) * e + 2 * zb,
         "dx_tc": (3 * hp + 2 * gn) * e, "scan_bwd_dx_tc": (3 * hp + 2 * gn) * e, "dBdC_tc": (2 * hp + 4 * gn) * e,
         "chunk_scan_ws": (2 * hp + 2 * gn) * e + zb, "chunk_scan_bwd_ws": (2 * hp + 2 * gn) * e + 2 * zb,

@@ -9,92 +9,83 @@ using namespace ssd;
 
 struct G { int B, G, hpg, nc; };
 
-#define REQUIRE(c)                                                                                          \
-  do {                                                                                                      \
-    if (!(c)) {                                                                                             \
-      std::printf("%s: units %d chunks %d sms %d (segments %d x %d, shares %d)\n", #c, units, nc, sms, p.nseg, p.seglen, (int)p.shares); \
-      return false;                                                                                         \
-    }                                                                                                       \
+#define REQUIRE(c)                                                                                              \
+  do {                                                                                                          \
+    if (!(c)) {                                                                                                 \
+      std::printf("%s: units %d chunks %d sms %d, plan %d\n", #c, units, nc, sms, (int)p);                      \
+      return false;                                                                                             \
+    }                                                                                                           \
   } while (0)
 
-static bool check_rule(int units, int nc, int sms, const StatePlan& p) {
-  REQUIRE(p.nseg >= 1 && p.seglen >= 1);
-  REQUIRE(!(p.shares && p.nseg > 1));
-  REQUIRE((long long)p.nseg * p.seglen >= nc && (long long)(p.nseg - 1) * p.seglen < nc);
-  REQUIRE(p.nseg == 1 || 2 * p.nseg <= nc);   // totals and decays of the segments fit the scratch of one state per chunk
-  REQUIRE(units <= sms || p.nseg == 1);
-  REQUIRE(!p.shares || (long long)units * nc / sms > nc);
+static bool check_rule(int units, int nc, int sms, StatePlan p) {
+  REQUIRE(p != StatePlan::shares || (units > sms && (long long)units * nc / sms > nc));   // a unit is cut at most once
+  REQUIRE(p != StatePlan::split || (units < sms && nc > 1));
   return true;
 }
 
 // All blocks of one launch: every (unit, chunk) once and in order, the hand-over slots inside their array and used by
 // neighbouring blocks only (published by the one before as its first piece), the end of every unit reached once.
 template <int P, bool BAL>
-static bool check_walk(const G& g, int segs, int sms, const StatePlan& p) {
-  const int MT = g.hpg * P / 128, units = g.B * g.G * MT, nc = g.nc, nunits = units * segs, hand_len = g.B * g.G * g.hpg * P / 128;
-  const int grid = nunits < sms ? nunits : sms;
+static bool check_walk(const G& g, int sms, StatePlan p) {
+  const int MT = g.hpg * P / 128, units = g.B * g.G * MT, nc = g.nc, hand_len = g.B * g.G * g.hpg * P / 128;
+  const int grid = BAL || units > sms ? sms : units;
   std::vector<char> seen((size_t)units * nc, 0);
   std::vector<int> published(units, -1), cut(units, 0), ends(units, 0);
   long long all = 0;
   for (int blk = 0; blk < grid; ++blk) {
     using Walk = StateWalk<P, BAL>;
-    const int total = Walk::total(g, p.seglen, nunits, segs, blk, grid);
-    Walk t(g, p.seglen, nunits, blk, grid);
+    const int total = Walk::total(g, units, blk, grid);
+    Walk t(g, units, blk, grid);
     int pieces = 0, su = -1, ss = -1;
     all += total;
-    for (int k = 0; k < total; ++k, t.next(g, p.seglen, nunits, blk, grid)) {
-      REQUIRE(t.u >= 0 && t.u < (BAL ? hand_len : nunits));
+    for (int k = 0; k < total; ++k, t.next(g, units, blk, grid)) {
+      REQUIRE(t.u >= 0 && t.u < hand_len);
       REQUIRE(t.b >= 0 && t.b < g.B && t.grp >= 0 && t.grp < g.G && t.h0 >= 0 && t.h0 + 128 / P <= g.G * g.hpg);
-      REQUIRE(t.s >= t.s0 && t.s < t.s1 && t.s1 <= nc && t.seg >= 0 && t.seg < p.nseg);
-      const int unit = (t.b * g.G + t.grp) * MT + (t.h0 - t.grp * g.hpg) * P / 128;
-      if (BAL) REQUIRE(unit == t.u);
+      REQUIRE(t.s >= t.s0 && t.s < t.s1 && t.s1 <= nc);
+      REQUIRE((t.b * g.G + t.grp) * MT + (t.h0 - t.grp * g.hpg) * P / 128 == t.u);
       if (t.s == t.s0) {
         ++pieces;
-        if (BAL && t.s0 > 0) {   // taken over, by the last piece of the block behind the one that published it
-          REQUIRE(published[unit] == blk - 1 && cut[unit] == t.s0 && t.s1 == nc);
+        REQUIRE(BAL || t.s0 == 0);
+        if (t.s0 > 0) {   // taken over, by the last piece of the block behind the one that published it
+          REQUIRE(published[t.u] == blk - 1 && cut[t.u] == t.s0 && t.s1 == nc);
           REQUIRE(k + (t.s1 - t.s0) == total);
         }
       } else {
-        REQUIRE(su == unit && ss == t.s - 1);
+        REQUIRE(su == t.u && ss == t.s - 1);
       }
-      char& c = seen[(size_t)unit * nc + t.s];
+      char& c = seen[(size_t)t.u * nc + t.s];
       REQUIRE(!c);
       c = 1;
       if (t.s + 1 == t.s1) {
-        if (BAL && t.s1 < nc) {
-          REQUIRE(pieces == 1 && published[unit] < 0);
-          published[unit] = blk;
-          cut[unit] = t.s1;
-        } else if (t.seg == p.nseg - 1) {
-          REQUIRE(t.s1 == nc);
-          ++ends[unit];
+        if (t.s1 < nc) {
+          REQUIRE(BAL && pieces == 1 && published[t.u] < 0);
+          published[t.u] = blk;
+          cut[t.u] = t.s1;
+        } else {
+          ++ends[t.u];
         }
       }
-      su = unit;
+      su = t.u;
       ss = t.s;
     }
   }
-  const int walked = segs == p.nseg ? nc : segs * p.seglen;   // a launch over all segments but the last leaves that one out
-  REQUIRE(all == (long long)units * walked);
-  if (segs == p.nseg)
-    for (int u = 0; u < units; ++u) REQUIRE(ends[u] == 1);
+  REQUIRE(all == (long long)units * nc);
+  for (int u = 0; u < units; ++u) REQUIRE(ends[u] == 1);
   return true;
 }
 
 template <int P>
 static bool check_all(const G& g, int sms) {
-  const int units = g.B * g.G * (g.hpg * P / 128);
-  const StatePlan p = state_plan(g.nc, units, sms);
-  if (!check_rule(units, g.nc, sms, p)) return false;
-  if (p.nseg > 1 && !check_walk<P, false>(g, p.nseg - 1, sms, p)) return false;
-  return p.shares ? check_walk<P, true>(g, 1, sms, p) : check_walk<P, false>(g, p.nseg, sms, p);
+  const StatePlan p = state_plan(g.nc, g.B * g.G * (g.hpg * P / 128), 64, sms);
+  return p == StatePlan::shares ? check_walk<P, true>(g, sms, p) : check_walk<P, false>(g, sms, p);
 }
 
 int main() {
   for (int sms : {148, 132})
     for (int units = 1; units <= 2000; ++units)
       for (int nc = 1; nc <= 1200; ++nc)
-        if (!check_rule(units, nc, sms, state_plan(nc, units, sms))) return 1;
+        for (int n : {64, 128})
+          if (!check_rule(units, nc, sms, state_plan(nc, units, n, sms))) return 1;
   const int chunks[] = {1, 2, 3, 8, 15, 16, 17, 31, 32, 33, 63, 87, 88, 89, 120, 147, 148, 149, 255, 256, 511, 1024, 1200};
   for (int sms : {148, 132})
     for (int nc : chunks) {

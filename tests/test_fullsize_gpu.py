@@ -233,6 +233,61 @@ def test_batch_rows_are_independent(lib):
         assert torch.equal(g[k][sl], gs[k]), k
 
 
+@pytest.mark.parametrize("H,P,N,G,L,rows", [
+    (24, 64, 128, 1, 17 * 128, (1, 8, 14)),            # 12 units a row: two kernels; walks; even shares
+    (8, 32, 64, 1, 40 * 128 + 70, (1, 50, 90)),        # 2 units a row: the same three, a ragged last chunk
+    (24, 64, 128, 1, 40 * 128, (2, 6, 13)),
+    (8, 32, 128, 2, 3 * 128, (1, 45, 100)),
+    (4, 32, 64, 1, 200 * 128 + 5, (1, 90, 180)),       # long ones
+    (2, 64, 128, 1, 300 * 128, (1, 70)),
+])
+def test_row_bits_do_not_depend_on_the_batch(lib, H, P, N, G, L, rows):
+    """The state scans are run in another way for few rows, for about as many units as SMs, and for more; a row's results are
+    the same bits in each, with states entering at both ends."""
+    import trading_bot_0_b200 as T
+    B = max(rows)
+    d = bench.make_inputs(dict(bench.CFGS["cfg1"], H=H, P=P, N=N, G=G, Q=128), DEV, 11, batch=B, seqlen=L)
+    g = torch.Generator(device=DEV).manual_seed(5)
+    init, dfin = (0.1 * torch.randn(B, H, P, N, generator=g, device=DEV) for _ in range(2))
+
+    def run(n):   # the last n rows
+        s = slice(B - n, B)
+        a = (d["x"][s], d["dt"][s], d["A"], d["B"][s], d["C"][s], d["D"], None, init[s])
+        y, fin, ws = T.forward(*a, chunk=128, for_backward=True, check=True)
+        o = T.backward(d["dy"][s], *a, dfin[s], chunk=128, workspace=ws, fwd_saved=True, check=True)
+        return {"y": y, "final_state": fin, **{k: o[k] for k in ("dx", "ddt", "dB", "dC", "dinit")}}
+
+    whole = run(B)
+    for n in rows[:-1]:
+        part = run(n)
+        for k, v in part.items():
+            assert torch.equal(whole[k][B - n:], v), (n, k)
+
+
+@pytest.mark.parametrize("H,P,N,L,cut", [(8, 32, 64, 60 * 128, 7), (24, 64, 128, 300 * 128, 150), (2, 64, 128, 300 * 128, 1)])
+def test_prefix_bits_do_not_depend_on_the_length(lib, H, P, N, L, cut):
+    """The state scans run a short and a long sequence in different ways; the outputs of the first chunks are the same bits."""
+    import trading_bot_0_b200 as T
+    d = bench.make_inputs(dict(bench.CFGS["cfg1"], H=H, P=P, N=N), DEV, 13, batch=1, seqlen=L)
+    y = [T.forward(d["x"][:, :n], d["dt"][:, :n], d["A"], d["B"][:, :n], d["C"][:, :n], d["D"], chunk=128)[0] for n in (L, cut * 128)]
+    assert torch.equal(y[0][:, :cut * 128], y[1])
+
+
+@pytest.mark.parametrize("H,P,N,L", [(4, 32, 64, 256 * 128), (2, 64, 128, 300 * 128)])
+def test_long_sequences_match_oracle(lib, H, P, N, L):
+    """A few rows of several hundred chunks, states entering at both ends: the first row against the fp64 oracle."""
+    import trading_bot_0_b200 as T
+    d = bench.make_inputs(dict(bench.CFGS["cfg1"], H=H, P=P, N=N), DEV, 12, batch=3, seqlen=L)
+    g = torch.Generator(device=DEV).manual_seed(6)
+    init, dfin = (0.1 * torch.randn(3, H, P, N, generator=g, device=DEV) for _ in range(2))
+    a = (d["x"], d["dt"], d["A"], d["B"], d["C"], d["D"], None, init)
+    y, fin, ws = T.forward(*a, chunk=128, for_backward=True, check=True)
+    o = T.backward(d["dy"], *a, dfin, chunk=128, workspace=ws, fwd_saved=True, check=True)
+    ref = oracle_chunked64(dict(rows_to_cpu(d, [0]), init_state=init[:1].cpu()), dfinal=dfin[:1].cpu())
+    for k, v in (("y", y), ("final_state", fin), *((k, o[k]) for k in ("dx", "ddt", "dB", "dC", "dinit"))):
+        assert_close(k, v[:1], ref[k], "bf16")
+
+
 def test_prefill_then_steps_at_full_batch(lib):
     """cfg1 batch: chunk-scan over 896 tokens, then 128 single steps over all 512 x 8 states, against
     the chunk-scan over all 1024 tokens."""

@@ -1,4 +1,4 @@
-"""How the state scans are spread over the SMs: one host rule picks segments of the sequence or even shares of chunks."""
+"""How the state scans are spread over the SMs: one host rule, and the order in which a block walks its chunks."""
 import os
 import shutil
 import subprocess
@@ -8,9 +8,10 @@ import pytest
 HERE = os.path.dirname(os.path.abspath(__file__))
 
 
-def test_segments_and_even_shares_exclude_each_other(tmp_path):
-    """Rule and block walks (csrc/state_plan.h) compiled for the host: 1-2000 units x 1-1200 chunks never choose both, and
-    the replayed walks of all blocks visit every chunk once, keep their hand-over slots inside the array, and end every unit."""
+def test_state_plan_and_walks(tmp_path):
+    """Rule and block walks (csrc/state_plan.h) compiled for the host: even shares only where a share is longer than a unit (1-2000
+    units x 1-1200 chunks), and the replayed walks of all blocks visit every chunk once and in order, keep their hand-over slots
+    inside the array, and end every unit."""
     cxx = shutil.which("g++")
     if cxx is None:
         pytest.skip("no host compiler")

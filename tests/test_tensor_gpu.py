@@ -238,7 +238,8 @@ def test_ragged_operands_of_any_alignment(lib, which, N):
 @pytest.mark.parametrize("L", [1921, 2304, 4200])
 @pytest.mark.parametrize("H,P,N,G", [(8, 32, 64, 1), (4, 64, 128, 2), (12, 64, 128, 1)])
 def test_segmented_state_scan_matches_oracle(lib, L, H, P, N, G):
-    """Few units and many chunks: the state scans run in segments (a shorter last segment, a last chunk of one token)."""
+    """Few units and many chunks: the state scans run as two kernels (a last chunk of one token, fewer and more chunks than the
+    fold requests at once)."""
     import trading_bot_0_b200 as T
     Bn = 2
     cfg = O.SsdConfig("seg", Bn, L, H, P, N, G, 128, "bf16", False)

@@ -22,8 +22,8 @@ int tensor_state_passing(const Geo& g, float* st, const float* cs, const float* 
                          int reverse, bool write, const float* fwd_prev, const void* fwd_prev_bf, const float* fwd_fin,
                          float* sdot, int* sdot_nw,
                          cudaStream_t s);
-// both together where it applies (full pass): bf16 `st_bf` out; `scratch` = the fp32 chunk-state segment, for segment totals and
-// states handed over; `hand` = one counter per 128 (h,p) rows of a batch row, zeroed by the cumsum kernel
+// both together where it applies (full pass): bf16 `st_bf` out; `scratch` = the fp32 chunk-state segment, for the local
+// states of a scan in two kernels and for states handed over; `hand` = one counter per 128 (h,p) rows of a batch row, zeroed by the cumsum kernel
 bool tensor_state_fused_applies(const Geo& g);
 int tensor_state_fused(const Geo& g, int mode, const void* xdy, long long sb, long long sl, const void* bc, long long bsb,
                        long long bsl, const float* tab, float* scratch, int* hand, void* st_bf, const float* init, float* last, float* last2,

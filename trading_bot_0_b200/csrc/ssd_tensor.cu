@@ -541,8 +541,8 @@ struct PsCfg {
 template <int P, int N_, int MODE>
 __global__ void __launch_bounds__(PsCfg<P, N_>::THREADS, 1) k_state_ps(Geo g, const __grid_constant__ CUtensorMap tmX,
                                                                    const __grid_constant__ CUtensorMap tmB,
-                                                                   const float* __restrict__ tab, float* __restrict__ out,
-                                                                   int* __restrict__ status) {
+                                                                   const float* __restrict__ tab, float* __restrict__ out, int row_step,
+                                                                   int slice_step, int* __restrict__ status) {
   using Cfg = PsCfg<P, N_>;
   constexpr int N = Cfg::N, HT = Cfg::HT, NX = Cfg::NX;
   extern __shared__ uint8_t smem_raw[];
@@ -608,7 +608,7 @@ __global__ void __launch_bounds__(PsCfg<P, N_>::THREADS, 1) k_state_ps(Geo g, co
           if (n >= 2) w.wait(&b_free[n & 1], ((n >> 1) - 1) & 1, 15);
           mbar_expect_tx(&b_full[n & 1], Cfg::B_BYTES);
           for (int kb = 0; kb < Cfg::NBX; ++kb)
-            tma_load_3d(sB + (n & 1) * Cfg::B_BYTES + kb * BOX_BYTES, &tmB, grp * N + kb * 64, c * QT, b, &b_full[n & 1]);
+            tma_load_3d(sB + (n & 1) * Cfg::B_BYTES + kb * BOX_BYTES, &tmB, grp / g.hsplit * N + kb * 64, c * QT, b, &b_full[n & 1]);
         }
         if (++mt == MT) { mt = 0; ++n; }
       }
@@ -679,7 +679,7 @@ __global__ void __launch_bounds__(PsCfg<P, N_>::THREADS, 1) k_state_ps(Geo g, co
     auto epilogue = [&](int k, int b, int grp, int c, int mt) {   // accumulator of tile k -> global
       const int h0 = grp * g.hpg + mt * HT;
       const int row = tid & 127, part = tid >> 7;
-      float* o = out + (((size_t)(b * g.nc + c) * g.H + h0) * P + row) * N + part * (N / PARTS);
+      float* o = out + ((size_t)(b * g.nc + c) * g.H + h0) * P * N + row * row_step + part * (N / PARTS / 8) * slice_step;
 #pragma unroll
       for (int q = 0; q < N / PARTS / 16; ++q) {
         float v[16];
@@ -691,7 +691,7 @@ __global__ void __launch_bounds__(PsCfg<P, N_>::THREADS, 1) k_state_ps(Geo g, co
         }
 #pragma unroll
         for (int j = 0; j < 16; j += 8)
-          st_global_32B(o + q * 16 + j, make_uint4(__float_as_uint(v[j]), __float_as_uint(v[j + 1]), __float_as_uint(v[j + 2]), __float_as_uint(v[j + 3])),
+          st_global_32B(o + (2 * q + j / 8) * slice_step, make_uint4(__float_as_uint(v[j]), __float_as_uint(v[j + 1]), __float_as_uint(v[j + 2]), __float_as_uint(v[j + 3])),
                         make_uint4(__float_as_uint(v[j + 4]), __float_as_uint(v[j + 5]), __float_as_uint(v[j + 6]), __float_as_uint(v[j + 7])));
       }
     };
@@ -735,22 +735,18 @@ __global__ void __launch_bounds__(PsCfg<P, N_>::THREADS, 1) k_state_ps(Geo g, co
 //           <dS_end_c, S_end_c> (the per-chunk term of the dt*A gradient, S_end_c read from the forward pass's bf16 copy of
 //           the chunk-entry states, the fp32 final state for the last chunk), `nw` = 4 * P / 32 partials per (batch, chunk,
 //           head) in `sdot`; `last` receives the gradient w.r.t. the initial state.
-// Where there are too few units to fill the SMs, the sequence is cut into `nseg` segments of `seglen` chunks: a first launch
-// (TOT) walks every segment but the last from a zero state and leaves its total and its decay, the second folds the totals
-// before its segment into the state it starts from.  x and B are then read twice; fp32 states per chunk, written and read
-// back by a kernel of their own, would be twice that again (dstate 128) and leave the scan to a few hundred warps.
 // Where there are more units than SMs but the last wave is far from full (192 units on 148 SMs took the time of 296), every CTA
 // gets the same number of chunks instead (BAL): unit after unit, a unit that crosses the end of a CTA's share is continued by
 // the next CTA.  A CTA starts with that cut unit and publishes its state, then walks its whole units, and ends with the one it
 // takes over - by then long published, a share being longer than a unit.  CTA i waits only for CTA i - 1 and only for what that
 // one does first, so blocks placed in index order always get on; the wait is bounded all the same.  Same order of operations on
 // every unit: same bits.  16x4096, 24 heads: 154 -> 122 us forward, 210 -> 167 us backward.
+// Few units: k_state_ps and k_state_fold instead (state_plan() picks); same operations in the same order there as well.
 // Pipeline and barriers as in k_state_ps; the B (or C) tile changes with every tile, so it has a ring of its own.
-template <int P, int N_, int MODE, int KIND>
+template <int P, int N_, int MODE>
 struct PfCfg {
-  static constexpr bool TOT = KIND == 1, BAL = KIND == 2;
   // the backward kernel gives a slot of the x ring to the S_end tiles (128 rows x N bf16: one or two 16 KB boxes each)
-  static constexpr bool SE = MODE == 1 && !TOT;
+  static constexpr bool SE = MODE == 1;
   static constexpr int N = N_, HT = 128 / P, NBX = N / 64, NX = (N == 64 ? 4 : 3) - (SE ? 1 : 0), NB = N == 64 ? 3 : 2;
   static constexpr int X_BYTES = 2 * BOX_BYTES, B_BYTES = NBX * BOX_BYTES;
   static constexpr int TBH = 256;
@@ -763,6 +759,15 @@ struct PfCfg {
   static_assert(SMEM <= 232448, "shared-memory plan exceeds the 227 KB a CTA can have");
 };
 
+// <dS_end, S_end> in one order for both kernels that form it: four columns in a chain, sixteen as a tree, then over the columns
+// of a part and over 32 rows.
+__device__ __forceinline__ float dot4(const float* r, const float4& f) {
+  return fmaf(r[3], f.w, fmaf(r[2], f.z, fmaf(r[1], f.y, __fmul_rn(r[0], f.x))));
+}
+__device__ __forceinline__ float4 bf16x4(uint32_t a, uint32_t b) {
+  return make_float4(__uint_as_float(a << 16), __uint_as_float(a & 0xffff0000u), __uint_as_float(b << 16), __uint_as_float(b & 0xffff0000u));
+}
+
 struct StateScanArgs {
   const float* tab;
   void* st_bf;          // [B,nc,H,P,N] bf16 out
@@ -771,17 +776,15 @@ struct StateScanArgs {
   const void* fwd_prev_bf;  // MODE 1: bf16 copy of the forward pass's chunk-entry states (read through a tensor map)
   const float* fwd_fin;   // MODE 1: forward final state
   float* sdot;            // MODE 1: [B,nc,H,SDOT_NW]
-  int nseg, seglen;       // segments of the sequence, chunks in each (the last may be shorter)
-  float *tot, *tdec;      // [B,nseg,H,P,N] totals and [B,nseg,H] decays of the segments (nseg > 1); BAL: [B,H,P,N] states handed over
+  float* state;           // BAL: [B,H,P,N] states handed over; split: the fp32 states of all chunks
   int* hand;              // BAL: per unit, warps that have written (16), then read, its state; zero before and after the launch
 };
 
-template <int P, int N_, int MODE, int KIND>
-__global__ void __launch_bounds__(PfCfg<P, N_, MODE, KIND>::THREADS, 1)
+template <int P, int N_, int MODE, bool BAL>
+__global__ void __launch_bounds__(PfCfg<P, N_, MODE>::THREADS, 1)
 k_state_scan_ps(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmB,
                 const __grid_constant__ CUtensorMap tmS, StateScanArgs a, int* __restrict__ status) {
-  using Cfg = PfCfg<P, N_, MODE, KIND>;
-  constexpr bool TOT = Cfg::TOT, BAL = Cfg::BAL;
+  using Cfg = PfCfg<P, N_, MODE>;
   constexpr int N = Cfg::N, HT = Cfg::HT, NX = Cfg::NX, NB = Cfg::NB, NQ = Cfg::NQ, NSE = Cfg::NSE;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);   // 1 KB aligned, still known to be shared memory
@@ -819,15 +822,15 @@ k_state_scan_ps(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_con
   const bool want_sdot = Cfg::SE && a.sdot != nullptr;
 
   using Walk = StateWalk<P, BAL>;
-  const int segs = TOT ? a.nseg - 1 : a.nseg, nunits = g.B * g.G * (g.hpg * P / 128) * segs;
+  const int nunits = g.B * g.G * (g.hpg * P / 128);
   const int blk = blockIdx.x, grid = gridDim.x;
   auto chunk = [&](const Walk& t) { return MODE == 0 ? t.s : g.nc - 1 - t.s; };
-  const int total = Walk::total(g, a.seglen, nunits, segs, blk, grid);
+  const int total = Walk::total(g, nunits, blk, grid);
 
   if (warp == Cfg::W_PROD) {
     if (lane == 0) {
-      Walk t(g, a.seglen, nunits, blk, grid);
-      for (int k = 0; k < total; ++k, t.next(g, a.seglen, nunits, blk, grid)) {
+      Walk t(g, nunits, blk, grid);
+      for (int k = 0; k < total; ++k, t.next(g, nunits, blk, grid)) {
         const int c = chunk(t), slot = k % NX, bs = k % NB;
         if (k >= NX) w.wait(&x_free[slot], ((k / NX) - 1) & 1, 14);
         const int col = t.h0 * P;
@@ -850,8 +853,8 @@ k_state_scan_ps(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_con
     // the epilogue reads itself)
     if (lane == 0 && want_sdot) {
       int k = 0;
-      Walk t(g, a.seglen, nunits, blk, grid);
-      for (int n = 0; n < total; ++n, t.next(g, a.seglen, nunits, blk, grid)) {
+      Walk t(g, nunits, blk, grid);
+      for (int n = 0; n < total; ++n, t.next(g, nunits, blk, grid)) {
         const int c = chunk(t);
         if (c + 1 >= g.nc) continue;
         const int slot = k % NSE;
@@ -925,7 +928,6 @@ k_state_scan_ps(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_con
       if (lane == 0) mbar_arrive(&half_ready[h]);
     };
     float run[16 * NQ];          // running state of this thread's (row, N / 4 columns)
-    float pdec = 1.f;            // TOT: decay of the row's head over the chunks of the segment so far
     int kse = 0;
     auto put = [&](float* to) {
 #pragma unroll
@@ -943,12 +945,12 @@ k_state_scan_ps(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_con
         __threadfence();
 #pragma unroll
         for (int j = 0; j < 16 * NQ; j += 4) {
-          const float4 v = __ldcg(reinterpret_cast<const float4*>(a.tot + t.b * PNH + e + j));
+          const float4 v = __ldcg(reinterpret_cast<const float4*>(a.state + t.b * PNH + e + j));
           run[j] = v.x; run[j + 1] = v.y; run[j + 2] = v.z; run[j + 3] = v.w;
         }
         if (lane == 0 && atomicAdd(a.hand + t.u, 1) == 31) *(volatile int*)(a.hand + t.u) = 0;   // every warp has seen the count
       } else if (t.s == t.s0) {
-        if (!TOT && a.init) {
+        if (a.init) {
 #pragma unroll
           for (int j = 0; j < 16 * NQ; j += 4) {
             const float4 v = *reinterpret_cast<const float4*>(a.init + t.b * PNH + e + j);
@@ -957,19 +959,6 @@ k_state_scan_ps(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_con
         } else {
 #pragma unroll
           for (int j = 0; j < 16 * NQ; ++j) run[j] = 0.f;
-        }
-        pdec = 1.f;
-        if constexpr (!TOT) {
-          for (int sg = 0; sg < t.seg; ++sg) {   // the segments before this one
-            const size_t i = (size_t)t.b * a.nseg + sg;
-            const float d = a.tdec[i * g.H + t.h0 + row / P];
-#pragma unroll
-            for (int j = 0; j < 16 * NQ; j += 4) {
-              const float4 v = *reinterpret_cast<const float4*>(a.tot + i * PNH + e + j);
-              run[j] = fmaf(d, run[j], v.x); run[j + 1] = fmaf(d, run[j + 1], v.y);
-              run[j + 2] = fmaf(d, run[j + 2], v.z); run[j + 3] = fmaf(d, run[j + 3], v.w);
-            }
-          }
         }
       }
       const bool tail = c + 1 >= g.nc;   // MODE 1: this chunk's S_end is the final state, fp32
@@ -984,31 +973,29 @@ k_state_scan_ps(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_con
           __syncwarp();
           if (lane == 0) mbar_arrive(&acc_empty[k & 1]);
         }
-        if constexpr (!TOT)
-          st_global_32B((bf16*)a.st_bf + (size_t)(t.b * g.nc + c) * PNH + e + 16 * q,
-                        make_uint4(pack_bf16(r[0], r[1]), pack_bf16(r[2], r[3]), pack_bf16(r[4], r[5]), pack_bf16(r[6], r[7])),
-                        make_uint4(pack_bf16(r[8], r[9]), pack_bf16(r[10], r[11]), pack_bf16(r[12], r[13]), pack_bf16(r[14], r[15])));
+        st_global_32B((bf16*)a.st_bf + (size_t)(t.b * g.nc + c) * PNH + e + 16 * q,
+                      make_uint4(pack_bf16(r[0], r[1]), pack_bf16(r[2], r[3]), pack_bf16(r[4], r[5]), pack_bf16(r[6], r[7])),
+                      make_uint4(pack_bf16(r[8], r[9]), pack_bf16(r[10], r[11]), pack_bf16(r[12], r[13]), pack_bf16(r[14], r[15])));
         if (want_sdot) {
           if (q == 0 && !tail) w.wait(&se_full[kse % NSE], (kse / NSE) & 1, 21);
+          float t4[4] = {0.f, 0.f, 0.f, 0.f};   // four columns each
           if (tail) {
             if (a.init) {   // else the running gradient is still zero, and the reads (nothing fetched them ahead) are not needed
 #pragma unroll
-              for (int j = 0; j < 16; j += 4) {
-                const float4 f = *reinterpret_cast<const float4*>(a.fwd_fin + t.b * PNH + e + 16 * q + j);
-                d += r[j] * f.x + r[j + 1] * f.y + r[j + 2] * f.z + r[j + 3] * f.w;
-              }
+              for (int j = 0; j < 4; ++j)
+                t4[j] = dot4(r + 4 * j, *reinterpret_cast<const float4*>(a.fwd_fin + t.b * PNH + e + 16 * q + 4 * j));
             }
           } else {   // the bf16 copy: this thread's columns are 16-byte pieces of its row
             const uint32_t sb = smem_u32(sSE) + (kse % NSE) * Cfg::SE_BYTES + ((part * (N / PARTS)) / 64) * BOX_BYTES;
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
               const uint4 u = ld_shared_v4(sb + sw128_off(row, ((part * (N / PARTS)) % 64) / 8 + 2 * q + j));
-              const uint32_t uw[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-              for (int i = 0; i < 4; ++i)
-                d += r[8 * j + 2 * i] * __uint_as_float(uw[i] << 16) + r[8 * j + 2 * i + 1] * __uint_as_float(uw[i] & 0xffff0000u);
+              t4[2 * j] = dot4(r + 8 * j, bf16x4(u.x, u.y));
+              t4[2 * j + 1] = dot4(r + 8 * j + 4, bf16x4(u.z, u.w));
             }
           }
+          const float dq = __fadd_rn(__fadd_rn(t4[0], t4[1]), __fadd_rn(t4[2], t4[3]));
+          d = q == 0 ? dq : __fadd_rn(d, dq);
         }
 #pragma unroll
         for (int j = 0; j < 16; j += 2) {
@@ -1028,24 +1015,19 @@ k_state_scan_ps(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_con
           a.sdot[((size_t)(t.b * g.nc + c) * g.H + t.h0 + row / P) * Cfg::SDOT_NW + slot] = d;
         }
       }
-      if (TOT) pdec *= dec;
       if (t.s + 1 == t.s1) {
-        if constexpr (TOT) {
-          const size_t i = (size_t)t.b * a.nseg + t.seg;
-          put(a.tot + i * PNH + e);
-          if (part == 0 && row % P == 0) a.tdec[i * g.H + t.h0 + row / P] = pdec;
-        } else if (BAL && t.s1 < g.nc) {
-          put(a.tot + t.b * PNH + e);
+        if (BAL && t.s1 < g.nc) {
+          put(a.state + t.b * PNH + e);
           __threadfence();
           __syncwarp();
           if (lane == 0) atomicAdd(a.hand + t.u, 1);
-        } else if (t.seg == a.nseg - 1) {
+        } else {
           if (a.last) put(a.last + t.b * PNH + e);
           if (a.last2) put(a.last2 + t.b * PNH + e);
         }
       }
     };
-    Walk prev(g, a.seglen, nunits, blk, grid);
+    Walk prev(g, nunits, blk, grid);
     float dec_prev = 0.f;
     for (int k = 0; k < total; ++k) {
       const int slot = k % NX;
@@ -1062,7 +1044,7 @@ k_state_scan_ps(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_con
       scale_half(1, xs, tb);
       if (k > 0) {
         epilogue(k - 1, prev, dec_prev);
-        prev.next(g, a.seglen, nunits, blk, grid);
+        prev.next(g, nunits, blk, grid);
       }
       dec_prev = dec;
     }
@@ -3090,6 +3072,102 @@ __global__ void __launch_bounds__(256, BFDOT ? 3 : 1) k_state_passing_v4(Geo g, 
 }
 
 // ---------------------------------------------------------------------------------------------
+// The scan over chunks on local states that k_state_ps left in memory: the other way to run k_state_scan_ps, with the same
+// operations in the same order on every element, for calls whose few units would leave most SMs idle behind one another's
+// chunks.  The local states lie in the order in which both kernels' warps touch whole lines: per tile of 128 (h,p) rows, slices of
+// 8 columns of all its rows.  Block = 32 rows of one head x 32 columns, thread = a slice of one row; MODE, outputs and partial sums
+// as there.  A step's U chunks are requested while the step before is folded.  Bound by DRAM on long sequences (2 rows of 131072
+// tokens, 24 heads of 64 x 128: 2.4 GB in 430 us forward, 3.2 GB in 505 us backward; U = 8 380-500 and 680), by the round trip of
+// the steps on short ones.
+template <int N, int MODE, int U>
+__global__ void __launch_bounds__(128) k_state_fold(Geo g, const float* __restrict__ local, StateScanArgs a) {
+  constexpr int PP = 128 / N;   // parts (N / 4 columns) of a block
+  struct Step {
+    float4 v[U][2];
+    uint4 se[U];
+    float cs[U];
+  };
+  __shared__ float red[2][U][PP][32];
+  pdl_wait();
+  const int tid = threadIdx.x, lr = tid / 4, hp = blockIdx.x / (N / 32) * 32, h = hp / g.P, b = blockIdx.y, nc = g.nc;
+  const int col = blockIdx.x % (N / 32) * 32 + tid % 4 * 8;
+  const size_t cstride = (size_t)g.H * g.P * N, e = (size_t)(hp + lr) * N + col;
+  const size_t base = (size_t)b * nc * cstride, sbase = b * cstride + e;
+  const float* mine = local + base + (size_t)(hp / 128 * 128) * N + col * 128 + (hp % 128 + lr) * 8;
+  float r[8] = {};
+  float4 fin[2] = {};
+  if (a.init) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      *reinterpret_cast<float4*>(r + 4 * i) = *reinterpret_cast<const float4*>(a.init + sbase + 4 * i);
+      if (MODE == 1) fin[i] = *reinterpret_cast<const float4*>(a.fwd_fin + sbase + 4 * i);
+    }
+  }
+  auto request = [&](Step& n, int s0) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {   // index clamped: loads without a branch go out together
+      const int s = min(s0 + u, nc - 1), c = MODE == 0 ? s : nc - 1 - s;
+      n.cs[u] = a.tab[((size_t)(b * nc + c) * g.H + h) * TAB + T_CS + 127];
+      n.v[u][0] = *reinterpret_cast<const float4*>(mine + c * cstride);
+      n.v[u][1] = *reinterpret_cast<const float4*>(mine + c * cstride + 4);
+      if (MODE == 1) n.se[u] = *reinterpret_cast<const uint4*>((const bf16*)a.fwd_prev_bf + base + min(c + 1, nc - 1) * cstride + e);
+    }
+  };
+  auto fold = [&](const Step& n, int s0, float (&rd)[U][PP][32]) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (s0 + u >= nc) break;   // block-uniform
+      const int s = s0 + u, c = MODE == 0 ? s : nc - 1 - s;
+      const float dec = ex2(n.cs[u]);
+      *reinterpret_cast<uint4*>((bf16*)a.st_bf + base + c * cstride + e) =
+          make_uint4(pack_bf16(r[0], r[1]), pack_bf16(r[2], r[3]), pack_bf16(r[4], r[5]), pack_bf16(r[6], r[7]));
+      if (MODE == 1) {
+        const bool tail = c + 1 == nc;
+        const uint4& q = n.se[u];
+        float d = __fadd_rn(dot4(r, tail ? fin[0] : bf16x4(q.x, q.y)), dot4(r + 4, tail ? fin[1] : bf16x4(q.z, q.w)));
+#pragma unroll
+        for (int o = 1; o < N / 32; o <<= 1) d = __fadd_rn(d, __shfl_xor_sync(0xffffffffu, d, o));
+        if (tid % (N / 32) == 0) rd[u][tid % 4 / (N / 32)][lr] = d;
+      }
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const float4 v = n.v[u][i];
+        r[4 * i] = fmaf(dec, r[4 * i], v.x); r[4 * i + 1] = fmaf(dec, r[4 * i + 1], v.y);
+        r[4 * i + 2] = fmaf(dec, r[4 * i + 2], v.z); r[4 * i + 3] = fmaf(dec, r[4 * i + 3], v.w);
+      }
+    }
+    if (MODE == 1) {   // two buffers: the barrier of a step holds back the writes of the one after the next
+      __syncthreads();
+      if (tid < U * PP && s0 + tid / PP < nc) {
+        float f[32];
+#pragma unroll
+        for (int i = 0; i < 32; ++i) f[i] = rd[tid / PP][tid % PP][i];
+#pragma unroll
+        for (int o = 16; o; o >>= 1)
+#pragma unroll
+          for (int i = 0; i < o; ++i) f[i] = __fadd_rn(f[i], f[i + o]);
+        const int part = blockIdx.x % (N / 32) * PP + tid % PP;
+        a.sdot[((size_t)(b * nc + nc - 1 - (s0 + tid / PP)) * g.H + h) * (4 * (g.P / 32)) + part * (g.P / 32) + hp % g.P / 32] = f[0];
+      }
+    }
+  };
+  Step p, q;
+  request(p, 0);
+  for (int s0 = 0; s0 < nc; s0 += 2 * U) {
+    request(q, s0 + U);
+    fold(p, s0, red[0]);
+    if (s0 + U >= nc) break;
+    request(p, s0 + 2 * U);
+    fold(q, s0 + U, red[1]);
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    if (a.last) *reinterpret_cast<float4*>(a.last + sbase + 4 * i) = *reinterpret_cast<float4*>(r + 4 * i);
+    if (a.last2) *reinterpret_cast<float4*>(a.last2 + sbase + 4 * i) = *reinterpret_cast<float4*>(r + 4 * i);
+  }
+}
+
+// ---------------------------------------------------------------------------------------------
 typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                              const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                              CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -3147,11 +3225,18 @@ constexpr size_t dbc_smem() {
 
 template <int P, int N, int MODE>
 int launch_state(const Geo& g, const CUtensorMap& tx, const CUtensorMap& tb, const float* tab, float* out, int* status,
-                 cudaStream_t s) {
-  if (!g.onetile) {   // persistent, ring-fed version
-    const int nitems = g.B * g.G * g.nc;
-    const int grid = nitems < sm_count() ? nitems : sm_count();
-    launch<k_state_ps<P, N, MODE>>(grid, PsCfg<P, N>::THREADS, PsCfg<P, N>::SMEM, s, g, tx, tb, tab, out, status);
+                 cudaStream_t s, bool sliced = false) {
+  if (!g.onetile) {   // persistent, ring-fed version; `sliced`: the order k_state_fold reads, else [B,nc,H,P,N]
+    // few items: a group's tiles are cut into parts, as in split_heads (2 rows of 16 chunks, 24 heads of 64 x 128: 32 blocks of 12
+    // tiles one behind the other become 128 of 3)
+    const int MT = g.hpg * P / 128, items = g.B * g.G * g.nc, sms = sm_count();
+    int parts = 1;
+    for (int n = 2; n <= MT; ++n)
+      if (MT % n == 0 && (long long)cdiv(items * n, sms) * (MT / n) < (long long)cdiv(items * parts, sms) * (MT / parts)) parts = n;
+    Geo p = g;
+    p.G *= parts; p.hpg /= parts; p.hsplit = parts;
+    launch<k_state_ps<P, N, MODE>>(items * parts < sms ? items * parts : sms, PsCfg<P, N>::THREADS, PsCfg<P, N>::SMEM, s, p, tx, tb, tab, out,
+                                   sliced ? 8 : N, sliced ? 1024 : 8, status);
     SSD_CUDA_CHECK_LAUNCH(MODE == 0 ? "chunk_state_ps" : "dstates_local_ps");
     return SSD_OK;
   }
@@ -3361,21 +3446,21 @@ bool tensor_state_fused_applies(const Geo& g) { return !g.onetile; }
 
 template <int P, int N, int MODE>
 static int launch_state_scan(const Geo& g, const CUtensorMap& tx, const CUtensorMap& tb, const CUtensorMap& ts, const StateScanArgs& a,
-                             bool shares, int* status, cudaStream_t s) {
-  const int units = g.B * g.G * (g.hpg * P / 128), n1 = units * (a.nseg - 1), n2 = units * a.nseg, sms = sm_count();
-  if (shares && n1) { set_error("state scan: even shares of a sequence in segments"); return SSD_ERR_UNSUPPORTED; }
-  if (n1) {
-    using C1 = PfCfg<P, N, MODE, 1>;
-    launch<k_state_scan_ps<P, N, MODE, 1>>(n1 < sms ? n1 : sms, C1::THREADS, C1::SMEM, s, g, tx, tb, ts, a, status);
-    SSD_CUDA_CHECK_LAUNCH(MODE == 0 ? "chunk_state_totals" : "dstate_totals");
+                             int* status, cudaStream_t s) {
+  using Cfg = PfCfg<P, N, MODE>;
+  const int units = g.B * g.G * (g.hpg * P / 128), sms = sm_count();
+  const StatePlan plan = state_plan(g.nc, units, N, sms);
+  if (plan == StatePlan::split) {
+    const int rc = launch_state<P, N, MODE>(g, tx, tb, a.tab, a.state, status, s, true);
+    if (rc) return rc;
+    launch<k_state_fold<N, MODE, MODE == 0 ? 6 : 4>>(dim3(g.H * P / 32 * (N / 32), g.B), 128, 0, s, g, (const float*)a.state, a);
+    SSD_CUDA_CHECK_LAUNCH(MODE == 0 ? "state_fold" : "dstate_fold");
+    return SSD_OK;
   }
-  if (shares) {
-    using C3 = PfCfg<P, N, MODE, 2>;
-    launch<k_state_scan_ps<P, N, MODE, 2>>(sms, C3::THREADS, C3::SMEM, s, g, tx, tb, ts, a, status);
-  } else {
-    using C2 = PfCfg<P, N, MODE, 0>;
-    launch<k_state_scan_ps<P, N, MODE, 0>>(n2 < sms ? n2 : sms, C2::THREADS, C2::SMEM, s, g, tx, tb, ts, a, status);
-  }
+  if (plan == StatePlan::shares)
+    launch<k_state_scan_ps<P, N, MODE, true>>(sms, Cfg::THREADS, Cfg::SMEM, s, g, tx, tb, ts, a, status);
+  else
+    launch<k_state_scan_ps<P, N, MODE, false>>(units < sms ? units : sms, Cfg::THREADS, Cfg::SMEM, s, g, tx, tb, ts, a, status);
   SSD_CUDA_CHECK_LAUNCH(MODE == 0 ? "chunk_state_scan" : "dstate_scan");
   return SSD_OK;
 }
@@ -3388,9 +3473,7 @@ int tensor_state_fused(const Geo& g, int mode, const void* xdy, long long sb, lo
   if (rc) return rc;
   rc = make_seq_map(&tb, bc, (long long)g.G * g.N, g.L, g.B, bsl, bsb, "B/C");
   if (rc) return rc;
-  const StatePlan plan = state_plan(g.nc, g.B * g.G * (g.hpg * g.P / 128), sm_count());
-  const size_t PNH = (size_t)g.H * g.P * g.N;
-  StateScanArgs a{tab, st_bf, init, last, last2, fwd_prev_bf, fwd_fin, sdot, plan.nseg, plan.seglen, scratch, scratch + (size_t)g.B * plan.nseg * PNH, hand};
+  StateScanArgs a{tab, st_bf, init, last, last2, fwd_prev_bf, fwd_fin, sdot, scratch, hand};
   if (sdot_nw) *sdot_nw = 4 * (g.P / 32);
   CUtensorMap ts = tx;   // a placeholder unless the backward kernel reads the forward states
   if (mode == 1 && sdot) {
@@ -3398,8 +3481,8 @@ int tensor_state_fused(const Geo& g, int mode, const void* xdy, long long sb, lo
     rc = make_map3(&ts, fwd_prev_bf, g.N, rows, 1, g.N, rows * g.N, 128, "forward chunk-entry states (bf16 copy)");
     if (rc) return rc;
   }
-#define CALL(PP, NN) return mode == 0 ? launch_state_scan<PP, NN, 0>(g, tx, tb, ts, a, plan.shares, status, s) \
-                                      : launch_state_scan<PP, NN, 1>(g, tx, tb, ts, a, plan.shares, status, s);
+#define CALL(PP, NN) return mode == 0 ? launch_state_scan<PP, NN, 0>(g, tx, tb, ts, a, status, s) \
+                                      : launch_state_scan<PP, NN, 1>(g, tx, tb, ts, a, status, s);
   DISPATCH_PN(CALL)
 #undef CALL
 }

@@ -10,74 +10,64 @@
 
 namespace ssd {
 
-// A unit is the sequence of one batch row for 128 (h,p) rows of a group.
-struct StatePlan {
-  int nseg, seglen;   // segments that the sequence is cut into, chunks in each (the last may be shorter)
-  bool shares;        // every block gets the same number of chunks (only with one segment)
+// A unit is the sequence of one batch row for 128 (h,p) rows of a group.  Whichever way is taken, every element goes through the
+// same operations in the same order, chunk after chunk: a row's bits depend neither on how many rows a call has nor on how far
+// its sequence goes on.
+enum class StatePlan {
+  walks,    // a block walks whole units
+  shares,   // every block gets the same number of chunks; a unit cut between two is handed over
+  split     // products and scan as two kernels, the fp32 states of all chunks in memory between them
 };
 
-// The one rule for both.  More units than SMs: one segment, and even shares where they save more than a twentieth (a hand-over
-// costs a state's write and read per block); a share has to be longer than a unit, so that a unit is cut at most once.
-// Fewer units: segments.  A launch takes (units per block, rounded up) x (chunks of a segment) steps; cutting costs a second
-// launch over all segments but the last, whose steps are 0.7 of the others' (nothing is written), the launch itself (about
-// three steps) and a fold per segment.  Fewer than 16 chunks: one segment, the second launch would cost what it saves.
-inline StatePlan state_plan(int nc, int units, int sms) {
-  auto up = [](int a, int b) { return (a + b - 1) / b; };
-  StatePlan p{1, nc, false};
+// The one rule; `n` = dstate.  State kernels of a forward and a backward pass, us on 148 SMs, sequences of 64 chunks:
+//                  24 heads of 64 x 128 (12 units a row)       8 heads of 32 x 64 (2 units a row)
+//   units           12    24    48    60    72    96            8    32    64    74    84    96
+//   walks          339   341   340   340   335   342          271   277   277   277   279   280
+//   split           96   142   253   336   373   490           67   125   229   257   279   299
+// A walk takes the time of one unit's chunks behind one another, the two kernels the time of the states they move: the lines cross
+// near 60 and 84 units, at 8 to 128 chunks alike (bounds: 2/5 and 1/2 of the SMs).  Below 8 chunks the second launch weighs more, and
+// they cross near 50 (2 chunks, 48 units of 24 heads: 37 against 44 us, but whole passes 92.2 against 91.1; 1/3); a single chunk has
+// nothing to walk.  The longest sequences stay with it (1024 chunks, 24 units: 2030 against 4870).
+// More units than SMs: even shares where they save more than a twentieth (192 units of 32 chunks: 413 -> 311; a hand-over costs a
+// state's write and read per block); a share has to be longer than a unit, so that a unit is cut at most once.
+inline StatePlan state_plan(int nc, int units, int n, int sms) {
   if (units > sms) {
-    p.shares = up(units, sms) * sms > units + units / 20 && (long long)units * nc / sms > nc;
-    return p;
+    const int rounds = (units + sms - 1) / sms;
+    return rounds * sms > units + units / 20 && (long long)units * nc / sms > nc ? StatePlan::shares : StatePlan::walks;
   }
-  if (nc < 16) return p;
-  double least = 1e30;
-  for (int n = 1; n <= nc / 2; ++n) {
-    const int len = up(nc, n), seg = up(nc, len);
-    const double t = (double)up(units * seg, sms) * len + (seg > 1 ? 0.7 * up(units * (seg - 1), sms) * len + 3 + 0.3 * seg : 0.);
-    if (t < least) { least = t; p.nseg = seg; p.seglen = len; }
-    if ((long long)units * n > 4LL * sms) break;
-  }
-  return p;
+  const int per6 = nc < 8 ? 18 : n > 64 ? 15 : 12;   // a third, two fifths, a half of the SMs
+  return nc > 1 && units * per6 <= 6 * sms ? StatePlan::split : StatePlan::walks;
 }
 
-// A block's tiles in order: the chunks of a unit (or of a segment of one) in scan order, unit after unit; neighbouring units
-// share a B/C tile.  BAL (even shares): the unit cut at the end of the share first, then the whole units, then the rest of the
-// unit that the block before cut.  `nunits` counts segments; G has B, G, hpg and nc.  (Few members: the consumers hold a walk
-// beside the running state.)
+// A block's tiles in order: the chunks of a unit in scan order, unit after unit; neighbouring units share a B/C tile.  BAL (even
+// shares): the unit cut at the end of the share first, then the whole units, then the rest of the unit that the block before
+// cut.  G has B, G, hpg and nc.  (Few members: the consumers hold a walk beside the running state.)
 template <int P, bool BAL>
 struct StateWalk {
-  int u, b, h0, grp, seg, s, s0, s1;
+  int u, b, h0, grp, s, s0, s1;
   template <class G>
-  SSD_HD StateWalk(const G& g, int seglen, int nunits, int block, int grid) {
+  SSD_HD StateWalk(const G& g, int nunits, int block, int grid) {
     if constexpr (BAL) {
       const long long a1 = (long long)(block + 1) * nunits * g.nc / grid;
       u = (int)(a1 / g.nc);
       piece(g, 0, (int)(a1 - (long long)u * g.nc));
-      if (s == s1) next_unit(g, seglen, nunits, block, grid);
+      if (s == s1) next_unit(g, nunits, block, grid);
     } else {
       u = block;
-      place(g, seglen);
+      piece(g, 0, g.nc);
     }
   }
   template <class G>
-  SSD_HD void place(const G& g, int seglen) {
-    const int MT = g.hpg * P / 128;
-    int r = u / MT;
-    h0 = (u - r * MT) * (128 / P);
-    grp = r % g.G; r /= g.G;
-    h0 += grp * g.hpg;
-    b = r % g.B;
-    seg = BAL ? 0 : r / g.B;
-    s = s0 = seg * seglen;
-    s1 = s + seglen < g.nc ? s + seglen : g.nc;
-  }
-  template <class G>
   SSD_HD void piece(const G& g, int from, int to) {
-    place(g, g.nc);
+    const int MT = g.hpg * P / 128, r = u / MT;
+    grp = r % g.G;
+    b = r / g.G;
+    h0 = grp * g.hpg + (u - r * MT) * (128 / P);
     s = s0 = from;
     s1 = to;
   }
   template <class G>
-  SSD_HD void next_unit(const G& g, int seglen, int nunits, int block, int grid) {
+  SSD_HD void next_unit(const G& g, int nunits, int block, int grid) {
     if constexpr (BAL) {
       const long long T = (long long)nunits * g.nc, a0 = block * T / grid, a1 = (block + 1) * T / grid;
       const int first = (int)(a0 / g.nc), off = (int)(a0 - (long long)first * g.nc), last = (int)(a1 / g.nc);
@@ -90,27 +80,19 @@ struct StateWalk {
       }
     } else {
       u += grid;
-      place(g, seglen);
+      piece(g, 0, g.nc);
     }
   }
   template <class G>
-  SSD_HD void next(const G& g, int seglen, int nunits, int block, int grid) {
-    if (++s == s1) next_unit(g, seglen, nunits, block, grid);
+  SSD_HD void next(const G& g, int nunits, int block, int grid) {
+    if (++s == s1) next_unit(g, nunits, block, grid);
   }
-  // tiles of a block; `segs` = segments of a unit among the `nunits`
+  // tiles of a block
   template <class G>
-  static SSD_HD int total(const G& g, int seglen, int nunits, int segs, int block, int grid) {
-    if constexpr (BAL) {
-      const long long T = (long long)nunits * g.nc;
-      return (int)((block + 1) * T / grid - block * T / grid);
-    } else {
-      int n = 0;
-      for (int u = block; u < nunits; u += grid) {
-        const int s0 = u / (nunits / segs) * seglen;
-        n += seglen < g.nc - s0 ? seglen : g.nc - s0;
-      }
-      return n;
-    }
+  static SSD_HD int total(const G& g, int nunits, int block, int grid) {
+    const long long T = (long long)nunits * g.nc;
+    if constexpr (BAL) return (int)((block + 1) * T / grid - block * T / grid);
+    else return (nunits - block + grid - 1) / grid * g.nc;
   }
 };
 
