@@ -162,3 +162,27 @@ def test_state_tiles_of_every_width(lib, S, P, N, dtype):
     yr, Sr = O.state_update(inp["state"].double(), inp["x"][0], dt, inp["A"], inp["B"][0], inp["C"][0], inp["D"], z)
     assert_close("y", y, yr, dtype)
     assert_close("state", state, Sr, dtype)
+
+
+def test_state_update_checks_the_callers_y(lib):
+    """A y that the kernel would overrun (short, another type or device, inner dims or rows that do not fit) is refused before
+    anything is launched; rows that lie apart are written and nothing between them."""
+    import trading_bot_0_b200 as T
+    S, H, P, N = 6, 8, 32, 64
+    inp = O.make_decode_inputs(O.SsdConfig("dec", S, 1, H, P, N, 1, 1, "bf16"), 1)
+    d = to_dev(inp, DEV)
+    a = lambda st: (st, d["x"][0], d["dt"][0], d["A"], d["B"][0], d["C"][0], d["D"])
+    bf = dict(dtype=torch.bfloat16, device=DEV)
+    bad = [torch.empty(S - 1, H, P, **bf), torch.empty(S, H, P - 1, **bf), torch.empty(S * H * P, **bf),
+           torch.empty(S, H, P, dtype=torch.float16, device=DEV), torch.empty(S, H, P, device=DEV), torch.empty(S, H, P, dtype=torch.bfloat16),
+           torch.empty(S, H, 2 * P, **bf)[:, :, ::2], torch.empty(S, H, 2 * P, **bf)[:, :, :P], torch.empty(S, P, H, **bf).transpose(1, 2),
+           torch.empty(1, H, P, **bf).expand(S, H, P)]
+    state = d["state"].clone()
+    for y in bad:
+        with pytest.raises(ValueError, match="y: "):
+            T.state_update(*a(state), y=y)
+    assert torch.equal(state, d["state"])
+    ref = T.state_update(*a(state))
+    buf = torch.full((S, H + 1, P), 7.0, **bf)
+    y = T.state_update(*a(d["state"].clone()), y=buf[:, :H])
+    assert torch.equal(y, ref) and (buf[:, H] == 7.0).all()

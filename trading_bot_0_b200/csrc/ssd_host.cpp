@@ -520,6 +520,12 @@ PyObject* py_state_update(PyObject*, PyObject* const* argv, Py_ssize_t argc) {
                      a.opt(9, "dt_bias"), a.flag(10), dev);
     const Tensor* y_in = a.opt(8, "y");
     Tensor y = y_in ? *y_in : empty(Shape(s.S, s.H, s.P), x.scalar_type(), dev);
+    if (y_in) {   // rows may lie apart, but not over one another
+      const Shape shape(s.S, s.H, s.P);
+      if (!same(y, shape) || y.scalar_type() != x.scalar_type() || y.device() != dev)
+        fail("y: expected ", at::IntArrayRef(shape), " ", x.scalar_type(), " on ", dev, ", got ", y.sizes(), " ", y.scalar_type(), " on ", y.device());
+      if ((s.P > 1 && y.stride(2) != 1) || (s.H > 1 && y.stride(1) != s.P) || (s.S > 1 && y.stride(0) < s.H * s.P)) fail("y: inner dims must be dense and rows apart");
+    }
     s.d.y_stride_s = y.stride(0);
     s.p.y = ptr(&y);
     const c10::cuda::CUDAGuard guard(dev);
@@ -540,6 +546,7 @@ PyObject* py_state_update_host(PyObject*, PyObject* const* argv, Py_ssize_t argc
     for (const Tensor* t : {&y, &yh})
       if (!same(*t, Shape(s.S, s.H, s.P)) || t->scalar_type() != a.tensor(1, "x").scalar_type() || !t->is_contiguous())
         fail("y: expected a contiguous ", at::IntArrayRef(Shape(s.S, s.H, s.P)), " tensor");
+    if (y.device() != dev) fail("y: expected device ", dev, ", got ", y.device());
     s.d.y_stride_s = s.H * s.P;
     s.p.y = ptr(&y);
     const c10::cuda::CUDAGuard guard(dev);
