@@ -140,3 +140,38 @@ def test_mamba2_mixer_core_autograd_fp32_kernels(lib):
     assert_close("out", out, ref, "bf16")
     for name, got, want in zip(("dxBC", "ddt", "dz", "dconv_w", "dconv_b", "ddt_bias", "dA", "dD", "dnorm_w"), dl, grads):
         assert_close(name, got.grad.detach(), want, "bf16")
+
+
+def test_operands_that_do_not_fit_are_refused(lib):
+    """Outputs, weights, statistics, gradients and workspaces that a kernel would read or write past their end are a ValueError
+    before anything is launched; a weight of another shape with as many values is taken."""
+    import trading_bot_0_b200 as T
+    from trading_bot_0_b200 import prepost as PP
+    Bn, L, Cn = 2, 64, 128
+    bf = dict(dtype=torch.bfloat16, device=DEV)
+    x, w, b = torch.randn(Bn, L, Cn, **bf), torch.randn(Cn, 4, device=DEV), torch.zeros(Cn, device=DEV)
+    for kw in (dict(out=torch.empty(Bn, L - 1, Cn, **bf)), dict(out=torch.empty(Bn, L, Cn, dtype=torch.float16, device=DEV)),
+               dict(out=torch.empty(Bn, L, Cn, dtype=torch.bfloat16)), dict(bias=b[:-8]), dict(bias=b.bfloat16()), dict(bias=b.cpu()),
+               dict(weight=w.cpu()), dict(weight=w[:-8])):
+        with pytest.raises(ValueError, match="conv1d"):
+            PP.conv1d_forward(**{**dict(inp=x, weight=w, bias=b), **kw})
+    for weight, bias, dout in ((w.bfloat16(), b, x), (w[:-8], b, x), (w, b[:-8], x), (w, b, x.cpu())):
+        with pytest.raises(ValueError, match="conv1d"):
+            PP.conv1d_backward(x, weight, bias, [dout])
+    nw = torch.ones(Cn, device=DEV)
+    out, rstd = PP.rmsnorm_forward(x, nw.view(4, -1))
+    assert torch.equal(out, PP.rmsnorm_forward(x, nw)[0])
+    for weight in (nw[:-8], nw.bfloat16(), nw.cpu()):
+        with pytest.raises(ValueError, match="rmsnorm"):
+            PP.rmsnorm_forward(x, weight)
+    for weight, r, dout in ((nw[:-8], rstd, x), (nw, rstd[:-1], x), (nw, rstd.double(), x), (nw, rstd, x[:1]), (nw, rstd, x.float())):
+        with pytest.raises(ValueError, match="rmsnorm"):
+            PP.rmsnorm_backward(x, weight, r, dout)
+    d = {k: v.to(DEV) for k, v in O.make_inputs(O.SsdConfig("op", 1, 128, 8, 32, 64, 1, 128, "bf16", False)).items() if v is not None}
+    a = (d["x"], d["dt"], d["A"], d["B"], d["C"], d["D"])
+    _, _, ws = T.forward(*a, chunk=128, for_backward=True)
+    for bad in (torch.empty(ws.numel(), dtype=torch.uint8), torch.empty(2 * ws.numel(), dtype=torch.uint8, device=DEV)[::2]):
+        with pytest.raises(ValueError, match="workspace"):
+            T.forward(*a, chunk=128, workspace=bad)
+        with pytest.raises(ValueError, match="workspace"):
+            T.backward(d["dy"], *a, chunk=128, workspace=bad, fwd_saved=True)

@@ -151,6 +151,10 @@ void check_dense_f32(const char* name, const Tensor* t, const Shape& shape, cons
   if (t->scalar_type() != at::kFloat) fail(name, ": expected float32, got ", t->scalar_type());
   if (t->device() != dev || !t->is_contiguous()) fail(name, ": must be a contiguous tensor on ", dev);
 }
+void check_values_f32(const char* name, const Tensor* t, int64_t n, const at::Device& dev) {   // any shape
+  if (t && (t->numel() != n || t->scalar_type() != at::kFloat || t->device() != dev || !t->is_contiguous()))
+    fail(name, ": expected ", n, " contiguous fp32 values on ", dev, ", got ", t->sizes(), " ", t->scalar_type(), " on ", t->device());
+}
 Tensor empty(at::IntArrayRef shape, at::ScalarType dtype, const at::Device& dev) {
   return at::detail::empty_cuda(shape, dtype, dev, std::nullopt);
 }
@@ -211,6 +215,10 @@ Tensor workspace_for(const SsdDims& d, const at::Device& dev, bool backward) {
   return empty(at::IntArrayRef(&size, 1), at::kByte, dev);
 }
 
+void check_workspace(const Tensor& ws, const at::Device& dev) {
+  if (ws.device() != dev || !ws.is_contiguous()) fail("workspace: must be a contiguous tensor on ", dev);
+}
+
 // y, final_state, workspace; undefined ones among the three are allocated here (final_state only when `want_final`).
 void scan_forward(const Scan& s, Tensor& y, Tensor& fin, Tensor& ws, bool want_final, bool for_backward, int32_t stages) {
   const at::Device dev = s.x.device();
@@ -222,7 +230,8 @@ void scan_forward(const Scan& s, Tensor& y, Tensor& fin, Tensor& ws, bool want_f
   const Shape state(d.batch, d.nheads, d.headdim, d.dstate);
   if (fin.defined()) check_dense_f32("final_state", &fin, state, dev);
   else if (want_final) fin = empty(state, at::kFloat, dev);
-  if (!ws.defined()) ws = workspace_for(d, dev, for_backward);
+  if (ws.defined()) check_workspace(ws, dev);
+  else ws = workspace_for(d, dev, for_backward);
   SsdFwdPtrs p;
   std::memset(&p, 0, sizeof p);
   p.x = ptr(&s.x); p.dt = ptr(&s.dt); p.A = fptr(&s.A); p.Bm = ptr(&s.Bm); p.Cm = ptr(&s.Cm); p.D = fptr(s.D); p.z = ptr(s.z);
@@ -258,7 +267,9 @@ void scan_backward(const Scan& s, const Tensor& dy, const Tensor* dfin, Tensor& 
   if (s.z) out_slot("dz", o.dz, Shape(B, L, H, P), st, dev);
   if (want_dinit || s.init) out_slot("dinit", o.dinit, Shape(B, H, P, N), at::kFloat, dev);
   if (s.bias) out_slot("ddt_bias", o.dbias, Shape(H), at::kFloat, dev);
-  if (!ws.defined()) {
+  if (ws.defined()) {
+    check_workspace(ws, dev);
+  } else {
     if (fwd_saved) fail("fwd_saved=True needs the workspace the forward ran in");
     ws = workspace_for(d, dev, true);
   }
@@ -273,6 +284,13 @@ void scan_backward(const Scan& s, const Tensor& dy, const Tensor* dfin, Tensor& 
 }
 
 // ---- conv1d and RMS norm -----------------------------------------------------------------------------------------------
+void check_conv_weights(const Tensor& in, const Tensor& weight, const Tensor* bias) {
+  if (weight.scalar_type() != at::kFloat || !weight.is_contiguous() || weight.dim() != 2)
+    fail("conv1d: weight must be contiguous fp32 [channels, width]");
+  if (weight.device() != in.device()) fail("conv1d: weight: expected device ", in.device(), ", got ", weight.device());
+  if (weight.size(0) != in.size(2)) fail("conv1d: weight rows must equal the channel count");
+  check_values_f32("conv1d: bias", bias, weight.size(0), in.device());
+}
 SsdConvDims conv_dims(const Tensor& in, const Tensor& out, int64_t width, bool activation) {
   if (!in.is_cuda() || in.dim() != 3 || (in.scalar_type() != at::kBFloat16 && in.scalar_type() != at::kFloat))
     fail("conv1d: input must be a CUDA [batch, seqlen, channels] bf16/fp32 tensor");
@@ -285,21 +303,21 @@ SsdConvDims conv_dims(const Tensor& in, const Tensor& out, int64_t width, bool a
   return d;
 }
 void conv_forward(const Tensor& in, const Tensor& weight, const Tensor* bias, bool activation, Tensor& out) {
-  if (weight.scalar_type() != at::kFloat || !weight.is_contiguous() || weight.dim() != 2)
-    fail("conv1d: weight must be contiguous fp32 [channels, width]");
-  if (!out.defined()) {
-    if (!in.is_cuda()) fail("conv1d: input must be a CUDA [batch, seqlen, channels] bf16/fp32 tensor");
-    out = empty(in.sizes(), in.scalar_type(), in.device());
-  }
+  if (!in.is_cuda() || in.dim() != 3) fail("conv1d: input must be a CUDA [batch, seqlen, channels] bf16/fp32 tensor");
+  check_conv_weights(in, weight, bias);
+  if (!out.defined()) out = empty(in.sizes(), in.scalar_type(), in.device());
+  if (!same(out, in.sizes()) || out.scalar_type() != in.scalar_type() || out.device() != in.device())
+    fail("conv1d: out: expected ", in.sizes(), " ", in.scalar_type(), " on ", in.device(), ", got ", out.sizes(), " ", out.scalar_type(),
+         " on ", out.device());
   const SsdConvDims d = conv_dims(in, out, weight.size(1), activation);
-  if (weight.size(0) != d.channels) fail("conv1d: weight rows must equal the channel count");
   const c10::cuda::CUDAGuard guard(in.device());
   check_rc(api.conv1d_forward(&d, ptr(&in), fptr(&weight), fptr(bias), ptr(&out), stream_of(in.device())));
 }
 struct ConvGrads { Tensor din, dweight, dbias; };
 ConvGrads conv_backward(const Tensor& in, const Tensor& weight, const Tensor* bias, const Tensor* const* douts, int ndout, bool activation) {
   const at::Device dev = in.device();
-  if (!in.is_cuda()) fail("conv1d: input must be a CUDA [batch, seqlen, channels] bf16/fp32 tensor");
+  if (!in.is_cuda() || in.dim() != 3) fail("conv1d: input must be a CUDA [batch, seqlen, channels] bf16/fp32 tensor");
+  check_conv_weights(in, weight, bias);
   ConvGrads g;
   g.din = empty(in.sizes(), in.scalar_type(), dev);
   const SsdConvDims d = conv_dims(in, g.din, weight.size(1), activation);
@@ -308,7 +326,7 @@ ConvGrads conv_backward(const Tensor& in, const Tensor& weight, const Tensor* bi
   if (ndout > 3) fail("conv1d backward: 1 to 3 gradient segments, got ", (int64_t)ndout);
   for (int i = 0; i < ndout; ++i) {
     const Tensor& t = *douts[i];
-    if (t.dim() != 3 || t.scalar_type() != in.scalar_type() || t.stride(2) != 1 || t.size(0) != in.size(0) || t.size(1) != in.size(1))
+    if (t.dim() != 3 || t.scalar_type() != in.scalar_type() || t.stride(2) != 1 || t.size(0) != in.size(0) || t.size(1) != in.size(1) || t.device() != dev)
       fail("conv1d backward: bad gradient segment");
     segs[i].ptr = ptr(&t); segs[i].channels = (int32_t)t.size(2); segs[i].stride_b = t.stride(0); segs[i].stride_l = t.stride(1);
   }
@@ -323,6 +341,11 @@ ConvGrads conv_backward(const Tensor& in, const Tensor& weight, const Tensor* bi
   return g;
 }
 
+void check_norm(const Tensor& in, const Tensor* weight) {
+  if (!in.is_cuda() || (in.scalar_type() != at::kBFloat16 && in.scalar_type() != at::kFloat) || !in.is_contiguous() || in.dim() < 1)
+    fail("rmsnorm: input must be a contiguous CUDA bf16/fp32 tensor");
+  check_values_f32("rmsnorm: weight", weight, in.size(-1), in.device());
+}
 SsdNormDims norm_dims(const Tensor& in, double eps) {   // `in` contiguous: every dim but the last is a row
   SsdNormDims d;
   std::memset(&d, 0, sizeof d);
@@ -332,8 +355,7 @@ SsdNormDims norm_dims(const Tensor& in, double eps) {   // `in` contiguous: ever
   return d;
 }
 void norm_forward(const Tensor& in, const Tensor* weight, double eps, Tensor& out, Tensor& rstd) {
-  if (!in.is_cuda() || (in.scalar_type() != at::kBFloat16 && in.scalar_type() != at::kFloat) || !in.is_contiguous())
-    fail("rmsnorm: input must be a contiguous CUDA bf16/fp32 tensor");
+  check_norm(in, weight);
   const SsdNormDims d = norm_dims(in, eps);
   out = empty(in.sizes(), in.scalar_type(), in.device());
   rstd = empty(Shape(d.rows), at::kFloat, in.device());
@@ -341,8 +363,13 @@ void norm_forward(const Tensor& in, const Tensor* weight, double eps, Tensor& ou
   check_rc(api.rmsnorm_forward(&d, ptr(&in), fptr(weight), ptr(&out), fptr(&rstd), stream_of(in.device())));
 }
 void norm_backward(const Tensor& in, const Tensor* weight, const Tensor& rstd, const Tensor& dout_, double eps, Tensor& din, Tensor& dweight) {
+  check_norm(in, weight);
+  if (dout_.numel() != in.numel() || dout_.scalar_type() != in.scalar_type() || dout_.device() != in.device())
+    fail("rmsnorm: dout: expected ", in.sizes(), " ", in.scalar_type(), " on ", in.device(), ", got ", dout_.sizes(), " ", dout_.scalar_type(),
+         " on ", dout_.device());
   const Tensor dout = dout_.contiguous();
   const SsdNormDims d = norm_dims(in, eps);
+  check_values_f32("rmsnorm: rstd", &rstd, d.rows, in.device());
   const at::Device dev = in.device();
   din = empty(in.sizes(), in.scalar_type(), dev);
   Tensor ws;
