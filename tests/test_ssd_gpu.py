@@ -319,3 +319,53 @@ def test_misaligned_pointer_is_an_error_code_not_a_fault(lib):
     y_ok, _, _ = T.forward(d["x"], d["dt"], d["A"], d["B"], d["C"], d["D"], chunk=128, algo="tensor")
     y2, _, _ = T.forward(d["x"], d["dt"], d["A"], d["B"], d["C"], d["D"], chunk=128, algo="fp32_cores", y=y_off)
     assert (y2.float() - y_ok.float()).abs().max().item() <= 2e-2
+
+
+@pytest.mark.parametrize("dtype", ["fp32", "bf16"])
+@pytest.mark.parametrize("dim", [0, 1])
+@pytest.mark.parametrize("node", ["host", "libtorch"])
+def test_gradient_that_comes_expanded(lib, dtype, dim, node):
+    """The gradient of a sum over the batch (or over the sequence) arrives as a view of stride 0: it gives what the same values
+    in a dense tensor give."""
+    import trading_bot_0_b200 as T
+    from trading_bot_0_b200 import torch_node as TN
+    scan = T.ssd_scan if node == "host" else TN.ssd_scan
+    cfg = O.SsdConfig("exp", 3, 256, 8, 32, 64, 1, 128, dtype)
+    d = to_dev(O.make_inputs(cfg), DEV)
+    names = ("x", "dt", "A", "B", "C", "D")
+    w = torch.randn_like(d["x"].select(dim, 0))
+    out = []
+    for expanded in (True, False):
+        v = [d[k].detach().clone().requires_grad_() for k in names]
+        y, _ = scan(*v, chunk=128)
+        if expanded:
+            y.sum(dim).backward(w)
+        else:
+            y.backward(w.unsqueeze(dim).expand(y.shape).contiguous())
+        out.append([t.grad for t in v])
+    for k, a, b in zip(names, *out):
+        assert torch.equal(a, b), k
+
+
+def test_operands_that_come_expanded_are_refused(lib):
+    """The C structs take stride 0 as dense, so an expanded operand would be read past its end: an error before any launch."""
+    import trading_bot_0_b200 as T
+    from trading_bot_0_b200 import torch_node as TN
+    d = to_dev(O.make_inputs(O.SsdConfig("exp", 3, 256, 8, 32, 64, 1, 128, "bf16")), DEV)
+    a = {k: d[k] for k in ("x", "dt", "A", "B", "C", "D")}
+    for k in ("x", "dt", "B", "C"):
+        for e in (d[k][:1].expand(d[k].shape), d[k][:, :1].expand(d[k].shape)):
+            with pytest.raises(ValueError, match="expanded"):
+                T.forward(*{**a, k: e}.values(), chunk=128)
+            with pytest.raises(RuntimeError, match="expanded"):
+                TN.ssd_scan(*{**a, k: e}.values(), chunk=128)
+    with pytest.raises(ValueError, match="expanded"):
+        T.backward(d["dy"][:1].expand(d["dy"].shape), *a.values(), chunk=128)
+    st = torch.zeros(3, 8, 32, 64, device=DEV)
+    v = [d[k][:, 0].contiguous() for k in ("x", "dt", "B", "C")]
+    for i in range(4):
+        u = list(v)
+        u[i] = u[i][:1].expand(v[i].shape)
+        with pytest.raises(ValueError, match="expanded"):
+            T.state_update(st, u[0], u[1], d["A"], u[2], u[3], d["D"])
+    assert (st == 0).all()

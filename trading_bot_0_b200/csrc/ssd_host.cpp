@@ -135,6 +135,12 @@ struct Shape {   // small fixed-size shape, no allocation
 };
 bool same(const Tensor& t, at::IntArrayRef s) { return t.sizes() == s; }
 
+// The geometry structs take a stride of 0 as "dense", so rows that lie over one another cannot be described by them.
+bool overlaid(const Tensor& t, int dims) {
+  for (int i = 0; i < dims; ++i)
+    if (t.size(i) > 1 && t.stride(i) == 0) return true;
+  return false;
+}
 void check_seq(const char* name, const Tensor& t, const Shape& shape, at::ScalarType dtype, const at::Device& dev) {
   if (!same(t, shape)) {
     if (t.dim() != shape.n) fail(name, ": expected rank ", (int64_t)shape.n, ", got ", t.dim());
@@ -144,6 +150,7 @@ void check_seq(const char* name, const Tensor& t, const Shape& shape, at::Scalar
   if (t.device() != dev) fail(name, ": expected device ", dev, ", got ", t.device());
   if (t.stride(-1) != 1) fail(name, ": innermost stride must be 1");
   if (t.dim() == 4 && t.stride(2) != t.size(3)) fail(name, ": the last two dims must be dense");
+  if (overlaid(t, 2)) fail(name, ": expanded over a dim (stride 0); make it contiguous");
 }
 void check_dense_f32(const char* name, const Tensor* t, const Shape& shape, const at::Device& dev) {
   if (!t) return;
@@ -395,11 +402,12 @@ const Tensor* or_null(const Opt& t) { return t.has_value() ? &*t : nullptr; }
 Tensor or_undefined(const Opt& t) { return t.has_value() ? *t : Tensor(); }
 Tensor or_undefined(const Tensor* t) { return t ? *t : Tensor(); }
 const Tensor* or_null(const Tensor& t) { return t.defined() ? &t : nullptr; }
-// An incoming gradient in the layout the kernels read: x's dtype, inner dims dense.
+// An incoming gradient in the layout the kernels read: x's dtype, inner dims dense, rows apart (that of a sum or mean over the
+// batch comes expanded).
 Tensor usable_dy(const Tensor& g, const Tensor& x) {
   if (!g.defined()) return at::zeros(x.sizes(), x.options().requires_grad(false));
   Tensor dy = g.scalar_type() == x.scalar_type() ? g : g.to(x.scalar_type());
-  if (dy.stride(-1) != 1 || dy.stride(2) != dy.size(3)) dy = dy.contiguous();
+  if (dy.stride(-1) != 1 || dy.stride(2) != dy.size(3) || overlaid(dy, 2)) dy = dy.contiguous();
   return dy;
 }
 Tensor as_type(const Tensor& t, at::ScalarType st) { return t.scalar_type() == st ? t : t.to(st); }
@@ -519,6 +527,7 @@ Step step_of(const Tensor& state, const Tensor& x, const Tensor& dt, const Tenso
     if (!same(t, shape) || t.scalar_type() != x.scalar_type() || t.device() != where)
       fail(name, ": expected ", at::IntArrayRef(shape), " ", x.scalar_type(), " on ", where);
     if (t.stride(-1) != 1 || (t.dim() >= 3 && t.stride(1) != t.size(2))) fail(name, ": inner dims must be dense");
+    if (overlaid(t, 1)) fail(name, ": expanded over the streams (stride 0); make it contiguous");
   };
   vec("x", x, Shape(S, H, P)); vec("dt", dt, Shape(S, H)); vec("B", Bm, Shape(S, G, N)); vec("C", Cm, Shape(S, G, N));
   check_dense_f32("A", &A, Shape(H), dev);

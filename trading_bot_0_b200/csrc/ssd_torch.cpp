@@ -47,12 +47,19 @@ const void* ptr(const Tensor* t) { return t ? t->data_ptr() : nullptr; }
 const float* fptr(const Tensor* t) { return t ? t->data_ptr<float>() : nullptr; }
 
 using Shape = std::vector<int64_t>;
+// The geometry structs take a stride of 0 as "dense", so rows that lie over one another cannot be described by them.
+bool overlaid(const Tensor& t, int dims) {
+  for (int i = 0; i < dims; ++i)
+    if (t.size(i) > 1 && t.stride(i) == 0) return true;
+  return false;
+}
 void check_seq(const char* name, const Tensor& t, const Shape& shape, const Tensor& like) {
   TORCH_CHECK(t.defined() && t.sizes() == at::IntArrayRef(shape), "ssd: ", name, " must have shape ", at::IntArrayRef(shape),
               ", got ", t.sizes());
   TORCH_CHECK(t.scalar_type() == like.scalar_type() && t.device() == like.device(), "ssd: ", name,
               " must have x's dtype and device");
   TORCH_CHECK(t.stride(-1) == 1 && (t.dim() < 4 || t.stride(2) == t.size(3)), "ssd: ", name, ": the inner dims must be dense");
+  TORCH_CHECK(!overlaid(t, 2), "ssd: ", name, ": expanded over a dim (stride 0); make it contiguous");
 }
 void check_f32(const char* name, const Tensor* t, const Shape& shape, const Tensor& like) {
   if (!t) return;
@@ -144,7 +151,7 @@ struct SsdScanNode : public torch::autograd::Function<SsdScanNode> {
                  *pinit = s[7].defined() ? &s[7] : nullptr, *pbias = s[8].defined() ? &s[8] : nullptr;
     Tensor dy = grads[0].defined() ? grads[0] : at::zeros(x.sizes(), x.options());
     if (dy.scalar_type() != x.scalar_type()) dy = dy.to(x.scalar_type());
-    if (dy.stride(-1) != 1 || dy.stride(2) != dy.size(3)) dy = dy.contiguous();
+    if (dy.stride(-1) != 1 || dy.stride(2) != dy.size(3) || overlaid(dy, 2)) dy = dy.contiguous();   // a sum over the batch: expanded
     Tensor dfin = grads[1].defined() ? grads[1].to(at::kFloat).contiguous() : Tensor();
     SsdDims d = make_dims(x, dt, Bm, Cm, pz, dy, ctx->saved_data["chunk"].toInt(), ctx->saved_data["dt_softplus"].toBool(),
                           ctx->saved_data["algo"].toInt());
@@ -195,6 +202,7 @@ Tensor ssd_state_update_op(Tensor state, const Tensor& x, const Tensor& dt, cons
     TORCH_CHECK(t.sizes() == at::IntArrayRef(shape) && t.scalar_type() == x.scalar_type() && t.device() == state.device(),
                 "ssd: ", name, " must have shape ", at::IntArrayRef(shape), ", x's dtype and the state's device");
     TORCH_CHECK(t.stride(-1) == 1 && (t.dim() < 3 || t.stride(1) == t.size(2)), "ssd: ", name, ": the inner dims must be dense");
+    TORCH_CHECK(!overlaid(t, 1), "ssd: ", name, ": expanded over the streams (stride 0); make it contiguous");
   };
   seq("x", x, {S, H, P}); seq("dt", dt, {S, H}); seq("B", Bm, {S, G, N}); seq("C", Cm, {S, G, N});
   if (pz) seq("z", *pz, {S, H, P});
