@@ -108,15 +108,33 @@ def test_host_step_groups_match_oracle(lib, groups, graph):
     ref_y, ref_S = oracle_steps(inp, steps)
     d = to_dev(inp, DEV)
     state = d["state"].clone()
-    hs = HostStep(state, cfg.ngroups, groups=groups, graph=graph)
+    hs = HostStep(state, cfg.ngroups, groups=groups, graph=graph, in_place=False)
     ys = []
     for t in range(steps):
         hs.load_inputs(inp["x"][t], inp["dt"][t], inp["B"][t], inp["C"][t])
         hs.step(d["A"], d["D"])
         torch.cuda.synchronize()
         ys.append(hs.hy.clone())
+    assert (hs._graph is not None) == graph and (len(hs.ranges) > 1) == (groups > 1)
     assert_close("y", torch.stack(ys).to(DEV), ref_y, "bf16")
     assert_close("state", state, ref_S, "bf16")
+
+
+@pytest.mark.parametrize("in_place", [True, False])
+@pytest.mark.parametrize("N", [64, 40])
+def test_host_step_device_copies(lib, in_place, N):
+    """x, dt, Bm, Cm hold the step's vectors on the device after a step of either kind (N = 40 copies anyway)."""
+    from trading_bot_0_b200.host import HostStep
+    inp = O.make_decode_inputs(O.SsdConfig("dec", 33, 1, 8, 32, N, 1, 1, "bf16"), 2)
+    d = to_dev(inp, DEV)
+    hs = HostStep(d["state"].clone(), 1, in_place=in_place)
+    for t in range(2):
+        hs.load_inputs(inp["x"][t], inp["dt"][t], inp["B"][t], inp["C"][t])
+        hs.step(d["A"], d["D"])
+        for k, v in (("x", hs.x), ("dt", hs.dt), ("B", hs.Bm), ("C", hs.Cm)):
+            assert v.is_cuda and torch.equal(v.cpu(), inp[k][t]), k
+        torch.cuda.synchronize()
+        assert torch.equal(hs.y.cpu(), hs.hy)
 
 
 @pytest.mark.parametrize("S,H,P,N,G,dtype", [(1, 8, 32, 64, 1, "bf16"), (33, 8, 32, 64, 1, "fp32"), (1201, 8, 32, 64, 2, "bf16"),

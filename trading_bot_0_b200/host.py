@@ -114,20 +114,26 @@ class HostFwdBwd:
 
 class HostStep:
     """Streamed-rollout step with the per-step vectors in pinned host memory and the state resident on
-    the device: one call copies x, dt, B, C in, runs the state update and copies y out.
+    the device: one call takes x, dt, B, C in, runs the state update and brings y out.
 
     The object owns the pinned staging buffers: the caller writes the step's vectors into `hx`, `hdt`,
     `hB`, `hC` (views of ONE packed pinned buffer, one packed row per stream) and reads the result from `hy`.
     Where the library's host-memory step covers the shape, a step is one kernel that reads the packed rows and writes
-    `hy` over PCIe itself.  Other shapes copy: the streams (environments) are cut into `groups`
-    row ranges that flow through three CUDA streams (host->device copies, kernels, device->host copies),
+    `hy` over PCIe itself.  Other shapes, and all with `in_place=False`, copy: the streams (environments) are cut into
+    `groups` row ranges that flow through three CUDA streams (host->device copies, kernels, device->host copies),
     the way a rollout double-buffers groups of environments: while one group's kernel runs, the next
     group's inputs arrive and the previous group's outputs leave.  After one eager step the whole step is
-    captured into a CUDA graph and replayed, so a step costs one launch on the host
-    (trading_bots/src/torch/train/rollout.rs:209-235 is the per-step loop this stands in for).
-    `step` returns after enqueueing on the caller's current stream."""
+    captured into a CUDA graph and replayed (`graph`), so a step costs one launch on the host
+    (trading_bots/src/torch/train/rollout.rs:209-235 is the per-step loop this stands in for).  `groups` and `graph`
+    shape the copies only: the one kernel has neither.
+    `step` returns after enqueueing on the caller's current stream.
 
-    def __init__(self, state: torch.Tensor, ngroups: int, dtype=torch.bfloat16, groups: int = 8, graph: bool = True):
+    `y` is the device copy of the result, `x`, `dt`, `Bm`, `Cm` are device copies of the step's vectors.  A copying step
+    leaves them behind; after an in-place step they are fetched on the current stream when they are read, so read them
+    before the staging buffers are written again."""
+
+    def __init__(self, state: torch.Tensor, ngroups: int, dtype=torch.bfloat16, groups: int = 8, graph: bool = True,
+                 in_place: bool = True):
         S, H, P, N = state.shape
         dev = state.device
         self.state, self.dev = state, dev
@@ -136,22 +142,36 @@ class HostStep:
         o_dt, o_b, o_c = up(hp), up(hp) + up(H), up(hp) + up(H) + up(gn)
         self.row = o_c + up(gn)
         self.host_in = torch.zeros(S, self.row, dtype=dtype).pin_memory()
-        self.dev_in = torch.zeros(S, self.row, dtype=dtype, device=dev)
-        cut = lambda buf: (buf[:, :hp].unflatten(1, (H, P)), buf[:, o_dt:o_dt + H],
-                           buf[:, o_b:o_b + gn].unflatten(1, (ngroups, N)),
-                           buf[:, o_c:o_c + gn].unflatten(1, (ngroups, N)))
-        self.hx, self.hdt, self.hB, self.hC = cut(self.host_in)
-        self.x, self.dt, self.Bm, self.Cm = cut(self.dev_in)
+        self._cut = lambda buf: (buf[:, :hp].unflatten(1, (H, P)), buf[:, o_dt:o_dt + H],
+                                 buf[:, o_b:o_b + gn].unflatten(1, (ngroups, N)),
+                                 buf[:, o_c:o_c + gn].unflatten(1, (ngroups, N)))
+        self.hx, self.hdt, self.hB, self.hC = self._cut(self.host_in)
         self.y = torch.empty(S, H, P, dtype=dtype, device=dev)
         self.hy = torch.empty(S, H, P, dtype=dtype).pin_memory()
         groups = max(1, min(groups, S))
         per = (S + groups - 1) // groups
         self.ranges = [(lo, min(S, lo + per)) for lo in range(0, S, per)]
-        self.s_in, self.s_run, self.s_out = (torch.cuda.Stream(dev) for _ in range(3))
-        self.ev_in = [torch.cuda.Event() for _ in self.ranges]
-        self.ev_run = [torch.cuda.Event() for _ in self.ranges]
-        self._in_place = True
+        self._in_place = in_place
+        self._dev_in = self._copies = None                   # made by the first step that copies, or the first read
         self.use_graph, self._graph, self._calls, self._params = graph, None, 0, None
+
+    def _device_rows(self) -> torch.Tensor:
+        if self._dev_in is None:
+            self._dev_in = torch.zeros(self.host_in.shape, dtype=self.host_in.dtype, device=self.dev)
+        return self._dev_in
+
+    @property
+    def dev_in(self) -> torch.Tensor:
+        """The packed rows on the device (see the class)."""
+        rows = self._device_rows()
+        if self._in_place:
+            rows.copy_(self.host_in, non_blocking=True)
+        return rows
+
+    x = property(lambda self: self._cut(self.dev_in)[0])
+    dt = property(lambda self: self._cut(self.dev_in)[1])
+    Bm = property(lambda self: self._cut(self.dev_in)[2])
+    Cm = property(lambda self: self._cut(self.dev_in)[3])
 
     def bytes_per_call(self):
         """(host->device, device->host) bytes one step moves, counted from the buffers copied."""
@@ -165,21 +185,23 @@ class HostStep:
         self.hC.copy_(hC)
 
     def _enqueue(self, root, A, D) -> None:
-        for s in (self.s_in, self.s_run, self.s_out):
+        s_in, s_run, s_out, ev_in, ev_run = self._copies
+        rows = self._device_rows()
+        x, dt, Bm, Cm = self._cut(rows)
+        for s in (s_in, s_run, s_out):
             s.wait_stream(root)
         for gi, (lo, hi) in enumerate(self.ranges):
-            with torch.cuda.stream(self.s_in):
-                self.dev_in[lo:hi].copy_(self.host_in[lo:hi], non_blocking=True)
-                self.ev_in[gi].record(self.s_in)
-            with torch.cuda.stream(self.s_run):
-                self.s_run.wait_event(self.ev_in[gi])
-                ssd.state_update(self.state[lo:hi], self.x[lo:hi], self.dt[lo:hi], A, self.Bm[lo:hi], self.Cm[lo:hi], D,
-                                 y=self.y[lo:hi])
-                self.ev_run[gi].record(self.s_run)
-            with torch.cuda.stream(self.s_out):
-                self.s_out.wait_event(self.ev_run[gi])
+            with torch.cuda.stream(s_in):
+                rows[lo:hi].copy_(self.host_in[lo:hi], non_blocking=True)
+                ev_in[gi].record(s_in)
+            with torch.cuda.stream(s_run):
+                s_run.wait_event(ev_in[gi])
+                ssd.state_update(self.state[lo:hi], x[lo:hi], dt[lo:hi], A, Bm[lo:hi], Cm[lo:hi], D, y=self.y[lo:hi])
+                ev_run[gi].record(s_run)
+            with torch.cuda.stream(s_out):
+                s_out.wait_event(ev_run[gi])
                 self.hy[lo:hi].copy_(self.y[lo:hi], non_blocking=True)
-        for s in (self.s_in, self.s_run, self.s_out):
+        for s in (s_in, s_run, s_out):
             root.wait_stream(s)
 
     def _step_in_place(self, A, D) -> bool:
@@ -196,6 +218,8 @@ class HostStep:
         if self._in_place and self._step_in_place(A, D):
             return
         cur = torch.cuda.current_stream(self.dev)
+        if self._copies is None:
+            self._copies = (*(torch.cuda.Stream(self.dev) for _ in range(3)), *([torch.cuda.Event() for _ in self.ranges] for _ in range(2)))
         self._calls += 1
         if not self.use_graph or self._calls == 1:          # first step eagerly (also warms everything up)
             self._enqueue(cur, A, D)
