@@ -53,7 +53,14 @@ typedef enum SsdDtype { SSD_F32 = 0, SSD_BF16 = 1 } SsdDtype;
 typedef enum SsdPass { SSD_PASS_FWD = 0, SSD_PASS_BWD = 1 } SsdPass;
 
 /* Kernel family selection.  AUTO picks the tcgen05 tensor-core kernels when dtype is bf16 and
- * the shape is one they cover, else the exact-fp32 CUDA-core kernels.  TENSOR insists on the
+ * the shape is one they cover, else the exact-fp32 CUDA-core kernels.  Sequence lengths that are
+ * no multiple of 128 are among the covered ones (ABI version 1 evaluated those in fp32).  The
+ * tensor-core family multiplies bf16 operands (the decayed score tiles, the chunk-entry states
+ * and their gradients are rounded to bf16) and adds in fp32; FP32_CORES keeps every intermediate
+ * value in fp32, on bf16 storage as well, and is the way to ask for that.  The difference shows in
+ * the gradients: relative to fp64, ddt 2e-3 against 3e-7, dA (a sum of terms that mostly cancel)
+ * 3e-3 to 2e-2 against 3e-6, dB and dC 2.4e-3 to 3e-3 against the 1.7e-3 of their storage; y and
+ * the final state agree to their storage either way.  TENSOR insists on the
  * tensor-core family (an error where it does not apply).  TENSOR_ONETILE is the same family
  * restricted to its one-tile-per-CTA kernels (no persistent pipelines, chunk states and the
  * scan over chunks as two kernels): the comparison arm the persistent kernels are measured

@@ -369,3 +369,22 @@ def test_operands_that_come_expanded_are_refused(lib):
         with pytest.raises(ValueError, match="expanded"):
             T.state_update(st, u[0], u[1], d["A"], u[2], u[3], d["D"])
     assert (st == 0).all()
+
+
+@pytest.mark.parametrize("H,P,N,G,L,has_z", [(8, 32, 64, 1, 333, False), (24, 64, 128, 1, 200, True), (8, 32, 64, 1, 256, False)])
+def test_fp32_cores_on_bf16_storage_keep_fp32(lib, H, P, N, G, L, has_z):
+    """algo = fp32_cores evaluates bf16 calls that the tensor-core kernels would take in fp32 throughout: outputs stored in fp32
+    meet the fp32 gate, those in bf16 are within their rounding (half a unit in the last of 8 bits, doubled for the
+    value it is rounded from)."""
+    import trading_bot_0_b200 as T
+    inp = O.make_inputs(O.SsdConfig("f32", 2, L, H, P, N, G, 128, "bf16", has_z))
+    ref = oracle_all(inp)
+    d = to_dev(inp, DEV)
+    a = (d["x"], d["dt"], d["A"], d["B"], d["C"], d["D"], d.get("z"))
+    y, fin, ws = T.forward(*a, chunk=128, algo="fp32_cores", for_backward=True)
+    g = T.backward(d["dy"], *a, chunk=128, algo="fp32_cores", workspace=ws, fwd_saved=True)
+    for k, v in (("final_state", fin), ("ddt", g["ddt"]), ("dA", g["dA"]), ("dD", g["dD"])):
+        assert_close(k, v, ref[k], "fp32")
+    for k, v in (("y", y), *((k, g[k]) for k in ("dx", "dB", "dC") + (("dz",) if has_z else ()))):
+        e = (v.double().cpu() - ref[k]).abs()
+        assert (e <= 2.0 ** -8 * ref[k].abs() + 1e-4 * ref[k].abs().max()).all(), k

@@ -90,6 +90,7 @@ def mamba2_mixer_core(xBC, dt, z, conv_weight, conv_bias, dt_bias, A, D, norm_we
         x, B, C = split(silu(causal_conv1d(xBC)));  y = SSD(x, softplus(dt + dt_bias), A, B, C, D) * silu(z);
         out = rmsnorm(y) * norm_weight.
     xBC [B,L,H*P+2*G*N], dt [B,L,H], z [B,L,H,P].  One autograd node over this library's operators: conv, scan (with the
-    step-size activation and the gate inside; x, B, C are channel ranges of the conv's output), norm."""
+    step-size activation and the gate inside; x, B, C are channel ranges of the conv's output), norm.  `algo` is the
+    scan's (see ssd.py)."""
     return L.host().mixer(xBC, dt, z, conv_weight, conv_bias, dt_bias, A, D, norm_weight, init_state, nheads, headdim, dstate,
                           ngroups, chunk, eps, ALGOS[algo])
