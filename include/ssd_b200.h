@@ -54,7 +54,7 @@ typedef enum SsdPass { SSD_PASS_FWD = 0, SSD_PASS_BWD = 1 } SsdPass;
 
 /* Kernel family selection.  AUTO picks the tcgen05 tensor-core kernels when dtype is bf16 and
  * the shape is one they cover, else the exact-fp32 CUDA-core kernels.  Sequence lengths that are
- * no multiple of 128 are among the covered ones (ABI version 1 evaluated those in fp32).  The
+ * no multiple of 128 are among the covered ones (earlier builds evaluated those in fp32).  The
  * tensor-core family multiplies bf16 operands (the decayed score tiles, the chunk-entry states
  * and their gradients are rounded to bf16) and adds in fp32; FP32_CORES keeps every intermediate
  * value in fp32, on bf16 storage as well, and is the way to ask for that.  The difference shows in

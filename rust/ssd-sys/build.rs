@@ -81,7 +81,7 @@ fn build_library(csrc: &Path, out: &Path) {
         assert!(status.success(), "nvcc failed on {}", path.display());
         objects.push(obj);
     }
-    for h in ["common.cuh", "umma.cuh", "ssd_internal.h"] {
+    for h in ["common.cuh", "umma.cuh", "ssd_internal.h", "state_plan.h"] {
         println!("cargo:rerun-if-changed={}", csrc.join(h).display());
     }
     let status = Command::new(nvcc())

@@ -177,42 +177,49 @@ struct Scan {
   bool softplus;
 };
 
-SsdDims make_dims(const Scan& s, const Tensor* y) {
-  const Tensor& x = s.x;
+// Validates the sequence operands and fills the geometry struct.
+SsdDims seq_dims(const Tensor& x, const Tensor& dt, const Tensor& Bm, const Tensor& Cm, const Tensor* z, const Tensor* y, int64_t chunk,
+                 int64_t algo, bool softplus) {
   if (!x.is_cuda()) fail("x must be a CUDA tensor (there is no CPU path)");
   if (x.dim() != 4) fail("x must be [batch, seqlen, nheads, headdim]");
   const int32_t dtype = storage_type(x);
-  if (s.Bm.dim() != 4) fail("B must be [batch, seqlen, ngroups, dstate]");
-  const int64_t B = x.size(0), L = x.size(1), H = x.size(2), P = x.size(3), G = s.Bm.size(2), N = s.Bm.size(3);
+  if (Bm.dim() != 4) fail("B must be [batch, seqlen, ngroups, dstate]");
+  const int64_t B = x.size(0), L = x.size(1), H = x.size(2), P = x.size(3), G = Bm.size(2), N = Bm.size(3);
   const at::Device dev = x.device();
   const at::ScalarType st = x.scalar_type();
   check_seq("x", x, Shape(B, L, H, P), st, dev);
-  check_seq("dt", s.dt, Shape(B, L, H), st, dev);
-  check_seq("B", s.Bm, Shape(B, L, G, N), st, dev);
-  check_seq("C", s.Cm, Shape(B, L, G, N), st, dev);
+  check_seq("dt", dt, Shape(B, L, H), st, dev);
+  check_seq("B", Bm, Shape(B, L, G, N), st, dev);
+  check_seq("C", Cm, Shape(B, L, G, N), st, dev);
   if (G <= 0 || H % G) fail("nheads (", H, ") must be a multiple of ngroups (", G, ")");
-  if (s.chunk < 1 || s.chunk > 256) fail("chunk must be in [1, 256], got ", s.chunk);
+  if (chunk < 1 || chunk > 256) fail("chunk must be in [1, 256], got ", chunk);
   SsdDims d;
   std::memset(&d, 0, sizeof d);
   d.batch = (int32_t)B; d.seqlen = (int32_t)L; d.nheads = (int32_t)H; d.headdim = (int32_t)P;
-  d.dstate = (int32_t)N; d.ngroups = (int32_t)G; d.chunk = (int32_t)s.chunk;
-  d.dtype = dtype; d.algo = (int32_t)s.algo; d.device = dev.index(); d.has_z = s.z ? 1 : 0; d.dt_softplus = s.softplus ? 1 : 0;
+  d.dstate = (int32_t)N; d.ngroups = (int32_t)G; d.chunk = (int32_t)chunk;
+  d.dtype = dtype; d.algo = (int32_t)algo; d.device = dev.index(); d.has_z = z ? 1 : 0; d.dt_softplus = softplus ? 1 : 0;
   d.x_stride_b = x.stride(0); d.x_stride_l = x.stride(1);
-  d.dt_stride_b = s.dt.stride(0); d.dt_stride_l = s.dt.stride(1);
-  d.b_stride_b = s.Bm.stride(0); d.b_stride_l = s.Bm.stride(1);
-  d.c_stride_b = s.Cm.stride(0); d.c_stride_l = s.Cm.stride(1);
-  if (s.z) {
-    check_seq("z", *s.z, Shape(B, L, H, P), st, dev);
-    d.z_stride_b = s.z->stride(0); d.z_stride_l = s.z->stride(1);
+  d.dt_stride_b = dt.stride(0); d.dt_stride_l = dt.stride(1);
+  d.b_stride_b = Bm.stride(0); d.b_stride_l = Bm.stride(1);
+  d.c_stride_b = Cm.stride(0); d.c_stride_l = Cm.stride(1);
+  if (z) {
+    check_seq("z", *z, Shape(B, L, H, P), st, dev);
+    d.z_stride_b = z->stride(0); d.z_stride_l = z->stride(1);
   }
   if (y) {
     check_seq("y/dy", *y, Shape(B, L, H, P), st, dev);
     d.y_stride_b = y->stride(0); d.y_stride_l = y->stride(1);
   }
+  return d;
+}
+SsdDims make_dims(const Scan& s, const Tensor* y) {
+  const SsdDims d = seq_dims(s.x, s.dt, s.Bm, s.Cm, s.z, y, s.chunk, s.algo, s.softplus);
+  const at::Device dev = s.x.device();
+  const int64_t H = d.nheads;
   check_dense_f32("A", &s.A, Shape(H), dev);
   check_dense_f32("D", s.D, Shape(H), dev);
   check_dense_f32("dt_bias", s.bias, Shape(H), dev);
-  check_dense_f32("init_state", s.init, Shape(B, H, P, N), dev);
+  check_dense_f32("init_state", s.init, Shape(d.batch, H, d.headdim, d.dstate), dev);
   return d;
 }
 Tensor workspace_for(const SsdDims& d, const at::Device& dev, bool backward) {
@@ -596,6 +603,16 @@ Scan scan_of(const Args& a, int at, int chunk, int algo, int bias, int softplus)
           a.opt(at + 6, "z"), a.opt(at + 7, "init_state"), a.opt(bias, "dt_bias"), a.integer(chunk), a.integer(algo), a.flag(softplus)};
 }
 
+// x, dt, B, C, chunk, z, y, algo, dt_softplus -> the bytes of an SsdDims
+PyObject* py_dims(PyObject*, PyObject* const* argv, Py_ssize_t argc) {
+  return guarded([&]() -> PyObject* {
+    const Args a(argv, argc, 9);
+    const SsdDims d = seq_dims(a.tensor(0, "x"), a.tensor(1, "dt"), a.tensor(2, "B"), a.tensor(3, "C"), a.opt(5, "z"), a.opt(6, "y/dy"),
+                               a.integer(4), a.integer(7), a.flag(8));
+    return PyBytes_FromStringAndSize(reinterpret_cast<const char*>(&d), sizeof d);
+  });
+}
+
 // x, dt, A, B, C, D, z, init_state, chunk, algo, workspace, y, final_state, want_final, for_backward, stages, dt_bias, dt_softplus
 //   -> y, final_state, workspace
 PyObject* py_forward(PyObject*, PyObject* const* argv, Py_ssize_t argc) {
@@ -736,7 +753,7 @@ PyObject* py_bind(PyObject*, PyObject* const* argv, Py_ssize_t argc) {
 }
 
 #define FAST(name, fn) {name, (PyCFunction)(void (*)(void))fn, METH_FASTCALL, nullptr}
-PyMethodDef methods[] = {FAST("bind", py_bind), FAST("state_update", py_state_update), FAST("state_update_host", py_state_update_host), FAST("forward", py_forward),
+PyMethodDef methods[] = {FAST("bind", py_bind), FAST("dims", py_dims), FAST("state_update", py_state_update), FAST("state_update_host", py_state_update_host), FAST("forward", py_forward),
                          FAST("backward", py_backward), FAST("scan", py_scan), FAST("mixer", py_mixer),
                          FAST("conv1d_forward", py_conv_forward), FAST("conv1d_backward", py_conv_backward),
                          FAST("rmsnorm_forward", py_norm_forward), FAST("rmsnorm_backward", py_norm_backward), {nullptr, nullptr, 0, nullptr}};

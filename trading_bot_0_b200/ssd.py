@@ -22,7 +22,6 @@ import torch
 
 from . import _lib as L
 
-_DT = {torch.float32: L.SSD_F32, torch.bfloat16: L.SSD_BF16}
 ALGOS = {"auto": L.ALGO_AUTO, "fp32_cores": L.ALGO_FP32_CORES, "tensor": L.ALGO_TENSOR,
          "tensor_onetile": L.ALGO_TENSOR_ONETILE}
 
@@ -35,52 +34,9 @@ def _stream(device) -> C.c_void_p:
     return C.c_void_p(torch.cuda.current_stream(device).cuda_stream)
 
 
-def _need(cond: bool, msg: str):
-    if not cond:
-        raise ValueError(msg)
-
-
-def _check_seq(name, t, shape, dtype, device):
-    _need(t.dim() == len(shape), f"{name}: expected rank {len(shape)}, got {t.dim()}")
-    _need(tuple(t.shape) == tuple(shape), f"{name}: expected shape {tuple(shape)}, got {tuple(t.shape)}")
-    _need(t.dtype == dtype, f"{name}: expected dtype {dtype}, got {t.dtype}")
-    _need(t.device == device, f"{name}: expected device {device}, got {t.device}")
-    _need(t.stride(-1) == 1, f"{name}: innermost stride must be 1")
-    if t.dim() == 4:
-        _need(t.stride(2) == t.shape[3], f"{name}: the last two dims must be dense")
-
-
 def make_dims(x, dt, Bm, Cm, chunk, *, z=None, y=None, algo="auto", dt_softplus=False) -> L.SsdDims:
     """Validate the sequence operands and fill the geometry struct."""
-    _need(x.is_cuda, "x must be a CUDA tensor (there is no CPU path)")
-    _need(x.dim() == 4, "x must be [batch, seqlen, nheads, headdim]")
-    _need(x.dtype in _DT, f"unsupported dtype {x.dtype}")
-    Bn, Ln, H, P = x.shape
-    _need(Bm.dim() == 4, "B must be [batch, seqlen, ngroups, dstate]")
-    G, N = Bm.shape[2], Bm.shape[3]
-    dev = x.device
-    _check_seq("x", x, (Bn, Ln, H, P), x.dtype, dev)
-    _check_seq("dt", dt, (Bn, Ln, H), x.dtype, dev)
-    _check_seq("B", Bm, (Bn, Ln, G, N), x.dtype, dev)
-    _check_seq("C", Cm, (Bn, Ln, G, N), x.dtype, dev)
-    _need(H % G == 0, f"nheads ({H}) must be a multiple of ngroups ({G})")
-    _need(1 <= chunk <= 256, f"chunk must be in [1, 256], got {chunk}")
-    d = L.SsdDims()
-    d.batch, d.seqlen, d.nheads, d.headdim, d.dstate, d.ngroups, d.chunk = Bn, Ln, H, P, N, G, chunk
-    d.dtype, d.algo, d.device = _DT[x.dtype], ALGOS[algo], dev.index if dev.index is not None else torch.cuda.current_device()
-    d.has_z = 0 if z is None else 1
-    d.dt_softplus = 1 if dt_softplus else 0
-    d.x_stride_b, d.x_stride_l = x.stride(0), x.stride(1)
-    d.dt_stride_b, d.dt_stride_l = dt.stride(0), dt.stride(1)
-    d.b_stride_b, d.b_stride_l = Bm.stride(0), Bm.stride(1)
-    d.c_stride_b, d.c_stride_l = Cm.stride(0), Cm.stride(1)
-    if z is not None:
-        _check_seq("z", z, (Bn, Ln, H, P), x.dtype, dev)
-        d.z_stride_b, d.z_stride_l = z.stride(0), z.stride(1)
-    if y is not None:
-        _check_seq("y/dy", y, (Bn, Ln, H, P), x.dtype, dev)
-        d.y_stride_b, d.y_stride_l = y.stride(0), y.stride(1)
-    return d
+    return L.SsdDims.from_buffer_copy(L.host().dims(x, dt, Bm, Cm, chunk, z, y, ALGOS[algo], dt_softplus))
 
 
 def workspace_bytes(dims: L.SsdDims, backward: bool = False) -> int:
