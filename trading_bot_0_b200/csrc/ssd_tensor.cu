@@ -215,54 +215,26 @@ __device__ __forceinline__ void decay_diag_half(const uint32_t (&raw)[16], uint3
 // several groups run through it at different places); the two 16-column halves of the next block are
 // requested as soon as the registers of the current ones are free.  The table (in shared memory) is read through the
 // shared-memory pipe.
-template <int NCH>
-__device__ __forceinline__ void decay_row(int rb, int ch, uint32_t tm_row, const float* __restrict__ tab, int row, uint32_t mrow) {
+__device__ __forceinline__ void decay_row(int rb, uint32_t tm_row, const float* __restrict__ tab, int row, uint32_t mrow) {
   const uint32_t ts = smem_u32(tab);
   const float csi = lds_f32(ts + 4 * (T_CS + row));
-  if (NCH == 1) {
-    uint32_t a[16], b[16];
-    tmem_ld16_issue(tm_row, a);
-    tmem_ld16_issue(tm_row + 16, b);
+  uint32_t a[16], b[16];
+  tmem_ld16_issue(tm_row, a);
+  tmem_ld16_issue(tm_row + 16, b);
 #pragma unroll 1
-    for (int cb = 0; cb < rb; ++cb) {
-      const float rf = ex2(csi - lds_f32(ts + 4 * (T_CS + cb * 32 + 31)));
-      const uint32_t cf = ts + 4 * (T_CF + cb * 32);
-      const uint32_t dst = mrow + cb * 4 * 2048;
-      tmem_ld_wait_2x16(a, b);
-      decay_off_half(a, rf, cf, dst);
-      tmem_ld16_issue(tm_row + (cb + 1) * 32, a);
-      decay_off_half(b, rf, cf + 64, dst + 2 * 2048);
-      tmem_ld16_issue(tm_row + (cb + 1) * 32 + 16, b);
-    }
+  for (int cb = 0; cb < rb; ++cb) {
+    const float rf = ex2(csi - lds_f32(ts + 4 * (T_CS + cb * 32 + 31)));
+    const uint32_t cf = ts + 4 * (T_CF + cb * 32);
+    const uint32_t dst = mrow + cb * 4 * 2048;
     tmem_ld_wait_2x16(a, b);
-    decay_diag_half(a, ts, rb * 32, row, csi, mrow + rb * 4 * 2048);
-    decay_diag_half(b, ts, rb * 32 + 16, row, csi, mrow + rb * 4 * 2048 + 2 * 2048);
-  } else {
-    // two threads per row: this one owns columns [16 ch, 16 ch + 16) of every block; two register sets so that
-    // the load of the next block flies while the current one is worked on
-    uint32_t a[16], b[16];
-    const uint32_t tmc = tm_row + ch * 16;
-    const uint32_t mr = mrow + ch * 2 * 2048;
-    tmem_ld16_issue(tmc, a);
-    int cb = 0;
-#pragma unroll 1
-    for (; cb + 1 < rb; cb += 2) {
-      tmem_ld16_issue(tmc + (cb + 1) * 32, b);
-      tmem_ld_wait_2x16(a, b);
-      decay_off_half(a, ex2(csi - lds_f32(ts + 4 * (T_CS + cb * 32 + 31))), ts + 4 * (T_CF + cb * 32 + ch * 16), mr + cb * 4 * 2048);
-      tmem_ld16_issue(tmc + (cb + 2) * 32, a);
-      decay_off_half(b, ex2(csi - lds_f32(ts + 4 * (T_CS + cb * 32 + 63))), ts + 4 * (T_CF + cb * 32 + 32 + ch * 16), mr + (cb + 1) * 4 * 2048);
-    }
-    if (cb < rb) {   // one more block below the diagonal, then the diagonal block
-      tmem_ld16_issue(tmc + (cb + 1) * 32, b);
-      tmem_ld_wait_2x16(a, b);
-      decay_off_half(a, ex2(csi - lds_f32(ts + 4 * (T_CS + cb * 32 + 31))), ts + 4 * (T_CF + cb * 32 + ch * 16), mr + cb * 4 * 2048);
-      decay_diag_half(b, ts, rb * 32 + ch * 16, row, csi, mr + rb * 4 * 2048);
-    } else {
-      tmem_ld_wait_2x16(a, b);
-      decay_diag_half(a, ts, rb * 32 + ch * 16, row, csi, mr + rb * 4 * 2048);
-    }
+    decay_off_half(a, rf, cf, dst);
+    tmem_ld16_issue(tm_row + (cb + 1) * 32, a);
+    decay_off_half(b, rf, cf + 64, dst + 2 * 2048);
+    tmem_ld16_issue(tm_row + (cb + 1) * 32 + 16, b);
   }
+  tmem_ld_wait_2x16(a, b);
+  decay_diag_half(a, ts, rb * 32, row, csi, mrow + rb * 4 * 2048);
+  decay_diag_half(b, ts, rb * 32 + 16, row, csi, mrow + rb * 4 * 2048 + 2 * 2048);
 }
 
 // Variant used by the one-tile-per-CTA kernels (all 16 warps meet at a CTA barrier per head anyway):
@@ -1834,10 +1806,9 @@ struct WsCfg {
   static constexpr size_t SMEM = 1024 + NCBS * CB_BYTES + NM * 2 * BOX_BYTES + 2 * IN_BYTES + (SPLIT ? ST_BYTES : 0) +
                                  NTH * TAB_BYTES + RED_BYTES;
   static_assert(SMEM <= 232448, "shared-memory plan exceeds the 227 KB a CTA can have");
-  // warp roles: NM groups of 4 * NCH decay warps, then two MMA issuer warps (one per head of a head block) on the two
+  // warp roles: NM groups of four decay warps, then two MMA issuer warps (one per head of a head block) on the two
   // least loaded schedulers, the producer warp and an idle warp, then 8 epilogue warps
-  static constexpr int NCH = 1;                                       // threads per row of the decay pass
-  static constexpr int DW = 4 * NCH * NM, W_MMA = DW, W_PROD = DW + 2, W_EPI = DW + 4;
+  static constexpr int DW = 4 * NM, W_MMA = DW, W_PROD = DW + 2, W_EPI = DW + 4;
   // active issuers: warps W_MMA .. W_MMA + NI - 1, one per head of a head block; with one (64-wide) head per block and
   // dstate 128 the second lane issues the state term (8 instructions per head beside the head's own 8)
   static constexpr int NI = (SPLIT && HB == 1) ? 2 : HB;
@@ -1899,9 +1870,9 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
       mbar_init(&bars.acc_full[i], Cfg::NI); mbar_init(&bars.acc_empty[i], WS_EPI_WARPS);
       mbar_init(&bars.out_ready[i], WS_EPI_WARPS);
     }
-    for (int i = 0; i < 3; ++i) { mbar_init(&bars.m_full[i], 4 * Cfg::NCH); mbar_init(&bars.m_empty[i], 1); }
+    for (int i = 0; i < 3; ++i) { mbar_init(&bars.m_full[i], 4); mbar_init(&bars.m_empty[i], 1); }
     // a head's table is read by the warps of its decay group and by the epilogue warps of its columns
-    for (int i = 0; i < NTH; ++i) { mbar_init(&bars.tab_full[i], 1); mbar_init(&bars.tab_empty[i], 4 * Cfg::NCH + WS_EPI_WARPS / HB); }
+    for (int i = 0; i < NTH; ++i) { mbar_init(&bars.tab_full[i], 1); mbar_init(&bars.tab_empty[i], 4 + WS_EPI_WARPS / HB); }
     mbar_init(&bars.st_full, 1); mbar_init(&bars.st_empty, 1);
     for (int i = 0; i < 4; ++i) mbar_init(&bars.hz[i], 1);
     mbar_init(&bars.done, Cfg::NI);
@@ -2104,7 +2075,7 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
   } else if (warp < Cfg::DW) {
     // ------------------------------------------------------------------ decay pass: group wg owns heads kh = wg (mod NM)
     reg_inc<Cfg::R_DECAY>();
-    const int wg = warp / (4 * Cfg::NCH), ch = (warp >> 2) % Cfg::NCH, rb = warp & 3, row = rb * 32 + lane;
+    const int wg = warp / 4, rb = warp & 3, row = rb * 32 + lane;
     const uint32_t mrow = smem_u32(sM + wg * 2 * BOX_BYTES) + row * 16;
     int kh = 0;
     for (int t = 0; t < my_tiles; ++t) {
@@ -2117,7 +2088,7 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         const int ts = kh % NTH;
         w.wait(&bars.m_empty[wg], ((kh / NM) & 1) ^ 1, 53);
         w.wait(&bars.tab_full[ts], (kh / NTH) & 1, 52);
-        decay_row<Cfg::NCH>(rb, ch, tm_row, (const float*)(sTab + ts * TAB_BYTES), row, mrow);
+        decay_row(rb, tm_row, (const float*)(sTab + ts * TAB_BYTES), row, mrow);
         fence_async_smem(); __syncwarp(); if (lane == 0) { mbar_arrive(&bars.m_full[wg]); mbar_arrive(&bars.tab_empty[ts]); }
       }
       tc_fence_before();
