@@ -467,7 +467,7 @@ static bool launch_ring(const SsdStepDims& d, const SsdStepPtrs& p, cudaStream_t
   launch<k_state_update_ring<T, N, R, GATED>>((unsigned)grid, DEC_THREADS, smem, s, d, p, tph);
   return true;
 }
-// The largest tile up to 8 KB that divides the head.
+// The larger of two tile sizes that divides the head; false: neither does (or an operand cannot be copied in 16-byte pieces).
 template <typename T, int N>
 static bool launch_ring_n(const SsdStepDims& d, const SsdStepPtrs& p, cudaStream_t s) {
   // rows per thread: 8 KB tiles, 16 KB at N = 128 (a row there takes a whole warp, so a tile of four rows per thread is half

@@ -1,21 +1,21 @@
-// bf16 tensor-core kernels (tcgen05.mma, accumulators in TMEM, operands fed by TMA) for the
-// intra-chunk contractions of the SSD forward and backward, chunk length 128.
+// bf16 tensor-core kernels (tcgen05.mma, accumulators in TMEM, operands fed by TMA) for the SSD forward and backward, chunk
+// length 128, headdim 32 or 64, dstate 64 or 128.
 //
-//   k_state_tc : per (batch, chunk, group)   states[(h,p), n] = sum_l w[h,l] x[l,(h,p)] B[l,n]
-//                A = x tile, scaled in place in shared memory, read MN-major; B = B tile read
-//                MN-major; one 128 x N accumulator per 128 (h,p) rows.
-//   k_scan_tc  : per (batch, chunk, group)   G = C B^T once (128x128 in TMEM), then per head
-//                M_h = tril(G o exp(cs_i-cs_j) o dt_j) -> bf16 -> shared memory,
-//                Y = M_h X_h  (+)  exp(cs_i) * (C S_prev^T);  three epilogues (forward, backward
-//                recompute, dx).
-//   k_dbc_tc   : per (batch, chunk, group)   W_h = dY_h X_h^T, masked/decayed like M_h, then
-//                dC += W'_h B, dB += W'_h^T C accumulated over heads in TMEM, plus state terms.
+// Default path, persistent and warp-specialised (one CTA per SM walks over its tiles; roles hand over by mbarriers):
+//   k_state_scan_ps : chunk states states[(h,p), n] = sum_l w[h,l] x[l,(h,p)] B[l,n] and the scan over chunks in one kernel, the
+//                     running state in registers; k_state_ps + k_state_fold: the same as two kernels, for few units and (k_state_ps
+//                     + k_state_passing_v4) for staged calls;
+//   k_scan_ws       : per (batch, chunk, group) G = C B^T once, then per head M_h = tril(G o exp(cs_i-cs_j) o dt_j) -> bf16 ->
+//                     shared memory, Y = M_h X_h (+) exp(cs_i) * (C S_prev^T); epilogues: forward (gated or not), backward
+//                     recompute, dx;
+//   k_bwd_ws        : recompute and dx of the ungated backward from one decay pass per head;
+//   k_dbc_ws        : W_h = dY_h X_h^T, masked / decayed like M_h and summed over heads, dC += W' B, dB += W'^T C, state terms.
+// One-tile arm (SSD_ALGO_TENSOR_ONETILE), a CTA of 512 threads per tile (thread t owns accumulator row t % 128 and part t / 128 of
+// the columns), the comparison the persistent kernels are measured against: k_state_tc, k_scan_tc, k_bwd_tc, k_dbc_tc.
 //
-// Everything a CTA reads arrives asynchronously: sequence tiles and the bf16 copies of the
-// chunk-entry states by TMA, the per-head decay tables (written by the cumsum kernel) by 1-D
-// bulk copies; the next head block's inputs are in flight while the current one is computed.
-// Shared-memory tiles and descriptor conventions are described in umma.cuh.  Each CTA has 512
-// threads: thread t owns accumulator row (t % 128) and part (t / 128) of the columns.
+// Everything a CTA reads arrives asynchronously: sequence tiles and the bf16 copies of the chunk-entry states by TMA, the
+// per-head decay tables (written by the cumsum kernel) by 1-D bulk copies.  Shared-memory tiles and descriptor conventions are
+// described in umma.cuh.
 #include <stdlib.h>
 #include <string.h>
 
@@ -489,10 +489,10 @@ __global__ void __launch_bounds__(TC_THREADS, 2) k_state_tc(Geo g, const __grid_
 }
 
 // ---------------------------------------------------------------------------------------------
-// Persistent version of k_state_tc for dstate 64: one CTA per SM walks over (batch, chunk, group) items and their
-// 128-row accumulator tiles.  Roles:
-//   warp 17 (one lane)  producer: a four-deep ring of x tiles + the two table sections this kernel reads (TMA), so that
-//                       about 100 KB of loads are in flight per SM all the time, and a two-deep ring of B (or C) tiles;
+// Persistent version of k_state_tc: one CTA per SM walks over (batch, chunk, group) items and their 128-row accumulator tiles.
+// Roles:
+//   warp 17 (one lane)  producer: a ring of x tiles (four deep, three at dstate 128) + the two table sections this kernel reads
+//                       (TMA), so that about 100 KB of loads are in flight per SM all the time, and a two-deep ring of B (or C) tiles;
 //   warps 0-15          scale the tile in place (high bf16 part) and write the low part to a second buffer, one 64-token
 //                       half at a time, then store the PREVIOUS tile's accumulator;
 //   warp 16 (one lane)  issues the MMAs of a half as soon as that half is scaled, into one of two TMEM accumulators.
@@ -1272,7 +1272,7 @@ k_scan_tc(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
 }
 
 // ---------------------------------------------------------------------------------------------
-// Backward chunk_scan, ungated case, one tile per CTA (dstate 128): the recompute pass (MODE 1) and the dx pass (MODE 2) of
+// Backward chunk_scan, ungated case, one tile per CTA (the one-tile arm at dstate 128): the recompute pass (MODE 1) and the dx pass (MODE 2) of
 // k_scan_tc share G and every M_h, so this kernel forms G once and does both from one decay pass per head:
 //   Y  = M_h X_h    (+) exp(cs_i) C S_prev^T                   -> dcsp[i] = sum_p dy*Y, ddot[i] = sum_p dy*x
 //   U' = M_h^T dY_h (+) dt_j exp(cs_end-cs_j) B dS_end^T       -> dx = D dy + U', ddtd[j] = sum_p x*U' / dt_j
@@ -1754,17 +1754,17 @@ k_dbc_tc(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant__
 }
 
 // ---------------------------------------------------------------------------------------------
-// Persistent, warp-specialised version of the chunk_scan family for dstate 64: one CTA per SM walks
-// over (batch, chunk, group) tiles and keeps every stage busy at once:
-//   warp 16 lane 0    TMA producer: C/B tiles (2 slots) and per-head-block inputs (2 slots)
-//   warp 17 lane 0    MMA issuer:   G = C B^T of the NEXT tile early, then per head Y/U' and the state term
-//   warps 0-15        decay pass:   G (TMEM) -> M_h (ring of NM shared-memory tiles)
-//   warps 20-27       epilogue:     accumulators (2 TMEM slots) -> global, overlapped with the next block
-// Hand-offs are mbarriers: *_full arrive by TMA bytes / tcgen05.commit / one lane per producer warp,
-// *_empty by tcgen05.commit or one lane per consumer warp.  Slot use n (0,1,2,...) waits `full` with
-// parity n&1 and `empty` with parity (n&1)^1 (a fresh barrier passes a wait on parity 1).
-// TMEM: G x2 (256 columns) + {Y, Y_off} x2 (256 columns) = 512.  Same math and operand layouts as
-// k_scan_tc; MODE as there.
+// Persistent, warp-specialised version of the chunk_scan family: one CTA per SM walks over (batch, chunk, group) tiles and keeps
+// every stage busy at once (warp numbers follow from the number of decay groups: WsCfg):
+//   decay warps      two or three groups of four: G (TMEM) -> M_h, a ring of as many shared-memory tiles as groups
+//   MMA issuers      one or two lanes: G = C B^T of the next tile, then per head Y / U' and the state term
+//   TMA producer     one lane: C/B tiles (two slots, one at dstate 128), per-head-block inputs (two slots), tables, state boxes
+//   epilogue         eight warps: accumulators (two TMEM slots) -> global, overlapped with the next block
+// Hand-offs are mbarriers: *_full arrive by TMA bytes / tcgen05.commit / one lane per producer warp, *_empty by tcgen05.commit or
+// one lane per consumer warp.  Slot use n (0,1,2,...) waits `full` with parity n&1 and `empty` with parity (n&1)^1 (a fresh barrier
+// passes a wait on parity 1).
+// TMEM: G (128 columns; two at dstate 64) at 0, {Y, Y_off} x 2 (256 columns) at 256.  Same math and operand layouts as k_scan_tc;
+// MODE as there.
 // sigmoid through one tanh.approx (relative error 2^-11, below the bf16 resolution of the gated output): the exact
 // form costs an exp, an IEEE division and its slow path per element, which made the gated epilogue 2.4x the ungated one
 __device__ __forceinline__ float sigmoid_fast(float a) {
@@ -2257,12 +2257,12 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
 }
 
 // ---------------------------------------------------------------------------------------------
-// Backward chunk_scan, ungated case, dstate 64: the recompute pass (dcsp, ddot) and the dx pass of
+// Backward chunk_scan, ungated case: the recompute pass (dcsp, ddot) and the dx pass of
 // k_scan_ws share G and every M_h, so this kernel does both from one decay pass per head:
 //   Y  = M_h X_h    (+) exp(cs_i) C S_prev^T                   -> dcsp[i] = sum_p dy*Y, ddot[i] = sum_p dy*x
 //   U' = M_h^T dY_h (+) dt_j exp(cs_end-cs_j) B dS_end^T       -> dx = D dy + U', ddtd[j] = sum_p x*U' / dt_j
-// Same roles, rings and parities as k_scan_ws.  TMEM: G x2 (256) + {Y, Y_off, U, U_off} (256, one
-// slot: the epilogue hands it back as soon as it has read it).  The two state boxes (S_prev, dS_end)
+// Same roles, rings and parities as k_scan_ws.  TMEM: G x2 (dstate 128: x1, columns 128-255 are idle) + {Y, Y_off, U, U_off}
+// (256 columns, one slot: the epilogue hands it back as soon as it has read it).  The two state boxes (S_prev, dS_end)
 // have a buffer of their own that is refilled while the second head of a block is worked on.
 // dstate 128 (SPLIT): one C/B slot and one G; the S_prev and dS_end boxes (32 KB per head block at this width) pass as four
 // 8 KB pieces through a two-slot ring with a producer lane and an issuer lane of their own (warps 19 and 18), so the state
@@ -2973,9 +2973,6 @@ __global__ void __launch_bounds__(256, BFDOT ? 3 : 1) k_state_passing_v4(Geo g, 
   const size_t boff = ((size_t)b * g.nc * g.H + h) * PN + eo;
   float* base = st + boff;
   const int nw = gridDim.x * 8, wslot = blockIdx.x * 8 + (threadIdx.x >> 5);
-  // chunks in flight per thread.  The scan is bound by the bytes it keeps in flight (B * H * P * N / 4 threads, each with U
-  // loads per stream outstanding): the narrower bf16 loads need more steps to keep as many, within the 85 registers
-  // that leave three blocks per SM (two would put the 384 blocks of a B2 H24 pass into two waves)
   // chunks in flight per thread.  The scan is bound by the bytes it keeps in flight (B * H * P * N / 4 threads): the
   // narrower bf16 loads get six steps instead of four, within the 85 registers that leave three blocks per SM (two would
   // put the 384 blocks of a B2 H24 pass into two waves)
@@ -3509,7 +3506,7 @@ int tensor_dx(const Geo& g, const SsdBwdPtrs& p, const void* dyp, bool dy_dense,
 #undef CALL
 }
 
-// ungated backward: recompute pass and dx pass in one kernel (persistent for dstate 64, one tile per CTA for dstate 128)
+// ungated backward: recompute pass and dx pass in one kernel (the one-tile arm has one at dstate 128 only)
 bool tensor_bwd_merged_applies(const Geo& g, const SsdBwdPtrs& p) { return !p.z && (g.N == 128 || !g.onetile); }
 int tensor_bwd_merged(const Geo& g, const SsdBwdPtrs& p, const float* tab, const void* prev_bf, const void* ds_bf,
                       float* dcsp, float* ddot, float* ddtd, int* status, cudaStream_t s) {
