@@ -78,7 +78,7 @@ __global__ void k_selftest_wait(int* status, long long max_cycles) {
   if (!mbar_wait(&bar, 0, max_cycles) && threadIdx.x == 0) atomicExch(status, 99);
 }
 
-// a0 *= y0, a1 *= y1 as one packed instruction, same rounding as two (the decay passes are bound by issue slots)
+// a0 *= y0, a1 *= y1 as one packed instruction, same rounding as two (the decay passes are mostly such arithmetic)
 __device__ __forceinline__ void mul2(float& a0, float& a1, float y0, float y1) {
   asm("{\n\t.reg .b64 a, y;\n\tmov.b64 a, {%0, %1};\n\tmov.b64 y, {%2, %3};\n\tmul.rn.f32x2 a, a, y;\n\tmov.b64 {%0, %1}, a;\n\t}"
       : "+f"(a0), "+f"(a1) : "f"(y0), "f"(y1));
@@ -2657,9 +2657,10 @@ k_bwd_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant__
 // TMEM: the W accumulators, dC, dB = 512 columns.
 // dstate 128: 2x131072 with 24 heads 0.97 -> 0.64 ms = 5.1 TB/s, what a pure TMA stream of boxes reaches; 16x4096 0.27 -> 0.185
 // ms (3.46 waves of tiles take the time of four).  dstate 64, 512x1024 with 8 heads: 0.278 ms whatever the decay; a kernel that
-// carried the decay on the operands where its range allowed took 0.290, and 0.394 with one head beyond the range.  There the
-// issue slots bound it: 0.339 with 32 columns of W in registers beside the sums (spills), 0.306 with 16, 0.301 with packed
-// scaling of the boxes, 0.278 with packed FMAs and without the six warps whose blocks lie above the diagonal.
+// carried the decay on the operands where its range allowed took 0.290, and 0.394 with one head beyond the range.  No unit is full
+// there (128x1024: issue slots 0.43, DRAM 42 %, tensor pipe 14 %); a block waits for its decay pass, so what that pass issues
+// counts: 0.339 with 32 columns of W in registers beside the sums (spills), 0.306 with 16, 0.301 with packed scaling of the
+// boxes, 0.278 with packed FMAs and without the six warps whose blocks lie above the diagonal.
 template <int P, int N_>
 struct DbCfg {
   static constexpr int N = N_, NB64 = N / 64, HB = 64 / P, NT = 4, NIN = N == 64 ? 4 : 3, NST = N == 64 ? 3 : 2;
