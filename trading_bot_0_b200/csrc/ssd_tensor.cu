@@ -3046,10 +3046,10 @@ __global__ void __launch_bounds__(256, BFDOT ? 3 : 1) k_state_passing_v4(Geo g, 
 // chunks.  The local states lie in the order in which both kernels' warps touch whole lines: per tile of 128 (h,p) rows, slices of
 // 8 columns of all its rows.  Block = 32 rows of one head x 32 columns, thread = a slice of one row; MODE, outputs and partial sums
 // as there.  A step's U chunks are requested while the step before is folded.  Bound by DRAM on long sequences (2 rows of 131072
-// tokens, 24 heads of 64 x 128: 2.4 GB in 430 us forward, 3.2 GB in 505 us backward; U = 8 380-500 and 680), by the round trip of
-// the steps on short ones.
+// tokens, 24 heads of 64 x 128: 2.4 GB in 410 us forward, 3.2 GB in 510 us backward; 460-700 with U = 6 or 8, whose registers leave
+// fewer blocks), by the round trip of the steps on short ones.
 template <int N, int MODE, int U>
-__global__ void __launch_bounds__(128) k_state_fold(Geo g, const float* __restrict__ local, StateScanArgs a) {
+__global__ void __launch_bounds__(128, 12 / U) k_state_fold(Geo g, const float* __restrict__ local, StateScanArgs a) {
   constexpr int PP = 128 / N;   // parts (N / 4 columns) of a block
   struct Step {
     float4 v[U][2];
@@ -3422,7 +3422,12 @@ static int launch_state_scan(const Geo& g, const CUtensorMap& tx, const CUtensor
   if (plan == StatePlan::split) {
     const int rc = launch_state<P, N, MODE>(g, tx, tb, a.tab, a.state, status, s, true);
     if (rc) return rc;
-    launch<k_state_fold<N, MODE, MODE == 0 ? 6 : 4>>(dim3(g.H * P / 32 * (N / 32), g.B), 128, 0, s, g, (const float*)a.state, a);
+    // three blocks of the deeper form fit an SM, six of the other: 4 rows of 32 chunks, 24 heads of 64 x 128 (768 blocks) 39 + 45 us
+    // deep, 33 + 41 shallow; 2 rows of 1024 chunks (384 blocks) 408 + 519 and 514 + 665
+    const int blocks = g.H * P / 32 * (N / 32) * g.B;
+    const dim3 grid(blocks / g.B, g.B);
+    if (blocks > 4 * sm_count()) launch<k_state_fold<N, MODE, 2>>(grid, 128, 0, s, g, (const float*)a.state, a);
+    else launch<k_state_fold<N, MODE, 4>>(grid, 128, 0, s, g, (const float*)a.state, a);
     SSD_CUDA_CHECK_LAUNCH(MODE == 0 ? "state_fold" : "dstate_fold");
     return SSD_OK;
   }
