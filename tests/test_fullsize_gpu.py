@@ -234,7 +234,7 @@ def test_batch_rows_are_independent(lib):
 
 
 @pytest.mark.parametrize("H,P,N,G,L,rows", [
-    (24, 64, 128, 1, 17 * 128, (1, 8, 14)),            # 12 units a row: two kernels; walks; even shares
+    (24, 64, 128, 1, 17 * 128, (1, 4, 8, 14)),         # 12 units a row: two kernels, with few and many blocks; walks; even shares
     (8, 32, 64, 1, 40 * 128 + 70, (1, 50, 90)),        # 2 units a row: the same three, a ragged last chunk
     (24, 64, 128, 1, 40 * 128, (2, 6, 13)),
     (8, 32, 128, 2, 3 * 128, (1, 45, 100)),

@@ -130,10 +130,10 @@ def test_chunk_256_runs_on_the_tensor_family_as_two_128_chunks(lib):
     assert torch.equal(y, y128)
 
 
-@pytest.mark.parametrize("Bn,L,H,P,G", [(1, 128, 8, 32, 1), (3, 1280, 4, 64, 2), (2, 384, 16, 32, 2)])
+@pytest.mark.parametrize("Bn,L,H,P,G", [(1, 128, 8, 32, 1), (3, 1280, 4, 64, 2), (2, 384, 16, 32, 2), (50, 256, 8, 32, 1)])
 def test_fused_state_scan_matches_the_staged_two_kernel_path(lib, Bn, L, H, P, G):
     """A full pass at dstate 64 computes the chunk states inside the scan over chunks (one kernel per pass, running state
-    in registers); the staged entry points (sequence-parallel callers) keep chunk-state kernel + scan kernel.  Same inputs,
+    in registers: one chunk, or 100 units of the last case) or, for few units, folds them in a kernel of its own; the staged entry points (sequence-parallel callers) keep chunk-state kernel + scan kernel.  Same inputs,
     both ways, incl. one chunk only, fewer units than SMs, an initial state and a gradient entering the final state:
     results agree to fp32 rounding of the chunk decay (exp2 of the table value against expf of the cumsum) and both match
     the oracle."""

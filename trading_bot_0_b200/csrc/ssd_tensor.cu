@@ -3423,10 +3423,11 @@ static int launch_state_scan(const Geo& g, const CUtensorMap& tx, const CUtensor
     const int rc = launch_state<P, N, MODE>(g, tx, tb, a.tab, a.state, status, s, true);
     if (rc) return rc;
     // three blocks of the deeper form fit an SM, six of the other: 4 rows of 32 chunks, 24 heads of 64 x 128 (768 blocks) 39 + 45 us
-    // deep, 33 + 41 shallow; 2 rows of 1024 chunks (384 blocks) 408 + 519 and 514 + 665
+    // deep, 33 + 41 shallow; 2 rows of 1024 chunks (384 blocks) 408 + 519 and 514 + 665.  (dstate 64 never has that many here.)
     const int blocks = g.H * P / 32 * (N / 32) * g.B;
     const dim3 grid(blocks / g.B, g.B);
-    if (blocks > 4 * sm_count()) launch<k_state_fold<N, MODE, 2>>(grid, 128, 0, s, g, (const float*)a.state, a);
+    constexpr int SHALLOW = N == 128 ? 2 : 4;
+    if (blocks > 4 * sm_count()) launch<k_state_fold<N, MODE, SHALLOW>>(grid, 128, 0, s, g, (const float*)a.state, a);
     else launch<k_state_fold<N, MODE, 4>>(grid, 128, 0, s, g, (const float*)a.state, a);
     SSD_CUDA_CHECK_LAUNCH(MODE == 0 ? "state_fold" : "dstate_fold");
     return SSD_OK;
