@@ -91,6 +91,10 @@ fn check_seq(name: &str, t: &Tensor, shape: &[i64], kind: Kind, device: Device) 
     if st[n - 1] != 1 || (n == 4 && st[2] != shape[3]) {
         bail!("SSD {name}: the inner dimensions must be dense (strides {st:?})");
     }
+    // the C structs take a stride of 0 as "dense"
+    if (0..2).any(|i| shape[i] > 1 && st[i] == 0) {
+        bail!("SSD {name}: expanded over a dimension (strides {st:?}); make it contiguous");
+    }
     Ok(())
 }
 
@@ -259,9 +263,15 @@ pub fn state_update(state: &mut Tensor, x: &Tensor, dt: &Tensor, a: &Tensor, b: 
     }
     let g = b.size()[1];
     let kind = x.kind();
-    for (name, t, shape) in [("x", x, vec![s, h, p]), ("dt", dt, vec![s, h]), ("B", b, vec![s, g, n]), ("C", c, vec![s, g, n])] {
-        if t.size() != shape || t.kind() != kind || t.device() != dev || *t.stride().last().unwrap() != 1 {
-            bail!("SSD step {name} must be {shape:?} {kind:?} on {dev:?} with a dense inner dimension");
+    let mut operands = vec![("x", x, vec![s, h, p]), ("dt", dt, vec![s, h]), ("B", b, vec![s, g, n]), ("C", c, vec![s, g, n])];
+    if let Some(z) = z {
+        operands.push(("z", z, vec![s, h, p]));
+    }
+    for (name, t, shape) in operands {
+        let st = t.stride();
+        if t.size() != shape || t.kind() != kind || t.device() != dev || *st.last().unwrap() != 1 || (shape.len() == 3 && st[1] != shape[2])
+            || (s > 1 && st[0] == 0) {
+            bail!("SSD step {name} must be {shape:?} {kind:?} on {dev:?} with dense inner dimensions and rows apart");
         }
     }
     check_f32("A", a, &[h], dev)?;
