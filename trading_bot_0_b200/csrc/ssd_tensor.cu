@@ -2262,7 +2262,8 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
 //   Y  = M_h X_h    (+) exp(cs_i) C S_prev^T                   -> dcsp[i] = sum_p dy*Y, ddot[i] = sum_p dy*x
 //   U' = M_h^T dY_h (+) dt_j exp(cs_end-cs_j) B dS_end^T       -> dx = D dy + U', ddtd[j] = sum_p x*U' / dt_j
 // Same roles, rings and parities as k_scan_ws.  TMEM: G x2 (dstate 128: x1, columns 128-255 are idle) + {Y, Y_off, U, U_off}
-// (256 columns, one slot: the epilogue hands it back as soon as it has read it).  The two state boxes (S_prev, dS_end)
+// (256 columns, one slot; at dstate 128 its Y and U halves are handed back one by one as soon as the epilogue has read them:
+// 1150 -> 1053 us at 2 x 131072 tokens).  The two state boxes (S_prev, dS_end)
 // have a buffer of their own that is refilled while the second head of a block is worked on.
 // dstate 128 (SPLIT): one C/B slot and one G; the S_prev and dS_end boxes (32 KB per head block at this width) pass as four
 // 8 KB pieces through a two-slot ring with a producer lane and an issuer lane of their own (warps 19 and 18), so the state
@@ -2283,7 +2284,7 @@ struct BwCfg {
 
 struct BwBars {
   uint64_t cb_full[2], cb_empty[2], g_full[2], g_empty[2], in_full[2], in_empty[2], m_full[2], m_empty[2];
-  uint64_t tab_full[4], tab_empty[4], st_full, st_empty, acc_full, acc_empty, done;
+  uint64_t tab_full[4], tab_empty[4], st_full, st_empty, y_full, y_empty, u_full, u_empty, done;
   uint64_t stp_full[2], stp_empty[2];
 };
 
@@ -2320,7 +2321,8 @@ k_bwd_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant__
     }
     for (int i = 0; i < 4; ++i) { mbar_init(&bars.tab_full[i], 1); mbar_init(&bars.tab_empty[i], WS_SCALE_WARPS + WS_EPI_WARPS); }
     mbar_init(&bars.st_full, 1); mbar_init(&bars.st_empty, 1);
-    mbar_init(&bars.acc_full, SPLIT ? 2 : 1); mbar_init(&bars.acc_empty, WS_EPI_WARPS);
+    mbar_init(&bars.y_full, SPLIT ? 2 : 1); mbar_init(&bars.y_empty, WS_EPI_WARPS);
+    mbar_init(&bars.u_full, SPLIT ? 2 : 1); mbar_init(&bars.u_empty, WS_EPI_WARPS);
     mbar_init(&bars.done, 1);
     mbar_fence_init();
   }
@@ -2437,9 +2439,10 @@ k_bwd_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant__
         w.wait(&bars.cb_full[0], t & 1, 61);
         const uint32_t ct = smem_u32(sCB);
         for (int blk = 0; blk < nblk; ++blk, ++kb) {
-          w.wait(&bars.acc_empty, (kb & 1) ^ 1, 62);
           for (int p = 0; p < 4; ++p, ++q) {
             const int slot = q & 1;
+            if (p == 0) w.wait(&bars.y_empty, (kb & 1) ^ 1, 62);
+            if (p == 2) w.wait(&bars.u_empty, (kb & 1) ^ 1, 62);
             w.wait(&bars.stp_full[slot], (q >> 1) & 1, 63);
             tc_fence_after();
             // C boxes 0,1 then B boxes 0,1 lie one after the other in the C/B slot: piece p multiplies box p
@@ -2448,9 +2451,10 @@ k_bwd_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant__
             for (int ks = 0; ks < 4; ++ks)
               mma_bf16(p < 2 ? tmYo_ : tmUo_, desc_adv(dA, ks * 32), desc_adv(dS, ks * 32), idO, ((p & 1) | ks) > 0);
             mma_commit(&bars.stp_empty[slot]);
+            if (p == 1) mma_commit(&bars.y_full);
           }
           if (blk == nblk - 1) mma_commit(&bars.cb_empty[0]);
-          mma_commit(&bars.acc_full);
+          mma_commit(&bars.u_full);
         }
       }
     }
@@ -2483,33 +2487,60 @@ k_bwd_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant__
           const int ib = kb & 1;
           const uint32_t inb = smem_u32(sIn + ib * Cfg::IN_BYTES);
           w.wait(&bars.in_full[ib], (kb >> 1) & 1, 45);
-          if (!SPLIT) w.wait(&bars.st_full, kb & 1, 57);
-          w.wait(&bars.acc_empty, (kb & 1) ^ 1, 46);
-          for (int hl = 0; hl < HB; ++hl, ++kh) {
-            const int ms = kh % NM;
-            w.wait(&bars.m_full[ms], (kh / NM) & 1, 47);
+          if constexpr (SPLIT) {
+            // the Y half, then the U half: each goes out as soon as the epilogue has drained its columns of the block before, so
+            // products and epilogue run side by side although there is one accumulator set
+            w.wait(&bars.y_empty, (kb & 1) ^ 1, 46);
+            for (int hl = 0; hl < HB; ++hl) {
+              const int ms = (kh + hl) % NM;
+              w.wait(&bars.m_full[ms], ((kh + hl) / NM) & 1, 47);
+              tc_fence_after();
+              const uint64_t dMk = desc_plain_k(smem_u32(sM + ms * 2 * BOX_BYTES), 128, 0), dX0 = desc_sw128_mn(inb, 0, hl * P * 2, 16);
+#pragma unroll
+              for (int ks = 0; ks < 8; ++ks) mma_bf16(tmYd + hl * P, desc_adv(dMk, ks * 4096), desc_adv(dX0, ks * 2048), idY, ks > 0);
+            }
+            mma_commit(&bars.y_full);
+            w.wait(&bars.u_empty, (kb & 1) ^ 1, 66);
             tc_fence_after();
-            const uint32_t mt = smem_u32(sM + ms * 2 * BOX_BYTES);
-            const uint64_t dMk = desc_plain_k(mt, 128, 0), dMt = desc_plain_mn(mt, 128, 0, 0);
-            const uint64_t dX0 = desc_sw128_mn(inb, 0, hl * P * 2, 16), dY0 = desc_sw128_mn(inb + BOX_BYTES, 0, hl * P * 2, 16);
+            for (int hl = 0; hl < HB; ++hl, ++kh) {
+              const int ms = kh % NM;
+              const uint64_t dMt = desc_plain_mn(smem_u32(sM + ms * 2 * BOX_BYTES), 128, 0, 0),
+                             dY0 = desc_sw128_mn(inb + BOX_BYTES, 0, hl * P * 2, 16);
 #pragma unroll
-            for (int ks = 0; ks < 8; ++ks) {
-              mma_bf16(tmYd + hl * P, desc_adv(dMk, ks * 4096), desc_adv(dX0, ks * 2048), idY, ks > 0);
-              mma_bf16(tmUd + hl * P, desc_adv(dMt, ks * 256), desc_adv(dY0, ks * 2048), idU, ks > 0);
+              for (int ks = 0; ks < 8; ++ks) mma_bf16(tmUd + hl * P, desc_adv(dMt, ks * 256), desc_adv(dY0, ks * 2048), idU, ks > 0);
+              mma_commit(&bars.m_empty[ms]);
             }
-            if (!SPLIT && hl == 0) {
+          } else {
+            // dstate 64: both products of a head together; a block needs both M_h tiles, and holding them for a second round
+            // keeps the decay pass from running ahead (361 us against 349 at 512 x 1024 tokens)
+            w.wait(&bars.st_full, kb & 1, 57);
+            w.wait(&bars.u_empty, (kb & 1) ^ 1, 46);
+            for (int hl = 0; hl < HB; ++hl, ++kh) {
+              const int ms = kh % NM;
+              w.wait(&bars.m_full[ms], (kh / NM) & 1, 47);
+              tc_fence_after();
+              const uint32_t mt = smem_u32(sM + ms * 2 * BOX_BYTES);
+              const uint64_t dMk = desc_plain_k(mt, 128, 0), dMt = desc_plain_mn(mt, 128, 0, 0);
+              const uint64_t dX0 = desc_sw128_mn(inb, 0, hl * P * 2, 16), dY0 = desc_sw128_mn(inb + BOX_BYTES, 0, hl * P * 2, 16);
 #pragma unroll
-              for (int ks = 0; ks < 4; ++ks) {
-                mma_bf16(tmYo, desc_adv(dC0, ks * 32), desc_adv(dS0, ks * 32), idO, ks > 0);
-                mma_bf16(tmUo, desc_adv(dB0, ks * 32), desc_adv(dDS0, ks * 32), idO, ks > 0);
+              for (int ks = 0; ks < 8; ++ks) {
+                mma_bf16(tmYd + hl * P, desc_adv(dMk, ks * 4096), desc_adv(dX0, ks * 2048), idY, ks > 0);
+                mma_bf16(tmUd + hl * P, desc_adv(dMt, ks * 256), desc_adv(dY0, ks * 2048), idU, ks > 0);
               }
-              mma_commit(&bars.st_empty);
+              if (hl == 0) {
+#pragma unroll
+                for (int ks = 0; ks < 4; ++ks) {
+                  mma_bf16(tmYo, desc_adv(dC0, ks * 32), desc_adv(dS0, ks * 32), idO, ks > 0);
+                  mma_bf16(tmUo, desc_adv(dB0, ks * 32), desc_adv(dDS0, ks * 32), idO, ks > 0);
+                }
+                mma_commit(&bars.st_empty);
+              }
+              mma_commit(&bars.m_empty[ms]);
             }
-            mma_commit(&bars.m_empty[ms]);
           }
           mma_commit(&bars.in_empty[ib]);
           if (blk == nblk - 1) mma_commit(&bars.cb_empty[t % NCBS]);
-          mma_commit(&bars.acc_full);
+          mma_commit(&bars.u_full);
           if (!SPLIT && blk == 0 && t + 1 < my_tiles) issue_g(t + 1);
         }
         if (SPLIT && t + 1 < my_tiles) issue_g(t + 1);
@@ -2568,7 +2599,7 @@ k_bwd_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant__
         const float osc_y = ex2(cs_r), osc_u = dt_r * ex2(lds_f32(tbs + 4 * (T_CS + 127)) - cs_r);
         if (reads_done(__float_as_uint(cs_r) ^ __float_as_uint(osc_u), lane)) mbar_arrive(&bars.tab_empty[ts]);
         w.wait(&bars.in_full[ib], (kb >> 1) & 1, 54);
-        w.wait(&bars.acc_full, kb & 1, 55);
+        w.wait(SPLIT ? &bars.y_full : &bars.u_full, kb & 1, 55);
         tc_fence_after();
         const size_t dense = ((size_t)b * g.L + t_row) * g.H * P + (size_t)h0 * P + half * 32;
         float s0 = 0.f, s1 = 0.f, s2 = 0.f;
@@ -2578,6 +2609,7 @@ k_bwd_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant__
           const bool upass = ph >= 2;
           uint4 xv[2], dv[2];
           float a16[16], o16[16];
+          if (SPLIT && ph == 2) { w.wait(&bars.u_full, kb & 1, 67); tc_fence_after(); }
 #pragma unroll
           for (int q = 0; q < 2; ++q) {
             xv[q] = ld_shared_v4(xt + sw128_off(row, half * 4 + h16 * 2 + q));
@@ -2591,9 +2623,14 @@ k_bwd_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant__
 #pragma unroll
             for (int k = 0; k < 16; ++k) { a16[k] = __uint_as_float(ra[k]); o16[k] = __uint_as_float(ro[k]); }
           }
-          if (ph == 3) {   // everything read: hand the accumulators and the input slot back
+          if (SPLIT && ph == 1) {   // the Y half is read: the next block's products may overwrite it
             tc_fence_before();
-            if (reads_done(xv[0].x ^ xv[1].x ^ dv[0].x ^ dv[1].x, lane)) { mbar_arrive(&bars.acc_empty); mbar_arrive(&bars.in_empty[ib]); }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bars.y_empty);
+          }
+          if (ph == 3) {   // everything read: hand the U half and the input slot back
+            tc_fence_before();
+            if (reads_done(xv[0].x ^ xv[1].x ^ dv[0].x ^ dv[1].x, lane)) { mbar_arrive(&bars.u_empty); mbar_arrive(&bars.in_empty[ib]); }
           }
           const float osc = upass ? osc_u : osc_y;
           uint4 ov[2];
