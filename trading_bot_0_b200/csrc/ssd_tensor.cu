@@ -1795,6 +1795,20 @@ struct WsCfg {
   static constexpr int ST_BYTES = NB64 * SBOX_BYTES;                 // state boxes of one head block
   static constexpr int ZOFF = NBOX * BOX_BYTES + (SPLIT ? 0 : ST_BYTES);       // the gate's box comes last in a slot
   static constexpr int IN_BYTES = ZOFF + ZB * BOX_BYTES;                       // x [, dy] box [+ state box] [+ z box]
+  // Input slots.  A slot is held from the request of its boxes until its output block has been read by the tile store (about 4 us
+  // against 2 us of work per block), so two of them leave the issuers waiting for boxes.  dstate 128: the tile that only G reads
+  // (32 KB) is free from the tile's G until the next tile's; it holds further slots meanwhile.  The last two blocks of a tile
+  // use the first two slots, so that those are drained when the next tile's C and B are requested.
+  // dstate 128, the state boxes: a ring of 8 KB pieces (64 state columns each).  One buffer for a block's 16 KB was a chain of load,
+  // product, load that took as long as a block.  Three pieces of their own, or (forward without a gate, where three M_h tiles
+  // leave room for two) two more in the tile that only G reads.  (Two heads per block: the tables leave room for two.)
+  static constexpr int NSP = !SPLIT ? 0 : (NM == 3 ? 4 : HB == 1 ? 3 : 2), NSP_OWN = NSP == 4 ? 2 : NSP;
+  static constexpr int NX = SPLIT && MODE != 1 ? 2 + (NB64 * BOX_BYTES - (NSP - NSP_OWN) * SBOX_BYTES) / IN_BYTES : 2;
+  // slot of piece j of a block; q counts the pieces before it
+  static __device__ __forceinline__ int piece(int blk, int nblk, int j, int q) {
+    return NSP == 4 ? (((blk & 1) && nblk - blk > 1) ? 2 : 0) + j : q % (NSP ? NSP : 1);
+  }
+  static __device__ __forceinline__ int slot(int blk, int nblk) { return (NX == 2 || nblk - blk <= 2) ? (blk & 1) : blk % NX; }
   // table ring depth (one 2 KB table per head): a multiple of the number of decay groups, so that a slot is always read by
   // the same group.  With a depth of 4 and three groups the slot of head 5 had last been head 1's, read by another group:
   // the group of head 5, coming from head 2, could reach the slot's barrier before head 1's table had landed, pass the wait
@@ -1802,10 +1816,10 @@ struct WsCfg {
   // of that head wrong about once in 10^4 CTAs).
   static constexpr int NTH = (NM == 3) ? 6 : 4 * HB;
   static_assert(NTH % NM == 0 && NTH % HB == 0 && NTH <= 8, "a table slot must belong to one decay group and one column half");
-  static constexpr int RED_BYTES = (P == 64 && MODE != 0) ? 2 * 256 * 4 : 0;
-  static constexpr size_t SMEM = 1024 + NCBS * CB_BYTES + NM * 2 * BOX_BYTES + 2 * IN_BYTES + (SPLIT ? ST_BYTES : 0) +
+  static constexpr int RED_BYTES = (P == 64 && MODE != 0) ? 2 * 128 * 4 : 0;
+  static constexpr size_t SMEM = 1024 + NCBS * CB_BYTES + NM * 2 * BOX_BYTES + 2 * IN_BYTES + NSP_OWN * SBOX_BYTES +
                                  NTH * TAB_BYTES + RED_BYTES;
-  static_assert(SMEM <= 232448, "shared-memory plan exceeds the 227 KB a CTA can have");
+  static_assert(SMEM <= 232448 - 512, "shared-memory plan exceeds the 227 KB a CTA can have");
   // warp roles: NM groups of four decay warps, then two MMA issuer warps (one per head of a head block) on the two
   // least loaded schedulers, the producer warp and an idle warp, then 8 epilogue warps
   static constexpr int DW = 4 * NM, W_MMA = DW, W_PROD = DW + 2, W_EPI = DW + 4;
@@ -1821,15 +1835,14 @@ struct WsCfg {
   // apart for the same reason, so four report slots never wrap.)
   static constexpr bool HEAD_ORDER = HB == 2 && NM == 3;
   static constexpr int THREADS = (DW + 4 + WS_EPI_WARPS) * 32;
-  // registers per thread after re-balancing (launch share: 80 at 768 threads, 96 at 640)
-  static constexpr int R_DECAY = (THREADS == 768) ? 88 : (THREADS == 640 ? 128 : (MODE == 0 ? 80 : 72)),
-                       R_SPECIAL = (THREADS > 768) ? 48 : 56,
-                       R_EPI = (THREADS > 768) ? (MODE == 0 ? 64 : 72) : ((MODE == 0) ? 72 : 80);
+  // registers per thread after re-balancing (launch share: 80 at 768 threads, 96 at 640; never the share itself)
+  static constexpr int R_SHARE = NM == 3 ? 80 : 96, R_SPECIAL = 56, R_DECAY = 88, R_EPI = NM == 3 ? 72 : 120;
+  static_assert(DW * R_DECAY + 4 * R_SPECIAL + WS_EPI_WARPS * R_EPI <= THREADS / 32 * R_SHARE, "more registers than the launch has");
 };
 
 struct WsBars {
-  uint64_t cb_full[2], cb_empty[2], g_full[2], g_empty[2], in_full[2], in_empty[2], acc_full[2], acc_empty[2];
-  uint64_t m_full[3], m_empty[3], tab_full[8], tab_empty[8], st_full, st_empty, out_ready[2], hz[4], done;
+  uint64_t cb_full[2], cb_empty[2], g_full[2], g_empty[2], in_full[4], in_empty[4], acc_full[2], acc_empty[2];
+  uint64_t m_full[3], m_empty[3], tab_full[8], tab_empty[8], st_full[4], st_empty[4], out_ready[4], hz[4], done;
 };
 
 template <int P, int MODE, int N_ = 64, bool GATED = false>
@@ -1854,9 +1867,9 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
   uint8_t* sCB = smem;                                   // NCBS x {keep tile, other tile}
   uint8_t* sM = sCB + NCBS * Cfg::CB_BYTES;              // NM x 32 KB
   uint8_t* sIn = sM + NM * 2 * BOX_BYTES;                // 2 x {x [, dy] [, state box]}
-  uint8_t* sSt = sIn + 2 * Cfg::IN_BYTES;                // dstate 128: the state boxes of one head block
-  uint8_t* sTab = sSt + (SPLIT ? Cfg::ST_BYTES : 0);     // NTH x decay table of one head (they run further ahead)
-  float* sRed = (float*)(sTab + NTH * TAB_BYTES);          // [2][256] (P = 64 row-sum exchange)
+  uint8_t* sSt = sIn + 2 * Cfg::IN_BYTES;                // dstate 128: state pieces
+  uint8_t* sTab = sSt + Cfg::NSP_OWN * SBOX_BYTES;       // NTH x decay table of one head (they run further ahead)
+  float* sRed = (float*)(sTab + NTH * TAB_BYTES);          // [2][128] (P = 64 row-sum exchange)
   __shared__ __align__(8) WsBars bars;
   __shared__ uint32_t tmem_slot;
   __shared__ int s_abort;
@@ -1866,15 +1879,16 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
     for (int i = 0; i < 2; ++i) {
       mbar_init(&bars.cb_full[i], 1); mbar_init(&bars.cb_empty[i], Cfg::NI);
       mbar_init(&bars.g_full[i], 1); mbar_init(&bars.g_empty[i], Cfg::DW);
-      mbar_init(&bars.in_full[i], 1); mbar_init(&bars.in_empty[i], Cfg::NI + (TSTORE ? 1 : WS_EPI_WARPS));
       mbar_init(&bars.acc_full[i], Cfg::NI); mbar_init(&bars.acc_empty[i], WS_EPI_WARPS);
+    }
+    for (int i = 0; i < Cfg::NX; ++i) {
+      mbar_init(&bars.in_full[i], 1); mbar_init(&bars.in_empty[i], Cfg::NI + (TSTORE ? 1 : WS_EPI_WARPS));
       mbar_init(&bars.out_ready[i], WS_EPI_WARPS);
     }
     for (int i = 0; i < 3; ++i) { mbar_init(&bars.m_full[i], 4); mbar_init(&bars.m_empty[i], 1); }
     // a head's table is read by the warps of its decay group and by the epilogue warps of its columns
     for (int i = 0; i < NTH; ++i) { mbar_init(&bars.tab_full[i], 1); mbar_init(&bars.tab_empty[i], 4 + WS_EPI_WARPS / HB); }
-    mbar_init(&bars.st_full, 1); mbar_init(&bars.st_empty, 1);
-    for (int i = 0; i < 4; ++i) mbar_init(&bars.hz[i], 1);
+    for (int i = 0; i < 4; ++i) { mbar_init(&bars.hz[i], 1); mbar_init(&bars.st_full[i], 1); mbar_init(&bars.st_empty[i], 1); }
     mbar_init(&bars.done, Cfg::NI);
     mbar_fence_init();
   }
@@ -1907,6 +1921,11 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
     b = r / g.G;
   };
 
+  constexpr int NPX = Cfg::NX - 2, NSP = Cfg::NSP, NSP_OWN = Cfg::NSP_OWN;
+  auto st_piece = [&](int s_) { return s_ < NSP_OWN ? sSt + s_ * SBOX_BYTES : sCB + NB64 * BOX_BYTES + NPX * Cfg::IN_BYTES + (s_ - NSP_OWN) * SBOX_BYTES; };
+  // input slot s; uses: bit s of a role's `used` counts the uses of slot s that it has seen, modulo 2
+  auto in_slot = [&](int s_) { return s_ < 2 ? sIn + s_ * Cfg::IN_BYTES : sCB + NB64 * BOX_BYTES + (s_ - 2) * Cfg::IN_BYTES; };
+
   if (warp >= Cfg::DW && warp < Cfg::W_EPI) reg_dec<Cfg::R_SPECIAL>();
   if (warp == Cfg::W_PROD) {
     // ------------------------------------------------------------------ TMA producer
@@ -1937,7 +1956,8 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
           bulk_load(sTab + ts * TAB_BYTES, tab + ((size_t)(b * g.nc + c) * g.H + h0 + hl) * TAB, TAB_BYTES, &bars.tab_full[ts]);
         }
       };
-      int kb = 0;
+      int kb = 0, sq = 0;
+      uint32_t used = 0, sused = 0;
       load_cb(0);
       load_tab(0);
       load_tab(1);
@@ -1945,9 +1965,11 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         int b, grp, c;
         tile_coords(t, b, grp, c);
         for (int blk = 0; blk < nblk; ++blk, ++kb) {
-          const int ib = kb & 1;
-          w.wait(&bars.in_empty[ib], ((kb >> 1) & 1) ^ 1, 42);
-          uint8_t* dst = sIn + ib * Cfg::IN_BYTES;
+          const int ib = Cfg::slot(blk, nblk);
+          if (NPX > 0 && blk == 2 && ib == 2) w.wait(&bars.g_full[0], t & 1, 66);   // G has read the tile these slots share
+          w.wait(&bars.in_empty[ib], ((used >> ib) & 1) ^ 1, 42);
+          used ^= 1u << ib;
+          uint8_t* dst = in_slot(ib);
           const int h0 = grp * g.hpg + blk * HB;
           const int col = grp * g.hpg * P + blk * 64;
           mbar_expect_tx(&bars.in_full[ib], Cfg::IN_BYTES);
@@ -1963,15 +1985,25 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
             // the next G while this tile is still being worked on
             if (blk == 0 && t + 1 < my_tiles) load_cb(t + 1);
           } else {
-            w.wait(&bars.st_empty, (kb & 1) ^ 1, 57);
-            mbar_expect_tx(&bars.st_full, Cfg::ST_BYTES);
 #pragma unroll
-            for (int j = 0; j < NB64; ++j)
-              tma_load_3d(sSt + j * SBOX_BYTES, &tmS, 64 * j, h0 * P, b * g.nc + c, &bars.st_full);
+            for (int j = 0; j < NB64; ++j, ++sq) {
+              const int sp = Cfg::piece(blk, nblk, j, sq);
+              if (NSP > NSP_OWN && blk == 1 && sp == NSP_OWN) w.wait(&bars.g_full[0], t & 1, 68);
+              w.wait(&bars.st_empty[sp], ((sused >> sp) & 1) ^ 1, 57);
+              sused ^= 1u << sp;
+              mbar_expect_tx(&bars.st_full[sp], SBOX_BYTES);
+              tma_load_3d(st_piece(sp), &tmS, 64 * j, h0 * P, b * g.nc + c, &bars.st_full[sp]);
+            }
           }
         }
         // one C/B slot: the next tile's C/B can only follow this tile's last block
-        if (SPLIT && t + 1 < my_tiles) load_cb(t + 1);
+        if (SPLIT && t + 1 < my_tiles) {
+#pragma unroll
+          for (int s_ = 2; s_ < Cfg::NX; ++s_) w.wait(&bars.in_empty[s_], ((used >> s_) & 1) ^ 1, 67);
+#pragma unroll
+          for (int s_ = NSP_OWN; s_ < NSP; ++s_) w.wait(&bars.st_empty[s_], ((sused >> s_) & 1) ^ 1, 69);
+          load_cb(t + 1);
+        }
       }
     }
   } else if (warp >= Cfg::W_MMA && warp < Cfg::W_MMA + Cfg::NI) {
@@ -1998,7 +2030,8 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         mma_commit(&bars.g_full[s_]);
       };
       if (mi == 0) issue_g(0);
-      int kb = 0, kh = 0;
+      int kb = 0, kh = 0, sq = 0;
+      uint32_t used = 0, sused = 0;
       for (int t = 0; t < my_tiles; ++t) {
         const uint32_t keep_t = smem_u32(sCB + (t % NCBS) * Cfg::CB_BYTES);
         const uint64_t dK0 = desc_sw128_k(keep_t, 0);
@@ -2006,22 +2039,25 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         // for the tile there), it has to see the tile's arrival itself: the first x box of a tile can land before its C/B
         if (mi == 1) w.wait(&bars.cb_full[t % NCBS], (t / NCBS) & 1, 64);
         for (int blk = 0; blk < nblk; ++blk, ++kb) {
-          const int ib = kb & 1, ab = kb & 1;
-          const uint32_t inb = smem_u32(sIn + ib * Cfg::IN_BYTES);
+          const int ib = Cfg::slot(blk, nblk), ab = kb & 1;
+          const uint32_t inb = smem_u32(in_slot(ib));
           const uint32_t tmYd = tm + 256 + ab * 128, tmYo = tmYd + 64;
-          w.wait(&bars.in_full[ib], (kb >> 1) & 1, 45);
+          w.wait(&bars.in_full[ib], (used >> ib) & 1, 45);
+          used ^= 1u << ib;
           w.wait(&bars.acc_empty[ab], ((kb >> 1) & 1) ^ 1, 46);
           if constexpr (SPLIT) {
             if (mi == (Cfg::STATE_LANE ? 1 : 0)) {    // the state term first: it needs the keep tile and the state boxes, not M_h
-              w.wait(&bars.st_full, kb & 1, 58);
-              tc_fence_after();
 #pragma unroll 1
-              for (int j = 0; j < NB64; ++j) {
-                const uint64_t dKj = desc_sw128_k(keep_t + j * BOX_BYTES, 0), dSj = desc_sw128_k(smem_u32(sSt + j * SBOX_BYTES), 0);
+              for (int j = 0; j < NB64; ++j, ++sq) {
+                const int sp = Cfg::piece(blk, nblk, j, sq);
+                w.wait(&bars.st_full[sp], (sused >> sp) & 1, 58);
+                sused ^= 1u << sp;
+                tc_fence_after();
+                const uint64_t dKj = desc_sw128_k(keep_t + j * BOX_BYTES, 0), dSj = desc_sw128_k(smem_u32(st_piece(sp)), 0);
 #pragma unroll 1
                 for (int ks = 0; ks < 4; ++ks) mma_bf16(tmYo, desc_adv(dKj, ks * 32), desc_adv(dSj, ks * 32), idO, (j | ks) > 0);
+                mma_commit(&bars.st_empty[sp]);
               }
-              mma_commit(&bars.st_empty);
             }
           }
           for (int hl = 0; hl < HB; ++hl, ++kh) {
@@ -2057,14 +2093,15 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
   } else if (TSTORE && warp == Cfg::W_PROD + 1) {
     // ------------------------------------------------------------------ store lane: output blocks leave as TMA tiles
     if (lane == 0) {
-      int kb = 0;
+      uint32_t used = 0;
       for (int t = 0; t < my_tiles; ++t) {
         int b, grp, c;
         tile_coords(t, b, grp, c);
-        for (int blk = 0; blk < nblk; ++blk, ++kb) {
-          const int ib = kb & 1;
-          w.wait(&bars.out_ready[ib], (kb >> 1) & 1, 59);
-          tma_store_3d(&tmOut, sIn + ib * Cfg::IN_BYTES + (NBOX - 1) * BOX_BYTES, grp * g.hpg * P + blk * 64, c * QT, b);
+        for (int blk = 0; blk < nblk; ++blk) {
+          const int ib = Cfg::slot(blk, nblk);
+          w.wait(&bars.out_ready[ib], (used >> ib) & 1, 59);
+          used ^= 1u << ib;
+          tma_store_3d(&tmOut, in_slot(ib) + (NBOX - 1) * BOX_BYTES, grp * g.hpg * P + blk * 64, c * QT, b);
           bulk_commit();
           bulk_wait_read0();            // the box has been read: the slot may be refilled
           mbar_arrive(&bars.in_empty[ib]);
@@ -2074,7 +2111,7 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
     }
   } else if (warp < Cfg::DW) {
     // ------------------------------------------------------------------ decay pass: group wg owns heads kh = wg (mod NM)
-    reg_inc<Cfg::R_DECAY>();
+    if constexpr (Cfg::R_DECAY > Cfg::R_SHARE) reg_inc<Cfg::R_DECAY>(); else reg_dec<Cfg::R_DECAY>();
     const int wg = warp / 4, rb = warp & 3, row = rb * 32 + lane;
     const uint32_t mrow = smem_u32(sM + wg * 2 * BOX_BYTES) + row * 16;
     int kh = 0;
@@ -2097,13 +2134,15 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
     }
   } else if (warp >= Cfg::W_EPI) {
     // ------------------------------------------------------------------ epilogue warps
-    reg_dec<Cfg::R_EPI>();
+    if constexpr (Cfg::R_EPI > Cfg::R_SHARE) reg_inc<Cfg::R_EPI>(); else reg_dec<Cfg::R_EPI>();
     const int ew = warp - Cfg::W_EPI;
     const int row = (ew & 3) * 32 + lane, half = ew >> 2;     // 32 of the block's 64 columns
     const int hl_e = (half * 32) / P;
     int kb = 0;
+    uint32_t used = 0;
     // gated recompute (MODE 1): the gate is the one operand the epilogue reads from global memory; this thread's 64 bytes
-    // of it are requested at the start of the block, before the waits (the forward gets the gate's box by TMA)
+    // of it are requested at the start of the block, before the waits (the forward gets the gate's box by TMA); a block ahead was
+    // no faster
     uint4 zq[GATED ? 4 : 1] = {};
     auto load_z = [&](int t_, int blk_, auto& dst) {
       if constexpr (GATED) {
@@ -2126,8 +2165,8 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
       const int t_row = c * QT + row;
       for (int blk = 0; blk < nblk; ++blk, ++kb) {
         if constexpr (GATED && !ZSMEM) load_z(t, blk, zq);
-        const int ib = kb & 1, ab = kb & 1;
-        uint8_t* xt = sIn + ib * Cfg::IN_BYTES;
+        const int ib = Cfg::slot(blk, nblk), ab = kb & 1;
+        uint8_t* xt = in_slot(ib);
         uint8_t* dyt = xt + (NBOX - 1) * BOX_BYTES;
         const int khe = kb * HB + hl_e, ts = khe % NTH;
         const float* tb = (const float*)(sTab + ts * TAB_BYTES);
@@ -2139,7 +2178,8 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         const float cs_r = lds_f32(tbs + 4 * (T_CS + row)), dt_r = lds_f32(tbs + 4 * (T_DT + row));
         const float osc = (MODE == 2) ? dt_r * ex2(lds_f32(tbs + 4 * (T_CS + 127)) - cs_r) : ex2(cs_r);
         if (reads_done(__float_as_uint(cs_r) ^ __float_as_uint(dt_r) ^ __float_as_uint(osc), lane)) mbar_arrive(&bars.tab_empty[ts]);
-        w.wait(&bars.in_full[ib], (kb >> 1) & 1, 54);
+        w.wait(&bars.in_full[ib], (used >> ib) & 1, 54);
+        used ^= 1u << ib;
         w.wait(&bars.acc_full[ab], (kb >> 1) & 1, 55);
         tc_fence_after();
         const long long colo = (long long)h0 * P + half * 32;
@@ -2234,9 +2274,9 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         if (MODE != 0) {
           if (P == 64) {   // the two column halves of a row belong to one head: combine through shared memory
             asm volatile("bar.sync 1, 256;" ::: "memory");   // previous block's exchange fully read
-            if (half == 1) { sRed[row] = s0; sRed[256 + row] = s1; }
+            if (half == 1) { sRed[row] = s0; sRed[128 + row] = s1; }
             asm volatile("bar.sync 1, 256;" ::: "memory");
-            if (half == 0) { s0 += sRed[row]; s1 += sRed[256 + row]; }
+            if (half == 0) { s0 += sRed[row]; s1 += sRed[128 + row]; }
           }
           if (P == 32 || half == 0) {
             const size_t co = ((size_t)(b * g.H + h_e) * g.nc + c) * QT + row;
