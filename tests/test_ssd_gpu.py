@@ -123,6 +123,22 @@ def test_autograd_function_matches_oracle(lib):
         assert_close(r, leaves[k].grad, ref[r], "fp32")
 
 
+@pytest.mark.parametrize("dtype", ["fp32", "bf16"])
+@pytest.mark.parametrize("used", ["y", "final_state"])
+def test_autograd_with_one_output_used(lib, dtype, used):
+    """An output that takes no part in the loss has no gradient; the node is not handed zeros for it.  Same bits as with zeros."""
+    import trading_bot_0_b200 as T
+    cfg = cfg_like(0 if dtype == "fp32" else 1, batch=2, seqlen=256)
+    d = to_dev(O.make_inputs(cfg, O.SEED, batch=2, seqlen=256, with_init_state=True), DEV)
+    leaves = [d[k].requires_grad_() for k in ("x", "dt", "A", "B", "C", "D", "init_state")]
+    y, fin = T.ssd_scan(*leaves[:6], init_state=leaves[6], chunk=cfg.chunk)
+    dy, dfin = (d["dy"], torch.zeros_like(fin)) if used == "y" else (torch.zeros_like(y), torch.ones_like(fin))
+    want = torch.autograd.grad([y, fin], leaves, [dy, dfin], retain_graph=True)
+    out, g = (y, dy) if used == "y" else (fin, dfin)
+    got = torch.autograd.grad(out, leaves, g)
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
 def test_cuda_graph_capture_on_side_stream(lib):
     """Forward + backward captured into a CUDA graph on a non-default stream and replayed: the
     contract the reference's PPO update imposes on anything inside its graph body."""

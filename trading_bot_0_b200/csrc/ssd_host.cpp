@@ -426,6 +426,7 @@ struct ScanNode : public torch::autograd::Function<ScanNode> {
     const Scan s{x, dt, A, Bm, Cm, or_null(D), or_null(z), or_null(init), or_null(bias), chunk, algo, softplus};
     Tensor y, fin, ws;
     scan_forward(s, y, fin, ws, true, true, kAllStages);
+    ctx->set_materialize_grads(false);   // an unused final state has no gradient: no zeros to allocate, fill and read
     ctx->save_for_backward({x, dt, A, Bm, Cm, or_undefined(D), or_undefined(z), or_undefined(init), or_undefined(bias), ws});
     ctx->saved_data["how"] = pack(chunk, algo, softplus);
     return {y, fin};
@@ -463,6 +464,7 @@ struct MixerNode : public torch::autograd::Function<MixerNode> {
     scan_forward(s, y, fin, ws, true, save, kAllStages);
     norm_forward(y.view({y.size(0), y.size(1), H * P}), or_null(nw), eps, out, rstd);
     if (save) {
+      ctx->set_materialize_grads(false);
       ctx->save_for_backward({xBC, dt, or_undefined(z), cw, or_undefined(cb), or_undefined(bias), A, or_undefined(D), or_undefined(nw),
                               or_undefined(init), conv, y, rstd, ws});
       ctx->saved_data["how"] = pack(chunk, algo, true);

@@ -135,6 +135,7 @@ struct SsdScanNode : public torch::autograd::Function<SsdScanNode> {
       check_rc(ssd_forward(&d, &p, ws.data_ptr(), (size_t)ws.numel(), c10::cuda::getCurrentCUDAStream().stream()));
     }
     if (needs_grad) {
+      ctx->set_materialize_grads(false);   // an unused final state has no gradient: no zeros to allocate, fill and read
       ctx->save_for_backward({x, dt, A, Bm, Cm, or_undefined(D), or_undefined(z), or_undefined(init_state),
                               or_undefined(dt_bias), ws});
       ctx->saved_data["chunk"] = chunk;
