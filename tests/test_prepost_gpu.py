@@ -43,6 +43,25 @@ def test_conv1d_forward_backward(lib, dtype, K, activation, use_bias, Bn, L, Cn)
         assert_close("dbias", db, db_r, dtype)
 
 
+@pytest.mark.parametrize("dtype", ["fp32", "bf16"])
+@pytest.mark.parametrize("K", [4, 3, 2])
+@pytest.mark.parametrize("Bn,L,Cn", [(300, 1, 128), (90, 3, 136), (5, 333, 200), (1, 2111, 384), (3, 1024, 128), (2, 17, 520)])
+def test_conv1d_backward_in_warp_shares(lib, dtype, K, Bn, L, Cn):
+    """Shares of the tokens that begin and end anywhere: sequences shorter than the window, several per share, several shares per
+    sequence, a channel block that is partly empty; activation on (whole stages have a form of their own) and off."""
+    from trading_bot_0_b200 import prepost as PP
+    g = torch.Generator().manual_seed(11)
+    td = O.torch_dtype(dtype)
+    x, dout = torch.randn(Bn, L, Cn, generator=g).to(td), torch.randn(Bn, L, Cn, generator=g).to(td)
+    w, b = torch.randn(Cn, K, generator=g) / K ** 0.5, 0.3 * torch.randn(Cn, generator=g)
+    for activation in (True, False):
+        _, (dx_r, dw_r, db_r) = _autograd_ref(lambda a, ww, bb: O.causal_conv1d_ref(a, ww, bb, activation), [x, w, b], dout)
+        din, dw, db = PP.conv1d_backward(x.to(DEV), w.to(DEV), b.to(DEV), [dout.to(DEV)], activation=activation)
+        assert_close("din", din, dx_r, dtype)
+        assert_close("dweight", dw, dw_r, dtype)
+        assert_close("dbias", db, db_r, dtype)
+
+
 def test_conv1d_output_views_feed_the_scan(lib):
     """The three channel ranges of the conv output are handed to the scan as strided views (no copies)."""
     import trading_bot_0_b200 as T

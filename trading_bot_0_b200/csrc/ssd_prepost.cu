@@ -7,6 +7,8 @@
 //
 // The step-size activation softplus(dt + dt_bias) and the gate y*silu(z) need no kernel here: they are
 // evaluated inside the scan's own kernels.
+#include <type_traits>
+
 #include "common.cuh"
 #include "ssd_internal.h"
 
@@ -433,79 +435,77 @@ __global__ void __launch_bounds__(CONV_THREADS, CONV_BWD_MINB) k_conv_bwd(SsdCon
 }
 
 // ---------------------------------------------------------------------------------------------
-// conv backward, shared-memory staged.  Grid = (tile walkers, channel blocks of 256 bytes); a CTA walks (batch, 32-token
-// tile) pairs of its channel block with the next tile's input rows and gradient rows arriving by cp.async while the
-// current tile is worked on in two phases:
-//   1. thread = (8 bytes of channels, 5 consecutive rows): recompute the pre-activation from a sliding input window,
-//      dpre = dout * act'(pre) into a shared fp32 tile, and the weight / bias gradient of the rows this tile owns;
-//   2. thread = (8 bytes of channels, 4 consecutive tokens): din from a sliding window over the dpre tile.
-// The tile carries K-1 halo rows on either side (zero-filled outside the sequence), so no row is recomputed in
-// registers and nothing is re-read from global memory but the halo.  A CTA leaves one partial weight-gradient row.
-constexpr int CONVB_STAGES = 2;
-constexpr int CONVB_CTAS_PER_SM = 3;
-// 32-token tiles: 55 KB of shared memory and 80 registers per thread let three blocks (24 warps) share an SM, which an
-// issue-bound kernel needs more than it needs long tiles (64-token tiles, two blocks of 126 registers: 0.424 ms; this:
-// 0.357 ms; four blocks at 64 registers spill: 0.51 ms)
-constexpr int CONVB_TT = 32;
+// conv backward, shared-memory staged.  Grid = (walkers, channel blocks of 256 bytes).  The tokens of all sequences are shared out
+// evenly over the warps of a channel block; a warp streams its share in time order, thread = 8 bytes of channels, through a ring
+// of its own (stages of eight input and eight gradient rows, two requested ahead by cp.async), so warps never wait for one
+// another.  Row s: the pre-activation from the input window, dpre = dout * act'(pre) into a window in registers, the weight and
+// bias gradient, and din[s - K + 1], which is then complete.  A share re-reads K - 1 rows on either side.  A CTA leaves one
+// partial weight-gradient row.
+// Bound by the FMA pipe and issue (issue slots 0.54 busy, math throttle the first stall): 64 x 1024 tokens of 384 channels 36.8 us;
+// 50.6 as tiles of 32 tokens whose dpre went through shared memory between two CTA barriers, 38.6 without the form for whole stages.
+constexpr int CONVB_STAGES = 3, CONVB_RS = 8, CONVB_CTAS_PER_SM = 2, CONVB_WARPS = CONVS_THREADS / 32;
+constexpr int CONVB_STAGE_BYTES = 2 * CONVB_RS * CONVS_ROWB;
+constexpr int CONVB_SMEM = CONVB_WARPS * CONVB_STAGES * CONVB_STAGE_BYTES;
+constexpr int CONVB_MIN_ROWS = 16;   // tokens of a warp's share at least (its halo is 2 (K - 1) rows)
+
+// Where a warp stands in its share [r0, r1) of the tokens: the piece [t0, t1) of sequence b, and the first row of its next stage.
+template <int K> struct ConvWalk {
+  long long left;
+  int b, t0, t1, s, L;
+  __device__ __forceinline__ ConvWalk(long long r0, long long r1, int L_) : L(L_) {
+    b = (int)(r0 / L);
+    t0 = (int)(r0 - (long long)b * L);
+    left = r1 - r0;
+    take();
+  }
+  __device__ __forceinline__ void take() {
+    t1 = (int)min((long long)L, t0 + left);
+    left -= t1 - t0;
+    s = t0 - (K - 1);
+  }
+  __device__ __forceinline__ bool live() const { return t1 > t0; }
+  __device__ __forceinline__ void next() {
+    s += CONVB_RS;
+    if (s > t1 + K - 2) { ++b; t0 = 0; take(); }
+  }
+};
 
 template <typename T, int K>
 __global__ void __launch_bounds__(CONVS_THREADS, CONVB_CTAS_PER_SM)
 k_conv_bwd_sm(SsdConvDims d, const T* __restrict__ in, const float* __restrict__ weight, const float* __restrict__ bias,
-              ConvSegs segs, T* __restrict__ din, long long din_stride_b, long long din_stride_l,
-              float* __restrict__ partial, int ntt) {
+              ConvSegs segs, T* __restrict__ din, long long din_stride_b, long long din_stride_l, float* __restrict__ partial) {
   pdl_wait();
   constexpr int NC = 16 / (int)sizeof(T);            // channels per 16-byte copy piece
-  constexpr int NP = 8 / (int)sizeof(T);             // channels per thread in the arithmetic phases
-  constexpr int CB = CONVS_ROWB / (int)sizeof(T);    // channels per tile
-  constexpr int IN_ROWS = CONVB_TT + 2 * (K - 1), GO_ROWS = CONVB_TT + K - 1;
-  constexpr int STAGE_BYTES = (IN_ROWS + GO_ROWS) * CONVS_ROWB;
-  constexpr int DPRE_ROWB = CB * 4;
-  constexpr int R1 = (GO_ROWS + 7) / 8;              // rows per thread in phase 1
+  constexpr int NP = 8 / (int)sizeof(T);             // channels per thread in the arithmetic
+  constexpr int CB = CONVS_ROWB / (int)sizeof(T);    // channels of a block
   extern __shared__ __align__(128) unsigned char conv_smem[];
-  unsigned char* dpre = conv_smem + CONVB_STAGES * STAGE_BYTES;
-  const int tid = threadIdx.x, cv = tid & 15, seg = tid >> 4, hv = tid & 31, rs = tid >> 5;
-  const int cb = blockIdx.y;
+  const int tid = threadIdx.x, hv = tid & 31, rs = tid >> 5, cb = blockIdx.y;
+  unsigned char* ring = conv_smem + rs * CONVB_STAGES * CONVB_STAGE_BYTES;
 
-  // copy role: the 16-byte piece `cv` of rows seg, seg+16, ...
-  const int cc = cb * CB + cv * NC;
+  // copy role: the 16-byte piece `cv` of rows rr, rr + 2, ...
+  const int cv = hv & 15, rr = hv >> 4, cc = cb * CB + cv * NC;
   const bool cok = cc < d.channels;
   int si = 0;
   for (int i = 1; i < segs.n; ++i) if (cc >= segs.c_begin[i]) si = i;
-  const T* gseg = (const T*)segs.ptr[si] + (cok ? cc - segs.c_begin[si] : 0);
+  const T* gbase = (const T*)segs.ptr[si] + (cok ? cc - segs.c_begin[si] : 0);
   const long long gsb = segs.stride_b[si], gsl = segs.stride_l[si];
-  const int npairs = d.batch * ntt;
   const T* ibase = in + (cok ? cc : 0);
-  auto request = [&](const PairWalk& pw, int stage) {
-    if (pw.b < d.batch) {
-      const int t0 = pw.tt * CONVB_TT;
-      unsigned char* sp = conv_smem + stage * STAGE_BYTES + cv * 16 + seg * CONVS_ROWB;
-      {
-        const T* src = ibase + (long long)pw.b * d.in_stride_b + (long long)(t0 - (K - 1) + seg) * d.in_stride_l;
-        int t = t0 - (K - 1) + seg;
+  auto request = [&](const ConvWalk<K>& a, int stage) {
+    if (a.live()) {
+      const int t = a.s + rr, end = min(a.t1 + K - 1, d.seqlen);
+      unsigned char* sp = ring + stage * CONVB_STAGE_BYTES + rr * CONVS_ROWB + cv * 16;
+      const T* si_ = ibase + (long long)a.b * d.in_stride_b + (long long)t * d.in_stride_l;
+      const T* sg = gbase + (long long)a.b * gsb + (long long)t * gsl;
 #pragma unroll
-        for (int j = 0; j < (IN_ROWS + 15) / 16; ++j) {
-          if (seg + 16 * j < IN_ROWS) {
-            const bool ok = cok && t >= 0 && t < d.seqlen;
-            cp_async16(sp + j * 16 * CONVS_ROWB, ok ? (const void*)src : (const void*)in, ok);
-          }
-          src += 16 * d.in_stride_l; t += 16;
-        }
-      }
-      sp += IN_ROWS * CONVS_ROWB;
-      {
-        const T* src = gseg + (long long)pw.b * gsb + (long long)(t0 + seg) * gsl;
-        int t = t0 + seg;
-#pragma unroll
-        for (int j = 0; j < (GO_ROWS + 15) / 16; ++j) {
-          if (seg + 16 * j < GO_ROWS) {
-            const bool ok = cok && t < d.seqlen;
-            cp_async16(sp + j * 16 * CONVS_ROWB, ok ? (const void*)src : (const void*)in, ok);
-          }
-          src += 16 * gsl; t += 16;
-        }
+      for (int j = 0; j < CONVB_RS / 2; ++j) {
+        const int tj = t + 2 * j;
+        const bool iok = cok && tj >= 0 && tj < end, gok = cok && tj >= a.t0 && tj < end;
+        cp_async16(sp + 2 * j * CONVS_ROWB, iok ? (const void*)si_ : (const void*)in, iok);
+        cp_async16(sp + (CONVB_RS + 2 * j) * CONVS_ROWB, gok ? (const void*)sg : (const void*)in, gok);
+        si_ += 2 * d.in_stride_l; sg += 2 * gsl;
       }
     }
-    cp_async_commit();
+    cp_async_commit();   // a group per stage even when it is empty: the wait below counts groups
   };
 
   // arithmetic role: NP channels starting at c0, held as NP/2 packed pairs
@@ -524,104 +524,86 @@ k_conv_bwd_sm(SsdConvDims d, const T* __restrict__ in, const float* __restrict__
     db[j] = 0ull;
   }
 
-  PairWalk ahead((int)blockIdx.x, (int)gridDim.x, ntt), cur = ahead;
-  request(ahead, 0);
-  ahead.next();
+  const long long rows = (long long)d.batch * d.seqlen, nw = (long long)gridDim.x * CONVB_WARPS, wi = (long long)blockIdx.x * CONVB_WARPS + rs;
+  ConvWalk<K> cur(rows * wi / nw, rows * (wi + 1) / nw, d.seqlen), ahead = cur;
+  int fill = 0;
+#pragma unroll
+  for (int i = 0; i < CONVB_STAGES - 1; ++i) {
+    request(ahead, fill++);
+    if (ahead.live()) ahead.next();
+  }
+  f32x2 win[K][NH] = {}, dwin[K][NH] = {};   // input rows s - K + 1 .. s; dpre of the same rows
   int stage = 0;
-  for (int pair = blockIdx.x; pair < npairs; pair += gridDim.x) {
-    cp_async_wait<0>();
-    __syncthreads();     // the tile has landed; phase 2 of the previous tile is over (dpre and the other stage are free)
-    request(ahead, stage ^ 1);
-    ahead.next();
-    const int b = cur.b, t0 = cur.tt * CONVB_TT;
-    cur.next();
-    const unsigned char* sin = conv_smem + stage * STAGE_BYTES + hv * 8;
-    const unsigned char* sgo = sin + IN_ROWS * CONVS_ROWB;
-    stage ^= 1;
-    // ---- phase 1: rows r0 .. r0+R1-1 of the gradient tile (row r <-> token t0 + r; input rows r .. r+K-1) ----
-    {
-      const int r0 = rs * R1;
-      f32x2 win[K][NH];
+  for (; cur.live(); cur.next()) {
+    cp_async_wait<CONVB_STAGES - 2>();
+    __syncwarp();           // this stage has landed for every lane; every lane is done with the previous one
+    request(ahead, fill);
+    if (ahead.live()) ahead.next();
+    fill = fill + 1 == CONVB_STAGES ? 0 : fill + 1;
+    const unsigned char* sin = ring + stage * CONVB_STAGE_BYTES + hv * 8;
+    const unsigned char* sgo = sin + CONVB_RS * CONVS_ROWB;
+    stage = stage + 1 == CONVB_STAGES ? 0 : stage + 1;
+    const int end = min(cur.t1 + K - 1, d.seqlen);
+    T* dp = din + (long long)cur.b * din_stride_b + (long long)(cur.s - (K - 1)) * din_stride_l + c0;
+    auto rows8 = [&](auto whole) {   // WHOLE: every row of the stage is the share's own and completes a row of din
+      constexpr bool WHOLE = decltype(whole)::value;
+      const bool act = WHOLE || d.activation;
 #pragma unroll
-      for (int k = 0; k < K - 1; ++k) {
+      for (int i = 0; i < CONVB_RS; ++i) {
+        const int s = cur.s + i;
         RawN<T, NP> raw;
-        if (r0 + k < IN_ROWS) lds_raw<T, NP>(sin + (r0 + k) * CONVS_ROWB, raw); else zero_raw(raw);
-        unpack_pairs(raw, win[k]);
-      }
+        lds_raw<T, NP>(sin + i * CONVS_ROWB, raw);
+        unpack_pairs(raw, win[K - 1]);
 #pragma unroll
-      for (int i = 0; i < R1; ++i) {
-        const int r = r0 + i;
-        if (r < GO_ROWS) {
-          RawN<T, NP> raw, rg;
-          lds_raw<T, NP>(sin + (r + K - 1) * CONVS_ROWB, raw);
-          unpack_pairs(raw, win[K - 1]);
-          lds_raw<T, NP>(sgo + r * CONVS_ROWB, rg);
-          f32x2 go[NH], dp[NH];
-          unpack_pairs(rg, go);
-          const bool own = r < CONVB_TT;    // each row's weight / bias gradient is counted by exactly one tile
+        for (int j = 0; j < NH; ++j) dwin[K - 1][j] = 0ull;
+        if (WHOLE || (s >= cur.t0 && s < end)) {
+          lds_raw<T, NP>(sgo + i * CONVS_ROWB, raw);
+          f32x2 go[NH];
+          unpack_pairs(raw, go);
 #pragma unroll
           for (int j = 0; j < NH; ++j) {
-            f32x2 a2 = bs[j];
-#pragma unroll
-            for (int k = 0; k < K; ++k) a2 = fma2(w[j][k], win[k][j], a2);
             f32x2 g = go[j];
-            if (d.activation) {
+            if (act) {
+              f32x2 a2 = bs[j];
+#pragma unroll
+              for (int k = 0; k < K; ++k) a2 = fma2(w[j][k], win[k][j], a2);
               float a0, a1;
               unpack2(a2, a0, a1);
               const float s0 = sig_<T>(a0), s1 = sig_<T>(a1);
               // silu'(a) = s (1 + a (1 - s))
               g = fma2(g, pack2(fmaf(s0, fmaf(-a0, s0, a0), s0), fmaf(s1, fmaf(-a1, s1, a1), s1)), 0ull);
             }
-            dp[j] = g;
-            if (own) {
-              db[j] = add2(db[j], g);
+            dwin[K - 1][j] = g;
+          }
+          if (WHOLE || s < cur.t1) {    // each row's weight / bias gradient is counted by exactly one share
 #pragma unroll
-              for (int k = 0; k < K; ++k) dw[j][k] = fma2(g, win[k][j], dw[j][k]);
+            for (int j = 0; j < NH; ++j) {
+              db[j] = add2(db[j], dwin[K - 1][j]);
+#pragma unroll
+              for (int k = 0; k < K; ++k) dw[j][k] = fma2(dwin[K - 1][j], win[k][j], dw[j][k]);
             }
           }
-          f32x2* dst = reinterpret_cast<f32x2*>(dpre + r * DPRE_ROWB) + hv * NH;
-          if constexpr (NH == 2) *reinterpret_cast<ulonglong2*>(dst) = make_ulonglong2(dp[0], dp[1]);
-          else dst[0] = dp[0];
-#pragma unroll
-          for (int k = 0; k < K - 1; ++k)
-#pragma unroll
-            for (int j = 0; j < NH; ++j) win[k][j] = win[k + 1][j];
         }
-      }
-    }
-    __syncthreads();
-    // ---- phase 2: din[t0 + i] = sum_q w[K-1-q] * dpre[i + q], tokens i0 .. i0+7 ----
-    if (live) {
-      const int i0 = rs * (CONVB_TT / 8);
-      const f32x2* dpp = reinterpret_cast<const f32x2*>(dpre) + hv * NH;
-      auto load_row = [&](int row, f32x2 (&v)[NH]) {
-        const f32x2* q = dpp + (size_t)row * (DPRE_ROWB / 8);
-        if constexpr (NH == 2) { const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(q); v[0] = t.x; v[1] = t.y; }
-        else v[0] = q[0];
-      };
-      T* dp = din + (long long)b * din_stride_b + (long long)(t0 + i0) * din_stride_l + c0;
-      f32x2 dwin[K][NH];
+        if ((WHOLE || (s - (K - 1) >= cur.t0 && s - (K - 1) < cur.t1)) && live) {   // din[s - K + 1] = sum_q w[K-1-q] dpre[s - K + 1 + q]
+          float o[NP];
 #pragma unroll
-      for (int q = 0; q < K - 1; ++q) load_row(i0 + q, dwin[q]);
+          for (int j = 0; j < NH; ++j) {
+            f32x2 a2 = 0ull;
 #pragma unroll
-      for (int i = 0; i < CONVB_TT / 8; ++i) {
-        load_row(i0 + i + K - 1, dwin[K - 1]);
-        float o[NP];
-#pragma unroll
-        for (int j = 0; j < NH; ++j) {
-          f32x2 a2 = 0ull;
-#pragma unroll
-          for (int q = 0; q < K; ++q) a2 = fma2(w[j][K - 1 - q], dwin[q][j], a2);
-          unpack2(a2, o[2 * j], o[2 * j + 1]);
+            for (int q = 0; q < K; ++q) a2 = fma2(w[j][K - 1 - q], dwin[q][j], a2);
+            unpack2(a2, o[2 * j], o[2 * j + 1]);
+          }
+          store_n(dp, o);
         }
-        if (t0 + i0 + i < d.seqlen) store_n(dp, o);
         dp += din_stride_l;
 #pragma unroll
-        for (int q = 0; q < K - 1; ++q)
+        for (int k = 0; k < K - 1; ++k)
 #pragma unroll
-          for (int j = 0; j < NH; ++j) dwin[q][j] = dwin[q + 1][j];
+          for (int j = 0; j < NH; ++j) { win[k][j] = win[k + 1][j]; dwin[k][j] = dwin[k + 1][j]; }
       }
-    }
+    };
+    if (d.activation && cur.s >= cur.t0 + K - 1 && cur.s + CONVB_RS <= cur.t1) rows8(std::true_type());
+    else rows8(std::false_type());
   }
   cp_async_wait<0>();
   __syncthreads();
@@ -1088,18 +1070,16 @@ int32_t ssd_conv1d_backward(const SsdConvDims* dims, const void* in, const float
   cudaStream_t s = (cudaStream_t)cuda_stream;
   float* partial = (float*)workspace;
   if ((long long)dims->channels * es >= CONVS_ROWB / 2) {
-    const int ntt = (dims->seqlen + CONVB_TT - 1) / CONVB_TT;
     const int ncb = (dims->channels * es + CONVS_ROWB - 1) / CONVS_ROWB;
-    const int sms = sm_count();
-    long long nx = ((long long)sms * CONVB_CTAS_PER_SM + ncb - 1) / ncb;
-    const long long pairs = (long long)dims->batch * ntt;
-    if (pairs > 0x7fffffffLL || ncb > 65535) { set_error("conv1d backward: batch x token tiles exceeds 2^31"); return SSD_ERR_UNSUPPORTED; }
-    if (nx > pairs) nx = pairs;
+    const long long rows = (long long)dims->batch * dims->seqlen;
+    if (ncb > 65535) { set_error("conv1d backward: too many channels"); return SSD_ERR_UNSUPPORTED; }
+    long long nx = ((long long)sm_count() * CONVB_CTAS_PER_SM) / ncb;
+    if (nx > rows / (CONVB_WARPS * CONVB_MIN_ROWS)) nx = rows / (CONVB_WARPS * CONVB_MIN_ROWS);
     if (nx > nblk) nx = nblk;     // the workspace holds nblk partial rows
+    if (nx < 1) nx = 1;
     const dim3 grid((unsigned)nx, (unsigned)ncb);
-#define CONV_BWD_SM(T, K) do { \
-      constexpr int smem = CONVB_STAGES * (2 * CONVB_TT + 3 * (K - 1)) * CONVS_ROWB + (CONVB_TT + K - 1) * (CONVS_ROWB / (int)sizeof(T)) * 4; \
-      launch<k_conv_bwd_sm<T, K>>(grid, CONVS_THREADS, smem, s, *dims, (const T*)in, weight, bias, segs, (T*)din, din_stride_b, din_stride_l, partial, ntt); } while (0)
+#define CONV_BWD_SM(T, K) \
+      launch<k_conv_bwd_sm<T, K>>(grid, CONVS_THREADS, CONVB_SMEM, s, *dims, (const T*)in, weight, bias, segs, (T*)din, din_stride_b, din_stride_l, partial)
     if (dims->dtype == SSD_BF16) {
       if (dims->width == 4) CONV_BWD_SM(__nv_bfloat16, 4); else if (dims->width == 3) CONV_BWD_SM(__nv_bfloat16, 3); else CONV_BWD_SM(__nv_bfloat16, 2);
     } else {
