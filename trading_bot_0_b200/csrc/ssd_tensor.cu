@@ -2356,13 +2356,13 @@ k_bwd_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant__
       mbar_init(&bars.cb_full[i], 1); mbar_init(&bars.cb_empty[i], SPLIT ? 2 : 1);
       mbar_init(&bars.stp_full[i], 1); mbar_init(&bars.stp_empty[i], 1);
       mbar_init(&bars.g_full[i], 1); mbar_init(&bars.g_empty[i], WS_SCALE_WARPS);
-      mbar_init(&bars.in_full[i], 1); mbar_init(&bars.in_empty[i], 1 + WS_EPI_WARPS);
+      mbar_init(&bars.in_full[i], 1); mbar_init(&bars.in_empty[i], WS_EPI_WARPS);   // the epilogue is behind the block's products
       mbar_init(&bars.m_full[i], WS_SCALE_WARPS); mbar_init(&bars.m_empty[i], 1);
     }
     for (int i = 0; i < 4; ++i) { mbar_init(&bars.tab_full[i], 1); mbar_init(&bars.tab_empty[i], WS_SCALE_WARPS + WS_EPI_WARPS); }
     mbar_init(&bars.st_full, 1); mbar_init(&bars.st_empty, 1);
     mbar_init(&bars.y_full, SPLIT ? 2 : 1); mbar_init(&bars.y_empty, WS_EPI_WARPS);
-    mbar_init(&bars.u_full, SPLIT ? 2 : 1); mbar_init(&bars.u_empty, WS_EPI_WARPS);
+    mbar_init(&bars.u_full, 2); mbar_init(&bars.u_empty, WS_EPI_WARPS);
     mbar_init(&bars.done, 1);
     mbar_fence_init();
   }
@@ -2498,11 +2498,49 @@ k_bwd_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant__
         }
       }
     }
+  } else if (!SPLIT && warp == 18) {
+    // ------------------------------------------------------------------ dstate 64: issuer of G and of the state products
+    // (512 x 1024 tokens of 8 heads: 351 us with one issuer for everything, 342 like this, 363 with one more for U' alone)
+    if (lane == 0) {
+      const uint32_t idG = make_idesc(128, 128, 0, 0), idO = make_idesc(128, 64, 0, 0);
+      const uint64_t dS0 = desc_sw128_k(smem_u32(sSt), 0), dDS0 = desc_sw128_k(smem_u32(sSt + SBOX_BYTES), 0);
+      auto issue_g = [&](int t) {
+        const int s_ = t & 1;
+        w.wait(&bars.cb_full[s_], (t >> 1) & 1, 43);
+        w.wait(&bars.g_empty[s_], ((t >> 1) & 1) ^ 1, 44);
+        tc_fence_after();
+        const uint32_t ct = smem_u32(sCB + s_ * Cfg::CB_BYTES);
+        const uint64_t dc = desc_sw128_k(ct, 0), db = desc_sw128_k(ct + BOX_BYTES, 0);
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks) mma_bf16(tm + s_ * 128, desc_adv(dc, ks * 32), desc_adv(db, ks * 32), idG, ks > 0);
+        mma_commit(&bars.g_full[s_]);
+      };
+      issue_g(0);
+      int kb = 0;
+      for (int t = 0; t < my_tiles; ++t) {
+        const uint32_t ct = smem_u32(sCB + (t & 1) * Cfg::CB_BYTES);
+        const uint64_t dC0 = desc_sw128_k(ct, 0), dB0 = desc_sw128_k(ct + BOX_BYTES, 0);
+        for (int blk = 0; blk < nblk; ++blk, ++kb) {
+          w.wait(&bars.st_full, kb & 1, 57);
+          w.wait(&bars.u_empty, (kb & 1) ^ 1, 62);
+          tc_fence_after();
+#pragma unroll
+          for (int ks = 0; ks < 4; ++ks) {
+            mma_bf16(tmYo, desc_adv(dC0, ks * 32), desc_adv(dS0, ks * 32), idO, ks > 0);
+            mma_bf16(tmUo, desc_adv(dB0, ks * 32), desc_adv(dDS0, ks * 32), idO, ks > 0);
+          }
+          mma_commit(&bars.st_empty);
+          if (blk == nblk - 1) mma_commit(&bars.cb_empty[t & 1]);
+          mma_commit(&bars.u_full);
+          if (blk == 0 && t + 1 < my_tiles) issue_g(t + 1);
+        }
+      }
+    }
   } else if (warp == 17) {
     // ------------------------------------------------------------------ MMA issuer
     if (lane == 0) {
       const uint32_t idG = make_idesc(128, 128, 0, 0);
-      const uint32_t idY = make_idesc(128, P, 0, 1), idU = make_idesc(128, P, 1, 1), idO = make_idesc(128, 64, 0, 0);
+      const uint32_t idY = make_idesc(128, P, 0, 1), idU = make_idesc(128, P, 1, 1);
       auto issue_g = [&](int t) {
         const int s_ = t % NCBS;
         w.wait(&bars.cb_full[s_], (t / NCBS) & 1, 43);
@@ -2517,12 +2555,9 @@ k_bwd_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant__
         }
         mma_commit(&bars.g_full[s_]);
       };
-      issue_g(0);
-      const uint64_t dS0 = desc_sw128_k(smem_u32(sSt), 0), dDS0 = desc_sw128_k(smem_u32(sSt + SBOX_BYTES), 0);
+      if constexpr (SPLIT) issue_g(0);
       int kb = 0, kh = 0;
       for (int t = 0; t < my_tiles; ++t) {
-        const uint32_t ct = smem_u32(sCB + (t % NCBS) * Cfg::CB_BYTES);
-        const uint64_t dC0 = desc_sw128_k(ct, 0), dB0 = desc_sw128_k(ct + BOX_BYTES, 0);
         for (int blk = 0; blk < nblk; ++blk, ++kb) {
           const int ib = kb & 1;
           const uint32_t inb = smem_u32(sIn + ib * Cfg::IN_BYTES);
@@ -2553,7 +2588,6 @@ k_bwd_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant__
           } else {
             // dstate 64: both products of a head together; a block needs both M_h tiles, and holding them for a second round
             // keeps the decay pass from running ahead (361 us against 349 at 512 x 1024 tokens)
-            w.wait(&bars.st_full, kb & 1, 57);
             w.wait(&bars.u_empty, (kb & 1) ^ 1, 46);
             for (int hl = 0; hl < HB; ++hl, ++kh) {
               const int ms = kh % NM;
@@ -2567,21 +2601,11 @@ k_bwd_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant__
                 mma_bf16(tmYd + hl * P, desc_adv(dMk, ks * 4096), desc_adv(dX0, ks * 2048), idY, ks > 0);
                 mma_bf16(tmUd + hl * P, desc_adv(dMt, ks * 256), desc_adv(dY0, ks * 2048), idU, ks > 0);
               }
-              if (hl == 0) {
-#pragma unroll
-                for (int ks = 0; ks < 4; ++ks) {
-                  mma_bf16(tmYo, desc_adv(dC0, ks * 32), desc_adv(dS0, ks * 32), idO, ks > 0);
-                  mma_bf16(tmUo, desc_adv(dB0, ks * 32), desc_adv(dDS0, ks * 32), idO, ks > 0);
-                }
-                mma_commit(&bars.st_empty);
-              }
               mma_commit(&bars.m_empty[ms]);
             }
           }
-          mma_commit(&bars.in_empty[ib]);
-          if (blk == nblk - 1) mma_commit(&bars.cb_empty[t % NCBS]);
+          if (SPLIT && blk == nblk - 1) mma_commit(&bars.cb_empty[0]);
           mma_commit(&bars.u_full);
-          if (!SPLIT && blk == 0 && t + 1 < my_tiles) issue_g(t + 1);
         }
         if (SPLIT && t + 1 < my_tiles) issue_g(t + 1);
       }
@@ -2728,21 +2752,26 @@ k_bwd_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant__
 //   * warp 16: TMA.  A ring of three (dstate 64: four) 32 KB slots holds {x box, dy box} of a head block, and after a tile's
 //     last block its C and B tiles (needed once, at the end of the tile: a buffer of their own would cost slots); a ring for
 //     the {S_prev, dS_end} boxes, one of four for the decay tables;
-//   * warp 17: MMA issue.  W products one block ahead into two (three) accumulators, state products, the tile's two products;
+//   * warp 17: issue of the W products into two (three) accumulators; warp 18 (dstate 128: and 19): of the state products and the
+//     tile's two products.  An instruction costs its lane over 100 cycles beside the other warps' work: one lane for all of them was
+//     busy 72 % of the time (dstate 64: 273 us where the two take 248; dstate 128: 620, 572);
 //   * warps 0-15: W -> decay -> register sum (thread = row x 32 columns) -> the M tile;
 //   * warps 20-27: scale the boxes in place for the state products, and drain dC / dB of a finished tile.
 // TMEM: the W accumulators, dC, dB = 512 columns.
-// dstate 128: 2x131072 with 24 heads 0.97 -> 0.64 ms = 5.1 TB/s, what a pure TMA stream of boxes reaches; 16x4096 0.27 -> 0.185
-// ms (3.46 waves of tiles take the time of four).  dstate 64, 512x1024 with 8 heads: 0.278 ms whatever the decay; a kernel that
+// dstate 128: 2x131072 with 24 heads 0.97 -> 0.57 ms = 5.7 TB/s; 16x4096 0.27 -> 0.169
+// ms (3.46 waves of tiles take the time of four).  dstate 64, 512x1024 with 8 heads: 0.248 ms whatever the decay; a kernel that
 // carried the decay on the operands where its range allowed took 0.290, and 0.394 with one head beyond the range.  No unit is full
 // there (128x1024: issue slots 0.43, DRAM 42 %, tensor pipe 14 %); a block waits for its decay pass, so what that pass issues
-// counts: 0.339 with 32 columns of W in registers beside the sums (spills), 0.306 with 16, 0.301 with packed scaling of the
-// boxes, 0.278 with packed FMAs and without the six warps whose blocks lie above the diagonal.
+// counts (with one issuer lane): 0.339 with 32 columns of W in registers beside the sums (spills), 0.306 with 16, 0.301 with
+// packed scaling of the boxes, 0.278 with packed FMAs and without the six warps whose blocks lie above the diagonal.
 template <int P, int N_>
 struct DbCfg {
   static constexpr int N = N_, NB64 = N / 64, HB = 64 / P, NT = 4, NIN = N == 64 ? 4 : 3, NST = N == 64 ? 3 : 2;
   static constexpr int NCB = NB64;                           // uses of the input ring for a tile's C and B (dstate 64: both in one)
   static constexpr int NW = N == 64 ? 3 : 2;                 // W accumulators
+  // issuer lanes of the products that add to dC and dB.  dstate 128: one each (2 x 131072 tokens of 24 heads 583 -> 572 us); dstate
+  // 64: one for both (512 x 1024 of 8 heads 248 us against 261)
+  static constexpr int NL = N == 64 ? 1 : 2;
   static constexpr int IN_BYTES = 2 * BOX_BYTES;             // x box, dy box; or C and B of a tile
   static constexpr int ST_BYTES = 2 * NB64 * SBOX_BYTES;     // S_prev, dS_end
   static constexpr int TB_BYTES = HB * TAB_BYTES;
@@ -2773,14 +2802,14 @@ k_dbc_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant__
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) {
     for (int i = 0; i < NIN; ++i) {
-      mbar_init(&in_full[i], 1); mbar_init(&in_empty[i], 1);
+      mbar_init(&in_full[i], 1); mbar_init(&in_empty[i], 1 + Cfg::NL);
       mbar_init(&raw_done[i], 1); mbar_init(&sc_full[i], Cfg::NSCALE);
     }
-    for (int i = 0; i < NST; ++i) { mbar_init(&st_full[i], 1); mbar_init(&st_empty[i], 1); }
+    for (int i = 0; i < NST; ++i) { mbar_init(&st_full[i], 1); mbar_init(&st_empty[i], Cfg::NL); }
     for (int i = 0; i < NT; ++i) { mbar_init(&tab_full[i], 1); mbar_init(&tab_empty[i], Cfg::NDECAY + Cfg::NSCALE); }
     for (int i = 0; i < NW; ++i) { mbar_init(&w_full[i], 1); mbar_init(&w_empty[i], Cfg::NDECAY); }
-    mbar_init(&m_full, Cfg::NDECAY); mbar_init(&m_empty, 1);
-    mbar_init(&acc_full, 1); mbar_init(&acc_empty, Cfg::NSCALE);
+    mbar_init(&m_full, Cfg::NDECAY); mbar_init(&m_empty, Cfg::NL);
+    mbar_init(&acc_full, Cfg::NL); mbar_init(&acc_empty, Cfg::NSCALE);
     mbar_fence_init();
   }
   if (warp == 17) tmem_alloc(&tmem_slot, 512);
@@ -2856,31 +2885,45 @@ k_dbc_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant__
       }
     }
   } else if (warp == 17) {
-    // ------------------------------------------------------------------ MMA issuer
+    // ------------------------------------------------------------------ issuer of the W products, as far ahead as boxes and W
+    // accumulators allow.  It arrives on in_empty for every use of the ring that it has seen, C and B included: a slot cannot
+    // come round to a lane that is two phases behind.
     if (lane == 0) {
-      const uint32_t idW = make_idesc(128, 128, 0, 0), idC = make_idesc(128, N, 0, 1), idB = make_idesc(128, N, 1, 1);
-      const uint64_t dMk = desc_plain_k(smem_u32(sM), 128, 0), dMt = desc_plain_mn(smem_u32(sM), 128, 0, 0);
+      const uint32_t idW = make_idesc(128, 128, 0, 0);
       int kb = 0, ki = 0, kw = 0;
-      auto issue_w = [&](int kbn, int kin) {   // the W products of block kbn, whose boxes are use kin of the input ring
-        const int ib = kin % NIN;
-        w.wait(&in_full[ib], par(kin, NIN), 45);
-        const uint32_t inb = smem_u32(sIn + ib * Cfg::IN_BYTES);
-        const uint64_t dX0 = desc_sw128_k(inb, 0), dDY0 = desc_sw128_k(inb + BOX_BYTES, 0);
-        for (int hl = 0; hl < HB; ++hl, ++kw) {
-          w.wait(&w_empty[kw % NW], par(kw, NW) ^ 1, 58);
-          tc_fence_after();
-#pragma unroll
-          for (int ks = 0; ks < P / 16; ++ks)
-            mma_bf16(tm + (kw % NW) * 128, desc_adv(dDY0, hl * P * 2 + ks * 32), desc_adv(dX0, hl * P * 2 + ks * 32), idW, ks > 0);
-          mma_commit(&w_full[kw % NW]);
-        }
-        mma_commit(&raw_done[kbn % NIN]);
-      };
       for (int t = 0; t < my_tiles; ++t) {
-        issue_w(kb, ki);   // after the previous tile's last products: its first box reuses the slot of that tile's last block
+        for (int blk = 0; blk < nblk; ++blk, ++kb, ++ki) {
+          const int ib = ki % NIN;
+          w.wait(&in_full[ib], par(ki, NIN), 45);
+          mbar_arrive(&in_empty[ib]);   // (the products are done before the boxes are scaled, the scaling before the other lane's products)
+          const uint32_t inb = smem_u32(sIn + ib * Cfg::IN_BYTES);
+          const uint64_t dX0 = desc_sw128_k(inb, 0), dDY0 = desc_sw128_k(inb + BOX_BYTES, 0);
+          for (int hl = 0; hl < HB; ++hl, ++kw) {
+            w.wait(&w_empty[kw % NW], par(kw, NW) ^ 1, 58);
+            tc_fence_after();
+#pragma unroll
+            for (int ks = 0; ks < P / 16; ++ks)
+              mma_bf16(tm + (kw % NW) * 128, desc_adv(dDY0, hl * P * 2 + ks * 32), desc_adv(dX0, hl * P * 2 + ks * 32), idW, ks > 0);
+            mma_commit(&w_full[kw % NW]);
+          }
+          mma_commit(&raw_done[kb % NIN]);
+        }
+        for (int n = 0; n < NCB; ++n, ++ki) {
+          w.wait(&in_full[ki % NIN], par(ki, NIN), 43);
+          mbar_arrive(&in_empty[ki % NIN]);
+        }
+      }
+    }
+  } else if (warp >= 18 && warp < 18 + Cfg::NL) {
+    // ------------------------------------------------------------------ issuers of everything that adds to dC (warp 18) and dB
+    if (lane == 0) {
+      const bool cside = warp == 18, bside = Cfg::NL == 1 || !cside;
+      const uint32_t idC = make_idesc(128, N, 0, 1), idB = make_idesc(128, N, 1, 1);
+      const uint64_t dMk = desc_plain_k(smem_u32(sM), 128, 0), dMt = desc_plain_mn(smem_u32(sM), 128, 0, 0);
+      int kb = 0, ki = 0;
+      for (int t = 0; t < my_tiles; ++t) {
         w.wait(&acc_empty, (t & 1) ^ 1, 46);
         for (int blk = 0; blk < nblk; ++blk, ++kb, ++ki) {
-          if (blk + 1 < nblk) issue_w(kb + 1, ki + 1);
           const int ib = ki % NIN, sb = kb % NST;
           const uint32_t inb = smem_u32(sIn + ib * Cfg::IN_BYTES), stb = smem_u32(sSt + sb * Cfg::ST_BYTES);
           const uint64_t dXk = desc_sw128_k(inb, 0), dDYk = desc_sw128_k(inb + BOX_BYTES, 0);
@@ -2890,8 +2933,8 @@ k_dbc_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant__
           tc_fence_after();
 #pragma unroll
           for (int ks = 0; ks < 4; ++ks) {
-            mma_bf16(tmDC, desc_adv(dDYk, ks * 32), desc_adv(dSm0, ks * 2048), idC, blk > 0 || ks > 0);
-            mma_bf16(tmDB, desc_adv(dXk, ks * 32), desc_adv(dDSm0, ks * 2048), idC, blk > 0 || ks > 0);
+            if (cside) mma_bf16(tmDC, desc_adv(dDYk, ks * 32), desc_adv(dSm0, ks * 2048), idC, blk > 0 || ks > 0);
+            if (bside) mma_bf16(tmDB, desc_adv(dXk, ks * 32), desc_adv(dDSm0, ks * 2048), idC, blk > 0 || ks > 0);
           }
           mma_commit(&in_empty[ib]);
           mma_commit(&st_empty[sb]);
@@ -2904,8 +2947,8 @@ k_dbc_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant__
         const uint64_t dCm0 = desc_sw128_mn(ct, 0, 0, BOX_BYTES), dBm0 = desc_sw128_mn(bt, 0, 0, BOX_BYTES);
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks) {
-          mma_bf16(tmDC, desc_adv(dMk, ks * 4096), desc_adv(dBm0, ks * 2048), idC, true);
-          mma_bf16(tmDB, desc_adv(dMt, ks * 256), desc_adv(dCm0, ks * 2048), idB, true);
+          if (cside) mma_bf16(tmDC, desc_adv(dMk, ks * 4096), desc_adv(dBm0, ks * 2048), idC, true);
+          if (bside) mma_bf16(tmDB, desc_adv(dMt, ks * 256), desc_adv(dCm0, ks * 2048), idB, true);
         }
         for (int n = 0; n < NCB; ++n) mma_commit(&in_empty[(ki + n) % NIN]);
         mma_commit(&m_empty);
