@@ -150,12 +150,18 @@ __device__ __forceinline__ void zero_upper_blocks(int row, int part, int warp, u
     if (cb > (warp & 3)) st_shared_v4(mtile + plain_off(128, row, cb * 32 + part * 8), 0u, 0u, 0u, 0u);
 }
 
-// Whole-row variant for the persistent kernels.  A group of four warps (one per TMEM lane quarter)
+// Whole-row variant for k_scan_ws.  A group of four warps (one per TMEM lane quarter)
 // owns one head at a time and different groups work on different heads, so the latency of one group's
-// TMEM loads, table loads and stores hides behind another group's arithmetic.  Thread = accumulator
-// row; it walks the 32x32 blocks of its block row left to right (blocks below the diagonal first, the
+// TMEM loads, table loads and stores hides behind another group's arithmetic.  A warp
+// walks the 32x32 blocks of its block row left to right (blocks below the diagonal first, the
 // diagonal block last) with the next block's TMEM load in flight while the current one is scaled,
-// converted and stored.  Same factorisation as decay_mask_tile.
+// converted and stored.  Same factorisation as decay_mask_tile below the diagonal; elements of the diagonal block take
+// exp(cs_i - cs_j) dt_j directly, so this variant does not need the T_DS section.
+// Blocks are read from TMEM in the layout of matrix fragments: a thread has two neighbouring columns of every group of eight,
+// in four rows (t / 4 + 8 a).  A read of shared memory costs what it delivers to registers, 128 bytes a cycle, broadcast or not;
+// with a row per thread every thread read every column's factor.  Here it reads a quarter of them, four rows share them, and
+// stmatrix writes the tile (512 x 1024 tokens of 8 heads 229 -> 224 us, 2 x 131072 of 24 heads 606 -> 590; in the backward
+// kernels, whose passes are shorter, it gained nothing: 349 against 354 and 273 against 290 us).
 __device__ __forceinline__ void tmem_ld16_issue(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
@@ -172,42 +178,47 @@ __device__ __forceinline__ void tmem_ld_wait_2x16(uint32_t (&r)[16], uint32_t (&
                  "+r"(q[9]), "+r"(q[10]), "+r"(q[11]), "+r"(q[12]), "+r"(q[13]), "+r"(q[14]), "+r"(q[15])
                :: "memory");
 }
-// 16 columns of a block below the diagonal: out[k] = raw[k] * rf * cf[k]; `cf` = shared-memory address of the column factors
-__device__ __forceinline__ void decay_off_half(const uint32_t (&raw)[16], float rf, uint32_t cf, uint32_t dst) {
+// One group of eight columns (first column c0 of the tile) of a 32x32 block: v[2 a + e] is row 8 a + t/4, column 2 (t % 4) + e.
+struct DecayRows {
+  float cs[4];   // of this thread's rows
+  __device__ __forceinline__ void load(uint32_t ts, int row0, int lane) {   // row0: first row of the block
 #pragma unroll
-  for (int j8 = 0; j8 < 16; j8 += 8) {
-    const float4 f0 = lds_v4f32(cf + 4 * j8), f1 = lds_v4f32(cf + 4 * (j8 + 4));
-    const float f[8] = {f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, f1.z, f1.w};
-    float v[8];
+    for (int a = 0; a < 4; ++a) cs[a] = lds_f32(ts + 4 * (T_CS + row0 + 8 * a + (lane >> 2)));
+  }
+};
+// below the diagonal; rf: exp(cs_i - cs_r) of the rows
+__device__ __forceinline__ void decay_off8(float (&v)[8], const float (&rf)[4], uint32_t ts, int c0, int lane) {
+  const float2 f = lds_v2f32(ts + 4 * (T_CF + c0 + 2 * (lane & 3)));
 #pragma unroll
-    for (int k = 0; k < 8; k += 2) {
-      v[k] = __uint_as_float(raw[j8 + k]); v[k + 1] = __uint_as_float(raw[j8 + k + 1]);
-      mul2(v[k], v[k + 1], f[k], f[k + 1]);
-      mul2(v[k], v[k + 1], rf, rf);
-    }
-    st_shared_v4(dst + (j8 >> 3) * 2048, pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
+  for (int a = 0; a < 4; ++a) {
+    mul2(v[2 * a], v[2 * a + 1], f.x, f.y);
+    mul2(v[2 * a], v[2 * a + 1], rf[a], rf[a]);
   }
 }
-// 16 columns (starting at column c0) of the diagonal block: two independent 8-column walks; `ts` = shared-memory address
-// of the head's table
-__device__ __forceinline__ void decay_diag_half(const uint32_t (&raw)[16], uint32_t ts, int c0, int row, float csi, uint32_t dst) {
+// group g of the diagonal block: rows 8 a + t/4 with a < g lie above it
+__device__ __forceinline__ void decay_diag8(float (&v)[8], const DecayRows& r, uint32_t ts, int c0, int g, int lane) {
+  const float2 c = lds_v2f32(ts + 4 * (T_CS + c0 + 2 * (lane & 3))), t = lds_v2f32(ts + 4 * (T_DT + c0 + 2 * (lane & 3)));
 #pragma unroll
-  for (int s = 0; s < 2; ++s) {
-    const int cs0 = c0 + 8 * s, je = cs0 + 7;
-    const float4 d0 = lds_v4f32(ts + 4 * (T_DS + cs0)), d1 = lds_v4f32(ts + 4 * (T_DS + cs0 + 4));
-    const float4 t0 = lds_v4f32(ts + 4 * (T_DT + cs0)), t1 = lds_v4f32(ts + 4 * (T_DT + cs0 + 4));
-    const float ds[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};   // ds[k] = decay of step cs0+k+1
-    float v[8] = {t0.x, t0.y, t0.z, t0.w, t1.x, t1.y, t1.z, t1.w}, run[8];
-    run[7] = (row >= je) ? ex2(csi - lds_f32(ts + 4 * (T_CS + je))) : 0.f;
-#pragma unroll
-    for (int k = 6; k >= 0; --k) run[k] = (cs0 + k == row) ? 1.f : run[k + 1] * ds[k];
-#pragma unroll
-    for (int k = 0; k < 8; k += 2) {
-      mul2(v[k], v[k + 1], run[k], run[k + 1]);
-      mul2(v[k], v[k + 1], __uint_as_float(raw[8 * s + k]), __uint_as_float(raw[8 * s + k + 1]));
-    }
-    st_shared_v4(dst + s * 2048, pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
+  for (int a = 0; a < 4; ++a) {
+    if (a < g) { v[2 * a] = v[2 * a + 1] = 0.f; continue; }
+    const int d = 8 * (a - g) + (lane >> 2) - 2 * (lane & 3);   // row - column of the left element
+    float f0 = d >= 0 ? ex2(r.cs[a] - c.x) : 0.f, f1 = d >= 1 ? ex2(r.cs[a] - c.y) : 0.f;
+    mul2(f0, f1, t.x, t.y);
+    mul2(v[2 * a], v[2 * a + 1], f0, f1);
   }
+}
+__device__ __forceinline__ void store8(const float (&v)[8], uint32_t addr) {   // addr: this lane's row of the group's 32 rows
+  st_matrix_x4(addr, pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
+}
+
+// 16 columns of a block in fragment layout: registers 0-7 hold rows 0-15, 8-15 rows 16-31
+__device__ __forceinline__ void tmem_ld_half_issue(uint32_t taddr, uint32_t (&r)[16]) {
+  tmem_ld_frag16_issue(taddr, r);
+  tmem_ld_frag16_issue(tmem_addr(taddr, 16, 0), r + 8);
+}
+__device__ __forceinline__ void half_group(const uint32_t (&raw)[16], int k, float (&v)[8]) {   // its k-th group of eight columns
+#pragma unroll
+  for (int e = 0; e < 4; ++e) { v[e] = __uint_as_float(raw[4 * k + e]); v[4 + e] = __uint_as_float(raw[8 + 4 * k + e]); }
 }
 // rb: block row of the warp (warp-uniform); tm_row: TMEM address of (first lane of this warp's quarter, first
 // source column); mrow: shared-memory address of this row's first 16 bytes in the plain 128x128 bf16 tile.
@@ -217,24 +228,33 @@ __device__ __forceinline__ void decay_diag_half(const uint32_t (&raw)[16], uint3
 // shared-memory pipe.
 __device__ __forceinline__ void decay_row(int rb, uint32_t tm_row, const float* __restrict__ tab, int row, uint32_t mrow) {
   const uint32_t ts = smem_u32(tab);
-  const float csi = lds_f32(ts + 4 * (T_CS + row));
+  const int lane = row & 31;
   uint32_t a[16], b[16];
-  tmem_ld16_issue(tm_row, a);
-  tmem_ld16_issue(tm_row + 16, b);
+  tmem_ld_half_issue(tm_row, a);
+  tmem_ld_half_issue(tm_row + 16, b);
+  DecayRows r;
+  r.load(ts, rb * 32, lane);
+  float v[8];
 #pragma unroll 1
   for (int cb = 0; cb < rb; ++cb) {
-    const float rf = ex2(csi - lds_f32(ts + 4 * (T_CS + cb * 32 + 31)));
-    const uint32_t cf = ts + 4 * (T_CF + cb * 32);
+    const float ref = lds_f32(ts + 4 * (T_CS + cb * 32 + 31));
+    const float rf[4] = {ex2(r.cs[0] - ref), ex2(r.cs[1] - ref), ex2(r.cs[2] - ref), ex2(r.cs[3] - ref)};
     const uint32_t dst = mrow + cb * 4 * 2048;
     tmem_ld_wait_2x16(a, b);
-    decay_off_half(a, rf, cf, dst);
-    tmem_ld16_issue(tm_row + (cb + 1) * 32, a);
-    decay_off_half(b, rf, cf + 64, dst + 2 * 2048);
-    tmem_ld16_issue(tm_row + (cb + 1) * 32 + 16, b);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) { half_group(a, k, v); decay_off8(v, rf, ts, cb * 32 + 8 * k, lane); store8(v, dst + k * 2048); }
+    tmem_ld_half_issue(tm_row + (cb + 1) * 32, a);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) { half_group(b, k, v); decay_off8(v, rf, ts, cb * 32 + 16 + 8 * k, lane); store8(v, dst + (2 + k) * 2048); }
+    tmem_ld_half_issue(tm_row + (cb + 1) * 32 + 16, b);
   }
   tmem_ld_wait_2x16(a, b);
-  decay_diag_half(a, ts, rb * 32, row, csi, mrow + rb * 4 * 2048);
-  decay_diag_half(b, ts, rb * 32 + 16, row, csi, mrow + rb * 4 * 2048 + 2 * 2048);
+#pragma unroll
+  for (int g = 0; g < 4; ++g) {
+    if (g < 2) half_group(a, g, v); else half_group(b, g - 2, v);
+    decay_diag8(v, r, ts, rb * 32 + 8 * g, g, lane);
+    store8(v, mrow + (rb * 4 + g) * 2048);
+  }
 }
 
 // Variant used by the one-tile-per-CTA kernels (all 16 warps meet at a CTA barrier per head anyway):
@@ -1778,47 +1798,41 @@ constexpr int WS_SCALE_WARPS = 16, WS_EPI_WARPS = 8;
 template <int P, int MODE, int N_ = 64, bool GATED_ = false>
 struct WsCfg {
   static constexpr int N = N_, HB = 64 / P, NB64 = N_ / 64;
-  // dstate 128: the C and B tiles are 32 KB each, so there is ONE C/B slot (and one G), and the state boxes of a head
-  // block live in a buffer of their own whose MMA is issued first in the block (it does not depend on M_h)
+  // The tile that the whole walk over the heads needs ("keep": C; dx: B) and the one that only G reads ("other").  dstate 64: two
+  // keep tiles and two G, one other tile, so that the next tile's G is formed during this tile.  dstate 128: the tiles are 32 KB
+  // each, one of either and one G.
   static constexpr bool SPLIT = N_ == 128;
-  static constexpr int NCBS = SPLIT ? 1 : 2;                          // C/B slots = G buffers
-  static constexpr int NBOX = (MODE == 0) ? 1 : 2;
-  // gated forward: the gate's box arrives by TMA beside the x box (a thread-per-row read of it from global memory costs one
-  // L1 wavefront per lane and instruction); its 2 x 16 KB take the place of the third M_h slot
-  static constexpr int ZB = (GATED_ && MODE == 0) ? 1 : 0;
+  static constexpr int NCBS = SPLIT ? 1 : 2;                          // keep slots = G buffers
+  // Boxes of a head block.  A: the operand of its products, over which the epilogue writes the output block (x; dx: dy).  E: what
+  // only the epilogue reads (gated forward: the gate; recompute: dy; dx: x); a thread-per-row read of it from global memory
+  // costs one L1 wavefront per lane and instruction.
+  static constexpr bool E = MODE != 0 || GATED_;
   // M_h ring depth = decay groups.  A wait by parity is only right for a waiter that is at most one phase behind.  Slot
   // kh % NM always belongs to decay group kh % NM.  On the issuing side, with two heads per block lane hl issues head hl of
   // every block: with two slots a slot then always meets the same lane; with three it alternates between the lanes, and
   // HEAD_ORDER (below) is what keeps the second lane from reaching a slot before the first lane's head has been written.
-  static constexpr int NM = (MODE == 0 && !ZB) ? 3 : 2;
-  static constexpr int CB_BYTES = 2 * NB64 * BOX_BYTES;              // keep + other tile
-  static constexpr int ST_BYTES = NB64 * SBOX_BYTES;                 // state boxes of one head block
-  static constexpr int ZOFF = NBOX * BOX_BYTES + (SPLIT ? 0 : ST_BYTES);       // the gate's box comes last in a slot
-  static constexpr int IN_BYTES = ZOFF + ZB * BOX_BYTES;                       // x [, dy] box [+ state box] [+ z box]
-  // Input slots.  A slot is held from the request of its boxes until its output block has been read by the tile store (about 4 us
-  // against 2 us of work per block), so two of them leave the issuers waiting for boxes.  dstate 128: the tile that only G reads
-  // (32 KB) is free from the tile's G until the next tile's; it holds further slots meanwhile.  The last two blocks of a tile
-  // use the first two slots, so that those are drained when the next tile's C and B are requested.
-  // dstate 128, the state boxes: a ring of 8 KB pieces (64 state columns each).  One buffer for a block's 16 KB was a chain of load,
-  // product, load that took as long as a block.  Three pieces of their own, or (forward without a gate, where three M_h tiles
-  // leave room for two) two more in the tile that only G reads.  (Two heads per block: the tables leave room for two.)
-  static constexpr int NSP = !SPLIT ? 0 : (NM == 3 ? 4 : HB == 1 ? 3 : 2), NSP_OWN = NSP == 4 ? 2 : NSP;
-  static constexpr int NX = SPLIT && MODE != 1 ? 2 + (NB64 * BOX_BYTES - (NSP - NSP_OWN) * SBOX_BYTES) / IN_BYTES : 2;
-  // slot of piece j of a block; q counts the pieces before it
-  static __device__ __forceinline__ int piece(int blk, int nblk, int j, int q) {
-    return NSP == 4 ? (((blk & 1) && nblk - blk > 1) ? 2 : 0) + j : q % (NSP ? NSP : 1);
-  }
-  static __device__ __forceinline__ int slot(int blk, int nblk) { return (NX == 2 || nblk - blk <= 2) ? (blk & 1) : blk % NX; }
-  // table ring depth (one 2 KB table per head): a multiple of the number of decay groups, so that a slot is always read by
+  static constexpr int NM = E ? 2 : 3;
+  static constexpr int TILE_BYTES = NB64 * BOX_BYTES;                // a C or B tile
+  static constexpr int CB_BYTES = (NCBS + 1) * TILE_BYTES;           // keep tiles, other tile
+  // Rings.  An A slot is held from the request of its box until its output block has been read by the tile store: about 4 us against
+  // 2 us of work per block, so with two of them the issuers wait for boxes.  Three; dstate 128: two, and two more in the other tile
+  // from the tile's G until the next tile's (the last two blocks of a tile use the first two slots, so that those are drained
+  // when the next tile's C and B are requested).  An E slot is given back by the epilogue: two.
+  // The state boxes pass as 8 KB pieces (64 state columns each); one buffer for a block was a chain of load, product, load that
+  // took as long as a block.
+  static constexpr int NA = SPLIT ? 4 : 3, NA_OWN = SPLIT ? 2 : 3, NE = E ? 2 : 0, NSP = SPLIT && !(HB == 2 && NM == 2) ? 3 : 2;
+  static __device__ __forceinline__ int a_slot(int kb, int blk, int nblk) { return !SPLIT ? kb % NA : nblk - blk <= 2 ? (blk & 1) : blk % NA; }
+  // table ring depth (the first 1.5 KB of a head's table: all but T_DS): a multiple of the number of decay groups, so that a slot is always read by
   // the same group.  With a depth of 4 and three groups the slot of head 5 had last been head 1's, read by another group:
   // the group of head 5, coming from head 2, could reach the slot's barrier before head 1's table had landed, pass the wait
   // on the parity of a phase that had not even begun, and read the slot while head 5's table was still arriving (rows 0-31
   // of that head wrong about once in 10^4 CTAs).
+  static constexpr int TBL_BYTES = T_DS * 4;
   static constexpr int NTH = (NM == 3) ? 6 : 4 * HB;
   static_assert(NTH % NM == 0 && NTH % HB == 0 && NTH <= 8, "a table slot must belong to one decay group and one column half");
   static constexpr int RED_BYTES = (P == 64 && MODE != 0) ? 2 * 128 * 4 : 0;
-  static constexpr size_t SMEM = 1024 + NCBS * CB_BYTES + NM * 2 * BOX_BYTES + 2 * IN_BYTES + NSP_OWN * SBOX_BYTES +
-                                 NTH * TAB_BYTES + RED_BYTES;
+  static constexpr size_t SMEM = 1024 + CB_BYTES + NM * 2 * BOX_BYTES + (NA_OWN + NE) * BOX_BYTES + NSP * SBOX_BYTES + NTH * TBL_BYTES +
+                                 RED_BYTES;
   static_assert(SMEM <= 232448 - 512, "shared-memory plan exceeds the 227 KB a CTA can have");
   // warp roles: NM groups of four decay warps, then two MMA issuer warps (one per head of a head block) on the two
   // least loaded schedulers, the producer warp and an idle warp, then 8 epilogue warps
@@ -1841,7 +1855,7 @@ struct WsCfg {
 };
 
 struct WsBars {
-  uint64_t cb_full[2], cb_empty[2], g_full[2], g_empty[2], in_full[4], in_empty[4], acc_full[2], acc_empty[2];
+  uint64_t cb_full[2], cb_empty[2], ot_full, ot_empty, g_full[2], g_empty[2], a_full[4], a_empty[4], e_full[2], e_empty[2], acc_full[2], acc_empty[2];
   uint64_t m_full[3], m_empty[3], tab_full[8], tab_empty[8], st_full[4], st_empty[4], out_ready[4], hz[4], done;
 };
 
@@ -1855,21 +1869,23 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
           bf16* __restrict__ dx, float* __restrict__ rs0, float* __restrict__ rs1, int* __restrict__ status) {
   using Cfg = WsCfg<P, MODE, N_, GATED>;
   const bf16* __restrict__ z = GATED ? z_ : nullptr;     // the ungated instantiation carries none of the gate's registers
-  constexpr bool ZSMEM = Cfg::ZB != 0;                    // forward: the gate's box is in the input slot
+  constexpr bool ZSMEM = GATED && MODE == 0;              // forward: the gate's box is in the E ring
   // Forward and dx: the output block (128 rows x 64 columns bf16) has the shape and layout of the x (dy) box the epilogue
   // reads, so the epilogue writes it over that box and a spare lane sends it out as ONE TMA tile store.  A row-per-thread
   // global store costs one L1 wavefront per lane and instruction, and the L1 data stage is what these kernels share.
   constexpr bool TSTORE = MODE != 1;
-  constexpr int N = Cfg::N, HB = Cfg::HB, NBOX = Cfg::NBOX, NM = Cfg::NM, NTH = Cfg::NTH, NB64 = Cfg::NB64, NCBS = Cfg::NCBS;
+  constexpr int N = Cfg::N, HB = Cfg::HB, NM = Cfg::NM, NTH = Cfg::NTH, NB64 = Cfg::NB64, NCBS = Cfg::NCBS, NSP = Cfg::NSP;
   constexpr bool SPLIT = Cfg::SPLIT;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);   // 1 KB aligned, still known to be shared memory
-  uint8_t* sCB = smem;                                   // NCBS x {keep tile, other tile}
-  uint8_t* sM = sCB + NCBS * Cfg::CB_BYTES;              // NM x 32 KB
-  uint8_t* sIn = sM + NM * 2 * BOX_BYTES;                // 2 x {x [, dy] [, state box]}
-  uint8_t* sSt = sIn + 2 * Cfg::IN_BYTES;                // dstate 128: state pieces
-  uint8_t* sTab = sSt + Cfg::NSP_OWN * SBOX_BYTES;       // NTH x decay table of one head (they run further ahead)
-  float* sRed = (float*)(sTab + NTH * TAB_BYTES);          // [2][128] (P = 64 row-sum exchange)
+  uint8_t* sCB = smem;                                   // NCBS keep tiles, then the other tile
+  uint8_t* sOther = sCB + NCBS * Cfg::TILE_BYTES;
+  uint8_t* sM = sCB + Cfg::CB_BYTES;                     // NM x 32 KB
+  uint8_t* sA = sM + NM * 2 * BOX_BYTES;                 // NA_OWN x A box
+  uint8_t* sE = sA + Cfg::NA_OWN * BOX_BYTES;            // NE x E box
+  uint8_t* sSt = sE + Cfg::NE * BOX_BYTES;               // state pieces
+  uint8_t* sTab = sSt + NSP * SBOX_BYTES;                // NTH x decay table of one head (they run further ahead)
+  float* sRed = (float*)(sTab + NTH * Cfg::TBL_BYTES);          // [2][128] (P = 64 row-sum exchange)
   __shared__ __align__(8) WsBars bars;
   __shared__ uint32_t tmem_slot;
   __shared__ int s_abort;
@@ -1881,10 +1897,12 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
       mbar_init(&bars.g_full[i], 1); mbar_init(&bars.g_empty[i], Cfg::DW);
       mbar_init(&bars.acc_full[i], Cfg::NI); mbar_init(&bars.acc_empty[i], WS_EPI_WARPS);
     }
-    for (int i = 0; i < Cfg::NX; ++i) {
-      mbar_init(&bars.in_full[i], 1); mbar_init(&bars.in_empty[i], Cfg::NI + (TSTORE ? 1 : WS_EPI_WARPS));
+    for (int i = 0; i < 4; ++i) {
+      mbar_init(&bars.a_full[i], 1); mbar_init(&bars.a_empty[i], TSTORE ? 1 : WS_EPI_WARPS);   // the epilogue is behind the block's products
       mbar_init(&bars.out_ready[i], WS_EPI_WARPS);
     }
+    for (int i = 0; i < 2; ++i) { mbar_init(&bars.e_full[i], 1); mbar_init(&bars.e_empty[i], WS_EPI_WARPS); }
+    mbar_init(&bars.ot_full, 1); mbar_init(&bars.ot_empty, 1);
     for (int i = 0; i < 3; ++i) { mbar_init(&bars.m_full[i], 4); mbar_init(&bars.m_empty[i], 1); }
     // a head's table is read by the warps of its decay group and by the epilogue warps of its columns
     for (int i = 0; i < NTH; ++i) { mbar_init(&bars.tab_full[i], 1); mbar_init(&bars.tab_empty[i], 4 + WS_EPI_WARPS / HB); }
@@ -1921,10 +1939,8 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
     b = r / g.G;
   };
 
-  constexpr int NPX = Cfg::NX - 2, NSP = Cfg::NSP, NSP_OWN = Cfg::NSP_OWN;
-  auto st_piece = [&](int s_) { return s_ < NSP_OWN ? sSt + s_ * SBOX_BYTES : sCB + NB64 * BOX_BYTES + NPX * Cfg::IN_BYTES + (s_ - NSP_OWN) * SBOX_BYTES; };
-  // input slot s; uses: bit s of a role's `used` counts the uses of slot s that it has seen, modulo 2
-  auto in_slot = [&](int s_) { return s_ < 2 ? sIn + s_ * Cfg::IN_BYTES : sCB + NB64 * BOX_BYTES + (s_ - 2) * Cfg::IN_BYTES; };
+  auto a_box = [&](int s_) { return s_ < Cfg::NA_OWN ? sA + s_ * BOX_BYTES : sOther + (s_ - Cfg::NA_OWN) * BOX_BYTES; };
+  // `used` of a role: bit s counts the uses of A slot s that it has seen, modulo 2
 
   if (warp >= Cfg::DW && warp < Cfg::W_EPI) reg_dec<Cfg::R_SPECIAL>();
   if (warp == Cfg::W_PROD) {
@@ -1935,13 +1951,15 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         tile_coords(t, b, grp, c);
         const int cs_ = t % NCBS;
         w.wait(&bars.cb_empty[cs_], ((t / NCBS) & 1) ^ 1, 41);
-        uint8_t* keep = sCB + cs_ * Cfg::CB_BYTES;
-        mbar_expect_tx(&bars.cb_full[cs_], Cfg::CB_BYTES);
+        mbar_expect_tx(&bars.cb_full[cs_], Cfg::TILE_BYTES);
 #pragma unroll
-        for (int j = 0; j < NB64; ++j) {
-          tma_load_3d(keep + j * BOX_BYTES, (MODE == 2) ? &tmB : &tmC, grp / g.hsplit * N + 64 * j, c * QT, b, &bars.cb_full[cs_]);
-          tma_load_3d(keep + (NB64 + j) * BOX_BYTES, (MODE == 2) ? &tmC : &tmB, grp / g.hsplit * N + 64 * j, c * QT, b, &bars.cb_full[cs_]);
-        }
+        for (int j = 0; j < NB64; ++j)
+          tma_load_3d(sCB + cs_ * Cfg::TILE_BYTES + j * BOX_BYTES, (MODE == 2) ? &tmB : &tmC, grp / g.hsplit * N + 64 * j, c * QT, b, &bars.cb_full[cs_]);
+        w.wait(&bars.ot_empty, (t & 1) ^ 1, 66);
+        mbar_expect_tx(&bars.ot_full, Cfg::TILE_BYTES);
+#pragma unroll
+        for (int j = 0; j < NB64; ++j)
+          tma_load_3d(sOther + j * BOX_BYTES, (MODE == 2) ? &tmC : &tmB, grp / g.hsplit * N + 64 * j, c * QT, b, &bars.ot_full);
       };
       const int total_blocks = my_tiles * nblk;
       auto load_tab = [&](int kg) {        // tables of the heads of global block kg: they run two blocks ahead of the boxes
@@ -1952,12 +1970,12 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         for (int hl = 0; hl < HB; ++hl) {
           const int kh = kg * HB + hl, ts = kh % NTH;
           w.wait(&bars.tab_empty[ts], ((kh / NTH) & 1) ^ 1, 49);
-          mbar_expect_tx(&bars.tab_full[ts], TAB_BYTES);
-          bulk_load(sTab + ts * TAB_BYTES, tab + ((size_t)(b * g.nc + c) * g.H + h0 + hl) * TAB, TAB_BYTES, &bars.tab_full[ts]);
+          mbar_expect_tx(&bars.tab_full[ts], Cfg::TBL_BYTES);
+          bulk_load(sTab + ts * Cfg::TBL_BYTES, tab + ((size_t)(b * g.nc + c) * g.H + h0 + hl) * TAB, Cfg::TBL_BYTES, &bars.tab_full[ts]);
         }
       };
       int kb = 0, sq = 0;
-      uint32_t used = 0, sused = 0;
+      uint32_t used = 0;
       load_cb(0);
       load_tab(0);
       load_tab(1);
@@ -1965,43 +1983,38 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         int b, grp, c;
         tile_coords(t, b, grp, c);
         for (int blk = 0; blk < nblk; ++blk, ++kb) {
-          const int ib = Cfg::slot(blk, nblk);
-          if (NPX > 0 && blk == 2 && ib == 2) w.wait(&bars.g_full[0], t & 1, 66);   // G has read the tile these slots share
-          w.wait(&bars.in_empty[ib], ((used >> ib) & 1) ^ 1, 42);
+          const int ib = Cfg::a_slot(kb, blk, nblk);
+          if (SPLIT && blk == 2 && ib == 2) w.wait(&bars.g_full[0], t & 1, 68);   // G has read the tile these slots share
+          w.wait(&bars.a_empty[ib], ((used >> ib) & 1) ^ 1, 42);
           used ^= 1u << ib;
-          uint8_t* dst = in_slot(ib);
           const int h0 = grp * g.hpg + blk * HB;
           const int col = grp * g.hpg * P + blk * 64;
-          mbar_expect_tx(&bars.in_full[ib], Cfg::IN_BYTES);
-          tma_load_3d(dst, &tmX, col, c * QT, b, &bars.in_full[ib]);
-          if (NBOX == 2) tma_load_3d(dst + BOX_BYTES, &tmDY, col, c * QT, b, &bars.in_full[ib]);
-          if (ZSMEM) tma_load_3d(dst + Cfg::ZOFF, &tmZ, col, c * QT, b, &bars.in_full[ib]);
-          if constexpr (!SPLIT) tma_load_3d(dst + NBOX * BOX_BYTES, &tmS, 0, h0 * P, b * g.nc + c, &bars.in_full[ib]);
+          mbar_expect_tx(&bars.a_full[ib], BOX_BYTES);
+          tma_load_3d(a_box(ib), (MODE == 2) ? &tmDY : &tmX, col, c * QT, b, &bars.a_full[ib]);
+#pragma unroll
+          for (int j = 0; j < NB64; ++j, ++sq) {
+            const int sp = sq % NSP;
+            w.wait(&bars.st_empty[sp], ((sq / NSP) & 1) ^ 1, 57);
+            mbar_expect_tx(&bars.st_full[sp], SBOX_BYTES);
+            tma_load_3d(sSt + sp * SBOX_BYTES, &tmS, 64 * j, h0 * P, b * g.nc + c, &bars.st_full[sp]);
+          }
+          if constexpr (Cfg::E) {
+            const int eb = kb & 1;
+            w.wait(&bars.e_empty[eb], ((kb >> 1) & 1) ^ 1, 50);
+            mbar_expect_tx(&bars.e_full[eb], BOX_BYTES);
+            tma_load_3d(sE + eb * BOX_BYTES, MODE == 0 ? &tmZ : MODE == 1 ? &tmDY : &tmX, col, c * QT, b, &bars.e_full[eb]);
+          }
           // tables two blocks ahead, behind this block's boxes: with a ring of three blocks of tables the slot's previous
           // readers (block kb - 1) start only when the box slot of block kb - 2 comes free, and the boxes must not wait for them
           load_tab(kb + 2);
-          if constexpr (!SPLIT) {
-            // the next tile's C/B go out right behind this tile's first block, so the MMA warp can form
-            // the next G while this tile is still being worked on
-            if (blk == 0 && t + 1 < my_tiles) load_cb(t + 1);
-          } else {
-#pragma unroll
-            for (int j = 0; j < NB64; ++j, ++sq) {
-              const int sp = Cfg::piece(blk, nblk, j, sq);
-              if (NSP > NSP_OWN && blk == 1 && sp == NSP_OWN) w.wait(&bars.g_full[0], t & 1, 68);
-              w.wait(&bars.st_empty[sp], ((sused >> sp) & 1) ^ 1, 57);
-              sused ^= 1u << sp;
-              mbar_expect_tx(&bars.st_full[sp], SBOX_BYTES);
-              tma_load_3d(st_piece(sp), &tmS, 64 * j, h0 * P, b * g.nc + c, &bars.st_full[sp]);
-            }
-          }
+          // the next tile's C/B go out right behind this tile's first block, so the MMA warp can form
+          // the next G while this tile is still being worked on
+          if (!SPLIT && blk == 0 && t + 1 < my_tiles) load_cb(t + 1);
         }
-        // one C/B slot: the next tile's C/B can only follow this tile's last block
+        // one keep tile: the next tile's C/B can only follow this tile's last block
         if (SPLIT && t + 1 < my_tiles) {
 #pragma unroll
-          for (int s_ = 2; s_ < Cfg::NX; ++s_) w.wait(&bars.in_empty[s_], ((used >> s_) & 1) ^ 1, 67);
-#pragma unroll
-          for (int s_ = NSP_OWN; s_ < NSP; ++s_) w.wait(&bars.st_empty[s_], ((sused >> s_) & 1) ^ 1, 69);
+          for (int s_ = Cfg::NA_OWN; s_ < Cfg::NA; ++s_) w.wait(&bars.a_empty[s_], ((used >> s_) & 1) ^ 1, 67);
           load_cb(t + 1);
         }
       }
@@ -2017,9 +2030,9 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
       constexpr uint32_t M_STEP = (MODE == 2) ? 256 : 4096;
       auto issue_g = [&](int t) {
         const int s_ = t % NCBS;
-        w.wait(&bars.cb_full[s_], (t / NCBS) & 1, 43); w.wait(&bars.g_empty[s_], ((t / NCBS) & 1) ^ 1, 44);
+        w.wait(&bars.cb_full[s_], (t / NCBS) & 1, 43); w.wait(&bars.ot_full, t & 1, 44); w.wait(&bars.g_empty[s_], ((t / NCBS) & 1) ^ 1, 44);
         tc_fence_after();
-        const uint32_t keep = smem_u32(sCB + s_ * Cfg::CB_BYTES), other = keep + NB64 * BOX_BYTES;
+        const uint32_t keep = smem_u32(sCB + s_ * Cfg::TILE_BYTES), other = smem_u32(sOther);
 #pragma unroll 1
         for (int j = 0; j < NB64; ++j) {
           const uint64_t dc = desc_sw128_k(((MODE == 2) ? other : keep) + j * BOX_BYTES, 0),
@@ -2027,37 +2040,34 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
 #pragma unroll 1
           for (int ks = 0; ks < 4; ++ks) mma_bf16(tm + s_ * 128, desc_adv(dc, ks * 32), desc_adv(db, ks * 32), idG, (j | ks) > 0);
         }
+        mma_commit(&bars.ot_empty);
         mma_commit(&bars.g_full[s_]);
       };
       if (mi == 0) issue_g(0);
       int kb = 0, kh = 0, sq = 0;
-      uint32_t used = 0, sused = 0;
+      uint32_t used = 0;
       for (int t = 0; t < my_tiles; ++t) {
-        const uint32_t keep_t = smem_u32(sCB + (t % NCBS) * Cfg::CB_BYTES);
-        const uint64_t dK0 = desc_sw128_k(keep_t, 0);
+        const uint32_t keep_t = smem_u32(sCB + (t % NCBS) * Cfg::TILE_BYTES);
         // the lane that issues the state term reads the keep tile; when that is not the lane that formed G (and waited
         // for the tile there), it has to see the tile's arrival itself: the first x box of a tile can land before its C/B
         if (mi == 1) w.wait(&bars.cb_full[t % NCBS], (t / NCBS) & 1, 64);
         for (int blk = 0; blk < nblk; ++blk, ++kb) {
-          const int ib = Cfg::slot(blk, nblk), ab = kb & 1;
-          const uint32_t inb = smem_u32(in_slot(ib));
+          const int ib = Cfg::a_slot(kb, blk, nblk), ab = kb & 1;
+          const uint32_t inb = smem_u32(a_box(ib));
           const uint32_t tmYd = tm + 256 + ab * 128, tmYo = tmYd + 64;
-          w.wait(&bars.in_full[ib], (used >> ib) & 1, 45);
+          w.wait(&bars.a_full[ib], (used >> ib) & 1, 45);
           used ^= 1u << ib;
           w.wait(&bars.acc_empty[ab], ((kb >> 1) & 1) ^ 1, 46);
-          if constexpr (SPLIT) {
-            if (mi == (Cfg::STATE_LANE ? 1 : 0)) {    // the state term first: it needs the keep tile and the state boxes, not M_h
-#pragma unroll 1
-              for (int j = 0; j < NB64; ++j, ++sq) {
-                const int sp = Cfg::piece(blk, nblk, j, sq);
-                w.wait(&bars.st_full[sp], (sused >> sp) & 1, 58);
-                sused ^= 1u << sp;
-                tc_fence_after();
-                const uint64_t dKj = desc_sw128_k(keep_t + j * BOX_BYTES, 0), dSj = desc_sw128_k(smem_u32(st_piece(sp)), 0);
-#pragma unroll 1
-                for (int ks = 0; ks < 4; ++ks) mma_bf16(tmYo, desc_adv(dKj, ks * 32), desc_adv(dSj, ks * 32), idO, (j | ks) > 0);
-                mma_commit(&bars.st_empty[sp]);
-              }
+          if (mi == Cfg::NI - 1) {    // the state term first: it needs the keep tile and the state boxes, not M_h
+#pragma unroll
+            for (int j = 0; j < NB64; ++j, ++sq) {
+              const int sp = sq % NSP;
+              w.wait(&bars.st_full[sp], (sq / NSP) & 1, 58);
+              tc_fence_after();
+              const uint64_t dKj = desc_sw128_k(keep_t + j * BOX_BYTES, 0), dSj = desc_sw128_k(smem_u32(sSt + sp * SBOX_BYTES), 0);
+#pragma unroll
+              for (int ks = 0; ks < 4; ++ks) mma_bf16(tmYo, desc_adv(dKj, ks * 32), desc_adv(dSj, ks * 32), idO, (j | ks) > 0);
+              mma_commit(&bars.st_empty[sp]);
             }
           }
           for (int hl = 0; hl < HB; ++hl, ++kh) {
@@ -2069,18 +2079,12 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
             tc_fence_after();
             const uint32_t mt = smem_u32(sM + ms * 2 * BOX_BYTES);
             const uint64_t dM0 = (MODE == 2) ? desc_plain_mn(mt, 128, 0, 0) : desc_plain_k(mt, 128, 0);
-            const uint64_t dO0 = desc_sw128_mn(inb + ((MODE == 2) ? BOX_BYTES : 0), 0, hl * P * 2, 16);
-#pragma unroll 1
+            const uint64_t dO0 = desc_sw128_mn(inb, 0, hl * P * 2, 16);
+#pragma unroll
             for (int ks = 0; ks < 8; ++ks)
               mma_bf16(tmYd + hl * P, desc_adv(dM0, ks * M_STEP), desc_adv(dO0, ks * 2048), idY, ks > 0);
-            if (!SPLIT && hl == 0) {
-              const uint64_t dS0 = desc_sw128_k(inb + NBOX * BOX_BYTES, 0);
-#pragma unroll 1
-              for (int ks = 0; ks < 4; ++ks) mma_bf16(tmYo, desc_adv(dK0, ks * 32), desc_adv(dS0, ks * 32), idO, ks > 0);
-            }
             mma_commit(&bars.m_empty[ms]);
           }
-          mma_commit(&bars.in_empty[ib]);
           if (blk == nblk - 1) mma_commit(&bars.cb_empty[t % NCBS]);
           mma_commit(&bars.acc_full[ab]);
           if (!SPLIT && mi == 0 && blk == 0 && t + 1 < my_tiles) issue_g(t + 1);
@@ -2093,18 +2097,19 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
   } else if (TSTORE && warp == Cfg::W_PROD + 1) {
     // ------------------------------------------------------------------ store lane: output blocks leave as TMA tiles
     if (lane == 0) {
+      int kb = 0;
       uint32_t used = 0;
       for (int t = 0; t < my_tiles; ++t) {
         int b, grp, c;
         tile_coords(t, b, grp, c);
-        for (int blk = 0; blk < nblk; ++blk) {
-          const int ib = Cfg::slot(blk, nblk);
+        for (int blk = 0; blk < nblk; ++blk, ++kb) {
+          const int ib = Cfg::a_slot(kb, blk, nblk);
           w.wait(&bars.out_ready[ib], (used >> ib) & 1, 59);
           used ^= 1u << ib;
-          tma_store_3d(&tmOut, in_slot(ib) + (NBOX - 1) * BOX_BYTES, grp * g.hpg * P + blk * 64, c * QT, b);
+          tma_store_3d(&tmOut, a_box(ib), grp * g.hpg * P + blk * 64, c * QT, b);
           bulk_commit();
           bulk_wait_read0();            // the box has been read: the slot may be refilled
-          mbar_arrive(&bars.in_empty[ib]);
+          mbar_arrive(&bars.a_empty[ib]);
         }
       }
       bulk_wait0();
@@ -2125,7 +2130,7 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         const int ts = kh % NTH;
         w.wait(&bars.m_empty[wg], ((kh / NM) & 1) ^ 1, 53);
         w.wait(&bars.tab_full[ts], (kh / NTH) & 1, 52);
-        decay_row(rb, tm_row, (const float*)(sTab + ts * TAB_BYTES), row, mrow);
+        decay_row(rb, tm_row, (const float*)(sTab + ts * Cfg::TBL_BYTES), row, mrow);
         fence_async_smem(); __syncwarp(); if (lane == 0) { mbar_arrive(&bars.m_full[wg]); mbar_arrive(&bars.tab_empty[ts]); }
       }
       tc_fence_before();
@@ -2165,11 +2170,11 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
       const int t_row = c * QT + row;
       for (int blk = 0; blk < nblk; ++blk, ++kb) {
         if constexpr (GATED && !ZSMEM) load_z(t, blk, zq);
-        const int ib = Cfg::slot(blk, nblk), ab = kb & 1;
-        uint8_t* xt = in_slot(ib);
-        uint8_t* dyt = xt + (NBOX - 1) * BOX_BYTES;
+        const int ib = Cfg::a_slot(kb, blk, nblk), ab = kb & 1, eb = kb & 1;
+        const uint32_t at = smem_u32(a_box(ib)), et = smem_u32(sE + eb * BOX_BYTES);
+        const uint32_t xt = MODE == 2 ? et : at, dyt = MODE == 2 ? at : et;
         const int khe = kb * HB + hl_e, ts = khe % NTH;
-        const float* tb = (const float*)(sTab + ts * TAB_BYTES);
+        const float* tb = (const float*)(sTab + ts * Cfg::TBL_BYTES);
         const uint32_t tmYd = tm + 256 + ab * 128, tmYo = tmYd + 64;
         const int h0 = grp * g.hpg + blk * HB, h_e = h0 + hl_e;
         const float Dh = D ? __ldg(D + h_e) : 0.f;
@@ -2178,8 +2183,9 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         const float cs_r = lds_f32(tbs + 4 * (T_CS + row)), dt_r = lds_f32(tbs + 4 * (T_DT + row));
         const float osc = (MODE == 2) ? dt_r * ex2(lds_f32(tbs + 4 * (T_CS + 127)) - cs_r) : ex2(cs_r);
         if (reads_done(__float_as_uint(cs_r) ^ __float_as_uint(dt_r) ^ __float_as_uint(osc), lane)) mbar_arrive(&bars.tab_empty[ts]);
-        w.wait(&bars.in_full[ib], (used >> ib) & 1, 54);
+        w.wait(&bars.a_full[ib], (used >> ib) & 1, 54);
         used ^= 1u << ib;
+        if (Cfg::E) w.wait(&bars.e_full[eb], (kb >> 1) & 1, 60);
         w.wait(&bars.acc_full[ab], (kb >> 1) & 1, 55);
         tc_fence_after();
         const long long colo = (long long)h0 * P + half * 32;
@@ -2189,12 +2195,12 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         for (int h16 = 0; h16 < 2; ++h16) {
           // pull this 16-column slice out of shared memory and TMEM; after the second slice the input
           // slot and the accumulator slot are handed back before the arithmetic and the stores
-          uint4 xv[2], dv[2];
+          uint4 xv[2], dv[2];   // dv: dy, forward: the gate
           float yd[16], yo[16];
 #pragma unroll
           for (int q = 0; q < 2; ++q) {
-            xv[q] = ld_shared_v4(smem_u32(xt) + sw128_off(row, half * 4 + h16 * 2 + q));
-            dv[q] = (MODE != 0) ? ld_shared_v4(smem_u32(dyt) + sw128_off(row, half * 4 + h16 * 2 + q)) : make_uint4(0u, 0u, 0u, 0u);
+            xv[q] = ld_shared_v4(xt + sw128_off(row, half * 4 + h16 * 2 + q));
+            dv[q] = Cfg::E ? ld_shared_v4(dyt + sw128_off(row, half * 4 + h16 * 2 + q)) : make_uint4(0u, 0u, 0u, 0u);
           }
           {   // both accumulator slices in flight, one wait (the two loads used to wait for one another)
             uint32_t rd[16], ro[16];
@@ -2206,12 +2212,13 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
           }
           if (h16 == 1) {
             tc_fence_before();
-            if (TSTORE) {
+            if (!Cfg::E) {
               __syncwarp();
               if (lane == 0) mbar_arrive(&bars.acc_empty[ab]);
             } else if (reads_done(xv[0].x ^ xv[1].x ^ dv[0].x ^ dv[1].x, lane)) {
               mbar_arrive(&bars.acc_empty[ab]);
-              mbar_arrive(&bars.in_empty[ib]);
+              mbar_arrive(&bars.e_empty[eb]);
+              if (!TSTORE) mbar_arrive(&bars.a_empty[ib]);
             }
           }
           uint4 ov[2], dpk[2];
@@ -2221,7 +2228,7 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
             unpack8(xv[q], xs);
 #pragma unroll
             for (int k = 0; k < 8; ++k) acc[k] = yd[q * 8 + k] + osc * yo[q * 8 + k];
-            if constexpr (ZSMEM) unpack8(ld_shared_v4(smem_u32(xt + Cfg::ZOFF) + sw128_off(row, half * 4 + h16 * 2 + q)), zs);
+            if constexpr (ZSMEM) unpack8(dv[q], zs);
             else if (GATED) unpack8(zq[GATED ? h16 * 2 + q : 0], zs);
             if (MODE != 0) unpack8(dv[q], dys);
             if (MODE == 0) {
@@ -2263,7 +2270,7 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
           if (TSTORE) {   // over the chunks of the x (dy) box this thread has just read
 #pragma unroll
             for (int q = 0; q < 2; ++q)
-              st_shared_v4(smem_u32(dyt) + sw128_off(row, half * 4 + h16 * 2 + q), ov[q].x, ov[q].y, ov[q].z, ov[q].w);
+              st_shared_v4(at + sw128_off(row, half * 4 + h16 * 2 + q), ov[q].x, ov[q].y, ov[q].z, ov[q].w);
           }
         }
         if (TSTORE) {
