@@ -1961,24 +1961,30 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         for (int j = 0; j < NB64; ++j)
           tma_load_3d(sOther + j * BOX_BYTES, (MODE == 2) ? &tmC : &tmB, grp / g.hsplit * N + 64 * j, c * QT, b, &bars.ot_full);
       };
-      const int total_blocks = my_tiles * nblk;
-      auto load_tab = [&](int kg) {        // tables of the heads of global block kg: they run two blocks ahead of the boxes
-        if (kg >= total_blocks) return;
-        int b, grp, c;
-        tile_coords(kg / nblk, b, grp, c);
-        const int h0 = grp * g.hpg + (kg % nblk) * HB;
-        for (int hl = 0; hl < HB; ++hl) {
-          const int kh = kg * HB + hl, ts = kh % NTH;
-          w.wait(&bars.tab_empty[ts], ((kh / NTH) & 1) ^ 1, 49);
-          mbar_expect_tx(&bars.tab_full[ts], Cfg::TBL_BYTES);
-          bulk_load(sTab + ts * Cfg::TBL_BYTES, tab + ((size_t)(b * g.nc + c) * g.H + h0 + hl) * TAB, Cfg::TBL_BYTES, &bars.tab_full[ts]);
+      // Tables of the next head block; they run two blocks ahead of the boxes.  The walk is kept, not computed: the divisions of a
+      // block index took this lane a third of a block's time.
+      int tt = 0, tblk = 0, tkh = 0;
+      const float* tsrc = nullptr;
+      auto load_tab = [&]() {
+        if (tt >= my_tiles) return;
+        if (tblk == 0) {
+          int b, grp, c;
+          tile_coords(tt, b, grp, c);
+          tsrc = tab + ((size_t)(b * g.nc + c) * g.H + grp * g.hpg) * TAB;
         }
+        for (int hl = 0; hl < HB; ++hl, ++tkh, tsrc += TAB) {
+          const int ts = tkh % NTH;
+          w.wait(&bars.tab_empty[ts], ((tkh / NTH) & 1) ^ 1, 49);
+          mbar_expect_tx(&bars.tab_full[ts], Cfg::TBL_BYTES);
+          bulk_load(sTab + ts * Cfg::TBL_BYTES, tsrc, Cfg::TBL_BYTES, &bars.tab_full[ts]);
+        }
+        if (++tblk == nblk) { tblk = 0; ++tt; }
       };
       int kb = 0, sq = 0;
       uint32_t used = 0;
       load_cb(0);
-      load_tab(0);
-      load_tab(1);
+      load_tab();
+      load_tab();
       for (int t = 0; t < my_tiles; ++t) {
         int b, grp, c;
         tile_coords(t, b, grp, c);
@@ -2006,7 +2012,7 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
           }
           // tables two blocks ahead, behind this block's boxes: with a ring of three blocks of tables the slot's previous
           // readers (block kb - 1) start only when the box slot of block kb - 2 comes free, and the boxes must not wait for them
-          load_tab(kb + 2);
+          load_tab();
           // the next tile's C/B go out right behind this tile's first block, so the MMA warp can form
           // the next G while this tile is still being worked on
           if (!SPLIT && blk == 0 && t + 1 < my_tiles) load_cb(t + 1);
@@ -2146,9 +2152,8 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
     int kb = 0;
     uint32_t used = 0;
     // gated recompute (MODE 1): the gate is the one operand the epilogue reads from global memory; this thread's 64 bytes
-    // of it are requested at the start of the block, before the waits (the forward gets the gate's box by TMA); a block ahead was
-    // no faster
-    uint4 zq[GATED ? 4 : 1] = {};
+    // of it are requested a block ahead (the forward gets the gate's box by TMA)
+    uint4 zq[GATED ? 4 : 1] = {}, zn[GATED && !ZSMEM ? 4 : 1] = {};
     auto load_z = [&](int t_, int blk_, auto& dst) {
       if constexpr (GATED) {
         if (t_ >= my_tiles) return;
@@ -2164,12 +2169,17 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         ld_global_32B(zp_ + 16, dst[2], dst[3]);
       }
     };
+    if constexpr (GATED && !ZSMEM) load_z(0, 0, zn);
     for (int t = 0; t < my_tiles; ++t) {
       int b, grp, c;
       tile_coords(t, b, grp, c);
       const int t_row = c * QT + row;
       for (int blk = 0; blk < nblk; ++blk, ++kb) {
-        if constexpr (GATED && !ZSMEM) load_z(t, blk, zq);
+        if constexpr (GATED && !ZSMEM) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) zq[q] = zn[q];
+          blk + 1 < nblk ? load_z(t, blk + 1, zn) : load_z(t + 1, 0, zn);
+        }
         const int ib = Cfg::a_slot(kb, blk, nblk), ab = kb & 1, eb = kb & 1;
         const uint32_t at = smem_u32(a_box(ib)), et = smem_u32(sE + eb * BOX_BYTES);
         const uint32_t xt = MODE == 2 ? et : at, dyt = MODE == 2 ? at : et;
@@ -2419,25 +2429,32 @@ k_bwd_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant__
           tma_load_3d(dst + (NB64 + j) * BOX_BYTES, &tmB, grp / g.hsplit * N + 64 * j, c * QT, b, &bars.cb_full[cs_]);
         }
       };
-      const int total_blocks = my_tiles * nblk;
-      auto load_tab = [&](int kg) {
-        if (kg >= total_blocks) return;
-        int b, grp, c;
-        tile_coords(kg / nblk, b, grp, c);
-        const int h0 = grp * g.hpg + (kg % nblk) * HB, ts = kg % Cfg::NT;
-        w.wait(&bars.tab_empty[ts], ((kg / Cfg::NT) & 1) ^ 1, 49);
+      int tt = 0, tblk = 0, tkb = 0;   // the next head block whose tables are requested (as in k_scan_ws)
+      const float* tsrc = nullptr;
+      auto load_tab = [&]() {
+        if (tt >= my_tiles) return;
+        if (tblk == 0) {
+          int b, grp, c;
+          tile_coords(tt, b, grp, c);
+          tsrc = tab + ((size_t)(b * g.nc + c) * g.H + grp * g.hpg) * TAB;
+        }
+        const int ts = tkb % Cfg::NT;
+        w.wait(&bars.tab_empty[ts], ((tkb / Cfg::NT) & 1) ^ 1, 49);
         mbar_expect_tx(&bars.tab_full[ts], Cfg::TB_BYTES);
-        bulk_load(sTab + ts * Cfg::TB_BYTES, tab + ((size_t)(b * g.nc + c) * g.H + h0) * TAB, Cfg::TB_BYTES, &bars.tab_full[ts]);
+        bulk_load(sTab + ts * Cfg::TB_BYTES, tsrc, Cfg::TB_BYTES, &bars.tab_full[ts]);
+        tsrc += HB * TAB;
+        ++tkb;
+        if (++tblk == nblk) { tblk = 0; ++tt; }
       };
       int kb = 0;
       load_cb(0);
-      load_tab(0);
-      load_tab(1);
+      load_tab();
+      load_tab();
       for (int t = 0; t < my_tiles; ++t) {
         int b, grp, c;
         tile_coords(t, b, grp, c);
         for (int blk = 0; blk < nblk; ++blk, ++kb) {
-          load_tab(kb + 2);
+          load_tab();
           const int ib = kb & 1;
           const int h0 = grp * g.hpg + blk * HB, col = grp * g.hpg * P + blk * 64;
           w.wait(&bars.in_empty[ib], ((kb >> 1) & 1) ^ 1, 42);
