@@ -3341,11 +3341,12 @@ int launch_state(const Geo& g, const CUtensorMap& tx, const CUtensorMap& tb, con
                  cudaStream_t s, bool sliced = false) {
   if (!g.onetile) {   // persistent, ring-fed version; `sliced`: the order k_state_fold reads, else [B,nc,H,P,N]
     // few items: a group's tiles are cut into parts, as in split_heads (2 rows of 16 chunks, 24 heads of 64 x 128: 32 blocks of 12
-    // tiles one behind the other become 128 of 3)
+    // tiles one behind the other become 128 of 3).  An item's B tile counts as half a tile: without it 2 rows of 1024 chunks were cut
+    // into single tiles for one wave in 168, and every tile loaded a B tile as large as itself (544 us; 443 with whole items).
     const int MT = g.hpg * P / 128, items = g.B * g.G * g.nc, sms = sm_count();
     int parts = 1;
     for (int n = 2; n <= MT; ++n)
-      if (MT % n == 0 && (long long)cdiv(items * n, sms) * (MT / n) < (long long)cdiv(items * parts, sms) * (MT / parts)) parts = n;
+      if (MT % n == 0 && (long long)cdiv(items * n, sms) * (2 * MT / n + 1) < (long long)cdiv(items * parts, sms) * (2 * MT / parts + 1)) parts = n;
     Geo p = g;
     p.G *= parts; p.hpg /= parts; p.hsplit = parts;
     launch<k_state_ps<P, N, MODE>>(items * parts < sms ? items * parts : sms, PsCfg<P, N>::THREADS, PsCfg<P, N>::SMEM, s, p, tx, tb, tab, out,
