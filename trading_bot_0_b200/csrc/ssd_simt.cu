@@ -816,7 +816,8 @@ __global__ void __launch_bounds__(ST) k_sdot(Geo g, const float* __restrict__ dS
 // 32-column strip of the chunk (strips; only those up to the position's own hold anything), one per 32 state columns, and one
 // part of ddtd per 32 features, `stride` elements apart.
 struct DdtParts { int strips, columns, features; size_t stride; };
-// HG heads at a time: 8 fill the sectors of a [B,L,H] row; 2 give a short batch four times the blocks (its time is one chain
+// HG heads at a time: 4 keep the registers low enough for a full SM (16 x 4096 tokens of 24 heads 19.5 us with 8, 13.7 with 4, and
+// k_cumsum 14.0, 9.7; 512 x 1024 of 8 heads the same); 2 give a short batch twice the blocks (its time is one chain
 // of loads and scans).  PARTS: the CUDA-core family's partial sums (their loops cost the other family 30 of 60 us at 512 x
 // 1024 tokens of 8 heads).  The two sums over the chunk fold 2 HG values across the warp together: 16 shuffles instead of 80.
 template <int HG, bool PARTS>
@@ -1022,10 +1023,10 @@ static int fwd_stages_t(const Geo& g, bool tc, const SsdFwdPtrs& p, char* ws, co
   if (stages & (SSD_STAGE_LOCAL | SSD_STAGE_LOCAL_STATES)) {
     const bool wide = (long long)g.nc * g.B >= 2LL * sm_count();
     auto cumsum = [&](auto kernel) {
-      launch<kernel.value>(dim3(g.nc, g.B, wide ? 1 : cdiv(g.H, 2)), g.Q <= 128 ? 128 : 256, 0, s, g, (const T*)p.dt, p.dt_bias, p.A, cs, dtf,
+      launch<kernel.value>(dim3(g.nc, g.B, wide ? cdiv(g.H, 4) : cdiv(g.H, 2)), g.Q <= 128 ? 128 : 256, 0, s, g, (const T*)p.dt, p.dt_bias, p.A, cs, dtf,
                            tc ? tab : nullptr, tc ? (int*)(ws + w.hand) : nullptr, status);
     };
-    wide ? cumsum(Fn<k_cumsum<T, 8>>()) : cumsum(Fn<k_cumsum<T, 2>>());
+    wide ? cumsum(Fn<k_cumsum<T, 4>>()) : cumsum(Fn<k_cumsum<T, 2>>());
     SSD_CUDA_CHECK_LAUNCH("cumsum");
     if (tc && fused) {
       // chunk states and the scan over chunks run as one kernel in the FINISH stage
@@ -1191,13 +1192,13 @@ static int bwd_stages_t(const Geo& g, bool tc, const SsdBwdPtrs& p, char* ws, co
     }
     const DdtParts parts = tc ? DdtParts{1, 0, 1, 0} : DdtParts{n.strips, cdiv(g.N, TN), cdiv(g.P, TN), n.nq};
     float* dbpart = p.ddt_bias ? (float*)(ws + w.dbpart) : nullptr;
-    const bool wide = (long long)g.nc * g.B >= 2LL * sm_count();   // eight heads per block fill the SMs twice
+    const bool wide = (long long)g.nc * g.B >= 2LL * sm_count();   // four heads per block fill the SMs twice
     auto ddt = [&](auto kernel) {
-      launch<kernel.value>(dim3(g.nc, g.B, wide ? 1 : cdiv(g.H, 2)), g.Q <= 128 ? 128 : 256, 0, s, g, p.A, dtf, parts, dcsp, ddtd, ddot, sdot,
+      launch<kernel.value>(dim3(g.nc, g.B, wide ? cdiv(g.H, 4) : cdiv(g.H, 2)), g.Q <= 128 ? 128 : 256, 0, s, g, p.A, dtf, parts, dcsp, ddtd, ddot, sdot,
                            sdot_nw, p.ddt, dapart, ddpart, dbpart);
     };
-    if (tc) wide ? ddt(Fn<k_ddt<8, false>>()) : ddt(Fn<k_ddt<2, false>>());
-    else wide ? ddt(Fn<k_ddt<8, true>>()) : ddt(Fn<k_ddt<2, true>>());
+    if (tc) wide ? ddt(Fn<k_ddt<4, false>>()) : ddt(Fn<k_ddt<2, false>>());
+    else wide ? ddt(Fn<k_ddt<4, true>>()) : ddt(Fn<k_ddt<2, true>>());
     SSD_CUDA_CHECK_LAUNCH("ddt");
     launch<k_reduce_heads>(g.H, RH_THREADS, 0, s, g.B * g.nc, g.H, dapart, ddpart, dbpart, p.dA, p.dD, p.ddt_bias);
     SSD_CUDA_CHECK_LAUNCH("reduce_heads");
