@@ -68,6 +68,23 @@ def test_fp32_groups_and_odd_dims(lib):
     run_case(cfg, with_init=True, with_dfinal=True)
 
 
+@pytest.mark.parametrize("chunk,seqlen", [(50, 333), (3, 40), (66, 200), (129, 300), (256, 256)])
+def test_fp32_decays_on_the_diagonal(lib, chunk, seqlen):
+    """Decays of the tiles on the diagonal are walked four columns at a time: chunk lengths that end inside a group of four, a tile or
+    a strip, with decays of several e-folds a step.  3e-6: sums of up to 256 rounded terms, an order below the parity gate."""
+    import trading_bot_0_b200 as T
+    cfg = cfg_like(0, chunk=chunk, seqlen=seqlen, batch=2)
+    inp = O.make_inputs(cfg, O.SEED, batch=2, seqlen=seqlen)
+    inp["dt"] = inp["dt"] * 8
+    ref = oracle_all(inp)
+    d = to_dev(inp, DEV)
+    a = (d["x"], d["dt"], d["A"], d["B"], d["C"], d.get("D"))
+    y, fin, ws = T.forward(*a, chunk=chunk, for_backward=True)
+    g = T.backward(d["dy"], *a, chunk=chunk, workspace=ws, fwd_saved=True)
+    for k, v in (("y", y), ("final_state", fin), ("dx", g["dx"]), ("dB", g["dB"]), ("dC", g["dC"])):
+        assert rel_err(v, ref[k]) < 3e-6, k
+
+
 def test_fp32_large_dims(lib):
     cfg = O.SsdConfig("large", 1, 512, 2, 128, 256, 1, 256, "fp32")
     run_case(cfg, with_dfinal=True)

@@ -293,6 +293,15 @@ __global__ void __launch_bounds__(256) k_cumsum(Geo g, const T* __restrict__ dt,
 }
 
 // ---------------------------------------------------------------------------------------------
+// Decays exp(cs_i - cs_j) of one row i and four columns j .. j + 3 (zero above the diagonal) from one exponential: that of the last
+// column, then leftwards by the steps st[c] = exp(dt_{j+c+1} A), restarting at 1 on the diagonal.  No exponent is positive; the
+// steps carry no rounding of the running sum, so an element is no less exact than exp(cs_i - cs_j) itself.
+// d = i - j.
+__device__ __forceinline__ void walk4(float ci, float c3, int d, const float (&st)[3], float (&o)[4]) {
+  o[3] = d >= 3 ? expf(ci - c3) : 0.f;
+#pragma unroll
+  for (int c = 2; c >= 0; --c) o[c] = d == c ? 1.f : o[c + 1] * st[c];
+}
 // Where a block stands: `u` counts tiles of a (batch, chunk, head) or (batch, chunk, group) entry, fastest first.
 struct Place { int tile, x, c, b; };   // x: head or group
 __device__ __forceinline__ Place place_of(unsigned u, int tiles, int nx, int nc) {
@@ -409,12 +418,12 @@ __global__ void __launch_bounds__(NT, 4) k_local(Geo g, unsigned n_state, const 
 //   GATE_BWD false (forward):      y = acc + D x, optional silu gate, store.
 //   GATE_BWD true (gated backward): from acc form dz and the pre-gate gradient dyp.
 template <typename T, bool GATE_BWD>
-__global__ void __launch_bounds__(NT, 4) k_chunk_scan(Geo g, const T* __restrict__ x, const T* __restrict__ Cm, const float* __restrict__ D,
-                                                      const T* __restrict__ z, const float* __restrict__ cs, const float* __restrict__ dtf,
+__global__ void __launch_bounds__(NT, 4) k_chunk_scan(Geo g, const T* __restrict__ x, const T* __restrict__ Cm, const float* __restrict__ A,
+                                                      const float* __restrict__ D, const T* __restrict__ z, const float* __restrict__ cs, const float* __restrict__ dtf,
                                                       const float* __restrict__ cb, const float* __restrict__ prev, T* __restrict__ y,
                                                       const T* __restrict__ dy, float* __restrict__ dyp, T* __restrict__ dz) {
   pdl_wait();
-  __shared__ __align__(16) float As[A_FLOATS], Bs[B_FLOATS], css[256], dts[256], fj[256];
+  __shared__ __align__(16) float As[A_FLOATS], Bs[B_FLOATS], css[256], dts[256], fj[256], stp[256];
   const int nti = (g.Q + TM - 1) / TM, ntp = (g.P + TN - 1) / TN;
   const Place q = place_of(blockIdx.x, nti * ntp, g.H, g.nc);
   // the last strip of a chunk has the most work: it starts first
@@ -427,6 +436,7 @@ __global__ void __launch_bounds__(NT, 4) k_chunk_scan(Geo g, const T* __restrict
     css[l] = c;
     dts[l] = d;
     if (l < i0) fj[l] = expf(ref - c) * d;
+    stp[l] = l + 1 < g.Q ? expf(dtf[co + l + 1] * A[h]) : 0.f;
   }
   const int pc = min(TN, g.P - p0);
   const Mat<float> M(cb + cb_idx(g, q.b, q.c, grp) + (size_t)i0 * g.Q, g.Q, min(TM, g.Q - i0), g.Q);
@@ -445,12 +455,11 @@ __global__ void __launch_bounds__(NT, 4) k_chunk_scan(Geo g, const T* __restrict
   contract<true, false>(acc, M, X, i0, min(i0 + TM, nv), As, Bs, [&](int k, int r, int c, float4 v) {
     const int i = i0 + r, j = k + c;
     if (i >= g.Q || j > i) return make_float4(0.f, 0.f, 0.f, 0.f);
-    const float ci = css[i];
-    v.x *= expf(ci - css[j]) * dts[j];
-    v.y = j + 1 <= i ? v.y * expf(ci - css[j + 1]) * dts[j + 1] : 0.f;
-    v.z = j + 2 <= i ? v.z * expf(ci - css[j + 2]) * dts[j + 2] : 0.f;
-    v.w = j + 3 <= i ? v.w * expf(ci - css[j + 3]) * dts[j + 3] : 0.f;
-    return v;
+    const float4 s4 = *reinterpret_cast<const float4*>(stp + j), d4 = *reinterpret_cast<const float4*>(dts + j);
+    const float st[3] = {s4.x, s4.y, s4.z};
+    float e[4];
+    walk4(css[i], css[min(j + 3, g.Q - 1)], i - j, st, e);
+    return make_float4(v.x * e[0] * d4.x, i - j >= 1 ? v.y * e[1] * d4.y : 0.f, i - j >= 2 ? v.z * e[2] * d4.z : 0.f, i - j >= 3 ? v.w * e[3] * d4.w : 0.f);
   }, Keep());
   float o[4][4];
   acc.get(o);
@@ -498,7 +507,7 @@ __global__ void __launch_bounds__(NT, 4) k_chunk_scan(Geo g, const T* __restrict
 // the dt / decay gradients fall out of it: dcs_i's intra-chunk part is sum_j W_h[i,j] cb[i,j] (one partial per column strip),
 // and ddot_i = dy[i,h,:] . x[i,h,:] is the undecayed diagonal.
 template <typename T, typename TD>
-__device__ __forceinline__ void w_tile(const Geo& g, unsigned u, const T* x, const TD* dy, long long dsb, long long dsl,
+__device__ __forceinline__ void w_tile(const Geo& g, unsigned u, const T* x, const TD* dy, long long dsb, long long dsl, const float* __restrict__ A,
                                        const float* __restrict__ cs, const float* __restrict__ dtf, const float* __restrict__ cb,
                                        float* __restrict__ wsum, float* __restrict__ dcs_part, float* __restrict__ ddot, float* As, float* Bs) {
   const Place q = place_of(u, tri_tiles(g.Q), g.G, g.nc);
@@ -553,18 +562,23 @@ __device__ __forceinline__ void w_tile(const Geo& g, unsigned u, const T* x, con
     float o[4][4], rs[4];
     acc.get(o);
     acc.zero();
-    float e[4], f[4];
+    float e[4], f[4], st[3];
     if (apart) {
 #pragma unroll
       for (int r = 0; r < 4; ++r) { e[r] = expf(ci[r] - ref); f[r] = expf(ref - cj[r]) * dj[r]; }
+    } else {
+#pragma unroll
+      for (int r = 0; r < 3; ++r) st[r] = expf(dj[r + 1] * A[h]);
     }
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
       rs[r] = 0.f;
+      float wk[4];
+      if (!apart) walk4(ci[r], cj[3], i + r - j, st, wk);
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         if (i + r == j + c && i + r < g.Q) ddot[co + i + r] = o[r][c];
-        const float l = apart ? e[r] * f[c] : (j + c <= i + r ? expf(ci[r] - cj[c]) * dj[c] : 0.f);
+        const float l = apart ? e[r] * f[c] : (j + c <= i + r ? wk[c] * dj[c] : 0.f);
         const float w = o[r][c] * l;
         sum[r][c] += w;
         rs[r] = fmaf(w, cbv[r][c], rs[r]);
@@ -586,27 +600,30 @@ __device__ __forceinline__ void w_tile(const Geo& g, unsigned u, const T* x, con
 // The part of a backward that needs no state gradient from other chunks, one launch: W, then the local state gradients.
 template <typename T, typename TD>
 __global__ void __launch_bounds__(NT, 4) k_bwd_local(Geo g, unsigned n_w, const T* __restrict__ x, const TD* __restrict__ dy, long long dsb,
-                                                     long long dsl, const T* __restrict__ Cm, const float* __restrict__ cs,
+                                                     long long dsl, const float* __restrict__ A, const T* __restrict__ Cm, const float* __restrict__ cs,
                                                      const float* __restrict__ dtf, const float* __restrict__ cb, float* __restrict__ wsum,
                                                      float* __restrict__ dcs_part, float* __restrict__ ddot, float* __restrict__ dstates) {
   pdl_wait();
   __shared__ __align__(16) float As[A_FLOATS], Bs[B_FLOATS], row[256];
-  if (blockIdx.x < n_w) w_tile(g, blockIdx.x, x, dy, dsb, dsl, cs, dtf, cb, wsum, dcs_part, ddot, As, Bs);
+  if (blockIdx.x < n_w) w_tile(g, blockIdx.x, x, dy, dsb, dsl, A, cs, dtf, cb, wsum, dcs_part, ddot, As, Bs);
   else state_tile<1>(g, blockIdx.x - n_w, dy, dsb, dsl, Cm, g.csb, g.csl, cs, dtf, dstates, As, Bs, row);
 }
 
 // dx:  u[j,p] = sum_{i>=j} cb[i,j] exp(cs_i-cs_j) dy[i,p] + exp(cs_end-cs_j) sum_n B[j,n] dS[p,n]
 //      dx = D dy + dt_j u ;  ddtd[j] = sum_p x[j,p] u[j,p] (one partial per 32 features)
 template <typename T, typename TD>
-__device__ __forceinline__ void dx_tile(const Geo& g, unsigned u, const T* x, const T* Bm, const float* D, const TD* dy, long long dsb,
+__device__ __forceinline__ void dx_tile(const Geo& g, unsigned u, const T* x, const T* Bm, const float* A, const float* D, const TD* dy, long long dsb,
                                         long long dsl, const float* __restrict__ cs, const float* __restrict__ dtf,
                                         const float* __restrict__ cb, const float* __restrict__ dS, T* dx, float* __restrict__ ddt_part,
-                                        float* As, float* Bs, float* css) {
+                                        float* As, float* Bs, float* css, float* stp) {
   const int ntj = (g.Q + TM - 1) / TM, ntp = (g.P + TN - 1) / TN;
   const Place q = place_of(u, ntj * ntp, g.H, g.nc);
   const int j0 = (q.tile % ntj) * TM, pt = q.tile / ntj, p0 = pt * TN, h = q.x, grp = h / g.hpg, t0 = q.c * g.Q, nv = valid_rows(g, q.c);
   const size_t co = cs_idx(g, q.b, h, q.c), nq = (size_t)g.B * g.H * g.nc * g.Q;
-  for (int l = threadIdx.x; l < g.Q; l += NT) css[l] = cs[co + l];
+  for (int l = threadIdx.x; l < g.Q; l += NT) {
+    css[l] = cs[co + l];
+    stp[l] = l + 1 < g.Q ? expf(dtf[co + l + 1] * A[h]) : 0.f;
+  }
   __syncthreads();
   const float ref = css[min(j0 + TM, g.Q) - 1], eend = expf(css[g.Q - 1] - ref);
   const int pc = min(TN, g.P - p0);
@@ -629,12 +646,11 @@ __device__ __forceinline__ void dx_tile(const Geo& g, unsigned u, const T* x, co
   contract<false, false>(acc, M, DY, j0, min(j0 + TM, g.Q), As, Bs, [&](int k, int r, int c, float4 v) {
     const int i = k + r, j = j0 + c;   // row i of cb, columns j .. j + 3
     if (i >= g.Q || j > i) return make_float4(0.f, 0.f, 0.f, 0.f);
-    const float ci = css[i];
-    v.x *= expf(ci - css[j]);
-    v.y = j + 1 <= i ? v.y * expf(ci - css[j + 1]) : 0.f;
-    v.z = j + 2 <= i ? v.z * expf(ci - css[j + 2]) : 0.f;
-    v.w = j + 3 <= i ? v.w * expf(ci - css[j + 3]) : 0.f;
-    return v;
+    const float4 s4 = *reinterpret_cast<const float4*>(stp + j);
+    const float st[3] = {s4.x, s4.y, s4.z};
+    float e[4];
+    walk4(css[i], css[min(j + 3, g.Q - 1)], i - j, st, e);
+    return make_float4(v.x * e[0], i - j >= 1 ? v.y * e[1] : 0.f, i - j >= 2 ? v.z * e[2] : 0.f, i - j >= 3 ? v.w * e[3] : 0.f);
   }, Keep());
   float o[4][4];
   acc.get(o);
@@ -745,18 +761,18 @@ __device__ __forceinline__ void dbc_tile(const Geo& g, unsigned u, const T* Othe
 // What follows the reverse scan over chunks, one launch: dC, dB (the longest tiles), dx.
 template <typename T, typename TD>
 __global__ void __launch_bounds__(NT, 4) k_bwd_final(Geo g, unsigned n_bc, const T* __restrict__ x, const T* __restrict__ Bm,
-                                                     const T* __restrict__ Cm, const float* __restrict__ D, const TD* __restrict__ dy,
-                                                     long long dsb, long long dsl, const float* __restrict__ cs, const float* __restrict__ dtf,
-                                                     const float* __restrict__ cb, const float* __restrict__ wsum,
+                                                     const T* __restrict__ Cm, const float* __restrict__ A, const float* __restrict__ D,
+                                                     const TD* __restrict__ dy, long long dsb, long long dsl, const float* __restrict__ cs,
+                                                     const float* __restrict__ dtf, const float* __restrict__ cb, const float* __restrict__ wsum,
                                                      const float* __restrict__ prev, const float* __restrict__ dS, T* __restrict__ dx,
                                                      T* __restrict__ dB, T* __restrict__ dC, float* __restrict__ dcs_part,
                                                      float* __restrict__ ddt_part) {
   pdl_wait();
-  __shared__ __align__(16) float As[A_FLOATS], Bs[B_FLOATS], css[256];
+  __shared__ __align__(16) float As[A_FLOATS], Bs[B_FLOATS], css[256], stp[256];
   const unsigned u = blockIdx.x;
   if (u < n_bc) dbc_tile<0>(g, u, Bm, g.bsb, g.bsl, Cm, dy, dsb, dsl, cs, dtf, wsum, prev, dC, dcs_part, As, Bs);
   else if (u < 2 * n_bc) dbc_tile<1>(g, u - n_bc, Cm, g.csb, g.csl, Cm, x, g.xsb, g.xsl, cs, dtf, wsum, dS, dB, dcs_part, As, Bs);
-  else dx_tile(g, u - 2 * n_bc, x, Bm, D, dy, dsb, dsl, cs, dtf, cb, dS, dx, ddt_part, As, Bs, css);
+  else dx_tile(g, u - 2 * n_bc, x, Bm, A, D, dy, dsb, dsl, cs, dtf, cb, dS, dx, ddt_part, As, Bs, css, stp);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1065,7 +1081,7 @@ static int fwd_stages_t(const Geo& g, bool tc, const SsdFwdPtrs& p, char* ws, co
       int rc = tensor_chunk_scan(g, p, tab, prev_bf, status, s);
       if (rc) return rc;
     } else if (p.y) {
-      launch<k_chunk_scan<T, false>>(Tiles(g).scan, NT, 0, s, g, x, (const T*)p.Cm, p.D, (const T*)p.z, cs, dtf, cb, states, (T*)p.y,
+      launch<k_chunk_scan<T, false>>(Tiles(g).scan, NT, 0, s, g, x, (const T*)p.Cm, p.A, p.D, (const T*)p.z, cs, dtf, cb, states, (T*)p.y,
                                      nullptr, nullptr, nullptr);
       SSD_CUDA_CHECK_LAUNCH("chunk_scan");
     }
@@ -1128,7 +1144,7 @@ static int bwd_stages_t(const Geo& g, bool tc, const SsdBwdPtrs& p, char* ws, co
     } else {
       // only the gate needs the forward's outputs again: dz and the pre-gate dy (the row sums come out of W and dC)
       if (p.z) {
-        launch<k_chunk_scan<T, true>>(Tiles(g).scan, NT, 0, s, g, x, (const T*)p.Cm, p.D, (const T*)p.z, cs, dtf, cb, states, nullptr,
+        launch<k_chunk_scan<T, true>>(Tiles(g).scan, NT, 0, s, g, x, (const T*)p.Cm, p.A, p.D, (const T*)p.z, cs, dtf, cb, states, nullptr,
                                       (const T*)p.dy, dyp, (T*)p.dz);
         SSD_CUDA_CHECK_LAUNCH("chunk_scan_bwd_epilogue");
       }
@@ -1145,9 +1161,9 @@ static int bwd_stages_t(const Geo& g, bool tc, const SsdBwdPtrs& p, char* ws, co
       }
     } else {
       if (p.z)
-        launch<k_bwd_local<T, float>>(n.state + n.cb, NT, 0, s, g, n.cb, x, dyp, HP * g.L, HP, (const T*)p.Cm, cs, dtf, cb, wsum, dcsp, ddot, dst);
+        launch<k_bwd_local<T, float>>(n.state + n.cb, NT, 0, s, g, n.cb, x, dyp, HP * g.L, HP, p.A, (const T*)p.Cm, cs, dtf, cb, wsum, dcsp, ddot, dst);
       else
-        launch<k_bwd_local<T, T>>(n.state + n.cb, NT, 0, s, g, n.cb, x, (const T*)p.dy, g.ysb, g.ysl, (const T*)p.Cm, cs, dtf, cb, wsum, dcsp,
+        launch<k_bwd_local<T, T>>(n.state + n.cb, NT, 0, s, g, n.cb, x, (const T*)p.dy, g.ysb, g.ysl, p.A, (const T*)p.Cm, cs, dtf, cb, wsum, dcsp,
                                   ddot, dst);
       SSD_CUDA_CHECK_LAUNCH("bwd_local");
     }
@@ -1183,10 +1199,10 @@ static int bwd_stages_t(const Geo& g, bool tc, const SsdBwdPtrs& p, char* ws, co
       float* dcs_cols = dcsp + (size_t)n.strips * n.nq;
       const unsigned blocks = 2 * n.bc + n.scan;
       if (p.z)
-        launch<k_bwd_final<T, float>>(blocks, NT, 0, s, g, n.bc, x, (const T*)p.Bm, (const T*)p.Cm, p.D, dyp, HP * g.L, HP, cs, dtf, cb, wsum,
+        launch<k_bwd_final<T, float>>(blocks, NT, 0, s, g, n.bc, x, (const T*)p.Bm, (const T*)p.Cm, p.A, p.D, dyp, HP * g.L, HP, cs, dtf, cb, wsum,
                                       states, dst, (T*)p.dx, (T*)p.dB, (T*)p.dC, dcs_cols, ddtd);
       else
-        launch<k_bwd_final<T, T>>(blocks, NT, 0, s, g, n.bc, x, (const T*)p.Bm, (const T*)p.Cm, p.D, (const T*)p.dy, g.ysb, g.ysl, cs, dtf, cb,
+        launch<k_bwd_final<T, T>>(blocks, NT, 0, s, g, n.bc, x, (const T*)p.Bm, (const T*)p.Cm, p.A, p.D, (const T*)p.dy, g.ysb, g.ysl, cs, dtf, cb,
                                   wsum, states, dst, (T*)p.dx, (T*)p.dB, (T*)p.dC, dcs_cols, ddtd);
       SSD_CUDA_CHECK_LAUNCH("bwd_final");
     }
