@@ -2691,17 +2691,21 @@ k_bwd_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant__
         tc_fence_after();
         const size_t dense = ((size_t)b * g.L + t_row) * g.H * P + (size_t)h0 * P + half * 32;
         float s0 = 0.f, s1 = 0.f, s2 = 0.f;
+        // 16 columns at a time.  dstate 128: ph 0,1 Y slices, ph 2,3 U' slices; dstate 64: Y, U' of one slice, then of the other,
+        // which reads the boxes once (512 x 1024 tokens of 8 heads 334 -> 307 us)
+        uint4 xv[2], dv[2];
 #pragma unroll
-        for (int ph = 0; ph < 4; ++ph) {          // ph 0,1: Y slices; ph 2,3: U' slices (16 columns each)
-          const int h16 = ph & 1;
-          const bool upass = ph >= 2;
-          uint4 xv[2], dv[2];
+        for (int ph = 0; ph < 4; ++ph) {
+          const int h16 = SPLIT ? (ph & 1) : (ph >> 1);
+          const bool upass = SPLIT ? ph >= 2 : (ph & 1);
           float a16[16], o16[16];
           if (SPLIT && ph == 2) { w.wait(&bars.u_full, kb & 1, 67); tc_fence_after(); }
+          if (SPLIT || !upass) {
 #pragma unroll
-          for (int q = 0; q < 2; ++q) {
-            xv[q] = ld_shared_v4(xt + sw128_off(row, half * 4 + h16 * 2 + q));
-            dv[q] = ld_shared_v4(dyt + sw128_off(row, half * 4 + h16 * 2 + q));
+            for (int q = 0; q < 2; ++q) {
+              xv[q] = ld_shared_v4(xt + sw128_off(row, half * 4 + h16 * 2 + q));
+              dv[q] = ld_shared_v4(dyt + sw128_off(row, half * 4 + h16 * 2 + q));
+            }
           }
           {   // both accumulator slices in flight, one wait
             uint32_t ra[16], ro[16];
