@@ -331,3 +331,27 @@ def test_more_units_than_sms_and_many_chunks(lib, H, P, N, G, Bn):
         ref = oracle_all(row, dfinal[r:r + 1])
         for k, v in (("y", y), ("final_state", fin), *((k, g[k]) for k in ("dx", "ddt", "dB", "dC", "dinit"))):
             assert_close(k, v[r:r + 1], ref[k], "bf16")
+
+
+@pytest.mark.parametrize("gate", [False, True])
+@pytest.mark.parametrize("H,P,N", [(2, 64, 128), (4, 64, 128), (6, 64, 128), (10, 64, 128), (4, 32, 128), (12, 32, 128), (4, 32, 64), (12, 32, 64),
+                                   (2, 64, 64), (6, 64, 64)])
+def test_rings_at_tile_ends(lib, H, P, N, gate):
+    """Several tiles per block with one to ten head blocks each: slots that a tile lends out, pieces and rings that end in the middle of a
+    tile.  Against the one-tile kernels, which have no rings; bf16 operands and sums rounded in another order: 1e-2."""
+    import trading_bot_0_b200 as T
+    B, L, bf = 70, 512, torch.bfloat16
+    g = torch.Generator(device="cuda").manual_seed(3)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    A = -torch.exp(2 * torch.rand(H, generator=g, device="cuda"))
+    a = (r(B, L, H, P).to(bf), torch.nn.functional.softplus(r(B, L, H) - 2).to(bf), A, (r(B, L, 1, N) / N ** 0.5).to(bf),
+         (r(B, L, 1, N) / N ** 0.5).to(bf), torch.ones(H, device="cuda"), r(B, L, H, P).to(bf) if gate else None)
+    dy = r(B, L, H, P).to(bf)
+    out = []
+    for algo in ("tensor", "tensor_onetile"):
+        y, fin, ws = T.forward(*a, chunk=128, algo=algo, for_backward=True)
+        o = T.backward(dy, *a, chunk=128, algo=algo, workspace=ws, fwd_saved=True)
+        out.append({"y": y, "fin": fin, **{k: o[k] for k in ("dx", "ddt", "dB", "dC") + (("dz",) if gate else ())}})
+    for k, v in out[0].items():
+        w = out[1][k].double()
+        assert float((v.double() - w).norm() / w.norm()) < 1e-2, k
