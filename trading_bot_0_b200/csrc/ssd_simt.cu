@@ -219,7 +219,7 @@ __device__ __forceinline__ size_t cb_idx(const Geo& g, int b, int c, int grp) {
 // Stage 1: cs = inclusive within-chunk cumsum of dt*A (fp32), dtf = dt as fp32, both [B,H,nc,Q]; dt here is the
 // step size after the optional bias / softplus, which every later stage reads from dtf or the decay tables.
 // One block per (chunk, batch): thread q reads the H contiguous dt values of position q once and
-// the block scans 8 heads at a time with warp shuffles.
+// the block scans HG heads at a time with warp shuffles.
 // HG heads at a time, as in k_ddt.
 template <typename T, int HG>
 __global__ void __launch_bounds__(256) k_cumsum(Geo g, const T* __restrict__ dt, const float* __restrict__ dt_bias,
@@ -827,7 +827,7 @@ __global__ void __launch_bounds__(ST) k_sdot(Geo g, const float* __restrict__ dS
 // Backward: da_k = sum_{i>=k in chunk}(dcsp_i - dt_i*ddtd_i) + sdot ; ddt_k = ddtd_k + A*da_k (times the derivative
 // of the step-size activation when dt_softplus is set) ;
 // per-chunk partial sums for dA (= sum dt*da) and dD (= sum ddot).  One block per (chunk, batch),
-// 8 heads at a time; sdot arrives as `nw` partial sums per (batch, chunk, head), added in fixed order.
+// HG heads at a time; sdot arrives as `nw` partial sums per (batch, chunk, head), added in fixed order.
 // How dcsp and ddtd arrive: the tensor family sums them itself ({1, 0, 1}); the CUDA-core family leaves one part of dcsp per
 // 32-column strip of the chunk (strips; only those up to the position's own hold anything), one per 32 state columns, and one
 // part of ddtd per 32 features, `stride` elements apart.
