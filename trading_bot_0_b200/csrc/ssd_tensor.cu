@@ -155,8 +155,7 @@ __device__ __forceinline__ void zero_upper_blocks(int row, int part, int warp, u
 // TMEM loads, table loads and stores hides behind another group's arithmetic.  A warp
 // walks the 32x32 blocks of its block row left to right (blocks below the diagonal first, the
 // diagonal block last) with the next block's TMEM load in flight while the current one is scaled,
-// converted and stored.  Same factorisation as decay_mask_tile below the diagonal; elements of the diagonal block take
-// exp(cs_i - cs_j) dt_j directly, so this variant does not need the T_DS section.
+// converted and stored.  Same factorisation and the same operations as decay_mask_tile.
 // Blocks are read from TMEM in the layout of matrix fragments: a thread has two neighbouring columns of every group of eight,
 // in four rows (t / 4 + 8 a).  A read of shared memory costs what it delivers to registers, 128 bytes a cycle, broadcast or not;
 // with a row per thread every thread read every column's factor.  Here it reads a quarter of them, four rows share them, and
@@ -195,14 +194,31 @@ __device__ __forceinline__ void decay_off8(float (&v)[8], const float (&rf)[4], 
     mul2(v[2 * a], v[2 * a + 1], rf[a], rf[a]);
   }
 }
-// group g of the diagonal block: rows 8 a + t/4 with a < g lie above it
+// group g of the diagonal block: rows 8 a + t/4 with a < g lie above it.  The same walk as in decay_mask_tile, operation for
+// operation: from the last column of the group leftwards by the steps, restarting at 1 on the diagonal.  A thread walks to its
+// own two columns (steps beyond them are 1) for all its rows at once; in the rows of a == g the walk starts on the diagonal.
 __device__ __forceinline__ void decay_diag8(float (&v)[8], const DecayRows& r, uint32_t ts, int c0, int g, int lane) {
-  const float2 c = lds_v2f32(ts + 4 * (T_CS + c0 + 2 * (lane & 3))), t = lds_v2f32(ts + 4 * (T_DT + c0 + 2 * (lane & 3)));
+  const int q = lane & 3, i = lane >> 2;
+  const float2 t = lds_v2f32(ts + 4 * (T_DT + c0 + 2 * q));
+  const float4 d0 = lds_v4f32(ts + 4 * (T_DS + c0)), d1 = lds_v4f32(ts + 4 * (T_DS + c0 + 4));
+  const float ds[7] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z};   // ds[k] = decay of step c0 + k + 1
+  const float left = q == 0 ? ds[0] : q == 1 ? ds[2] : q == 2 ? ds[4] : ds[6];
+  const float end = lds_f32(ts + 4 * (T_CS + c0 + 7));
+  float f[4];
+#pragma unroll
+  for (int a = g; a < 4; ++a) f[a] = a == g ? 1.f : ex2(r.cs[a] - end);
+#pragma unroll
+  for (int k = 6; k >= 1; --k) {
+    const float m = k > 2 * q ? ds[k] : 1.f, md = k < i ? m : 1.f;
+    if (g == 3) f[3] *= md; else mul2(f[g], f[g + 1], md, m);
+    if (g == 0) mul2(f[2], f[3], m, m);
+    if (g == 1) f[3] *= m;
+  }
 #pragma unroll
   for (int a = 0; a < 4; ++a) {
     if (a < g) { v[2 * a] = v[2 * a + 1] = 0.f; continue; }
-    const int d = 8 * (a - g) + (lane >> 2) - 2 * (lane & 3);   // row - column of the left element
-    float f0 = d >= 0 ? ex2(r.cs[a] - c.x) : 0.f, f1 = d >= 1 ? ex2(r.cs[a] - c.y) : 0.f;
+    float f0 = f[a] * (a > g || 2 * q < i ? left : 1.f), f1 = f[a];
+    if (a == g) { f0 = 2 * q <= i ? f0 : 0.f; f1 = 2 * q < i ? f1 : 0.f; }
     mul2(f0, f1, t.x, t.y);
     mul2(v[2 * a], v[2 * a + 1], f0, f1);
   }
@@ -1820,18 +1836,17 @@ struct WsCfg {
   // when the next tile's C and B are requested).  An E slot is given back by the epilogue: two.
   // The state boxes pass as 8 KB pieces (64 state columns each); one buffer for a block was a chain of load, product, load that
   // took as long as a block.
-  static constexpr int NA = SPLIT ? 4 : 3, NA_OWN = SPLIT ? 2 : 3, NE = E ? 2 : 0, NSP = SPLIT && !(HB == 2 && NM == 2) ? 3 : 2;
+  static constexpr int NA = SPLIT ? 4 : 3, NA_OWN = SPLIT ? 2 : 3, NE = E ? 2 : 0, NSP = SPLIT && HB == 1 ? 3 : 2;
   static __device__ __forceinline__ int a_slot(int kb, int blk, int nblk) { return !SPLIT ? kb % NA : nblk - blk <= 2 ? (blk & 1) : blk % NA; }
-  // table ring depth (the first 1.5 KB of a head's table: all but T_DS): a multiple of the number of decay groups, so that a slot is always read by
+  // table ring depth (one 2 KB table per head): a multiple of the number of decay groups, so that a slot is always read by
   // the same group.  With a depth of 4 and three groups the slot of head 5 had last been head 1's, read by another group:
   // the group of head 5, coming from head 2, could reach the slot's barrier before head 1's table had landed, pass the wait
   // on the parity of a phase that had not even begun, and read the slot while head 5's table was still arriving (rows 0-31
   // of that head wrong about once in 10^4 CTAs).
-  static constexpr int TBL_BYTES = T_DS * 4;
-  static constexpr int NTH = (NM == 3) ? 6 : 4 * HB;
+  static constexpr int NTH = (NM == 3) ? (SPLIT && HB == 1 ? 3 : 6) : 4 * HB;
   static_assert(NTH % NM == 0 && NTH % HB == 0 && NTH <= 8, "a table slot must belong to one decay group and one column half");
   static constexpr int RED_BYTES = (P == 64 && MODE != 0) ? 2 * 128 * 4 : 0;
-  static constexpr size_t SMEM = 1024 + CB_BYTES + NM * 2 * BOX_BYTES + (NA_OWN + NE) * BOX_BYTES + NSP * SBOX_BYTES + NTH * TBL_BYTES +
+  static constexpr size_t SMEM = 1024 + CB_BYTES + NM * 2 * BOX_BYTES + (NA_OWN + NE) * BOX_BYTES + NSP * SBOX_BYTES + NTH * TAB_BYTES +
                                  RED_BYTES;
   static_assert(SMEM <= 232448 - 512, "shared-memory plan exceeds the 227 KB a CTA can have");
   // warp roles: NM groups of four decay warps, then two MMA issuer warps (one per head of a head block) on the two
@@ -1885,7 +1900,7 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
   uint8_t* sE = sA + Cfg::NA_OWN * BOX_BYTES;            // NE x E box
   uint8_t* sSt = sE + Cfg::NE * BOX_BYTES;               // state pieces
   uint8_t* sTab = sSt + NSP * SBOX_BYTES;                // NTH x decay table of one head (they run further ahead)
-  float* sRed = (float*)(sTab + NTH * Cfg::TBL_BYTES);          // [2][128] (P = 64 row-sum exchange)
+  float* sRed = (float*)(sTab + NTH * TAB_BYTES);          // [2][128] (P = 64 row-sum exchange)
   __shared__ __align__(8) WsBars bars;
   __shared__ uint32_t tmem_slot;
   __shared__ int s_abort;
@@ -1975,8 +1990,8 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         for (int hl = 0; hl < HB; ++hl, ++tkh, tsrc += TAB) {
           const int ts = tkh % NTH;
           w.wait(&bars.tab_empty[ts], ((tkh / NTH) & 1) ^ 1, 49);
-          mbar_expect_tx(&bars.tab_full[ts], Cfg::TBL_BYTES);
-          bulk_load(sTab + ts * Cfg::TBL_BYTES, tsrc, Cfg::TBL_BYTES, &bars.tab_full[ts]);
+          mbar_expect_tx(&bars.tab_full[ts], TAB_BYTES);
+          bulk_load(sTab + ts * TAB_BYTES, tsrc, TAB_BYTES, &bars.tab_full[ts]);
         }
         if (++tblk == nblk) { tblk = 0; ++tt; }
       };
@@ -2136,7 +2151,7 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         const int ts = kh % NTH;
         w.wait(&bars.m_empty[wg], ((kh / NM) & 1) ^ 1, 53);
         w.wait(&bars.tab_full[ts], (kh / NTH) & 1, 52);
-        decay_row(rb, tm_row, (const float*)(sTab + ts * Cfg::TBL_BYTES), row, mrow);
+        decay_row(rb, tm_row, (const float*)(sTab + ts * TAB_BYTES), row, mrow);
         fence_async_smem(); __syncwarp(); if (lane == 0) { mbar_arrive(&bars.m_full[wg]); mbar_arrive(&bars.tab_empty[ts]); }
       }
       tc_fence_before();
@@ -2184,7 +2199,7 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         const uint32_t at = smem_u32(a_box(ib)), et = smem_u32(sE + eb * BOX_BYTES);
         const uint32_t xt = MODE == 2 ? et : at, dyt = MODE == 2 ? at : et;
         const int khe = kb * HB + hl_e, ts = khe % NTH;
-        const float* tb = (const float*)(sTab + ts * Cfg::TBL_BYTES);
+        const float* tb = (const float*)(sTab + ts * TAB_BYTES);
         const uint32_t tmYd = tm + 256 + ab * 128, tmYo = tmYd + 64;
         const int h0 = grp * g.hpg + blk * HB, h_e = h0 + hl_e;
         const float Dh = D ? __ldg(D + h_e) : 0.f;
