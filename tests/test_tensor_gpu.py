@@ -333,28 +333,56 @@ def test_more_units_than_sms_and_many_chunks(lib, H, P, N, G, Bn):
             assert_close(k, v[r:r + 1], ref[k], "bf16")
 
 
+def block_errors(v, w, tokens=32):
+    """2-norm of the difference over the 2-norm of the reference, for every block of `tokens` rows of one batch row and one head (or
+    group); blocks whose reference is small are held to the average block's norm."""
+    B, L = v.shape[:2]
+    pad = -L % tokens
+
+    def blocks(t):
+        t = torch.nn.functional.pad(t.double().reshape(B, L, v.shape[2], -1), (0, 0, 0, 0, 0, pad))
+        return t.view(B, (L + pad) // tokens, tokens, v.shape[2], -1).square().sum((2, 4))
+
+    ref = blocks(w)
+    return (blocks(v.double() - w.double()) / torch.maximum(ref, ref.mean())).sqrt()
+
+
 @pytest.mark.parametrize("gate", [False, True])
-@pytest.mark.parametrize("H,P,N", [(2, 64, 128), (4, 64, 128), (6, 64, 128), (10, 64, 128), (4, 32, 128), (12, 32, 128), (4, 32, 64), (12, 32, 64),
-                                   (2, 64, 64), (6, 64, 64)])
-def test_rings_at_tile_ends(lib, H, P, N, gate):
-    """Several tiles per block with one to ten head blocks each: slots that a tile lends out, pieces and rings that end in the middle of a
-    tile.  Against the one-tile kernels, which have no rings; bf16 operands and sums rounded in another order: 1e-2."""
+@pytest.mark.parametrize("H,P,N,B,L", [
+    (2, 64, 128, 200, 512), (4, 64, 128, 200, 475), (6, 64, 128, 40, 512), (10, 64, 128, 150, 512), (10, 64, 128, 150, 475), (12, 64, 128, 200, 512),
+    (4, 32, 128, 200, 475), (12, 32, 128, 200, 512), (4, 32, 64, 200, 475), (12, 32, 64, 200, 512), (2, 64, 64, 200, 475), (6, 64, 64, 200, 512)])
+def test_rings_at_tile_ends(lib, H, P, N, B, L, gate):
+    """Five tiles and more per block (40 rows: two or three), of two to twelve head blocks each - 150 rows of 10 heads run as two parts of five
+    blocks, 40 rows of 6 as two parts of three - in whole and in ragged chunks: slots that a tile lends out, pieces and rings that end in
+    the middle of a tile, every barrier used many times over.  Against the one-tile kernels, which have no rings, block by block of 32
+    rows of a head: a wrong block is off by about its own norm, two roundings of the bf16 operands of a sum (2^-9 each) by less than a
+    hundredth.  And twice with the same bits."""
     import trading_bot_0_b200 as T
-    B, L, bf = 70, 512, torch.bfloat16
+    bf, Lp = torch.bfloat16, L + -L % 128
     g = torch.Generator(device="cuda").manual_seed(3)
     r = lambda *s: torch.randn(*s, generator=g, device="cuda")
     A = -torch.exp(2 * torch.rand(H, generator=g, device="cuda"))
-    a = (r(B, L, H, P).to(bf), torch.nn.functional.softplus(r(B, L, H) - 2).to(bf), A, (r(B, L, 1, N) / N ** 0.5).to(bf),
-         (r(B, L, 1, N) / N ** 0.5).to(bf), torch.ones(H, device="cuda"), r(B, L, H, P).to(bf) if gate else None)
-    dy = r(B, L, H, P).to(bf)
+    seq = [r(B, Lp, H, P).to(bf), torch.nn.functional.softplus(r(B, Lp, H) - 2).to(bf), (r(B, Lp, 1, N) / N ** 0.5).to(bf),
+           (r(B, Lp, 1, N) / N ** 0.5).to(bf), r(B, Lp, H, P).to(bf) if gate else None, r(B, Lp, H, P).to(bf)]
+    for v in seq:   # the one-tile kernels take whole chunks only: steps of size zero behind the end
+        if v is not None:
+            v[:, L:] = 0
     out = []
-    for algo in ("tensor", "tensor_onetile"):
+    for algo, n in (("tensor", L), ("tensor", L), ("tensor_onetile", Lp)):
+        x, dt, Bm, Cm, z, dy = (v if v is None else v[:, :n].contiguous() for v in seq)
+        a = (x, dt, A, Bm, Cm, torch.ones(H, device="cuda"), z)
         y, fin, ws = T.forward(*a, chunk=128, algo=algo, for_backward=True)
         o = T.backward(dy, *a, chunk=128, algo=algo, workspace=ws, fwd_saved=True)
-        out.append({"y": y, "fin": fin, **{k: o[k] for k in ("dx", "ddt", "dB", "dC") + (("dz",) if gate else ())}})
+        torch.cuda.synchronize()
+        assert status_word(ws) == 0
+        keys = ("dx", "ddt", "dB", "dC") + (("dz",) if gate else ())
+        out.append({"y": y[:, :L], **{k: o[k][:, :L] for k in keys}, "fin": fin, "dA": o["dA"], "dD": o["dD"]})
     for k, v in out[0].items():
-        w = out[1][k].double()
-        assert float((v.double() - w).norm() / w.norm()) < 1e-2, k
+        assert torch.equal(v, out[1][k]), k
+        if k not in ("fin", "dA", "dD"):
+            e = float(block_errors(v, out[2][k]).max())
+            print(k, f"{e:.2e}")
+            assert e < 5e-2, (k, e)
 
 
 @pytest.mark.parametrize("gate", [False, True])
@@ -380,6 +408,5 @@ def test_large_steps_next_to_the_diagonal(lib, H, P, N, gate):
         o = T.backward(d["dy"], *a, chunk=128, algo=algo, workspace=ws, fwd_saved=True)
         out = {"y": y, "dx": o["dx"], **({"dz": o["dz"]} if gate else {})}
         err.append({k: float((v.double().cpu() - ref[k]).norm() / ref[k].norm()) for k, v in out.items()})
-    print(err)
     for k, e in err[0].items():
         assert e < 1.07 * err[1][k], (k, e, err[1][k])

@@ -1223,8 +1223,11 @@ k_scan_tc(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
     // off-diagonal scale: exp(cs_i) for Y, dt_j exp(cs_end - cs_j) for U'
     const float osc = (MODE == 2) ? dt_r * ex2(tb[hl_e * TAB + T_CS + 127] - cs_r) : ex2(cs_r);
     if (IBUF == 1) {
-      __syncthreads();
-      if (tid == 0 && blk + 1 < nblk) load_block(blk + 1, 0);
+      // A barrier alone does not wait for reads that are still behind the last block's stores: the refill overtook them (rows of a
+      // head took the next block's x or dy at 200 x 512 tokens, 12 heads of 32 x 64).  So its count depends on what was read.
+      const int warps = __syncthreads_count(
+          reads_done(xv[0].x ^ xv[1].x ^ dv[0].x ^ dv[1].x ^ __float_as_uint(osc) ^ __float_as_uint(dt_r), tid & 31));
+      if (tid == 0 && warps > 0 && blk + 1 < nblk) load_block(blk + 1, 0);
     }
     float s0 = 0.f, s1 = 0.f;
     {
