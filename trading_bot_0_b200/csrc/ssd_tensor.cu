@@ -1835,12 +1835,15 @@ struct WsCfg {
   static constexpr int CB_BYTES = (NCBS + 1) * TILE_BYTES;           // keep tiles, other tile
   // Rings.  An A slot is held from the request of its box until its output block has been read by the tile store: about 4 us against
   // 2 us of work per block, so with two of them the issuers wait for boxes.  Three; dstate 128: two, and two more in the other tile
-  // from the tile's G until the next tile's (the last two blocks of a tile use the first two slots, so that those are drained
+  // from the tile's G until the next tile's (the last two blocks of a tile use the slots of their own, so that the lent ones are drained
   // when the next tile's C and B are requested).  An E slot is given back by the epilogue: two.
   // The state boxes pass as 8 KB pieces (64 state columns each); one buffer for a block was a chain of load, product, load that
   // took as long as a block.
   static constexpr int NA = SPLIT ? 4 : 3, NA_OWN = SPLIT ? 2 : 3, NE = E ? 2 : 0, NSP = SPLIT && HB == 1 ? 3 : 2;
-  static __device__ __forceinline__ int a_slot(int kb, int blk, int nblk) { return !SPLIT ? kb % NA : nblk - blk <= 2 ? (blk & 1) : blk % NA; }
+  // The slots of their own alternate through all tiles; `own` counts their uses so far.
+  static __device__ __forceinline__ int a_slot(uint32_t& own, int kb, int blk, int nblk) {
+    return !SPLIT ? kb % NA : (blk & 2) && blk < nblk - 2 ? blk % NA : (int)(own++ & 1);
+  }
   // table ring depth (one 2 KB table per head): a multiple of the number of decay groups, so that a slot is always read by
   // the same group.  With a depth of 4 and three groups the slot of head 5 had last been head 1's, read by another group:
   // the group of head 5, coming from head 2, could reach the slot's barrier before head 1's table had landed, pass the wait
@@ -1999,7 +2002,7 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         if (++tblk == nblk) { tblk = 0; ++tt; }
       };
       int kb = 0, sq = 0;
-      uint32_t used = 0;
+      uint32_t used = 0, own = 0;
       load_cb(0);
       load_tab();
       load_tab();
@@ -2007,7 +2010,7 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         int b, grp, c;
         tile_coords(t, b, grp, c);
         for (int blk = 0; blk < nblk; ++blk, ++kb) {
-          const int ib = Cfg::a_slot(kb, blk, nblk);
+          const int ib = Cfg::a_slot(own, kb, blk, nblk);
           if (SPLIT && blk == 2 && ib == 2) w.wait(&bars.g_full[0], t & 1, 68);   // G has read the tile these slots share
           w.wait(&bars.a_empty[ib], ((used >> ib) & 1) ^ 1, 42);
           used ^= 1u << ib;
@@ -2069,14 +2072,14 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
       };
       if (mi == 0) issue_g(0);
       int kb = 0, kh = 0, sq = 0;
-      uint32_t used = 0;
+      uint32_t used = 0, own = 0;
       for (int t = 0; t < my_tiles; ++t) {
         const uint32_t keep_t = smem_u32(sCB + (t % NCBS) * Cfg::TILE_BYTES);
         // the lane that issues the state term reads the keep tile; when that is not the lane that formed G (and waited
         // for the tile there), it has to see the tile's arrival itself: the first x box of a tile can land before its C/B
         if (mi == 1) w.wait(&bars.cb_full[t % NCBS], (t / NCBS) & 1, 64);
         for (int blk = 0; blk < nblk; ++blk, ++kb) {
-          const int ib = Cfg::a_slot(kb, blk, nblk), ab = kb & 1;
+          const int ib = Cfg::a_slot(own, kb, blk, nblk), ab = kb & 1;
           const uint32_t inb = smem_u32(a_box(ib));
           const uint32_t tmYd = tm + 256 + ab * 128, tmYo = tmYd + 64;
           w.wait(&bars.a_full[ib], (used >> ib) & 1, 45);
@@ -2122,12 +2125,12 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
     // ------------------------------------------------------------------ store lane: output blocks leave as TMA tiles
     if (lane == 0) {
       int kb = 0;
-      uint32_t used = 0;
+      uint32_t used = 0, own = 0;
       for (int t = 0; t < my_tiles; ++t) {
         int b, grp, c;
         tile_coords(t, b, grp, c);
         for (int blk = 0; blk < nblk; ++blk, ++kb) {
-          const int ib = Cfg::a_slot(kb, blk, nblk);
+          const int ib = Cfg::a_slot(own, kb, blk, nblk);
           w.wait(&bars.out_ready[ib], (used >> ib) & 1, 59);
           used ^= 1u << ib;
           tma_store_3d(&tmOut, a_box(ib), grp * g.hpg * P + blk * 64, c * QT, b);
@@ -2168,7 +2171,7 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
     const int row = (ew & 3) * 32 + lane, half = ew >> 2;     // 32 of the block's 64 columns
     const int hl_e = (half * 32) / P;
     int kb = 0;
-    uint32_t used = 0;
+    uint32_t used = 0, own = 0;
     // gated recompute (MODE 1): the gate is the one operand the epilogue reads from global memory; this thread's 64 bytes
     // of it are requested a block ahead (the forward gets the gate's box by TMA)
     uint4 zq[GATED ? 4 : 1] = {}, zn[GATED && !ZSMEM ? 4 : 1] = {};
@@ -2198,7 +2201,7 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
           for (int q = 0; q < 4; ++q) zq[q] = zn[q];
           blk + 1 < nblk ? load_z(t, blk + 1, zn) : load_z(t + 1, 0, zn);
         }
-        const int ib = Cfg::a_slot(kb, blk, nblk), ab = kb & 1, eb = kb & 1;
+        const int ib = Cfg::a_slot(own, kb, blk, nblk), ab = kb & 1, eb = kb & 1;
         const uint32_t at = smem_u32(a_box(ib)), et = smem_u32(sE + eb * BOX_BYTES);
         const uint32_t xt = MODE == 2 ? et : at, dyt = MODE == 2 ? at : et;
         const int khe = kb * HB + hl_e, ts = khe % NTH;
