@@ -40,6 +40,8 @@ constexpr int SBOX_BYTES = 64 * 128;  // state TMA box: 64 (h,p) rows x 64 bf16
 constexpr int TAB = SSD_TAB_FLOATS;   // floats per (batch, chunk, head) decay table
 constexpr int TAB_BYTES = TAB * 4;
 constexpr int T_CS = 0, T_DT = 128, T_CF = 256, T_DS = 384;   // table sections, 128 floats each
+// The 227 KB a CTA can have, without a kilobyte for a persistent kernel's barriers, the TMEM address and the abort flag.
+constexpr size_t SMEM_STATIC = 1024, SMEM_MOST = 232448 - SMEM_STATIC;
 
 // Bounded waits: after the first one gives up every later wait is skipped, so a broken
 // pipeline drains in bounded time instead of hanging; the status word tells the host.
@@ -543,6 +545,7 @@ struct PsCfg {
   static constexpr int W_MMA = 16, W_PROD = 17, THREADS = 18 * 32;
   static constexpr int B_BYTES = NBX * BOX_BYTES;
   static constexpr size_t SMEM = 1024 + NX * X_BYTES + X_BYTES + 2 * B_BYTES + NX * TB_BYTES;
+  static_assert(SMEM <= SMEM_MOST, "shared-memory plan exceeds the 227 KB a CTA can have");
   static_assert(T_CS == 0 && T_DT == 128, "the two sections must be the first 1 KB of a table");
 };
 
@@ -764,7 +767,7 @@ struct PfCfg {
   static constexpr int SDOT_NW = 4 * (P / 32);
   static constexpr int NQ = N / 64;   // 16-column slices per thread
   static constexpr size_t SMEM = 1024 + NX * X_BYTES + X_BYTES + NB * B_BYTES + NSE * SE_BYTES + NX * TB_BYTES;
-  static_assert(SMEM <= 232448, "shared-memory plan exceeds the 227 KB a CTA can have");
+  static_assert(SMEM <= SMEM_MOST, "shared-memory plan exceeds the 227 KB a CTA can have");
 };
 
 // <dS_end, S_end> in one order for both kernels that form it: four columns in a chain, sixteen as a tree, then over the columns
@@ -1854,7 +1857,7 @@ struct WsCfg {
   static constexpr int RED_BYTES = (P == 64 && MODE != 0) ? 2 * 128 * 4 : 0;
   static constexpr size_t SMEM = 1024 + CB_BYTES + NM * 2 * BOX_BYTES + (NA_OWN + NE) * BOX_BYTES + NSP * SBOX_BYTES + NTH * TAB_BYTES +
                                  RED_BYTES;
-  static_assert(SMEM <= 232448 - 512, "shared-memory plan exceeds the 227 KB a CTA can have");
+  static_assert(SMEM <= SMEM_MOST, "shared-memory plan exceeds the 227 KB a CTA can have");
   // warp roles: NM groups of four decay warps, then two MMA issuer warps (one per head of a head block) on the two
   // least loaded schedulers, the producer warp and an idle warp, then 8 epilogue warps
   static constexpr int DW = 4 * NM, W_MMA = DW, W_PROD = DW + 2, W_EPI = DW + 4;
@@ -1879,6 +1882,7 @@ struct WsBars {
   uint64_t cb_full[2], cb_empty[2], ot_full, ot_empty, g_full[2], g_empty[2], a_full[4], a_empty[4], e_full[2], e_empty[2], acc_full[2], acc_empty[2];
   uint64_t m_full[3], m_empty[3], tab_full[8], tab_empty[8], st_full[4], st_empty[4], out_ready[4], hz[4], done;
 };
+static_assert(sizeof(WsBars) + 16 <= SMEM_STATIC, "the barriers need more than their share");
 
 template <int P, int MODE, int N_ = 64, bool GATED = false>
 __global__ void __launch_bounds__(WsCfg<P, MODE, N_, GATED>::THREADS, 1)
@@ -2357,7 +2361,7 @@ struct BwCfg {
   static constexpr int TB_BYTES = HB * TAB_BYTES;
   static constexpr int RED_BYTES = (P == 64) ? 3 * 256 * 4 : 0;
   static constexpr size_t SMEM = 1024 + NCBS * CB_BYTES + NM * 2 * BOX_BYTES + 2 * IN_BYTES + ST_BYTES + NT * TB_BYTES + RED_BYTES;
-  static_assert(SMEM <= 232448, "shared-memory plan exceeds the 227 KB a CTA can have");
+  static_assert(SMEM <= SMEM_MOST, "shared-memory plan exceeds the 227 KB a CTA can have");
 };
 
 struct BwBars {
@@ -2365,6 +2369,7 @@ struct BwBars {
   uint64_t tab_full[4], tab_empty[4], st_full, st_empty, y_full, y_empty, u_full, u_empty, done;
   uint64_t stp_full[2], stp_empty[2];
 };
+static_assert(sizeof(BwBars) + 16 <= SMEM_STATIC, "the barriers need more than their share");
 
 template <int P, int N_ = 64>
 __global__ void __launch_bounds__(WS_THREADS, 1)
@@ -2826,7 +2831,7 @@ struct DbCfg {
   static constexpr int TB_BYTES = HB * TAB_BYTES;
   static constexpr int W_SCALE = 20, NSCALE = 8, NDECAY = 10;   // decay warps with a block on or below the diagonal
   static constexpr size_t SMEM = 1024 + 2 * BOX_BYTES + NIN * IN_BYTES + NST * ST_BYTES + NT * TB_BYTES;
-  static_assert(SMEM <= 232448 - 512, "shared-memory plan exceeds the 227 KB a CTA can have");
+  static_assert(SMEM <= SMEM_MOST, "shared-memory plan exceeds the 227 KB a CTA can have");
 };
 
 template <int P, int N_>
