@@ -154,15 +154,15 @@ __device__ __forceinline__ void zero_upper_blocks(int row, int part, int warp, u
 
 // Whole-row variant for k_scan_ws.  A group of four warps (one per TMEM lane quarter)
 // owns one head at a time and different groups work on different heads, so the latency of one group's
-// TMEM loads, table loads and stores hides behind another group's arithmetic.  A warp
-// walks the 32x32 blocks of its block row left to right (blocks below the diagonal first, the
+// TMEM loads, table loads and stores hides behind another group's arithmetic.  Thread = accumulator
+// row; it walks the 32x32 blocks of its block row left to right (blocks below the diagonal first, the
 // diagonal block last) with the next block's TMEM load in flight while the current one is scaled,
 // converted and stored.  Same factorisation and the same operations as decay_mask_tile.
-// Blocks are read from TMEM in the layout of matrix fragments: a thread has two neighbouring columns of every group of eight,
-// in four rows (t / 4 + 8 a).  A read of shared memory costs what it delivers to registers, 128 bytes a cycle, broadcast or not;
-// with a row per thread every thread read every column's factor.  Here it reads a quarter of them, four rows share them, and
-// stmatrix writes the tile (512 x 1024 tokens of 8 heads 229 -> 224 us, 2 x 131072 of 24 heads 606 -> 590; in the backward
-// kernels, whose passes are shorter, it gained nothing: 349 against 354 and 273 against 290 us).
+// A read of shared memory costs what it delivers to registers, broadcast or not, and here every thread reads every column's factor.  In
+// the layout of matrix fragments (tcgen05.ld.16x256b, stmatrix: a quarter of the factors per thread) the walk in the diagonal
+// block takes a select per step and costs more than that saves, in the diagonal block alone or in all: 16 x 4096 gated steps of 24
+// heads 1167 us as here, 1184 with fragments below the diagonal, 1191 with fragments throughout; 150 x 512 of 20 heads of 32 x 128
+// gated 758, 781, 791.
 __device__ __forceinline__ void tmem_ld16_issue(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
@@ -179,64 +179,42 @@ __device__ __forceinline__ void tmem_ld_wait_2x16(uint32_t (&r)[16], uint32_t (&
                  "+r"(q[9]), "+r"(q[10]), "+r"(q[11]), "+r"(q[12]), "+r"(q[13]), "+r"(q[14]), "+r"(q[15])
                :: "memory");
 }
-// One group of eight columns (first column c0 of the tile) of a 32x32 block: v[2 a + e] is row 8 a + t/4, column 2 (t % 4) + e.
-struct DecayRows {
-  float cs[4];   // of this thread's rows
-  __device__ __forceinline__ void load(uint32_t ts, int row0, int lane) {   // row0: first row of the block
+// 16 columns of a block below the diagonal: out[k] = raw[k] * rf * cf[k]; `cf` = shared-memory address of the column factors
+__device__ __forceinline__ void decay_off_half(const uint32_t (&raw)[16], float rf, uint32_t cf, uint32_t dst) {
 #pragma unroll
-    for (int a = 0; a < 4; ++a) cs[a] = lds_f32(ts + 4 * (T_CS + row0 + 8 * a + (lane >> 2)));
-  }
-};
-// below the diagonal; rf: exp(cs_i - cs_r) of the rows
-__device__ __forceinline__ void decay_off8(float (&v)[8], const float (&rf)[4], uint32_t ts, int c0, int lane) {
-  const float2 f = lds_v2f32(ts + 4 * (T_CF + c0 + 2 * (lane & 3)));
+  for (int j8 = 0; j8 < 16; j8 += 8) {
+    const float4 f0 = lds_v4f32(cf + 4 * j8), f1 = lds_v4f32(cf + 4 * (j8 + 4));
+    const float f[8] = {f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, f1.z, f1.w};
+    float v[8];
 #pragma unroll
-  for (int a = 0; a < 4; ++a) {
-    mul2(v[2 * a], v[2 * a + 1], f.x, f.y);
-    mul2(v[2 * a], v[2 * a + 1], rf[a], rf[a]);
-  }
-}
-// group g of the diagonal block: rows 8 a + t/4 with a < g lie above it.  The same walk as in decay_mask_tile, operation for
-// operation: from the last column of the group leftwards by the steps, restarting at 1 on the diagonal.  A thread walks to its
-// own two columns (steps beyond them are 1) for all its rows at once; in the rows of a == g the walk starts on the diagonal.
-__device__ __forceinline__ void decay_diag8(float (&v)[8], const DecayRows& r, uint32_t ts, int c0, int g, int lane) {
-  const int q = lane & 3, i = lane >> 2;
-  const float2 t = lds_v2f32(ts + 4 * (T_DT + c0 + 2 * q));
-  const float4 d0 = lds_v4f32(ts + 4 * (T_DS + c0)), d1 = lds_v4f32(ts + 4 * (T_DS + c0 + 4));
-  const float ds[7] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z};   // ds[k] = decay of step c0 + k + 1
-  const float left = q == 0 ? ds[0] : q == 1 ? ds[2] : q == 2 ? ds[4] : ds[6];
-  const float end = lds_f32(ts + 4 * (T_CS + c0 + 7));
-  float f[4];
-#pragma unroll
-  for (int a = g; a < 4; ++a) f[a] = a == g ? 1.f : ex2(r.cs[a] - end);
-#pragma unroll
-  for (int k = 6; k >= 1; --k) {
-    const float m = k > 2 * q ? ds[k] : 1.f, md = k < i ? m : 1.f;
-    if (g == 3) f[3] *= md; else mul2(f[g], f[g + 1], md, m);
-    if (g == 0) mul2(f[2], f[3], m, m);
-    if (g == 1) f[3] *= m;
-  }
-#pragma unroll
-  for (int a = 0; a < 4; ++a) {
-    if (a < g) { v[2 * a] = v[2 * a + 1] = 0.f; continue; }
-    float f0 = f[a] * (a > g || 2 * q < i ? left : 1.f), f1 = f[a];
-    if (a == g) { f0 = 2 * q <= i ? f0 : 0.f; f1 = 2 * q < i ? f1 : 0.f; }
-    mul2(f0, f1, t.x, t.y);
-    mul2(v[2 * a], v[2 * a + 1], f0, f1);
+    for (int k = 0; k < 8; k += 2) {
+      v[k] = __uint_as_float(raw[j8 + k]); v[k + 1] = __uint_as_float(raw[j8 + k + 1]);
+      mul2(v[k], v[k + 1], f[k], f[k + 1]);
+      mul2(v[k], v[k + 1], rf, rf);
+    }
+    st_shared_v4(dst + (j8 >> 3) * 2048, pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
   }
 }
-__device__ __forceinline__ void store8(const float (&v)[8], uint32_t addr) {   // addr: this lane's row of the group's 32 rows
-  st_matrix_x4(addr, pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
-}
-
-// 16 columns of a block in fragment layout: registers 0-7 hold rows 0-15, 8-15 rows 16-31
-__device__ __forceinline__ void tmem_ld_half_issue(uint32_t taddr, uint32_t (&r)[16]) {
-  tmem_ld_frag16_issue(taddr, r);
-  tmem_ld_frag16_issue(tmem_addr(taddr, 16, 0), r + 8);
-}
-__device__ __forceinline__ void half_group(const uint32_t (&raw)[16], int k, float (&v)[8]) {   // its k-th group of eight columns
+// 16 columns (starting at column c0) of the diagonal block: two independent 8-column walks; `ts` = shared-memory address
+// of the head's table
+__device__ __forceinline__ void decay_diag_half(const uint32_t (&raw)[16], uint32_t ts, int c0, int row, float csi, uint32_t dst) {
 #pragma unroll
-  for (int e = 0; e < 4; ++e) { v[e] = __uint_as_float(raw[4 * k + e]); v[4 + e] = __uint_as_float(raw[8 + 4 * k + e]); }
+  for (int s = 0; s < 2; ++s) {
+    const int cs0 = c0 + 8 * s, je = cs0 + 7;
+    const float4 d0 = lds_v4f32(ts + 4 * (T_DS + cs0)), d1 = lds_v4f32(ts + 4 * (T_DS + cs0 + 4));
+    const float4 t0 = lds_v4f32(ts + 4 * (T_DT + cs0)), t1 = lds_v4f32(ts + 4 * (T_DT + cs0 + 4));
+    const float ds[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};   // ds[k] = decay of step cs0+k+1
+    float v[8] = {t0.x, t0.y, t0.z, t0.w, t1.x, t1.y, t1.z, t1.w}, run[8];
+    run[7] = (row >= je) ? ex2(csi - lds_f32(ts + 4 * (T_CS + je))) : 0.f;
+#pragma unroll
+    for (int k = 6; k >= 0; --k) run[k] = (cs0 + k == row) ? 1.f : run[k + 1] * ds[k];
+#pragma unroll
+    for (int k = 0; k < 8; k += 2) {
+      mul2(v[k], v[k + 1], run[k], run[k + 1]);
+      mul2(v[k], v[k + 1], __uint_as_float(raw[8 * s + k]), __uint_as_float(raw[8 * s + k + 1]));
+    }
+    st_shared_v4(dst + s * 2048, pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
+  }
 }
 // rb: block row of the warp (warp-uniform); tm_row: TMEM address of (first lane of this warp's quarter, first
 // source column); mrow: shared-memory address of this row's first 16 bytes in the plain 128x128 bf16 tile.
@@ -246,33 +224,24 @@ __device__ __forceinline__ void half_group(const uint32_t (&raw)[16], int k, flo
 // shared-memory pipe.
 __device__ __forceinline__ void decay_row(int rb, uint32_t tm_row, const float* __restrict__ tab, int row, uint32_t mrow) {
   const uint32_t ts = smem_u32(tab);
-  const int lane = row & 31;
+  const float csi = lds_f32(ts + 4 * (T_CS + row));
   uint32_t a[16], b[16];
-  tmem_ld_half_issue(tm_row, a);
-  tmem_ld_half_issue(tm_row + 16, b);
-  DecayRows r;
-  r.load(ts, rb * 32, lane);
-  float v[8];
+  tmem_ld16_issue(tm_row, a);
+  tmem_ld16_issue(tm_row + 16, b);
 #pragma unroll 1
   for (int cb = 0; cb < rb; ++cb) {
-    const float ref = lds_f32(ts + 4 * (T_CS + cb * 32 + 31));
-    const float rf[4] = {ex2(r.cs[0] - ref), ex2(r.cs[1] - ref), ex2(r.cs[2] - ref), ex2(r.cs[3] - ref)};
+    const float rf = ex2(csi - lds_f32(ts + 4 * (T_CS + cb * 32 + 31)));
+    const uint32_t cf = ts + 4 * (T_CF + cb * 32);
     const uint32_t dst = mrow + cb * 4 * 2048;
     tmem_ld_wait_2x16(a, b);
-#pragma unroll
-    for (int k = 0; k < 2; ++k) { half_group(a, k, v); decay_off8(v, rf, ts, cb * 32 + 8 * k, lane); store8(v, dst + k * 2048); }
-    tmem_ld_half_issue(tm_row + (cb + 1) * 32, a);
-#pragma unroll
-    for (int k = 0; k < 2; ++k) { half_group(b, k, v); decay_off8(v, rf, ts, cb * 32 + 16 + 8 * k, lane); store8(v, dst + (2 + k) * 2048); }
-    tmem_ld_half_issue(tm_row + (cb + 1) * 32 + 16, b);
+    decay_off_half(a, rf, cf, dst);
+    tmem_ld16_issue(tm_row + (cb + 1) * 32, a);
+    decay_off_half(b, rf, cf + 64, dst + 2 * 2048);
+    tmem_ld16_issue(tm_row + (cb + 1) * 32 + 16, b);
   }
   tmem_ld_wait_2x16(a, b);
-#pragma unroll
-  for (int g = 0; g < 4; ++g) {
-    if (g < 2) half_group(a, g, v); else half_group(b, g - 2, v);
-    decay_diag8(v, r, ts, rb * 32 + 8 * g, g, lane);
-    store8(v, mrow + (rb * 4 + g) * 2048);
-  }
+  decay_diag_half(a, ts, rb * 32, row, csi, mrow + rb * 4 * 2048);
+  decay_diag_half(b, ts, rb * 32 + 16, row, csi, mrow + rb * 4 * 2048 + 2 * 2048);
 }
 
 // Variant used by the one-tile-per-CTA kernels (all 16 warps meet at a CTA barrier per head anyway):

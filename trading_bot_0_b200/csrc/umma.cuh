@@ -139,21 +139,6 @@ __device__ __forceinline__ void tmem_ld8_issue(uint32_t taddr, uint32_t (&r)[8])
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
                : "r"(taddr));
 }
-// 16 lanes x 8 or 16 consecutive fp32 columns, without the wait.  Thread t of the warp gets, for every group of eight columns,
-// columns 2 (t % 4) and 2 (t % 4) + 1 of lane t / 4 (r[4 g], r[4 g + 1]) and of lane t / 4 + 8 (r[4 g + 2], r[4 g + 3]): the layout
-// stmatrix takes.
-__device__ __forceinline__ void tmem_ld_frag8_issue(uint32_t taddr, uint32_t* r) {
-  asm volatile("tcgen05.ld.sync.aligned.16x256b.x1.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr));
-}
-__device__ __forceinline__ void tmem_ld_frag16_issue(uint32_t taddr, uint32_t* r) {
-  asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-               : "r"(taddr));
-}
-// Four 8 x 8 bf16 matrices in that layout (register m = matrix m) to shared memory: lane l gives the address of row l % 8 of matrix l / 8.
-__device__ __forceinline__ void st_matrix_x4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-  asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
-}
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ uint32_t tmem_addr(uint32_t base, int lane, int col) {
   return base + ((uint32_t)lane << 16) + (uint32_t)col;
@@ -279,11 +264,6 @@ __device__ __forceinline__ void st_global_32B(void* p, const uint4& a, const uin
 __device__ __forceinline__ float lds_f32(uint32_t addr) {
   float v;
   asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr));
-  return v;
-}
-__device__ __forceinline__ float2 lds_v2f32(uint32_t addr) {
-  float2 v;
-  asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr));
   return v;
 }
 __device__ __forceinline__ float4 lds_v4f32(uint32_t addr) {
