@@ -161,6 +161,26 @@ def test_mamba2_mixer_core_autograd_fp32_kernels(lib):
         assert_close(name, got.grad.detach(), want, "bf16")
 
 
+@pytest.mark.parametrize("dtype", ["fp32", "bf16"])
+@pytest.mark.parametrize("used", ["out", "final_state"])
+def test_mixer_with_one_output_used(lib, dtype, used):
+    """An output that takes no part in the loss has no gradient; the mixer's node is not handed zeros for it.  Same bits as with zeros."""
+    from trading_bot_0_b200 import prepost as PP
+    Bn, L, H, P, N, G = 2, 256, 8, 32, 64, 1
+    td = O.torch_dtype(dtype)
+    g = torch.Generator(device=DEV).manual_seed(23)
+    r = lambda *s: torch.randn(*s, generator=g, device=DEV)
+    hp, ch = H * P, H * P + 2 * G * N
+    leaves = [r(Bn, L, ch).to(td), (0.5 * r(Bn, L, H)).to(td), r(Bn, L, H, P).to(td), r(ch, 4) / 2, 0.1 * r(ch), r(H) - 3.0,
+              -torch.exp(r(H)), torch.ones(H, device=DEV), 1.0 + 0.1 * r(hp), 0.1 * r(Bn, H, P, N)]
+    leaves = [v.requires_grad_() for v in leaves]
+    out, fin = PP.mamba2_mixer_core(*leaves[:9], init_state=leaves[9], nheads=H, headdim=P, dstate=N, ngroups=G, chunk=128)
+    dout, dfin = (r(Bn, L, hp).to(td), torch.zeros_like(fin)) if used == "out" else (torch.zeros_like(out), torch.ones_like(fin))
+    want = torch.autograd.grad([out, fin], leaves, [dout, dfin], retain_graph=True)
+    got = torch.autograd.grad(*((out, leaves, dout) if used == "out" else (fin, leaves, dfin)))
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
 def test_operands_that_do_not_fit_are_refused(lib):
     """Outputs, weights, statistics, gradients and workspaces that a kernel would read or write past their end are a ValueError
     before anything is launched; a weight of another shape with as many values is taken."""

@@ -68,14 +68,16 @@ def test_fp32_groups_and_odd_dims(lib):
     run_case(cfg, with_init=True, with_dfinal=True)
 
 
+@pytest.mark.parametrize("speed", [8, 1 / 8])
 @pytest.mark.parametrize("chunk,seqlen", [(50, 333), (3, 40), (66, 200), (129, 300), (256, 256)])
-def test_fp32_decays_on_the_diagonal(lib, chunk, seqlen):
+def test_fp32_decays_on_the_diagonal(lib, chunk, seqlen, speed):
     """Decays of the tiles on the diagonal are walked four columns at a time: chunk lengths that end inside a group of four, a tile or
-    a strip, with decays of several e-folds a step.  3e-6: sums of up to 256 rounded terms, an order below the parity gate."""
+    a strip, with decays of several e-folds a step (running sums round most) and with slow ones (the walk's own products do).
+    3e-6: sums of up to 256 rounded terms, an order below the parity gate."""
     import trading_bot_0_b200 as T
     cfg = cfg_like(0, chunk=chunk, seqlen=seqlen, batch=2)
     inp = O.make_inputs(cfg, O.SEED, batch=2, seqlen=seqlen)
-    inp["dt"] = inp["dt"] * 8
+    inp["dt"] = inp["dt"] * speed
     ref = oracle_all(inp)
     d = to_dev(inp, DEV)
     a = (d["x"], d["dt"], d["A"], d["B"], d["C"], d.get("D"))

@@ -51,6 +51,21 @@ def test_node_matches_oracle_and_python_autograd(lib, base, kw):
     assert torch.equal(y, y2) and torch.equal(fin, fin2)
 
 
+@pytest.mark.parametrize("base", [0, 1])
+@pytest.mark.parametrize("used", ["y", "final_state"])
+def test_node_with_one_output_used(lib, base, used):
+    """An output that takes no part in the loss has no gradient; the node is not handed zeros for it.  Same bits as with zeros."""
+    from trading_bot_0_b200 import torch_node as TN
+    cfg = cfg_like(base, batch=2, seqlen=256)
+    d = to_dev(O.make_inputs(cfg, O.SEED, batch=2, seqlen=256, with_init_state=True), DEV)
+    leaves = [d[k].requires_grad_() for k in ("x", "dt", "A", "B", "C", "D", "init_state")]
+    y, fin = TN.ssd_scan(*leaves[:6], init_state=leaves[6], chunk=cfg.chunk)
+    dy, dfin = (d["dy"], torch.zeros_like(fin)) if used == "y" else (torch.zeros_like(y), torch.ones_like(fin))
+    want = torch.autograd.grad([y, fin], leaves, [dy, dfin], retain_graph=True)
+    got = torch.autograd.grad(*((y, leaves, dy) if used == "y" else (fin, leaves, dfin)))
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
 def test_node_forward_only_and_step(lib):
     """No input requires a gradient: the node takes the smaller forward workspace; the step operator updates in place."""
     from trading_bot_0_b200 import torch_node as TN
