@@ -218,9 +218,8 @@ __device__ __forceinline__ size_t cb_idx(const Geo& g, int b, int c, int grp) {
 // ---------------------------------------------------------------------------------------------
 // Stage 1: cs = inclusive within-chunk cumsum of dt*A (fp32), dtf = dt as fp32, both [B,H,nc,Q]; dt here is the
 // step size after the optional bias / softplus, which every later stage reads from dtf or the decay tables.
-// One block per (chunk, batch): thread q reads the H contiguous dt values of position q once and
-// the block scans HG heads at a time with warp shuffles.
-// HG heads at a time, as in k_ddt.
+// One block per (chunk, batch, HG heads), as k_ddt: thread q reads the HG contiguous dt values of position q and the block scans
+// them together with warp shuffles.
 template <typename T, int HG>
 __global__ void __launch_bounds__(256) k_cumsum(Geo g, const T* __restrict__ dt, const float* __restrict__ dt_bias,
                                                const float* __restrict__ A, float* __restrict__ cs,
@@ -294,8 +293,9 @@ __global__ void __launch_bounds__(256) k_cumsum(Geo g, const T* __restrict__ dt,
 
 // ---------------------------------------------------------------------------------------------
 // Decays exp(cs_i - cs_j) of one row i and four columns j .. j + 3 (zero above the diagonal) from one exponential: that of the last
-// column, then leftwards by the steps st[c] = exp(dt_{j+c+1} A), restarting at 1 on the diagonal.  No exponent is positive; the
-// steps carry no rounding of the running sum, so an element is no less exact than exp(cs_i - cs_j) itself.
+// column, then leftwards by the steps st[c] = exp(dt_{j+c+1} A), restarting at 1 on the diagonal.  No exponent is positive.  Against
+// exp(cs_i - cs_j) per element: up to three more rounded factors (a few ulp), but steps carry no rounding of the running sums, whose
+// difference loses ulp(cs) - more than those ulp as soon as |cs| exceeds a few units.
 // d = i - j.
 __device__ __forceinline__ void walk4(float ci, float c3, int d, const float (&st)[3], float (&o)[4]) {
   o[3] = d >= 3 ? expf(ci - c3) : 0.f;
@@ -826,8 +826,8 @@ __global__ void __launch_bounds__(ST) k_sdot(Geo g, const float* __restrict__ dS
 // ---------------------------------------------------------------------------------------------
 // Backward: da_k = sum_{i>=k in chunk}(dcsp_i - dt_i*ddtd_i) + sdot ; ddt_k = ddtd_k + A*da_k (times the derivative
 // of the step-size activation when dt_softplus is set) ;
-// per-chunk partial sums for dA (= sum dt*da) and dD (= sum ddot).  One block per (chunk, batch),
-// HG heads at a time; sdot arrives as `nw` partial sums per (batch, chunk, head), added in fixed order.
+// per-chunk partial sums for dA (= sum dt*da) and dD (= sum ddot).  One block per (chunk, batch, HG
+// heads); sdot arrives as `nw` partial sums per (batch, chunk, head), added in fixed order.
 // How dcsp and ddtd arrive: the tensor family sums them itself ({1, 0, 1}); the CUDA-core family leaves one part of dcsp per
 // 32-column strip of the chunk (strips; only those up to the position's own hold anything), one per 32 state columns, and one
 // part of ddtd per 32 features, `stride` elements apart.

@@ -2312,10 +2312,11 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
 // k_scan_ws share G and every M_h, so this kernel does both from one decay pass per head:
 //   Y  = M_h X_h    (+) exp(cs_i) C S_prev^T                   -> dcsp[i] = sum_p dy*Y, ddot[i] = sum_p dy*x
 //   U' = M_h^T dY_h (+) dt_j exp(cs_end-cs_j) B dS_end^T       -> dx = D dy + U', ddtd[j] = sum_p x*U' / dt_j
-// Same roles, rings and parities as k_scan_ws.  TMEM: G x2 (dstate 128: x1, columns 128-255 are idle) + {Y, Y_off, U, U_off}
+// Roles and hand-overs by parity as in k_scan_ws, with rings of its own: x and dy boxes of a block in one slot (two slots), C and B in
+// one slot, whole tables of a block.  TMEM: G x2 (dstate 128: x1, columns 128-255 are idle) + {Y, Y_off, U, U_off}
 // (256 columns, one slot; at dstate 128 its Y and U halves are handed back one by one as soon as the epilogue has read them:
 // 1150 -> 1053 us at 2 x 131072 tokens).  The two state boxes (S_prev, dS_end)
-// have a buffer of their own that is refilled while the second head of a block is worked on.
+// have a buffer of their own that is refilled as soon as the block's state products have read it.
 // dstate 128 (SPLIT): one C/B slot and one G; the S_prev and dS_end boxes (32 KB per head block at this width) pass as four
 // 8 KB pieces through a two-slot ring with a producer lane and an issuer lane of their own (warps 19 and 18), so the state
 // products run beside the head's own products and the whole plan stays inside 227 KB.
@@ -2784,7 +2785,7 @@ k_bwd_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant__
 // dstate 128: 2x131072 with 24 heads 0.97 -> 0.57 ms = 5.7 TB/s; 16x4096 0.27 -> 0.169
 // ms (3.46 waves of tiles take the time of four).  dstate 64, 512x1024 with 8 heads: 0.248 ms whatever the decay; a kernel that
 // carried the decay on the operands where its range allowed took 0.290, and 0.394 with one head beyond the range.  No unit is full
-// there (128x1024: issue slots 0.43, DRAM 42 %, tensor pipe 14 %); a block waits for its decay pass, so what that pass issues
+// there (128x1024: issue slots 0.48, DRAM 45 %, tensor pipe 15 %); a block waits for its decay pass, so what that pass issues
 // counts (with one issuer lane): 0.339 with 32 columns of W in registers beside the sums (spills), 0.306 with 16, 0.301 with
 // packed scaling of the boxes, 0.278 with packed FMAs and without the six warps whose blocks lie above the diagonal.
 template <int P, int N_>
