@@ -45,7 +45,7 @@ def test_conv1d_forward_backward(lib, dtype, K, activation, use_bias, Bn, L, Cn)
 
 @pytest.mark.parametrize("dtype", ["fp32", "bf16"])
 @pytest.mark.parametrize("K", [4, 3, 2])
-@pytest.mark.parametrize("Bn,L,Cn", [(300, 1, 128), (90, 3, 136), (5, 333, 200), (1, 2111, 384), (3, 1024, 128), (2, 17, 520)])
+@pytest.mark.parametrize("Bn,L,Cn", [(300, 1, 128), (90, 3, 136), (5, 333, 200), (1, 2111, 384), (3, 1024, 128), (2, 17, 520), (1, 1, 128), (1, 9, 200), (1, 70, 128)])
 def test_conv1d_backward_in_warp_shares(lib, dtype, K, Bn, L, Cn):
     """Shares of the tokens that begin and end anywhere: sequences shorter than the window, several per share, several shares per
     sequence, a channel block that is partly empty; activation on (whole stages have a form of their own) and off."""

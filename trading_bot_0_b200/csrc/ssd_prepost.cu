@@ -446,7 +446,6 @@ __global__ void __launch_bounds__(CONV_THREADS, CONV_BWD_MINB) k_conv_bwd(SsdCon
 constexpr int CONVB_STAGES = 3, CONVB_RS = 8, CONVB_CTAS_PER_SM = 2, CONVB_WARPS = CONVS_THREADS / 32;
 constexpr int CONVB_STAGE_BYTES = 2 * CONVB_RS * CONVS_ROWB;
 constexpr int CONVB_SMEM = CONVB_WARPS * CONVB_STAGES * CONVB_STAGE_BYTES;
-constexpr int CONVB_MIN_ROWS = 16;   // tokens of a warp's share at least (its halo is 2 (K - 1) rows)
 
 // Where a warp stands in its share [r0, r1) of the tokens: the piece [t0, t1) of sequence b, and the first row of its next stage.
 template <int K> struct ConvWalk {
@@ -953,6 +952,19 @@ int conv_rows(const SsdConvDims* d) {   // thread rows of the backward kernel = 
   const long long pairs = (long long)d->batch * ntile;
   return (int)(pairs < CONV_ROWS ? pairs : CONV_ROWS);
 }
+// Blocks of a channel block of the staged backward kernel: a warp's share is 16 tokens at least (its halo is 2 (K - 1) rows), but
+// below 1024 tokens, where a block's chain of stages is most of the time, eight blocks share them down to a token a warp.  More
+// of them there cost k_conv_reduce what they save, and from 33 rows on its groups walk two (384 channels of bf16, us: 32 tokens 7.5
+// with one block, 6.5 with four; 333 tokens 10.6 with two, 7.7 with eight; 4096 tokens 9.8 with 32, 11.6 with 64).
+long long conv_shares(const SsdConvDims* d) {
+  const long long rows = (long long)d->batch * d->seqlen, few = (rows + CONVB_WARPS - 1) / CONVB_WARPS, many = rows / (16 * CONVB_WARPS);
+  return many > 8 ? many : few < 8 ? few : 8;
+}
+// Rows of partial sums that the backward asks a workspace for; it takes conv_rows() of them at least.
+long long conv_partials(const SsdConvDims* d) {
+  const long long few = conv_shares(d) < 8 ? conv_shares(d) : 8;
+  return few > conv_rows(d) ? few : conv_rows(d);
+}
 int norm_blocks(const SsdNormDims* d) {
   const long long need = (d->rows + NORM_THREADS / 32 - 1) / (NORM_THREADS / 32);
   return (int)(need < 1184 ? need : 1184);
@@ -983,7 +995,7 @@ extern "C" {
 size_t ssd_conv1d_workspace_bytes(const SsdConvDims* dims) {
   clear_error();
   if (check_conv(dims)) return 0;
-  return (size_t)conv_rows(dims) * dims->channels * (dims->width + 1) * sizeof(float);
+  return (size_t)conv_partials(dims) * dims->channels * (dims->width + 1) * sizeof(float);
 }
 
 int32_t ssd_conv1d_forward(const SsdConvDims* dims, const void* in, const float* weight, const float* bias, void* out,
@@ -1071,11 +1083,12 @@ int32_t ssd_conv1d_backward(const SsdConvDims* dims, const void* in, const float
   float* partial = (float*)workspace;
   if ((long long)dims->channels * es >= CONVS_ROWB / 2) {
     const int ncb = (dims->channels * es + CONVS_ROWB - 1) / CONVS_ROWB;
-    const long long rows = (long long)dims->batch * dims->seqlen;
     if (ncb > 65535) { set_error("conv1d backward: too many channels"); return SSD_ERR_UNSUPPORTED; }
     long long nx = ((long long)sm_count() * CONVB_CTAS_PER_SM) / ncb;
-    if (nx > rows / (CONVB_WARPS * CONVB_MIN_ROWS)) nx = rows / (CONVB_WARPS * CONVB_MIN_ROWS);
-    if (nx > nblk) nx = nblk;     // the workspace holds nblk partial rows
+    if (nx > conv_shares(dims)) nx = conv_shares(dims);
+    const long long held = (long long)(workspace_bytes / ((size_t)dims->channels * (dims->width + 1) * sizeof(float)));
+    const long long most = conv_partials(dims) < held ? conv_partials(dims) : held;
+    if (nx > most) nx = most;     // partial rows
     if (nx < 1) nx = 1;
     const dim3 grid((unsigned)nx, (unsigned)ncb);
 #define CONV_BWD_SM(T, K) \
