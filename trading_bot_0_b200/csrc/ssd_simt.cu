@@ -620,9 +620,11 @@ __device__ __forceinline__ void dx_tile(const Geo& g, unsigned u, const T* x, co
   const Place q = place_of(u, ntj * ntp, g.H, g.nc);
   const int j0 = (q.tile % ntj) * TM, pt = q.tile / ntj, p0 = pt * TN, h = q.x, grp = h / g.hpg, t0 = q.c * g.Q, nv = valid_rows(g, q.c);
   const size_t co = cs_idx(g, q.b, h, q.c), nq = (size_t)g.B * g.H * g.nc * g.Q;
+  const float a = A[h];
   for (int l = threadIdx.x; l < g.Q; l += NT) {
-    css[l] = cs[co + l];
-    stp[l] = l + 1 < g.Q ? expf(dtf[co + l + 1] * A[h]) : 0.f;
+    const float c = cs[co + l], dn = dtf[co + min(l + 1, g.Q - 1)];
+    css[l] = c;
+    stp[l] = expf(dn * a);
   }
   __syncthreads();
   const float ref = css[min(j0 + TM, g.Q) - 1], eend = expf(css[g.Q - 1] - ref);
