@@ -28,6 +28,8 @@ enum class StatePlan {
 // near 60 and 84 units, at 8 to 128 chunks alike (bounds: 2/5 and 1/2 of the SMs).  Below 8 chunks the second launch weighs more, and
 // they cross near 50 (2 chunks, 48 units of 24 heads: 37 against 44 us, but whole passes 92.2 against 91.1; 1/3); a single chunk has
 // nothing to walk.  The longest sequences stay with it (1024 chunks, 24 units: 2030 against 4870).
+// Whole forwards since the products of k_state_ps got faster, walks and split: 64 chunks, 24 heads, 48, 60, 72 units 226, 248, 264 and
+// 198, 260, 300 us; 8 heads, 64, 74, 84 units 259, 279, 303 and 234, 266, 322; 16 chunks, 60 and 72 units 75, 78 and 74, 79.
 // More units than SMs: even shares where they save more than a twentieth (192 units of 32 chunks: 413 -> 311; a hand-over costs a
 // state's write and read per block); a share has to be longer than a unit, so that a unit is cut at most once.
 inline StatePlan state_plan(int nc, int units, int n, int sms) {
