@@ -1834,6 +1834,11 @@ struct WsCfg {
   // dstate 128 the second lane issues the state term (8 instructions per head beside the head's own 8)
   static constexpr int NI = (SPLIT && HB == 1) ? 2 : HB;
   static constexpr bool STATE_LANE = (SPLIT && HB == 1);             // the second lane issues the state term only
+  // The lanes' product loops: rolled where two lanes run beside the decay passes at dstate 64 (512 x 1024 tokens of 8 heads of 32 x 64,
+  // forward / gated forward / gated step 376 / 455 / 1623 us unrolled, 355 / 409 / 1519 rolled: unrolled they take instruction
+  // cache and issue slots that the decay warps are short of), unrolled elsewhere (16 x 4096 of 8 heads of 64 x 64 forward 99 us against
+  // 106, of 32 x 128 95 against 99).
+  static constexpr int MMA_UNROLL = HB == 2 && !SPLIT ? 1 : 8;
   // Head 2 kb + 1 (lane 1) takes the slot head 2 kb - 2 (lane 0) had.  Lane 1 has not waited on that use, so its wait by
   // parity could pass while the slot still shows the phase before it.  Lane 0 therefore reports "head 0 of block kb is
   // written" on hz[kb % 4] as soon as it has seen it, and lane 1 waits for block kb - 1's report first.  (Lane 0 needs no
@@ -2065,7 +2070,7 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
               w.wait(&bars.st_full[sp], (sq / NSP) & 1, 58);
               tc_fence_after();
               const uint64_t dKj = desc_sw128_k(keep_t + j * BOX_BYTES, 0), dSj = desc_sw128_k(smem_u32(sSt + sp * SBOX_BYTES), 0);
-#pragma unroll
+#pragma unroll Cfg::MMA_UNROLL
               for (int ks = 0; ks < 4; ++ks) mma_bf16(tmYo, desc_adv(dKj, ks * 32), desc_adv(dSj, ks * 32), idO, (j | ks) > 0);
               mma_commit(&bars.st_empty[sp]);
             }
@@ -2080,7 +2085,7 @@ k_scan_ws(Geo g, const __grid_constant__ CUtensorMap tmX, const __grid_constant_
             const uint32_t mt = smem_u32(sM + ms * 2 * BOX_BYTES);
             const uint64_t dM0 = (MODE == 2) ? desc_plain_mn(mt, 128, 0, 0) : desc_plain_k(mt, 128, 0);
             const uint64_t dO0 = desc_sw128_mn(inb, 0, hl * P * 2, 16);
-#pragma unroll
+#pragma unroll Cfg::MMA_UNROLL
             for (int ks = 0; ks < 8; ++ks)
               mma_bf16(tmYd + hl * P, desc_adv(dM0, ks * M_STEP), desc_adv(dO0, ks * 2048), idY, ks > 0);
             mma_commit(&bars.m_empty[ms]);
