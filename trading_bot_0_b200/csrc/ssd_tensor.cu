@@ -179,38 +179,53 @@ __device__ __forceinline__ void tmem_ld_wait_2x16(uint32_t (&r)[16], uint32_t (&
                  "+r"(q[9]), "+r"(q[10]), "+r"(q[11]), "+r"(q[12]), "+r"(q[13]), "+r"(q[14]), "+r"(q[15])
                :: "memory");
 }
-// 16 columns of a block below the diagonal: out[k] = raw[k] * rf * cf[k]; `cf` = shared-memory address of the column factors
+// 16 columns of a block below the diagonal: out[k] = raw[k] * rf * cf[k]; `cf` = shared-memory address of the column factors.
+// All reads come before the first store, here and below: a read cannot be moved over a store, and one after it would start a second
+// round trip.
 __device__ __forceinline__ void decay_off_half(const uint32_t (&raw)[16], float rf, uint32_t cf, uint32_t dst) {
+  float4 f[4];
 #pragma unroll
-  for (int j8 = 0; j8 < 16; j8 += 8) {
-    const float4 f0 = lds_v4f32(cf + 4 * j8), f1 = lds_v4f32(cf + 4 * (j8 + 4));
-    const float f[8] = {f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, f1.z, f1.w};
+  for (int q = 0; q < 4; ++q) f[q] = lds_v4f32(cf + 16 * q);
+#pragma unroll
+  for (int s = 0; s < 2; ++s) {
+    const float4 f0 = f[2 * s], f1 = f[2 * s + 1];
+    const float c[8] = {f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, f1.z, f1.w};
     float v[8];
 #pragma unroll
     for (int k = 0; k < 8; k += 2) {
-      v[k] = __uint_as_float(raw[j8 + k]); v[k + 1] = __uint_as_float(raw[j8 + k + 1]);
-      mul2(v[k], v[k + 1], f[k], f[k + 1]);
+      v[k] = __uint_as_float(raw[8 * s + k]); v[k + 1] = __uint_as_float(raw[8 * s + k + 1]);
+      mul2(v[k], v[k + 1], c[k], c[k + 1]);
       mul2(v[k], v[k + 1], rf, rf);
     }
-    st_shared_v4(dst + (j8 >> 3) * 2048, pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
+    st_shared_v4(dst + s * 2048, pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
   }
 }
-// 16 columns (starting at column c0) of the diagonal block: two independent 8-column walks; `ts` = shared-memory address
-// of the head's table
+// 16 columns (starting at column c0) of the diagonal block: two independent 8-column walks side by side; `ts` = shared-memory address
+// of the head's table.  Right of the diagonal a walk is zero, so the restart is an addend and not a select (and rounds the same).
 __device__ __forceinline__ void decay_diag_half(const uint32_t (&raw)[16], uint32_t ts, int c0, int row, float csi, uint32_t dst) {
+  float run[16];
+  float4 d[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) d[q] = lds_v4f32(ts + 4 * (T_DS + c0 + 4 * q));   // the decays of steps c0 + 4 q + 1 ..
+  const float e0 = lds_f32(ts + 4 * (T_CS + c0 + 7)), e1 = lds_f32(ts + 4 * (T_CS + c0 + 15));
+  const float ds[16] = {d[0].x, d[0].y, d[0].z, d[0].w, d[1].x, d[1].y, d[1].z, d[1].w, d[2].x, d[2].y, d[2].z, d[2].w, d[3].x, d[3].y, d[3].z, d[3].w};
+  const float fr = (float)(row - c0);
+  run[7] = row >= c0 + 7 ? ex2(csi - e0) : 0.f;
+  run[15] = row >= c0 + 15 ? ex2(csi - e1) : 0.f;
+#pragma unroll
+  for (int k = 6; k >= 0; --k) {
+    run[k] = fmaf(run[k + 1], ds[k], fr == (float)k ? 1.f : 0.f);
+    run[8 + k] = fmaf(run[9 + k], ds[8 + k], fr == (float)(8 + k) ? 1.f : 0.f);
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) d[q] = lds_v4f32(ts + 4 * (T_DT + c0 + 4 * q));
 #pragma unroll
   for (int s = 0; s < 2; ++s) {
-    const int cs0 = c0 + 8 * s, je = cs0 + 7;
-    const float4 d0 = lds_v4f32(ts + 4 * (T_DS + cs0)), d1 = lds_v4f32(ts + 4 * (T_DS + cs0 + 4));
-    const float4 t0 = lds_v4f32(ts + 4 * (T_DT + cs0)), t1 = lds_v4f32(ts + 4 * (T_DT + cs0 + 4));
-    const float ds[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};   // ds[k] = decay of step cs0+k+1
-    float v[8] = {t0.x, t0.y, t0.z, t0.w, t1.x, t1.y, t1.z, t1.w}, run[8];
-    run[7] = (row >= je) ? ex2(csi - lds_f32(ts + 4 * (T_CS + je))) : 0.f;
-#pragma unroll
-    for (int k = 6; k >= 0; --k) run[k] = (cs0 + k == row) ? 1.f : run[k + 1] * ds[k];
+    const float4 t0 = d[2 * s], t1 = d[2 * s + 1];
+    float v[8] = {t0.x, t0.y, t0.z, t0.w, t1.x, t1.y, t1.z, t1.w};
 #pragma unroll
     for (int k = 0; k < 8; k += 2) {
-      mul2(v[k], v[k + 1], run[k], run[k + 1]);
+      mul2(v[k], v[k + 1], run[8 * s + k], run[8 * s + k + 1]);
       mul2(v[k], v[k + 1], __uint_as_float(raw[8 * s + k]), __uint_as_float(raw[8 * s + k + 1]));
     }
     st_shared_v4(dst + s * 2048, pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
