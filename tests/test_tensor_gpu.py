@@ -381,7 +381,6 @@ def test_rings_at_tile_ends(lib, H, P, N, B, L, gate):
         assert torch.equal(v, out[1][k]), k
         if k not in ("fin", "dA", "dD"):
             e = float(block_errors(v, out[2][k]).max())
-            print(k, f"{e:.2e}")
             assert e < 5e-2, (k, e)
 
 

@@ -160,9 +160,9 @@ __device__ __forceinline__ void zero_upper_blocks(int row, int part, int warp, u
 // converted and stored.  Same factorisation and the same operations as decay_mask_tile.
 // A read of shared memory costs what it delivers to registers, broadcast or not, and here every thread reads every column's factor.  In
 // the layout of matrix fragments (tcgen05.ld.16x256b, stmatrix: a quarter of the factors per thread) the walk in the diagonal
-// block takes a select per step and costs more than that saves, in the diagonal block alone or in all: 16 x 4096 gated steps of 24
-// heads 1167 us as here, 1184 with fragments below the diagonal, 1191 with fragments throughout; 150 x 512 of 20 heads of 32 x 128
-// gated 758, 781, 791.
+// block takes a select per step and costs more than that saves, in the diagonal block alone or in all (gated steps, the rest alike:
+// 16 x 4096 of 24 heads 1167 us by rows, 1184 with fragments below the diagonal, 1191 with fragments throughout; 150 x 512 of 20
+// heads of 32 x 128 758, 781, 791).
 __device__ __forceinline__ void tmem_ld16_issue(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
